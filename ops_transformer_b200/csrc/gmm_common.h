@@ -77,14 +77,12 @@ struct Problem {
 struct Plan {
     int path = kPathSimt;
     int num_sms = 0;
-    int ctas = 1;                       // 1 = one CTA per 128-row tile, 2 = CTA pairs on 256-row tiles
-    bool hybrid = false;                // with ctas == 2: a second launch with 128-row tiles takes trailing blocks of <= 128 rows
+    int ctas = 2;                       // 2 = CTA pairs (256 channels per tile), 1 = single CTAs (128 channels)
     size_t ws_bytes = 0;
     size_t off_status = 0, off_amax = 0, off_stage = 0, off_done = 0;
     size_t off_wave = 0;                // 0 = no pacing counters in this workspace
     size_t zero_bytes = 0;              // leading bytes of the workspace cleared at launch
-    bool maps_ready = false;
-    alignas(64) CUtensorMap map_x;
+    alignas(64) CUtensorMap map_x[3];   // boxes of 32, 64 and 128 rows
     alignas(64) CUtensorMap map_w;
 };
 

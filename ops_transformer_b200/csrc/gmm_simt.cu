@@ -250,23 +250,20 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 void make_plan(const Problem &p, Plan *plan)
 {
     plan->path = sm100_shape_ok(p) ? kPathSm100 : kPathSimt;
-    // CTA pairs halve the weight traffic per SM but waste up to 255 rows at the end of every group, so they are
-    // used when groups are long on average.  GMM_B200_CTAS=1|2 overrides the choice (for measurements).
+    // Pairs stage 32 KB per 256 channels x 256 tokens and K block where single CTAs stage 48 KB per 128 x 256, but their CTAs
+    // meet at every tile, and a tile of few tokens or few K blocks has nothing to save.  Measured (us, pair / single):
+    //   swiglu K=7168 N=4096, 32 groups: 162 / 157 at 64 rows, 174 / 174 at 128, 195 / 225 at 192, 354 / 401 at 400
+    //   gmm    K=2048 N=7168, 32 groups:  86 /  85 at 64 rows,  92 /  91 at 128, 105 / 112 at 192, 171 / 191 at 400
+    //   gmm    K=1536 N=4096, 32 groups:  50 /  45 at 128 rows, 60 / 58 at 256, 88 / 88 at 400, 176 / 180 at 1000
+    //   gmm    K=768  N=2048, 64 groups:  43 /  37 at 192 rows, 70 / 62 at 400, 129 / 121 at 1000
+    //   swiglu K=1024 N=2048, 32 groups:  64 /  58 at 256 rows, 156 / 140 at 1000
+    // GMM_B200_CTAS=1|2 overrides the choice (for measurements and tests).
     const long long avg_rows = p.rows_per_group_hint > 0 ? p.rows_per_group_hint : (p.gl_len > 0 ? p.M / p.gl_len : 0);
-    plan->ctas = avg_rows >= 384 ? 2 : 1;
+    plan->ctas = avg_rows > 128 && p.K >= 2048 ? 2 : 1;
     if (const char *e = getenv("GMM_B200_CTAS")) {
         if (e[0] == '1') plan->ctas = 1;
         if (e[0] == '2') plan->ctas = 2;
     }
-    // A second launch with 128-row tiles for the trailing blocks pays only when there are many of them: about half of the
-    // groups end in such a block, and their tiles should fill the GPU several times over (measured: with 32 groups it loses
-    // 5-8 %).  GMM_B200_HYBRID=0|1 overrides.
-    {
-        const long long n_tiles = p.mode == kModeSwigluQuant ? (p.N / 2 + 127) / 128 : (p.N + 255) / 256;
-        constexpr long long kPlanSms = 148;  // a B200; phase 1 is host only and does not ask the device
-        plan->hybrid = plan->ctas == 2 && (long long)p.gl_len * n_tiles >= 16ll * kPlanSms;
-    }
-    if (const char *e = getenv("GMM_B200_HYBRID")) plan->hybrid = plan->ctas == 2 && e[0] != '0';
     plan->off_status = 0;
     plan->off_wave = 0;
     size_t off = 256;
@@ -289,7 +286,6 @@ void make_plan(const Problem &p, Plan *plan)
         plan->off_stage = off;
     }
     plan->ws_bytes = off;
-    plan->maps_ready = false;
 }
 
 cudaError_t simt_launch(const Problem &p, Plan &, void *, cudaStream_t stream)

@@ -1,5 +1,5 @@
 // Grouped int8 GEMM for sm_100a: TMA-staged tiles -> tcgen05.mma kind::i8 -> TMEM int32 accumulators ->
-// warp-specialised fused epilogue.  One persistent CTA per SM walks a tile list that every CTA derives
+// warp-specialised fused epilogue.  Persistent CTA pairs (one CTA per SM) walk a tile list that every CTA derives
 // from group_list on the device (empty experts produce no tiles).
 //
 // Replaces, for NVIDIA B200, the reference's AscendC kernels
@@ -8,25 +8,39 @@
 //   gmm/grouped_matmul_swiglu_quant/op_kernel/grouped_matmul_swiglu_quant.h:231-262, 367-474 (matmul, dequant, SwiGLU)
 // and the host tiling that feeds them (op_host/op_tiling/grouped_matmul_tiling.cpp:727-763).
 //
-// Tile: 128 rows x 256 accumulator columns, K consumed 128 bytes per pipeline stage (4 MMAs of K=32).
-//   grouped_matmul       : the 256 columns are 256 consecutive output columns.
-//   swiglu_quant         : columns [0,128) come from weight columns n0.. (activated half), columns [128,256)
-//                          from N/2+n0.. (linear half), so SwiGLU is tile-local and a tile yields 128 outputs.
+// Orientation: the weight columns ("channels") are the M side of the MMA, 128 per CTA (a TMEM lane is a channel); the
+// token rows are its N side, any multiple of 32 up to 256 (a TMEM column is a token).  A group of R rows is cut into
+// ceil(R / 256) tiles of nearly equal size, so what a tile costs follows the rows it has: with the tokens on the M side
+// a group's last tile multiplied up to 255 rows of other groups (12.5 % of all MMA work on 32 groups of ~1024 rows, half
+// of it on groups of ~250), and a decode tile of a few rows staged and multiplied 128.
+//   grouped_matmul       : a CTA's 128 channels are 128 consecutive output columns.
+//   swiglu_quant, pairs  : lanes [0,64) are weight columns j0.. (activated half), lanes [64,128) are N/2+j0.. (linear
+//                          half): a tile yields 64 outputs per CTA and token; the two halves meet through shared memory.
+//   swiglu_quant, one CTA: both halves of 128 columns in two accumulators of at most 128 tokens; a lane holds both values.
+// K is consumed 128 bytes per pipeline stage (4 MMAs of K=32).
 // Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2-9 = epilogue; swiglu_quant
 // adds warp 10, one lane of which keeps the books of the row blocks in global memory.
-// CTA pairs (cluster of 2, tcgen05 cta_group::2) compute 256-row tiles when groups are long; each CTA then stages its own
-// 128 rows of x and half of the weight columns.  Weight layouts: [E,K,N] (MN-major operand, 128-byte swizzle), the
-// transposed view [E,N,K] (K-major) and FRACTAL_NZ [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, 5-D tensor map).
-// Epilogue: the tile's per-column scales are staged in shared memory while the MMAs run; bf16 / fp16 results are
-// transposed through shared memory so that stores cover whole 128-byte row segments (optionally scattered by a row
-// index, also into other GPUs' buffers); the finalize-routing variant adds weighted fp32 rows into token rows with
-// 16-byte vector reductions; SwiGLU values go to an fp32 staging buffer (transposed the same way) with a per-row atomic
-// max, and a finished row block is requantised to int8 in row slices that the CTAs which worked on it claim from a
+// CTA pairs (cluster of 2, tcgen05 cta_group::2) compute 256 channels; each CTA stages its own 128 channels and half of the
+// tile's token rows.  A launch confined to one CTA runs the one-CTA instances.  Weight layouts: [E,K,N] (MN-major operand,
+// 128-byte swizzle; 64-byte for swiglu's 64-channel boxes), the transposed view [E,N,K] (K-major) and FRACTAL_NZ
+// [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, 5-D tensor map).
+// Epilogue: a lane holds one channel (its weight scale stays in a register), the tokens' scales come from shared memory.
+// bf16 / fp16 results are read as 16x256b fragments, packed by token pairs and transposed by stmatrix, so that the four
+// warps of a column half together hold 256 contiguous bytes of every result row; 32-bit results (SwiGLU values, the
+// combine's fp32 rows, int32 accumulators) are transposed 16 tokens at a time, 128 contiguous bytes per row and warp.
+// Rows are optionally scattered by a row index, also into other GPUs' buffers; the finalize-routing variant adds weighted
+// fp32 rows into token rows with 16-byte vector reductions; SwiGLU values go to an fp32 staging buffer with a per-row
+// atomic max, and a finished row block is requantised to int8 in row slices that the CTAs which worked on it claim from a
 // counter - no CTA ever waits for another one (see publish_and_collect).
-// What bounds the MMA loop is the shared-memory / L1 data path (TMA writes, operand reads of both CTAs of a pair, and
-// every load, store and shuffle of the epilogue), not the tensor pipe and not the feed: memory instructions of the
-// epilogue are kept wide and contiguous for that reason.  The producers pace themselves wave by wave so that the units
-// which share x rows and weight boxes through L2 stay together (a bounded hint).
+// What bounds it: long groups the power limit (the MMA loop runs at 550-570 cycles per K block of 512 where the epilogue is
+// idle; the SM clock falls to 1.5-1.6 GHz, at which the tensor pipe alone draws the board's 1 kW); groups of up to 128 rows
+// HBM; short K the epilogue.  Measured before (tokens on the M side, operations issued by one thread of a diverged warp,
+// every epilogue thread fencing for itself, requantisation inside the epilogue warps) and now, us:
+//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 881 (power), 1000 tokens x 8: layer 597 / 514,
+//     128 tokens x 8 over 256 experts 884 / 850 (HBM); K=2048 N=1536, 64 groups of 64 rows 66 / 54, of 400 rows 190 / 121
+//   gmm K=2048 N=7168: 4096 tokens x 8 449 / 430; 32 groups of 192 rows 120 / 105; K=768 N=2048, 64 x 400 rows 76 / 62
+// The producers pace themselves wave by wave so that the units which share x rows and weight boxes through L2 stay
+// together (a bounded hint).
 // Every wait on an mbarrier is bounded; on expiry the CTA records a status word, all roles leave their loops,
 // outstanding copies are drained with a second bounded wait, TMEM is released and the kernel returns.
 // -DGMM_TRACE builds in clock64 / globaltimer stamps of the roles of a few CTAs (a buffer address comes from the environment).
@@ -41,36 +55,38 @@
 namespace gmm {
 namespace {
 
-constexpr int BM = 128;
-constexpr int BN = 256;
+constexpr int BC = 128;                 // channels (weight columns) per CTA: the MMA's M side, one TMEM lane each
+constexpr int BT = 256;                 // most tokens of a tile: the MMA's N side, one TMEM column each
+constexpr int TOK_STEP = 32;            // the MMA's N is a multiple of this
 constexpr int BK = 128;
 constexpr int UMMA_K = 32;
-constexpr int A_STAGE = BM * BK;        // 128 rows x 128 bytes of K
-constexpr int B_BOX = 128 * BK;         // one weight box: 128 N-columns x 128 bytes of K
+constexpr int W_STAGE = BC * BK;        // a CTA's channels x 128 bytes of K
 constexpr int PIPE_BYTES = 196608;      // shared memory given to the TMA ring
 constexpr int MAX_STAGES = 6;
+constexpr int X_MAPS = 3;               // tensor maps of x with boxes of 32, 64 and 128 rows
 
-// CTAS = 1: one CTA computes a 128 x 256 tile; it stages A (16 KB) and both weight boxes (32 KB) per K block, 4 stages.
-// CTAS = 2: a pair of CTAs (one cluster) computes a 256 x 256 tile with cta_group::2 MMAs; each CTA stages its own 128
-//           rows of A and ONE weight box (its half of the 256 columns), so a K block costs 32 KB per SM and the ring
-//           holds 6 stages.  The pair's even CTA issues the MMAs for both.
-template <int CTAS>
-struct Cfg {
-    static constexpr int kBoxes = 2 / CTAS;                 // weight boxes staged per CTA and K block
-    static constexpr int kStageBytes = A_STAGE + kBoxes * B_BOX;
-    static constexpr int kStages = PIPE_BYTES / kStageBytes;
-    static constexpr int kTileM = BM * CTAS;
-    static constexpr uint32_t kTxBytes = (uint32_t)kStageBytes * CTAS;  // bytes landing per stage, both CTAs together
+// CTAS = 2: a pair of CTAs (one cluster) computes 256 channels with cta_group::2 MMAs; each CTA stages its own 128 channels
+//           (16 KB per K block) and half of the tile's tokens (at most 16 KB).  The pair's even CTA issues the MMAs for both.
+// CTAS = 1: one CTA, 128 channels, all tokens of the tile (at most 32 KB).
+//   swiglu_quant: 128 channels of either half (32 KB) into two accumulators of at most 128 tokens each, so that a lane holds
+//   both values of its column.
+// The ring has as many stages as PIPE_BYTES holds of the launch's largest token box, at most MAX_STAGES.
+template <int MODE, int CTAS>
+struct Shape {
+    static constexpr bool kDual = MODE == kModeSwigluQuant && CTAS == 1;
+    static constexpr int kWStage = kDual ? 2 * W_STAGE : W_STAGE;
+    static constexpr int kMaxTok = kDual ? BT / 2 : BT;
+    static constexpr int kCols = MODE == kModeSwigluQuant && !kDual ? BC / 2 : BC;   // result columns per CTA and tile
 };
-static_assert(Cfg<1>::kStages == 4 && Cfg<2>::kStages == 6 && Cfg<2>::kStages <= MAX_STAGES, "stage arithmetic");
 constexpr int MAX_GROUPS = 1024;
-constexpr int EPI_WARPS = 8;                 // two warps per TMEM lane quarter, each takes half of the columns
+constexpr int EPI_WARPS = 8;                 // two warps per TMEM lane quarter, each takes every second 32-token chunk
 // swiglu_quant only: one more warp, of which one lane keeps the books of the row blocks in global memory (arrivals, slice
 // claims) beside the epilogue, so that none of its round trips to L2 delays the next tile.  It hands the epilogue warps
 // lists of row ranges to requantise through a small ring.
 constexpr int WK_DEPTH = 4;                  // work lists the publishing lane may be ahead of the epilogue warps
+constexpr int RQ_WARPS = 5;                  // swiglu_quant: warps that requantise finished row blocks beside the epilogue
 constexpr int BASE_THREADS = 64 + 32 * EPI_WARPS;
-__host__ __device__ constexpr int num_threads(int mode) { return BASE_THREADS + (mode == kModeSwigluQuant ? 32 : 0); }
+__host__ __device__ constexpr int num_threads(int mode) { return BASE_THREADS + (mode == kModeSwigluQuant ? 32 + 32 * RQ_WARPS : 0); }
 constexpr int TMEM_COLS = 512;
 constexpr long long WAIT_LIMIT_CYCLES = 1ll << 31;   // about a second
 constexpr long long DRAIN_LIMIT_CYCLES = 1ll << 24;  // a few milliseconds
@@ -84,23 +100,28 @@ enum : int { kEpiPlain = 0, kEpiScatter = 1, kEpiGeneric = 2, kEpiCombine = 3 };
 // Weight layouts: [E,K,N]; [E,N,K] (the transposed view); FRACTAL_NZ [E, N/32, K/16, 16, 32] (32-byte runs along N).
 enum : int { kBRowMajor = 0, kBTransposed = 1, kBFractalNz = 2 };
 constexpr int MAX_PENDING = 6;         // unsettled row blocks a CTA keeps track of before it hands its share over
-constexpr int SCALE_BUFS = 3;          // an epilogue thread can run at most two tiles ahead of another one
-constexpr int OUT_STAGE_BYTES = 2048;  // per epilogue warp: 32 rows x 64 bytes of packed bf16
+// Epilogue staging: 32-bit results 16 tokens x 128 bytes per warp; 16-bit results 32 tokens per column half (four warps) of
+// 256 bytes each, 16 bytes apart so that the eight 16-byte rows of a stmatrix fall into different banks.
+constexpr int WARP_STAGE_BYTES = 2048;
+constexpr int ROW16_PITCH = 2 * BC + 16;
+constexpr int OUT_STAGE_BYTES = 2 * 32 * ROW16_PITCH;
+static_assert(OUT_STAGE_BYTES >= EPI_WARPS * WARP_STAGE_BYTES, "one staging area serves both forms");
 
 struct Shared {
     uint64_t full[MAX_STAGES];
     uint64_t empty[MAX_STAGES];
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
-    uint64_t scale_ready[SCALE_BUFS];  // all epilogue threads have stored their column's scale
+    uint64_t tok_ready[2];             // all epilogue threads have stored their token's scale
+    uint64_t grp_sync[4];              // epilogue warps that exchange values through out_stage (see group_sync)
     uint64_t wk_full[WK_DEPTH];        // a work list is written (swiglu_quant)
-    uint64_t wk_empty[WK_DEPTH];       // every epilogue warp is done with it
+    uint64_t wk_empty[WK_DEPTH];       // every requantising warp is done with it
     uint32_t tmem_base;
     int abort_flag;
     int total_tiles;
-    int pad;
+    int max_tok;                       // tokens of the largest tile
     long long wait_limit;              // bound of every wait, in cycles
-    // swiglu_quant: how many epilogue threads have stored (and fenced) their part of how many tiles; the row blocks this
+    // swiglu_quant: how many epilogue warps have stored their part of how many tiles; the row blocks this
     // CTA contributed to and has not yet settled (publishing lane only); a ring of work lists: the row ranges to requantise
     // (written by that lane, read by the epilogue warps after wk_full)
     unsigned stored_count;
@@ -111,13 +132,17 @@ struct Shared {
     int row_start[MAX_GROUPS];
     int rows[MAX_GROUPS];
     int tile_start[MAX_GROUPS + 1];
-    alignas(16) float scales[SCALE_BUFS][BN];  // dequant scale of every accumulator column of the tile (read as float4)
-    alignas(16) uint8_t out_stage[EPI_WARPS][OUT_STAGE_BYTES];
+    // per accumulator buffer: the factor of every token of the tile (x scale, for the combine times the routing weight) and
+    // the combine's routing weight on its own (for the bias term).  A buffer is written after acc_full of its tile, i.e.
+    // after every epilogue warp has left the tile before last, which used it.
+    alignas(16) float tok_scale[2][BT];
+    alignas(16) float tok_logit[2][BT];
+    alignas(16) uint8_t out_stage[OUT_STAGE_BYTES];
 };
 
 constexpr size_t SMEM_BYTES = 1024 + (size_t)PIPE_BYTES + sizeof(Shared);
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
-static_assert(offsetof(Shared, scales) % 16 == 0 && offsetof(Shared, out_stage) % 16 == 0, "vector accesses need 16-byte alignment");
+static_assert(offsetof(Shared, tok_scale) % 16 == 0 && offsetof(Shared, out_stage) % 16 == 0, "vector accesses need 16-byte alignment");
 
 // Debug build only (-DGMM_TRACE): clock64 stamps of the roles of a few CTAs, written to a buffer whose address comes from
 // the environment; layout [cta < 4][role < 4][tile < 64][slot < 8].
@@ -147,7 +172,7 @@ struct KParams {
     int gl_len, gl_type;
     int M, K, N;
     int half_n;        // N/2 (swiglu)
-    int n_tiles;       // tiles along N per row block
+    int n_tiles;       // channel tiles per row block
     int num_k_blocks;  // ceil(K / BK)
     const void *w_scale;
     int w_scale_dtype;
@@ -167,8 +192,6 @@ struct KParams {
     long long out_rows;        // rows of the fp32 result; indices outside [0, out_rows) are skipped
     unsigned *amax_bits;  // [M] row max of |S| as float bits (swiglu)
     int *rb_counter;      // per row block of a tile two words: arrivals + (hand-overs << 16), and the slice claim counter (swiglu)
-    int rb_base;          // first counter of this launch (two launches share the array)
-    int part;             // 0: all rows; 1: every group without its trailing rows if those are at most 128; 2: only those
     int8_t *q_out;        // int8 [M, N/2] (swiglu)
     float *q_scale_out;   // fp32 [M] (swiglu)
     int *status;
@@ -243,50 +266,37 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, Shared
     return mbar_wait_slow(a, parity, sh, status, who, sh->wait_limit);
 }
 
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar)
+// Tiled TMA loads into this CTA's shared memory.  CTAS == 2 is the pair form: the byte count is credited to the mbarrier at
+// `bar`, a shared::cluster address that may belong to the other CTA of the pair.
+template <int CTAS>
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint32_t bar)
 {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-        : "memory");
+    if (CTAS == 1)
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(bar) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar)
+template <int CTAS>
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint32_t bar)
 {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
-        : "memory");
+    if (CTAS == 1)
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4, uint64_t *bar)
+template <int CTAS>
+__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4, uint32_t bar)
 {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
-        : "memory");
-}
-// Pair (cta_group::2) forms: the copy lands in the executing CTA's shared memory, the byte count is credited to the
-// mbarrier at `bar_cluster_addr`, a shared::cluster address that may belong to the other CTA of the pair.
-__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int c0, int c1, uint32_t bar_cluster_addr)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(bar_cluster_addr)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar_cluster_addr)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(bar_cluster_addr)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_5d_pair(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
-                                                 uint32_t bar_cluster_addr)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar_cluster_addr)
-        : "memory");
+    if (CTAS == 1)
+        asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar) : "memory");
 }
 // L2 eviction policies for the fp32 SwiGLU staging rows: they are read back exactly once, about one tile after they were
 // written, while the operands of 74 other tiles stream through L2 in between.  Stored with evict_last and read back with
@@ -312,6 +322,15 @@ __device__ __forceinline__ float4 ld_global_cg_v4_hint(const float4 *a, uint64_t
     float4 v;
     asm volatile("ld.global.cg.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a), "l"(pol) : "memory");
     return v;
+}
+// One lane of a converged warp.  Copies and MMAs take their operands from uniform registers: issued under this predicate by
+// an otherwise converged warp they cost a few cycles each; in a branch that only one thread enters the compiler serialises
+// them (about 150 cycles per MMA, which held the whole MMA loop at 600 cycles per K block instead of 512 at 256 tokens).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
 }
 // shared::cluster address of `p` (a location in this CTA's shared memory) as seen in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(const void *p, uint32_t rank)
@@ -411,38 +430,95 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Shared-memory matrix descriptor, 128-byte swizzle (layout type 2), descriptor version 1.
-//   K-major operand : rows of 128 bytes, 8-row groups 1024 bytes apart (SBO); LBO unused.
-//   MN-major operand: 128-byte runs along M/N; the next 8 K-rows are SBO bytes on, the next 128 M/N LBO bytes on.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint64_t layout_type = 2)
+// 16 TMEM lanes x 32 consecutive columns as matrix fragments: of every 8 columns thread t receives row t/4 in v[4i], v[4i+1]
+// and row t/4 + 8 in v[4i+2], v[4i+3], columns 8i + 2 (t%4) and the next one.
+__device__ __forceinline__ void tmem_ld16x256b_x4(uint32_t taddr, uint32_t (&v)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+// Four 8x8 matrices of 16-bit values, each stored transposed: lane 8j + r names the row of matrix j that receives the
+// fragment's column r.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Shared-memory matrix descriptor, version 1.
+//   K-major operand : rows of 128 bytes, 8-row groups SBO bytes apart; LBO unused.
+//   MN-major operand: runs of one swizzle width along M/N; the next 8 K-rows are SBO bytes on, the next run LBO bytes on.
+enum : uint32_t { kSwizzle128 = 2, kSwizzle64 = 4, kSwizzle32 = 6 };
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout_type)
 {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
     d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
     d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
     d |= 1ull << 46;
-    d |= layout_type << 61;  // 2 = 128-byte swizzle, 6 = 32-byte swizzle
+    d |= (uint64_t)layout_type << 61;
     return d;
 }
 
-// Instruction descriptor for kind::i8: D = S32 (2 at bit 4), A = B = signed 8-bit (1 at bits 7 and 10),
-// A K-major, B major per flag (bit 16), N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t make_idesc(bool b_mn_major, int m)
+// Descriptor of the weight operand of a stage at `addr`; the next 32 K-rows are weight_k_step bytes on.
+template <bool SPLIT, int BL>
+__device__ __forceinline__ uint64_t weight_desc(uint32_t addr)
 {
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(BN >> 3) << 17) |
-           ((uint32_t)(m >> 4) << 24);
+    // transposed: rows of 128 K-bytes, one per channel.
+    if (BL == kBTransposed) return make_smem_desc(addr, 16, 1024, kSwizzle128);
+    // fractal: 32-byte runs along the channels, 8 K-rows = 256 B, next 32 channels 128 K-rows (4096 B) on.
+    if (BL == kBFractalNz) return make_smem_desc(addr, 4096, 256, kSwizzle32);
+    // [E,K,N], swiglu on a pair: two boxes of 64 channels, 8 K-rows = 512 B, next 64 channels one box on.
+    if (SPLIT) return make_smem_desc(addr, W_STAGE / 2, 512, kSwizzle64);
+    // [E,K,N]: one box of 128 channels, 8 K-rows = 1024 B.
+    return make_smem_desc(addr, W_STAGE, 1024, kSwizzle128);
+}
+__host__ __device__ constexpr uint32_t weight_k_step(bool split, int bl)
+{
+    return bl == kBTransposed ? UMMA_K : UMMA_K * (bl == kBFractalNz ? 32u : split ? 64u : 128u);
+}
+
+// Instruction descriptor for kind::i8: D = S32 (2 at bit 4), A = B = signed 8-bit (1 at bits 7 and 10), A (weights) major
+// per flag (bit 15), B (tokens) K-major, N >> 3 at bit 17, M >> 4 at bit 24.
+__host__ __device__ constexpr uint32_t make_idesc(bool a_mn_major, int m)
+{
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((a_mn_major ? 1u : 0u) << 15) | ((uint32_t)(m >> 4) << 24);
 }
 
 // ---------------------------------------------------------------------------------------------------------
 // Tile schedule, rebuilt by every CTA from group_list (<= 1024 entries)
 // ---------------------------------------------------------------------------------------------------------
 
+// Token rows per tile of a group of `rows` rows: as few tiles as MAX_TOK rows allow, of nearly equal size (a multiple of 32).
+// Equal tiles keep the units of a wave together; their sum costs the same as full tiles and a short one.
+template <int MAX_TOK>
+__device__ __forceinline__ int tile_tokens(int rows)
+{
+    const int nt = (rows + MAX_TOK - 1) / MAX_TOK;
+    return nt == 0 ? TOK_STEP : ((rows + nt - 1) / nt + TOK_STEP - 1) / TOK_STEP * TOK_STEP;
+}
+
 // Row ranges follow GetSplitValueFromGroupList (gmm/grouped_matmul/op_kernel/grouped_matmul_utils.h:243-257):
 // type 0 = running total, type 1 = count, values narrowed to int32; groups with no rows are skipped
 // (grouped_matmul.h:263).  Ranges are clipped to [0, M] so a malformed list cannot address other memory.
-__device__ void build_schedule(Shared *sh, const KParams &p, int tile_m)
+template <int MAX_TOK>
+__device__ void build_schedule(Shared *sh, const KParams &p)
 {
     const int tid = threadIdx.x, L = p.gl_len;
     for (int g = tid; g < L; g += (int)blockDim.x) {
@@ -475,25 +551,20 @@ __device__ void build_schedule(Shared *sh, const KParams &p, int tile_m)
                 run += max(sh->rows[g], 0);
             }
         }
-        int tsum = 0;
+        int tsum = 0, max_tok = TOK_STEP;
         for (int g = lo; g < hi; ++g) {
             long long start = sh->row_start[g], rows = sh->rows[g];
             if (rows < 0) rows = 0;
             if (start < 0) { rows += start; start = 0; if (rows < 0) rows = 0; }
             if (start > p.M) { start = p.M; rows = 0; }
             if (start + rows > p.M) rows = p.M - start;
-            if (p.part != 0) {
-                // A 256-row tile on a trailing block of at most 128 rows would leave the second CTA of the pair idle:
-                // the pair launch (part 1) stops short of such a block and a launch with 128-row tiles (part 2) takes it.
-                const long long r = rows % (2 * BM);
-                const bool small_tail = r > 0 && r <= BM;
-                if (p.part == 1) { if (small_tail) rows -= r; }
-                else if (small_tail) { start += rows - r; rows = r; }
-                else rows = 0;
-            }
             sh->row_start[g] = (int)start;
             sh->rows[g] = (int)rows;
-            tsum += (int)((rows + tile_m - 1) / tile_m) * p.n_tiles;
+            const int tt = tile_tokens<MAX_TOK>((int)rows);
+            const int tiles = (int)((rows + tt - 1) / tt) * p.n_tiles;
+            max_tok = max(max_tok, tt);
+            sh->tile_start[g] = tiles;
+            tsum += tiles;
         }
         int incl = tsum;
         for (int o = 1; o < 32; o <<= 1) {
@@ -502,10 +573,13 @@ __device__ void build_schedule(Shared *sh, const KParams &p, int tile_m)
         }
         int run = incl - tsum;
         for (int g = lo; g < hi; ++g) {
+            const int tiles = sh->tile_start[g];
             sh->tile_start[g] = run;
-            run += ((sh->rows[g] + tile_m - 1) / tile_m) * p.n_tiles;
+            run += tiles;
         }
+        max_tok = __reduce_max_sync(0xffffffffu, max_tok);
         if (lane == 31) {
+            sh->max_tok = max_tok;
             sh->tile_start[L] = incl;
             sh->total_tiles = incl;
         }
@@ -513,24 +587,36 @@ __device__ void build_schedule(Shared *sh, const KParams &p, int tile_m)
     __syncthreads();
 }
 
+// Rows of x a CTA loads per K block for its share of a tile: one box, the smallest of 32, 64 or 128 rows that covers the
+// share, or two of 128.
+template <int CTAS>
+__device__ __forceinline__ int x_box_rows(int share)
+{
+    return CTAS == 1 && share > 128 ? 256 : share > 64 ? 128 : share > 32 ? 64 : 32;
+}
+
 struct Tile {
     int g, row0, rows, n_idx;
 };
 
-__device__ __forceinline__ Tile decode_tile(const Shared *sh, int t, int n_tiles, int L, int tile_m)
+// `from`: the group of this unit's previous tile (tiles are visited in ascending order); normally the next one is near.
+template <int MAX_TOK>
+__device__ __forceinline__ Tile decode_tile(const Shared *sh, int t, int n_tiles, int L, int from = 0)
 {
-    int lo = 0, hi = L;  // largest g in [0, L) with tile_start[g] <= t
+    int lo = from, hi = min(from + 4, L);  // largest g in [0, L) with tile_start[g] <= t
+    if (sh->tile_start[hi] <= t) { lo = hi; hi = L; }
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (sh->tile_start[mid] <= t) lo = mid; else hi = mid;
     }
     const int local = t - sh->tile_start[lo];
     const int mb = local / n_tiles;
+    const int tt = tile_tokens<MAX_TOK>(sh->rows[lo]);
     Tile tl;
     tl.g = lo;
     tl.n_idx = local - mb * n_tiles;
-    tl.row0 = sh->row_start[lo] + mb * tile_m;
-    tl.rows = min(tile_m, sh->rows[lo] - mb * tile_m);
+    tl.row0 = sh->row_start[lo] + mb * tt;
+    tl.rows = min(tt, sh->rows[lo] - mb * tt);
     return tl;
 }
 
@@ -589,7 +675,7 @@ __device__ void requant_rows(const KParams &p, int r_begin, int r_end, int warp_
     const int H = p.half_n;
     const int nf = H >> 2;  // 16-byte pieces per row
     const float *stage = reinterpret_cast<const float *>(p.out);
-    for (int grow = r_begin + warp_r; grow < r_end; grow += EPI_WARPS) {
+    for (int grow = r_begin + warp_r; grow < r_end; grow += RQ_WARPS) {
         const float amax = __uint_as_float(__ldcg(p.amax_bits + grow));
         const float4 *src = reinterpret_cast<const float4 *>(stage + (size_t)grow * H);
         uint32_t *dst = reinterpret_cast<uint32_t *>(p.q_out + (size_t)grow * H);
@@ -720,72 +806,113 @@ __device__ void release_pending(const KParams &p, Shared *sh, int ws, int shares
     sh->pend_n = 0;
 }
 
-// Epilogue warp: requantise the row ranges of the next work list(s).  Every warp consumes every list, in order, and takes
-// the rows warp, warp + EPI_WARPS, ... of each range.  With `blocking` unset only lists that are already written are
-// taken; otherwise the call waits (bounded) for the next one.  Returns false when a wait gave up.
-__device__ __forceinline__ bool consume_work(const KParams &p, Shared *sh, int &lists_done, int warp_e, int lane, bool blocking)
+// Requantising warp: the row ranges of the next work list.  Every warp consumes every list, in order, and takes the rows
+// warp, warp + RQ_WARPS, ... of each range.  Returns false when the (bounded) wait for the list gave up.
+__device__ __forceinline__ bool consume_work(const KParams &p, Shared *sh, int list, int warp_r, int lane)
 {
-    while (true) {
-        const int ws = lists_done % WK_DEPTH;
-        const uint32_t parity = ((uint32_t)(lists_done / WK_DEPTH)) & 1u;
-        int ready = 0;
-        if (lane == 0) {
-            ready = mbar_try_wait(smem_u32(&sh->wk_full[ws]), parity) ? 1 : 0;
-            if (!ready && blocking) ready = mbar_wait(&sh->wk_full[ws], parity, sh, p.status, 650 + ws) ? 1 : -1;
-        }
-        ready = __shfl_sync(0xffffffffu, ready, 0);
-        if (ready <= 0) return ready == 0;
-        const int n = sh->n_work[ws];
-        for (int k = 0; k < n; ++k) requant_rows(p, sh->work_begin[ws][k], sh->work_end[ws][k], warp_e, lane);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->wk_empty[ws]);
-        ++lists_done;
-        if (blocking) return true;
-    }
+    const int ws = list % WK_DEPTH;
+    const bool ok = mbar_wait(&sh->wk_full[ws], ((uint32_t)(list / WK_DEPTH)) & 1u, sh, p.status, 650 + ws);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    const int n = sh->n_work[ws];
+    for (int k = 0; k < n; ++k) requant_rows(p, sh->work_begin[ws][k], sh->work_end[ws][k], warp_r, lane);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->wk_empty[ws]);
+    return true;
+}
+
+// a / (1 + exp(-a)), for a < 0 as a e / (1 + e), with e = exp(-|a|) so that nothing overflows:  e = 2^t (1 + d ln 2) with
+// t = fl(-|a| log2 e) and d the remainder of that product (log2 e in two parts), the quotient from an approximate reciprocal
+// r of the denominator in [1, 2] and one correction q + (n - q den) r (Markstein).  As exact as expf and a correctly rounded
+// division (the 2-ulp ex2 is what either form is left with), in half of the instructions and without a branch.  An infinite
+// quotient is kept as it is; NaN stays NaN.
+__device__ __forceinline__ float silu(float a)
+{
+    const float x = fminf(fabsf(a), 150.0f);
+    const float t = __fmul_rn(x, -1.44269502f);
+    const float d = __fmaf_rn(x, -1.92596303e-8f, __fmaf_rn(x, -1.44269502f, -t));
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+    e = __fmaf_rn(e, __fmul_rn(d, 0.693147181f), e);
+    const float den = __fadd_rn(1.0f, e);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+    const float n = a < 0.0f ? __fmul_rn(a, e) : a;
+    const float q = __fmul_rn(n, r);
+    const float c = __fmaf_rn(__fmaf_rn(-q, den, n), r, q);
+    return fabsf(q) <= 3.402823466e38f ? c : q;
+}
+
+// A meeting of the epilogue warps that exchange values through shared memory (2 or 4 of them per barrier): every warp's
+// earlier accesses to the staging area are done and visible to the others when it returns.  Bounded like every wait, and
+// the same answer for all lanes of a warp; false = give up.
+__device__ __forceinline__ bool group_sync(uint64_t *bar, uint32_t &phase, Shared *sh, int *status, int lane, int who)
+{
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+    const bool ok = mbar_wait(bar, phase, sh, status, who);
+    phase ^= 1u;
+    return __all_sync(0xffffffffu, ok);
+}
+
+// 16 tokens x 32 channels of 32-bit values, one channel per lane: afterwards eight lanes hold 128 contiguous bytes of one
+// token's row.  Piece i of lane l is token i * 4 + l / 8, channels 4 * (l % 8) .. + 3.
+__device__ __forceinline__ void transpose16(uint8_t *stage, const uint32_t (&v)[16], int lane, uint4 (&out)[4])
+{
+#pragma unroll
+    for (int t = 0; t < 16; ++t) *reinterpret_cast<uint32_t *>(stage + t * 128 + lane * 4) = v[t];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = *reinterpret_cast<const uint4 *>(stage + (i * 4 + (lane >> 3)) * 128 + (lane & 7) * 16);
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------------------------------------
 
+struct XMaps {
+    CUtensorMap box[X_MAPS];  // boxes of 32 << i rows
+};
+
 // EPI selects the epilogue variant: kEpiPlain = no bias, no activation, per-token scale present, rows stored in place
 // (the common case, compiled without per-element tests for the options); kEpiScatter = the same arithmetic with the
 // result rows scattered through out_row_index, optionally into other GPUs' memory; kEpiGeneric = every option
-// tested at run time.  CTAS: 1 = one CTA per tile, 2 = a cluster of two CTAs per 256-row tile.
+// tested at run time.  CTAS: 1 = one CTA per tile (128 channels), 2 = a cluster of two CTAs (256 channels).
 template <int MODE, int BL, int EPI, int CTAS>
 __global__ void __launch_bounds__(num_threads(MODE), 1)
-gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const KParams p)
+gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constant__ CUtensorMap map_w, const KParams p)
 {
-    constexpr bool B_MN_MAJOR = BL != kBTransposed;  // [E,K,N] and the fractal layout are N-contiguous
     constexpr bool PLAIN = EPI != kEpiGeneric;   // lean arithmetic
     constexpr bool SCATTER = EPI != kEpiPlain;  // rows go where out_row_index says
     constexpr bool COMBINE = EPI == kEpiCombine;  // fp32 rows combined into row_index[r] of a [out_rows, N] result
-    using C = Cfg<CTAS>;
-    constexpr int STAGES = C::kStages;
-    constexpr int STAGE_BYTES = C::kStageBytes;
+    constexpr bool SWIGLU = MODE == kModeSwigluQuant;
+    constexpr bool OUT16 = MODE == kModeDequantBf16 && !COMBINE;
+    using S = Shape<MODE, CTAS>;
+    constexpr bool DUAL = S::kDual;
+    constexpr int CH_CTA = S::kCols, MAX_TOK = S::kMaxTok, W_BYTES = S::kWStage;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     Shared *sh = reinterpret_cast<Shared *>(smem + PIPE_BYTES);
-    // stage s: A at smem + s * STAGE_BYTES, weight box(es) right behind it
+    // stage s: this CTA's channels at smem + s * stage_bytes, its token rows right behind them
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // known to be uniform
     const uint32_t rank = CTAS == 2 ? cluster_cta_rank() : 0u;  // position in the pair; rank 0 issues the MMAs
     const int unit = CTAS == 2 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;   // tile-processing unit (CTA or pair)
     const int n_units = CTAS == 2 ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
             mbar_init(&sh->full[s], 1);   // pair: only rank 0's is used; its producer arrives, both CTAs' copies credit it
             mbar_init(&sh->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sh->acc_full[b], 1);
             mbar_init(&sh->acc_empty[b], EPI_WARPS * CTAS);  // one arrival per epilogue warp of every CTA of the unit
+            mbar_init(&sh->tok_ready[b], EPI_THREADS);
         }
-        for (int b = 0; b < SCALE_BUFS; ++b) mbar_init(&sh->scale_ready[b], EPI_THREADS);
+        for (int b = 0; b < 4; ++b) mbar_init(&sh->grp_sync[b], SWIGLU ? 2 : 4);
         for (int b = 0; b < WK_DEPTH; ++b) {
             mbar_init(&sh->wk_full[b], 1);
-            mbar_init(&sh->wk_empty[b], EPI_WARPS);
+            mbar_init(&sh->wk_empty[b], RQ_WARPS);
         }
         sh->stored_count = 0;
         sh->abort_flag = 0;
@@ -793,97 +920,99 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         sh->wait_limit = p.wait_limit;
         sh->pend_n = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        prefetch_map(&map_x);
+        for (int i = 0; i < X_MAPS; ++i) prefetch_map(&maps_x.box[i]);
         prefetch_map(&map_w);
     }
     if (warp == 1) {
         tmem_alloc<CTAS>(&sh->tmem_base, TMEM_COLS);
         tc_fence_before();
     }
-    build_schedule(sh, p, C::kTileM);  // ends with __syncthreads()
+    build_schedule<MAX_TOK>(sh, p);  // ends with __syncthreads()
     if (CTAS == 2) cluster_sync_all();  // the partner's barriers exist before anything is sent to them
     tc_fence_after();
 
     const int total_tiles = sh->total_tiles;
+    const int stage_bytes = W_BYTES + x_box_rows<CTAS>(sh->max_tok / CTAS) * BK;
+    const int stages = min(PIPE_BYTES / stage_bytes, MAX_STAGES);
     const uint32_t tmem_base = sh->tmem_base;
     const int L = p.gl_len;
 
     if (warp == 0) {
-        // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
+        // ------------------------------ TMA producer (whole warp, one elected lane issues) ------------------------------
+        {
+            const bool leader = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             long long issued = 0;
             bool ok = true;
             // pair: rank 0's full barriers as shared::cluster addresses (barriers are 8 bytes apart)
             const uint32_t full_rank0 = CTAS == 2 ? map_to_cta(&sh->full[0], 0) : 0u;
-            // Pacing: the units of a wave (one round of the static schedule) share their operands through L2 - the N tiles
-            // of a row block read the same rows of x, the row blocks of an expert the same weight boxes - and one launch
+            // Pacing: the units of a wave (one round of the static schedule) share their operands through L2 - the channel
+            // tiles of a row block read the same rows of x, the row blocks of an expert the same weight boxes - and one launch
             // streams many times the L2's capacity, so a unit that drifts a tile or two away from the others finds the
             // shared data evicted and fetches it from DRAM again.  Every unit therefore announces the wave it starts and
             // waits, for at most about one tile's duration, until all units have started the wave before.  It is a hint,
             // never needed for correctness: when the wait runs out (units not resident together) pacing is switched off.
             bool pace = p.wave_cnt != nullptr && rank == 0;
             int wave = 0;
+            Tile next = unit < total_tiles ? decode_tile<MAX_TOK>(sh, unit, p.n_tiles, L) : Tile{};
             for (int t = unit; t < total_tiles && ok; t += n_units, ++wave) {
-                const Tile tl = decode_tile(sh, t, p.n_tiles, L, C::kTileM);
-                // A CTA none of whose 128 rows belong to the group (the second CTA of a pair on a trailing block of at most
-                // 128 rows) loads from beyond the last row of x instead: TMA then fills the box with zeros without touching
-                // memory, and the tensor core multiplies zeros instead of the next group's rows (less traffic, less power;
-                // the results of those rows are discarded either way).
-                const int my_row0 = tl.rows > (int)rank * BM ? tl.row0 + (int)rank * BM : p.M;
+                const Tile tl = next;
                 if (pace) {
-                    if (wave > 0) {
-                        const int expected = min(n_units, total_tiles - (wave - 1) * n_units);
-                        const long long t0 = clock64();
-                        while (ld_relaxed_gpu(p.wave_cnt + wave - 1) < expected) {
-                            if (clock64() - t0 > p.pace_cycles) { pace = false; break; }
-                            __nanosleep(500);
+                    if (lane == 0) {
+                        if (wave > 0) {
+                            const int expected = min(n_units, total_tiles - (wave - 1) * n_units);
+                            const long long t0 = clock64();
+                            while (ld_relaxed_gpu(p.wave_cnt + wave - 1) < expected) {
+                                if (clock64() - t0 > p.pace_cycles) { pace = false; break; }
+                                __nanosleep(500);
+                            }
                         }
+                        asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(p.wave_cnt + wave) : "memory");
                     }
-                    asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(p.wave_cnt + wave) : "memory");
+                    pace = __shfl_sync(0xffffffffu, pace ? 1 : 0, 0) != 0;
                 }
-                int n0, n1;
-                if (MODE == kModeSwigluQuant) { n0 = tl.n_idx * (BN / 2); n1 = p.half_n + n0; }
-                else { n0 = tl.n_idx * BN; n1 = n0 + BN / 2; }
-                const int nb = rank == 0 ? n0 : n1;  // pair: the weight box this CTA contributes
+                // This CTA's share of the tokens; rows beyond the group or the tensor (zero filled) are never stored.
+                const int my_tok = (tl.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP / CTAS;
+                const int my_row0 = tl.row0 + (int)rank * my_tok;
+                const int x_rows = x_box_rows<CTAS>(my_tok);
+                const CUtensorMap *map_x = &maps_x.box[x_rows >= 128 ? 2 : x_rows >= 64 ? 1 : 0];
+                const uint32_t tx_bytes = (uint32_t)CTAS * (uint32_t)(W_BYTES + x_rows * BK);
+                const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA;   // first weight column of this CTA
                 // test hook: leaving K blocks out of the last tile makes the MMA issuer's wait run out (nothing else is touched)
                 const int kb_end = p.num_k_blocks - (t + n_units >= total_tiles ? p.skip_k_blocks : 0);
                 for (int kb = 0; kb < kb_end; ++kb) {
-                    if (!mbar_wait(&sh->empty[stage], phase ^ 1u, sh, p.status, 100 + stage)) { ok = false; break; }
-                    uint8_t *adst = smem + stage * STAGE_BYTES;
-                    uint8_t *bdst = adst + A_STAGE;
-                    if (CTAS == 1) {
-                        mbar_arrive_expect_tx(&sh->full[stage], C::kTxBytes);
-                        tma_load_2d(adst, &map_x, kb * BK, my_row0, &sh->full[stage]);
-                        if (BL == kBFractalNz) {  // map dims {32 n, 16 k, K/16, N/32, E}: a box is 128 k x 128 n in 32-column slabs
-                            tma_load_5d(bdst, &map_w, 0, 0, kb * (BK / 16), n0 >> 5, tl.g, &sh->full[stage]);
-                            tma_load_5d(bdst + B_BOX, &map_w, 0, 0, kb * (BK / 16), n1 >> 5, tl.g, &sh->full[stage]);
-                        } else if (B_MN_MAJOR) {  // weight [E, K, N]: map dims {N, K, E}
-                            tma_load_3d(bdst, &map_w, n0, kb * BK, tl.g, &sh->full[stage]);
-                            tma_load_3d(bdst + B_BOX, &map_w, n1, kb * BK, tl.g, &sh->full[stage]);
-                        } else {           // weight [E, N, K]: map dims {K, N, E}
-                            tma_load_3d(bdst, &map_w, kb * BK, n0, tl.g, &sh->full[stage]);
-                            tma_load_3d(bdst + B_BOX, &map_w, kb * BK, n1, tl.g, &sh->full[stage]);
-                        }
-                    } else {
-                        if (rank == 0) mbar_arrive_expect_tx(&sh->full[stage], C::kTxBytes);
-                        tma_load_2d_pair(adst, &map_x, kb * BK, my_row0, full_rank0 + (uint32_t)stage * 8u);
-                        if (BL == kBFractalNz) tma_load_5d_pair(bdst, &map_w, 0, 0, kb * (BK / 16), nb >> 5, tl.g, full_rank0 + (uint32_t)stage * 8u);
-                        else if (B_MN_MAJOR) tma_load_3d_pair(bdst, &map_w, nb, kb * BK, tl.g, full_rank0 + (uint32_t)stage * 8u);
-                        else tma_load_3d_pair(bdst, &map_w, kb * BK, nb, tl.g, full_rank0 + (uint32_t)stage * 8u);
+#ifdef GMM_TRACE
+                    const long long tw0 = clock64();
+#endif
+                    if (!__all_sync(0xffffffffu, mbar_wait(&sh->empty[stage], phase ^ 1u, sh, p.status, 100 + stage))) { ok = false; break; }
+#ifdef GMM_TRACE
+                    if (lane == 0) TRACE_ADD(0, wave, 2, clock64() - tw0);
+#endif
+                    if (leader) {
+                        uint8_t *wdst = smem + stage * stage_bytes;
+                        const uint32_t bar = CTAS == 2 ? full_rank0 + (uint32_t)stage * 8u : smem_u32(&sh->full[stage]);
+                        if (rank == 0) mbar_arrive_expect_tx(&sh->full[stage], tx_bytes);
+                        if (BL == kBFractalNz) tma_load_5d<CTAS>(wdst, &map_w, 0, kb * BK, c0 >> 5, 0, tl.g, bar);
+                        else if (BL == kBTransposed) tma_load_4d<CTAS>(wdst, &map_w, kb * BK, c0, 0, tl.g, bar);
+                        else tma_load_4d<CTAS>(wdst, &map_w, c0, kb * BK, 0, tl.g, bar);
+                        tma_load_2d<CTAS>(wdst + W_BYTES, map_x, kb * BK, my_row0, bar);
+                        if (CTAS == 1 && x_rows > 128) tma_load_2d<CTAS>(wdst + W_BYTES + 128 * BK, map_x, kb * BK, my_row0 + 128, bar);
                     }
+                    __syncwarp();
+                    // the next tile is looked up while the ring is full, not between two tiles
+                    if (kb == 0 && t + n_units < total_tiles) next = decode_tile<MAX_TOK>(sh, t + n_units, p.n_tiles, L, tl.g);
                     ++issued;
-                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                    if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
             }
-            if ((!ok || *(volatile int *)&sh->abort_flag) && rank == 0) {
+            if (lane == 0 && (!ok || *(volatile int *)&sh->abort_flag) && rank == 0) {
                 // Drain: give the copies already issued a bounded chance to land before the CTA leaves.
-                const int n = (int)(issued < STAGES ? issued : STAGES);
+                const int n = (int)(issued < stages ? issued : stages);
                 int s2 = stage;
                 uint32_t ph = phase;
                 for (int i = 0; i < n; ++i) {
-                    if (--s2 < 0) { s2 = STAGES - 1; ph ^= 1u; }
+                    if (--s2 < 0) { s2 = stages - 1; ph ^= 1u; }
                     const uint32_t a = smem_u32(&sh->full[s2]);
                     const long long t0 = clock64();
                     while (!mbar_try_wait(a, ph) && clock64() - t0 < DRAIN_LIMIT_CYCLES) {}
@@ -891,9 +1020,15 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             }
         }
     } else if (warp == 1) {
-        // ------------------------------ MMA issuer (rank 0 of the unit) ------------------------------
-        if (lane == 0 && rank == 0) {
-            constexpr uint32_t idesc = make_idesc(B_MN_MAJOR, C::kTileM);
+        // ------------------------------ MMA issuer (rank 0 of the unit; whole warp, one elected lane issues) ------------------------------
+        if (rank == 0) {
+            constexpr uint32_t idesc0 = make_idesc(BL != kBTransposed, BC * CTAS);  // [E,K,N] and fractal are channel-contiguous
+            const bool leader = elect_one();
+            // descriptors of stage 0, MMA 0; the address field counts 16-byte units
+            const uint32_t smem0 = smem_u32(smem);
+            const uint64_t w_desc0 = weight_desc<SWIGLU && !DUAL, BL>(smem0);
+            const uint64_t x_desc0 = make_smem_desc(smem0 + W_BYTES, 16, 1024, kSwizzle128);
+            constexpr uint32_t W_STEP = weight_k_step(SWIGLU && !DUAL, BL) >> 4, X_STEP = UMMA_K >> 4;
             int stage = 0;
             uint32_t phase = 0;
             int buf = 0;
@@ -902,331 +1037,329 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             const uint32_t empty_peer = CTAS == 2 ? map_to_cta(&sh->empty[0], 1) : 0u;       // the partner's barriers
             const uint32_t acc_full_peer = CTAS == 2 ? map_to_cta(&sh->acc_full[0], 1) : 0u;
             int ti = 0;
-            TRACE_GT(0, 0, 0);
+            if (lane == 0) TRACE_GT(0, 0, 0);
+            Tile next = unit < total_tiles ? decode_tile<MAX_TOK>(sh, unit, p.n_tiles, L) : Tile{};
             for (int t = unit; t < total_tiles && ok; t += n_units, ++ti) {
-                TRACE(1, ti, 0);
-                if (!mbar_wait(&sh->acc_empty[buf], acc_phase ^ 1u, sh, p.status, 200 + buf)) { ok = false; break; }
-                TRACE(1, ti, 1);
+                const Tile tl = next;
+                const uint32_t idesc = idesc0 | (uint32_t)(((tl.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP) >> 3) << 17;
+                if (lane == 0) TRACE(1, ti, 0);
+                if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[buf], acc_phase ^ 1u, sh, p.status, 200 + buf))) { ok = false; break; }
+                if (lane == 0) TRACE(1, ti, 1);
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)buf * BN;
+                const uint32_t d_tmem = tmem_base + (uint32_t)buf * BT;
                 for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-                    if (!mbar_wait(&sh->full[stage], phase, sh, p.status, 300 + stage)) { ok = false; break; }
+#ifdef GMM_TRACE
+                    const long long tw0 = clock64();
+#endif
+                    if (!__all_sync(0xffffffffu, mbar_wait(&sh->full[stage], phase, sh, p.status, 300 + stage))) { ok = false; break; }
+#ifdef GMM_TRACE
+                    if (lane == 0) {
+                        TRACE_ADD(1, ti, 3, clock64() - tw0);
+                        TRACE_ADD(1, ti, 4, kb == 0 ? clock64() - tw0 : 0);
+                    }
+#endif
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + stage * STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + A_STAGE;
+                    if (leader) {
+                        const uint64_t w_desc = w_desc0 + (uint64_t)(stage * (stage_bytes >> 4));
+                        const uint64_t x_desc = x_desc0 + (uint64_t)(stage * (stage_bytes >> 4));
 #pragma unroll
-                    for (int j = 0; j < BK / UMMA_K; ++j) {
-                        const uint64_t a_desc = make_smem_desc(a_addr + j * UMMA_K, 16, 1024);
-                        // [E,K,N]: 128-byte runs along N, 8 K-rows = 1024 B, next 128 columns one box on.
-                        // fractal: 32-byte runs along N, 8 K-rows = 256 B, next 32 columns 128 K-rows (4096 B) on.
-                        const uint64_t b_desc = BL == kBFractalNz ? make_smem_desc(b_addr + j * UMMA_K * 32, 4096, 256, 6)
-                                                : B_MN_MAJOR      ? make_smem_desc(b_addr + j * UMMA_K * 128, B_BOX, 1024)
-                                                                  : make_smem_desc(b_addr + j * UMMA_K, 16, 1024);
-                        if (CTAS == 1) umma_i8(d_tmem, a_desc, b_desc, idesc, (kb | j) != 0 ? 1u : 0u);
-                        else umma_i8_pair(d_tmem, a_desc, b_desc, idesc, (kb | j) != 0 ? 1u : 0u);
+                        for (int j = 0; j < BK / UMMA_K; ++j) {
+                            if (CTAS == 1) umma_i8(d_tmem, w_desc + j * W_STEP, x_desc + j * X_STEP, idesc, (kb | j) != 0 ? 1u : 0u);
+                            if (DUAL) umma_i8(d_tmem + MAX_TOK, w_desc + (W_STAGE >> 4) + j * W_STEP, x_desc + j * X_STEP, idesc, (kb | j) != 0 ? 1u : 0u);
+                            if (CTAS == 2) umma_i8_pair(d_tmem, w_desc + j * W_STEP, x_desc + j * X_STEP, idesc, (kb | j) != 0 ? 1u : 0u);
+                        }
+                        if (CTAS == 1) {
+                            umma_commit(&sh->empty[stage]);
+                        } else {  // the stage is free in both CTAs once these MMAs have read it
+                            umma_commit_pair(smem_u32(&sh->empty[stage]));
+                            umma_commit_pair(empty_peer + (uint32_t)stage * 8u);
+                        }
+                        if (kb == p.num_k_blocks - 1) {  // the tile's accumulators are complete
+                            if (CTAS == 1) {
+                                umma_commit(&sh->acc_full[buf]);
+                            } else {
+                                umma_commit_pair(smem_u32(&sh->acc_full[buf]));
+                                umma_commit_pair(acc_full_peer + (uint32_t)buf * 8u);
+                            }
+                        }
                     }
-                    if (CTAS == 1) {
-                        umma_commit(&sh->empty[stage]);
-                    } else {  // the stage is free in both CTAs once these MMAs have read it
-                        umma_commit_pair(smem_u32(&sh->empty[stage]));
-                        umma_commit_pair(empty_peer + (uint32_t)stage * 8u);
-                    }
-                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                    __syncwarp();
+                    if (kb == 0 && t + n_units < total_tiles) next = decode_tile<MAX_TOK>(sh, t + n_units, p.n_tiles, L, tl.g);
+                    if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                TRACE(1, ti, 2);
-                TRACE_GT(0, 0, 1);
-                if (CTAS == 1) {
-                    umma_commit(&sh->acc_full[buf]);
-                } else {
-                    umma_commit_pair(smem_u32(&sh->acc_full[buf]));
-                    umma_commit_pair(acc_full_peer + (uint32_t)buf * 8u);
-                }
+                if (lane == 0) TRACE(1, ti, 2);
+                if (lane == 0) TRACE_GT(0, 0, 1);
                 buf ^= 1;
                 if (buf == 0) acc_phase ^= 1u;
             }
         }
     } else if (warp < 2 + EPI_WARPS) {
-        // ------------------------------ epilogue: warp -> (TMEM lane quarter, column half) ------------------------------
+        // ------------------------------ epilogue: warp -> (TMEM lane quarter, every second chunk of 32 tokens) ------------------------------
         const int quarter = warp & 3;
         const int chalf = (warp - 2) >> 2;
-        const int te = (int)threadIdx.x - 64;  // 0 .. EPI_THREADS-1
-        const int r = quarter * 32 + lane;     // row inside the tile == TMEM lane
-        uint8_t *my_stage = sh->out_stage[warp - 2];
+        const int te = (int)threadIdx.x - 64;  // 0 .. EPI_THREADS-1: the token whose factors this thread fetches
+        uint8_t *my_stage = sh->out_stage + (warp - 2) * WARP_STAGE_BYTES;
+        uint8_t *half_stage = sh->out_stage + chalf * (32 * ROW16_PITCH);
+        // swiglu: the warp of the other half (gate / up) with the same columns and tokens, two lane quarters on; the two share a
+        // barrier
+        const bool up = !DUAL && quarter >= 2;
+        const int ch0 = SWIGLU && !DUAL ? (quarter & 1) * 32 : quarter * 32;   // first of this warp's 32 columns
+        uint8_t *partner_stage = sh->out_stage + (chalf * 4 + ((quarter ^ 2) + 2) % 4) * WARP_STAGE_BYTES;
+        uint64_t *grp_bar = &sh->grp_sync[SWIGLU ? chalf * 2 + (quarter & 1) : chalf];
+        uint32_t grp_phase = 0;
         int buf = 0, it = 0;
         uint32_t acc_phase = 0;
-        int lists_done = 0, lists_total = 0;
         const uint64_t pol_last = policy_evict_last();
         const uint32_t acc_empty_rank0 = CTAS == 2 ? map_to_cta(&sh->acc_empty[0], 0) : 0u;
+        bool ok = true;
+        int g_prev = 0;
         for (int t = unit; t < total_tiles; t += n_units, ++it) {
-            const Tile tl = decode_tile(sh, t, p.n_tiles, L, C::kTileM);
-            const int my_row0 = tl.row0 + (int)rank * BM;                 // this CTA's 128 rows of the tile
-            const int my_rows = max(0, min(BM, tl.rows - (int)rank * BM));
-            const bool valid = r < my_rows;
-            const bool warp_has_rows = quarter * 32 < my_rows;
-            const int grow = my_row0 + r;
+            const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                g_prev = tl.g;
             const size_t sbase = (size_t)tl.g * p.N;
-            const int n0 = MODE == kModeSwigluQuant ? tl.n_idx * (BN / 2) : tl.n_idx * BN;
+            const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA;   // first result column of this CTA
 
-            // Stage this tile's per-column scales in shared memory; the loads overlap the wait for the MMAs.
-            const int sb = it % SCALE_BUFS;
-            if (MODE != kModeInt32) {
-                int col;
-                bool in_range;
-                if (MODE == kModeSwigluQuant) {
-                    const int j = te < BN / 2 ? te : te - BN / 2;
-                    in_range = n0 + j < p.half_n;
-                    col = (te < BN / 2 ? 0 : p.half_n) + n0 + j;
-                } else {
-                    col = n0 + te;
-                    in_range = col < p.N;
+            // Per-channel values of this lane, and the factors of token te: all loads overlap the wait for the MMAs.
+            constexpr int NCH = OUT16 ? 4 : 1;   // fragment rows lane/4 + 8j, else the lane's own channel
+            float wsc[NCH], wsc_up = 0.0f;       // wsc_up: the linear half's, where the lane holds both
+            float bias_f[NCH];
+            int bias_i[NCH];
+            if (MODE != kModeInt32 || !PLAIN) {
+#pragma unroll
+                for (int j = 0; j < NCH; ++j) {
+                    const int lc = OUT16 ? quarter * 32 + (lane >> 2) + 8 * j : ch0 + lane;
+                    const int c = c0 + lc;
+                    const bool in = c < (SWIGLU ? p.half_n : p.N);
+                    const size_t col = sbase + (size_t)(SWIGLU && up ? p.half_n + c : c);
+                    wsc[j] = MODE != kModeInt32 && in ? load_scale1(p.w_scale, p.w_scale_dtype, col) : 0.0f;
+                    if (DUAL && in) wsc_up = load_scale1(p.w_scale, p.w_scale_dtype, col + p.half_n);
+                    bias_f[j] = 0.0f;
+                    bias_i[j] = 0;
+                    if ((!PLAIN || COMBINE) && in) {
+                        if (p.bias_dtype == kBF16) bias_f[j] = __uint_as_float((uint32_t)__ldg(reinterpret_cast<const uint16_t *>(p.bias) + col) << 16);
+                        else if (!COMBINE && p.bias_dtype == kI32) bias_i[j] = __ldg(reinterpret_cast<const int *>(p.bias) + col);
+                    }
                 }
-                sh->scales[sb][te] = in_range ? load_scale1(p.w_scale, p.w_scale_dtype, sbase + col) : 0.0f;
-                mbar_arrive(&sh->scale_ready[sb]);
             }
-            const float xs = (valid && p.x_scale) ? __ldg(p.x_scale + grow) : 1.0f;
-            long long out_row = grow;
-            float lg = 1.0f;
-            if (COMBINE) {
-                out_row = -1;
-                if (valid) {
-                    out_row = p.row_index_i32 ? (long long)__ldg(reinterpret_cast<const int *>(p.row_index) + grow)
-                                              : __ldg(reinterpret_cast<const long long *>(p.row_index) + grow);
-                    if (p.logit) lg = __ldg(p.logit + grow);
-                }
-            } else if (MODE != kModeSwigluQuant && SCATTER && p.out_row_index && valid) out_row = __ldg(p.out_row_index + grow);
+            float xs = 1.0f, lg = 1.0f;
+            if (te < tl.rows) {
+                if (MODE != kModeInt32 && p.x_scale) xs = __ldg(p.x_scale + tl.row0 + te);
+                if (COMBINE && p.logit) lg = __ldg(p.logit + tl.row0 + te);
+            }
             if (te == 0) TRACE(2, it, 0);
-            if (MODE != kModeInt32 && !mbar_wait(&sh->scale_ready[sb], (uint32_t)(it / SCALE_BUFS) & 1u, sh, p.status, 500 + sb)) break;
-            if (!mbar_wait(&sh->acc_full[buf], acc_phase, sh, p.status, 400 + buf)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[buf], acc_phase, sh, p.status, 400 + buf))) { ok = false; break; }
             if (te == 0) TRACE(2, it, 1);
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * BN;
-            const float *tsc = sh->scales[sb];
+            if (MODE != kModeInt32) {
+                sh->tok_scale[buf][te] = COMBINE && p.logit ? (p.x_scale ? __fmul_rn(xs, lg) : lg) : xs;
+                if (COMBINE) sh->tok_logit[buf][te] = lg;
+                mbar_arrive(&sh->tok_ready[buf]);
+                if (!__all_sync(0xffffffffu, mbar_wait(&sh->tok_ready[buf], acc_phase, sh, p.status, 500 + buf))) { ok = false; break; }
+            }
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * BT;
+            const float *tok = sh->tok_scale[buf];
 
-            if (warp_has_rows) {
-                if (MODE == kModeSwigluQuant) {
+            // 16 tokens of S, one column per lane: fp32 rows to the staging buffer, row maxima
+            auto store_s = [&](const uint32_t (&v)[16], int t0) {
+                uint4 o[4];
+                transpose16(my_stage, v, lane, o);
+                const int col = c0 + ch0 + (lane & 7) * 4;
+                float *sout = reinterpret_cast<float *>(p.out);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int tk = t0 + i * 4 + (lane >> 3);
+                    const float4 val = make_float4(__uint_as_float(o[i].x), __uint_as_float(o[i].y), __uint_as_float(o[i].z), __uint_as_float(o[i].w));
                     float amax = 0.0f;
-                    float *sout = reinterpret_cast<float *>(p.out);
-#pragma unroll 1
-                    for (int c = chalf * 2; c < chalf * 2 + 2; ++c) {
-                        if (n0 + c * 32 >= p.half_n) break;
-                        uint32_t va[32], vb[32];
-                        tmem_ld32(taddr + c * 32, va);
-                        tmem_ld32(taddr + BN / 2 + c * 32, vb);
-                        tmem_ld_wait();
+                    if (col < p.half_n) amax = fmaxf(fmaxf(fmaxf(fmaxf(0.0f, fabsf(val.x)), fabsf(val.y)), fabsf(val.z)), fabsf(val.w));
 #pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            const float4 sa = *reinterpret_cast<const float4 *>(tsc + c * 32 + j4 * 4);
-                            const float4 sg = *reinterpret_cast<const float4 *>(tsc + BN / 2 + c * 32 + j4 * 4);
-                            const float sav[4] = {sa.x, sa.y, sa.z, sa.w}, sgv[4] = {sg.x, sg.y, sg.z, sg.w};
+                    for (int s = 1; s < 8; s <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
+                    if (tk < tl.rows) {
+                        if (col < p.half_n) st_global_v4_hint(sout + (size_t)(tl.row0 + tk) * p.half_n + col, val, pol_last);
+                        if ((lane & 7) == 0) atomicMax(p.amax_bits + tl.row0 + tk, __float_as_uint(amax));
+                    }
+                }
+            };
+            if (DUAL) {
+                for (int tc = chalf * 16; tc < tl.rows; tc += 32) {
+                    uint32_t va[16], vb[16];
+                    tmem_ld16(taddr + tc, va);
+                    tmem_ld16(taddr + MAX_TOK + tc, vb);
+                    tmem_ld_wait();
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                // (acc * x_scale) * w_scale, then S = gate * (act / (1 + exp(-act)))
-                                const float a = __fmul_rn(__fmul_rn(__int2float_rn((int)va[j4 * 4 + j]), xs), sav[j]);
-                                const float b = __fmul_rn(__fmul_rn(__int2float_rn((int)vb[j4 * 4 + j]), xs), sgv[j]);
-                                const float den = __fadd_rn(1.0f, expf(-a));
-                                const float sw = __fdiv_rn(a, den);
-                                const float sv = __fmul_rn(b, sw);
-                                va[j4 * 4 + j] = __float_as_uint(sv);
-                                if (n0 + c * 32 + j4 * 4 + j < p.half_n) amax = fmaxf(amax, fabsf(sv));
-                            }
-                        }
-                        // Transpose through shared memory, 16 rows per round, so that eight lanes store 128 contiguous bytes
-                        // of one row of S: a store instruction then touches 4 lines instead of 32 (the shared-memory / L1
-                        // data path is the one the tensor cores read their operands through).
-                        const int pc = lane & 7;
-                        const int col = n0 + c * 32 + pc * 4;
+                    for (int i = 0; i < 16; ++i) {
+                        // (acc * x_scale) * w_scale, then S = gate * (act / (1 + exp(-act)))
+                        const float a = __fmul_rn(__fmul_rn(__int2float_rn((int)va[i]), tok[tc + i]), wsc[0]);
+                        const float b = __fmul_rn(__fmul_rn(__int2float_rn((int)vb[i]), tok[tc + i]), wsc_up);
+                        va[i] = __float_as_uint(__fmul_rn(b, silu(a)));
+                    }
+                    store_s(va, tc);
+                }
+            }
+            for (int tc = chalf * 32; !DUAL && tc < tl.rows && ok; tc += 64) {  // a chunk of 32 tokens
+                if (SWIGLU) {
+                    uint32_t v[32], own[16];
+                    tmem_ld32(taddr + tc, v);
+                    tmem_ld_wait();
+                    // (acc * x_scale) * w_scale.  The gate warp finishes tokens 0..15 of the chunk, the up warp 16..31: each
+                    // sends the other its values of the other's tokens.
 #pragma unroll
-                        for (int round = 0; round < 2; ++round) {
-                            if ((lane >> 4) == round) {
+                    for (int t4 = 0; t4 < 4; ++t4) {
+                        const float4 s0 = *reinterpret_cast<const float4 *>(tok + tc + t4 * 4);
+                        const float4 s1 = *reinterpret_cast<const float4 *>(tok + tc + 16 + t4 * 4);
+                        const float sl[4] = {s0.x, s0.y, s0.z, s0.w}, sh4[4] = {s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-                                for (int q8 = 0; q8 < 8; ++q8)
-                                    *reinterpret_cast<uint4 *>(my_stage + (lane & 15) * 128 + (((q8 ^ lane) & 7) << 4)) =
-                                        make_uint4(va[q8 * 4], va[q8 * 4 + 1], va[q8 * 4 + 2], va[q8 * 4 + 3]);
-                            }
-                            __syncwarp();
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int r16 = i * 4 + (lane >> 3);
-                                const int rr = quarter * 32 + round * 16 + r16;
-                                const float4 val = *reinterpret_cast<const float4 *>(my_stage + r16 * 128 + (((pc ^ r16) & 7) << 4));
-                                if (rr < my_rows && col < p.half_n)
-                                    st_global_v4_hint(sout + (size_t)(my_row0 + rr) * p.half_n + col, val, pol_last);
-                            }
-                            __syncwarp();
+                        for (int k = 0; k < 4; ++k) {
+                            const int i = t4 * 4 + k;
+                            const float lo = __fmul_rn(__fmul_rn(__int2float_rn((int)v[i]), sl[k]), wsc[0]);
+                            const float hi = __fmul_rn(__fmul_rn(__int2float_rn((int)v[16 + i]), sh4[k]), wsc[0]);
+                            own[i] = __float_as_uint(up ? hi : lo);
+                            *reinterpret_cast<float *>(partner_stage + i * 128 + lane * 4) = up ? lo : hi;
                         }
                     }
-                    if (valid) atomicMax(p.amax_bits + grow, __float_as_uint(amax));
-                } else if (MODE == kModeInt32) {
-#pragma unroll 1
-                    for (int c = chalf * 4; c < chalf * 4 + 4; ++c) {
-                        if (n0 + c * 32 >= p.N) break;
-                        uint32_t v[32];
-                        tmem_ld32(taddr + c * 32, v);
-                        tmem_ld_wait();
+                    if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 700)) { ok = false; break; }
 #pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            const int col = n0 + c * 32 + j4 * 4;
-                            if (col < p.N && valid && (!SCATTER || (out_row >= 0 && (p.out_rows <= 0 || out_row < p.out_rows)))) {
-                                int acc[4];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    acc[j] = (int)v[j4 * 4 + j];
-                                    if (!PLAIN && p.bias_dtype == kI32) acc[j] += __ldg(reinterpret_cast<const int *>(p.bias) + sbase + col + j);
-                                }
-                                *reinterpret_cast<int4 *>(reinterpret_cast<int *>(p.out) + (size_t)out_row * p.N + col) =
-                                    make_int4(acc[0], acc[1], acc[2], acc[3]);
-                            }
-                        }
+                    for (int i = 0; i < 16; ++i) {
+                        const float other = *reinterpret_cast<const float *>(my_stage + i * 128 + lane * 4);
+                        const float act = up ? other : __uint_as_float(own[i]);
+                        const float gate = up ? __uint_as_float(own[i]) : other;
+                        own[i] = __float_as_uint(__fmul_rn(gate, silu(act)));  // S = gate * (act / (1 + exp(-act)))
                     }
-                } else if (COMBINE) {
-                    // grouped_matmul_finalize_routing: t = float(acc) * scale[n]; t *= (per_token[m] * logit[m]);
-                    // t += logit[m] * float(bias[n]); y[row_index[m], n] += t  (ComputeDequantAndActivate,
-                    // DataCopyPerTokenScaleAndBrcb, VectorAtomicProcess of
-                    // gmm/grouped_matmul_finalize_routing/op_kernel/grouped_matmul_finalize_routing.h:418-448, 497-545, 343-366).
-                    float *out = reinterpret_cast<float *>(p.out);
-                    const float rs = p.logit ? (p.x_scale ? __fmul_rn(xs, lg) : lg) : xs;
-                    // One 32-column chunk at a time: 32 fp32 = 128 bytes per row and pass.
-#pragma unroll 1
-                    for (int c = chalf * 4; c < chalf * 4 + 4; ++c) {
-                        if (n0 + c * 32 >= p.N) break;
-                        uint32_t v[32], pk[32];
-                        tmem_ld32(taddr + c * 32, v);
-                        tmem_ld_wait();
+                    store_s(own, tc + (up ? 16 : 0));
+                    // the partner may write the next chunk's values here
+                    if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 710)) { ok = false; break; }
+                } else if (!OUT16) {
+                    // 32-bit results: int32 accumulators, or the combine
+                    //   t = float(acc) * scale[n]; t *= (per_token[m] * logit[m]); t += logit[m] * float(bias[n]);
+                    //   y[row_index[m], n] += t  (ComputeDequantAndActivate, DataCopyPerTokenScaleAndBrcb, VectorAtomicProcess
+                    //   of gmm/grouped_matmul_finalize_routing/op_kernel/grouped_matmul_finalize_routing.h:418-448, 497-545, 343-366)
+                    uint32_t v[32];
+                    tmem_ld32(taddr + tc, v);
+                    tmem_ld_wait();
+                    const int col = c0 + quarter * 32 + (lane & 7) * 4;
 #pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            const float4 s4 = *reinterpret_cast<const float4 *>(tsc + c * 32 + j4 * 4);
-                            const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
+                    for (int h = 0; h < 2; ++h) {
+                        const int t0 = tc + h * 16;
+                        if (t0 >= tl.rows) break;
+                        // where this lane's four rows go
+                        long long orow[4];
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const int cc = c * 32 + j4 * 4 + j;
-                                float tv = __fmul_rn(__fmul_rn(__int2float_rn((int)v[j4 * 4 + j]), sv[j]), rs);
-                                if (p.bias_dtype == kBF16 && n0 + cc < p.N) {
-                                    const float b = __uint_as_float((uint32_t)__ldg(reinterpret_cast<const uint16_t *>(p.bias) + sbase + n0 + cc) << 16);
-                                    tv = __fadd_rn(tv, __fmul_rn(lg, b));
-                                }
-                                pk[j4 * 4 + j] = __float_as_uint(tv);
+                        for (int i = 0; i < 4; ++i) {
+                            const int tk = t0 + i * 4 + (lane >> 3);
+                            orow[i] = -1;
+                            if (tk < tl.rows) {
+                                orow[i] = tl.row0 + tk;
+                                if (COMBINE)
+                                    orow[i] = p.row_index_i32 ? (long long)__ldg(reinterpret_cast<const int *>(p.row_index) + tl.row0 + tk)
+                                                              : __ldg(reinterpret_cast<const long long *>(p.row_index) + tl.row0 + tk);
+                                else if (SCATTER && p.out_row_index) orow[i] = __ldg(p.out_row_index + tl.row0 + tk);
                             }
                         }
-                        // Same transposition as the bf16 path: eight lanes then hold 128 contiguous bytes of one row, so a
-                        // vector reduction covers whole 32-byte sectors of the fp32 result.
-                        const int pc = lane & 7;
-                        const int col = n0 + c * 32 + pc * 4;
+                        uint32_t r[16];
 #pragma unroll
-                        for (int round = 0; round < 2; ++round) {
-                            if ((lane >> 4) == round) {
-#pragma unroll
-                                for (int q8 = 0; q8 < 8; ++q8)
-                                    *reinterpret_cast<uint4 *>(my_stage + (lane & 15) * 128 + (((q8 ^ lane) & 7) << 4)) =
-                                        make_uint4(pk[q8 * 4], pk[q8 * 4 + 1], pk[q8 * 4 + 2], pk[q8 * 4 + 3]);
+                        for (int i = 0; i < 16; ++i) {
+                            const int acc = (int)v[h * 16 + i];
+                            if (COMBINE) {
+                                float tv = __fmul_rn(__fmul_rn(__int2float_rn(acc), wsc[0]), tok[t0 + i]);
+                                if (p.bias_dtype == kBF16) tv = __fadd_rn(tv, __fmul_rn(sh->tok_logit[buf][t0 + i], bias_f[0]));
+                                r[i] = __float_as_uint(tv);
+                            } else {
+                                r[i] = (uint32_t)(!PLAIN ? acc + bias_i[0] : acc);
                             }
-                            __syncwarp();
+                        }
+                        uint4 o[4];
+                        transpose16(my_stage, r, lane, o);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int r16 = i * 4 + (lane >> 3);
-                                const int rr = round * 16 + r16;
-                                const float4 val = *reinterpret_cast<const float4 *>(my_stage + r16 * 128 + (((pc ^ r16) & 7) << 4));
-                                const long long orow = __shfl_sync(0xffffffffu, out_row, rr);
-                                if (quarter * 32 + rr < my_rows && col < p.N && orow >= 0 && orow < p.out_rows) {
-                                    float *dst = out + (size_t)orow * p.N + col;
-                                    if (p.scatter_add) red_add_v4(dst, val);
-                                    else *reinterpret_cast<float4 *>(dst) = val;
-                                }
+                        for (int i = 0; i < 4; ++i) {
+                            if (col >= p.N || orow[i] < 0) continue;
+                            if (COMBINE) {
+                                if (orow[i] >= p.out_rows) continue;
+                                float *dst = reinterpret_cast<float *>(p.out) + (size_t)orow[i] * p.N + col;
+                                const float4 val = make_float4(__uint_as_float(o[i].x), __uint_as_float(o[i].y), __uint_as_float(o[i].z), __uint_as_float(o[i].w));
+                                if (p.scatter_add) red_add_v4(dst, val);
+                                else *reinterpret_cast<float4 *>(dst) = val;
+                            } else {
+                                if (SCATTER && p.out_rows > 0 && orow[i] >= p.out_rows) continue;
+                                *reinterpret_cast<uint4 *>(reinterpret_cast<int *>(p.out) + (size_t)orow[i] * p.N + col) = o[i];
                             }
-                            __syncwarp();
                         }
                     }
                 } else {
-                    uint16_t *out = reinterpret_cast<uint16_t *>(p.out);
-                    // Two 32-column chunks at a time: 64 bf16 = 128 bytes per row and pass.
-#pragma unroll 1
-                    for (int c = chalf * 4; c < chalf * 4 + 4; c += 2) {
-                        if (n0 + c * 32 >= p.N) break;
-                        uint32_t pk[32];
+                    // 16-bit results.  After the exchange lane l of this warp stores 16 bytes (8 channels) of rows
+                    // quarter * 8 + 2 i + l / 16 of the chunk: a store instruction covers 256 contiguous bytes of two rows.
+                    long long orow[4];
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            uint32_t v[32];
-                            tmem_ld32(taddr + (c + half) * 32, v);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int j4 = 0; j4 < 8; ++j4) {
-                                const float4 s4 = *reinterpret_cast<const float4 *>(tsc + (c + half) * 32 + j4 * 4);
-                                const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
-                                float o[4];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    // (acc * w_scale) * x_scale, optional bf16 bias, optional relu, then bf16 RNE
-                                    const int cc = (c + half) * 32 + j4 * 4 + j;
-                                    int acc = (int)v[j4 * 4 + j];
-                                    if (PLAIN) {
-                                        o[j] = __fmul_rn(__fmul_rn(__int2float_rn(acc), sv[j]), xs);
-                                    } else {
-                                        const bool in_n = n0 + cc < p.N;
-                                        if (p.bias_dtype == kI32 && in_n) acc += __ldg(reinterpret_cast<const int *>(p.bias) + sbase + n0 + cc);
-                                        float tv = __fmul_rn(__int2float_rn(acc), sv[j]);
-                                        if (p.x_scale) tv = __fmul_rn(tv, xs);
-                                        if (p.bias_dtype == kBF16 && in_n)
-                                            tv = __fadd_rn(tv, __uint_as_float((uint32_t)__ldg(reinterpret_cast<const uint16_t *>(p.bias) + sbase + n0 + cc) << 16));
-                                        tv = apply_activation(p.act_type, tv);
-                                        o[j] = tv;
-                                    }
-                                }
-                                if (!PLAIN && p.out_f16) {
-                                    pk[half * 16 + j4 * 2] = pack_f16x2(o[0], o[1]);
-                                    pk[half * 16 + j4 * 2 + 1] = pack_f16x2(o[2], o[3]);
-                                } else {
-                                    pk[half * 16 + j4 * 2] = pack_bf16x2(o[0], o[1]);
-                                    pk[half * 16 + j4 * 2 + 1] = pack_bf16x2(o[2], o[3]);
-                                }
-                            }
-                        }
-                        // Transpose through shared memory, 16 rows per round, so that eight lanes write 128 contiguous
-                        // bytes of one row (a full line for local memory, a full-size packet for a peer GPU).
-                        const int pc = lane & 7;
-                        const int col = n0 + c * 32 + pc * 8;
-#pragma unroll
-                        for (int round = 0; round < 2; ++round) {
-                            if ((lane >> 4) == round) {
-#pragma unroll
-                                for (int q8 = 0; q8 < 8; ++q8)
-                                    *reinterpret_cast<uint4 *>(my_stage + (lane & 15) * 128 + (((q8 ^ lane) & 7) << 4)) =
-                                        make_uint4(pk[q8 * 4], pk[q8 * 4 + 1], pk[q8 * 4 + 2], pk[q8 * 4 + 3]);
-                            }
-                            __syncwarp();
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int r16 = i * 4 + (lane >> 3);
-                                const int rr = round * 16 + r16;
-                                const uint4 val = *reinterpret_cast<const uint4 *>(my_stage + r16 * 128 + (((pc ^ r16) & 7) << 4));
-                                long long orow = my_row0 + quarter * 32 + rr;
-                                uint16_t *obase = out;
-                                bool in_rows = quarter * 32 + rr < my_rows;
-                                if (SCATTER) {
-                                    orow = __shfl_sync(0xffffffffu, out_row, rr);
-                                    long long gpu_field = 0;
-                                    if (p.num_peers > 0) {  // high bits: which GPU's buffer, low 40 bits: row in it
-                                        gpu_field = orow >> 40;
-                                        orow &= (1ll << 40) - 1;
-                                    }
-                                    // an index that names no peer or no row of the result is skipped and reported, not stored
-                                    if (in_rows && (orow < 0 || gpu_field >= (p.num_peers > 0 ? p.num_peers : 1) || (p.out_rows > 0 && orow >= p.out_rows))) {
-                                        if (pc == 0 && c == chalf * 4 && atomicCAS(p.status, kStatusOk, kStatusBadIndex) == kStatusOk) {
-                                            p.status[1] = (int)blockIdx.x;
-                                            p.status[2] = 800;
-                                            p.status[3] = my_row0 + quarter * 32 + rr;
-                                        }
-                                        in_rows = false;
-                                    } else if (p.num_peers > 0) {
-                                        obase = reinterpret_cast<uint16_t *>(p.out_peers[(int)gpu_field]);
-                                    }
-                                }
-                                if (in_rows && col < p.N) *reinterpret_cast<uint4 *>(obase + (size_t)orow * p.N + col) = val;
-                            }
-                            __syncwarp();
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        const int tk = tc + quarter * 8 + i * 2 + (lane >> 4);
+                        orow[i] = tk < tl.rows ? (long long)(tl.row0 + tk) : -1;
+                        if (SCATTER && p.out_row_index && tk < tl.rows) orow[i] = __ldg(p.out_row_index + tl.row0 + tk);
                     }
+                    uint32_t v0[16], v1[16];
+                    tmem_ld16x256b_x4(taddr + tc, v0);
+                    tmem_ld16x256b_x4(taddr + (16u << 16) + tc, v1);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {  // 8 tokens; this lane holds two of them for four channels
+                        const float2 ts = *reinterpret_cast<const float2 *>(tok + tc + i * 8 + (lane & 3) * 2);
+                        uint32_t pk[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            float o[2];
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                const int acc = (int)(j < 2 ? v0[i * 4 + j * 2 + k] : v1[i * 4 + (j - 2) * 2 + k]);
+                                const float s = k ? ts.y : ts.x;
+                                // (acc * w_scale) * x_scale, optional bias, optional activation, then one rounding
+                                if (PLAIN) {
+                                    o[k] = __fmul_rn(__fmul_rn(__int2float_rn(acc), wsc[j]), s);
+                                } else {
+                                    float tv = __fmul_rn(__int2float_rn(acc + bias_i[j]), wsc[j]);
+                                    if (p.x_scale) tv = __fmul_rn(tv, s);
+                                    if (p.bias_dtype == kBF16) tv = __fadd_rn(tv, bias_f[j]);
+                                    o[k] = apply_activation(p.act_type, tv);
+                                }
+                            }
+                            pk[j] = !PLAIN && p.out_f16 ? pack_f16x2(o[0], o[1]) : pack_bf16x2(o[0], o[1]);
+                        }
+                        stmatrix_x4_trans(smem_u32(half_stage + (i * 8 + (lane & 7)) * ROW16_PITCH + quarter * 64 + (lane >> 3) * 16),
+                                          pk[0], pk[1], pk[2], pk[3]);
+                    }
+                    if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 720)) { ok = false; break; }
+                    uint16_t *out = reinterpret_cast<uint16_t *>(p.out);
+                    const int pc = lane & 15;
+                    const int col = c0 + pc * 8;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int r = quarter * 8 + i * 2 + (lane >> 4);
+                        const uint4 val = *reinterpret_cast<const uint4 *>(half_stage + r * ROW16_PITCH + pc * 16);
+                        bool in_rows = tc + r < tl.rows;
+                        long long row = orow[i];
+                        uint16_t *obase = out;
+                        if (SCATTER) {
+                            long long gpu_field = 0;
+                            if (p.num_peers > 0) {  // high bits: which GPU's buffer, low 40 bits: row in it
+                                gpu_field = row >> 40;
+                                row &= (1ll << 40) - 1;
+                            }
+                            // an index that names no peer or no row of the result is skipped and reported, not stored
+                            if (in_rows && (row < 0 || gpu_field < 0 || gpu_field >= (p.num_peers > 0 ? p.num_peers : 1) || (p.out_rows > 0 && row >= p.out_rows))) {
+                                if (pc == 0 && atomicCAS(p.status, kStatusOk, kStatusBadIndex) == kStatusOk) {
+                                    p.status[1] = (int)blockIdx.x;
+                                    p.status[2] = 800;
+                                    p.status[3] = tl.row0 + tc + r;
+                                }
+                                in_rows = false;
+                            } else if (p.num_peers > 0 && in_rows) {
+                                obase = reinterpret_cast<uint16_t *>(p.out_peers[(int)gpu_field]);
+                            }
+                        }
+                        if (in_rows && col < p.N) *reinterpret_cast<uint4 *>(obase + (size_t)row * p.N + col) = val;
+                    }
+                    // the other warps may write the next chunk's values
+                    if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 730)) { ok = false; break; }
                 }
             }
+            if (!ok) break;
             if (te == 0) TRACE(2, it, 2);
             tc_fence_before();
             __syncwarp();
@@ -1237,29 +1370,33 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             buf ^= 1;
             if (buf == 0) acc_phase ^= 1u;
 
-            if (MODE == kModeSwigluQuant) {
-                // Tell the publishing lane that this thread's part of the tile is stored (the fence orders the stores and
-                // the row maximum before the count), then take the work list it writes for this tile.  That list comes
-                // within a few round trips to L2 (the lane waits for no other CTA) and names the row blocks that are
-                // complete by now - normally the block of this unit's previous tile, whose rows are then read while
-                // they are still in L2; one tile later they would have been evicted.
-                __threadfence();
+            if (SWIGLU) {
+                // Tell the publishing lane that this warp's part of the tile is stored.  A CTA-wide release is enough here: the
+                // lane's own fence is cumulative over what it has observed, so only one thread waits for the stores to reach
+                // L2 (with a device-wide fence in every epilogue thread the warps stood still for 5000 cycles per tile).
+                if (lane == 0) {
+                    __threadfence_block();
+                    atomicAdd(&sh->stored_count, 1u);
+                }
                 if (te == 0) TRACE(2, it, 3);
-                atomicAdd(&sh->stored_count, 1u);
-                if (!consume_work(p, sh, lists_done, warp - 2, lane, true)) break;
-                if (te == 0) { TRACE(2, it, 4); TRACE_ADD(2, it, 5, lists_done); }
             }
-        }
-        if (MODE == kModeSwigluQuant && !*(volatile int *)&sh->abort_flag) {
-            // one list per tile of this unit plus the closing one: wait (bounded) for those not seen yet
-            lists_total = it + 1;
-            while (lists_done < lists_total)
-                if (!consume_work(p, sh, lists_done, warp - 2, lane, true)) break;
         }
         if (SCATTER && p.num_peers > 0) __threadfence_system();  // rows stored into other GPUs' memory
     }
 
-    else if (MODE == kModeSwigluQuant) {
+    else if (SWIGLU && warp > 2 + EPI_WARPS) {
+        // ------------------------------ requantising warps (swiglu_quant) ------------------------------
+        // One list per tile of this unit plus the closing one.  A list names the row blocks that are complete by then -
+        // normally the block of this unit's previous tile, whose rows are read while they are still in L2.  These warps
+        // spend their time waiting for L2; beside the epilogue that costs nothing, inside it every tile of a C2-sized
+        // launch lost 13 of 36 thousand cycles to it, more than its MMAs take.
+        int lists = 1;
+        for (int t = unit; t < total_tiles; t += n_units) ++lists;
+        for (int i = 0; i < lists; ++i)
+            if (!consume_work(p, sh, i, warp - 3 - EPI_WARPS, lane)) break;
+    }
+
+    else if (SWIGLU) {
         // ------------------------------ publishing lane (swiglu_quant) ------------------------------
         // Per tile of this unit, in the epilogue's order: wait until every epilogue thread has stored the tile, arrive at its
         // row block, collect the row slices that fall to this CTA now (publish_and_collect) into the next work list.  After
@@ -1269,9 +1406,10 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             const int shares = p.n_tiles * CTAS;
             int it = 0;
             bool ok = true;
+            int g_prev = 0;
             for (int t = unit; t < total_tiles && ok; t += n_units, ++it) {
                 const int ws = it % WK_DEPTH;
-                const unsigned need = (unsigned)(it + 1) * EPI_THREADS;
+                const unsigned need = (unsigned)(it + 1) * EPI_WARPS;
                 if (*(volatile unsigned *)&sh->stored_count < need) {
                     const long long t0 = clock64();
                     while (*(volatile unsigned *)&sh->stored_count < need) {
@@ -1292,10 +1430,11 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 }
                 TRACE(3, it, 0);
                 if (!mbar_wait(&sh->wk_empty[ws], (((uint32_t)(it / WK_DEPTH)) & 1u) ^ 1u, sh, p.status, 630 + ws)) { ok = false; break; }
-                const Tile tl = decode_tile(sh, t, p.n_tiles, L, C::kTileM);
+                const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                g_prev = tl.g;
                 TRACE(3, it, 1);
                 __threadfence();
-                publish_and_collect(p, sh, ws, p.rb_base + t / p.n_tiles, tl.row0, tl.rows, shares);
+                publish_and_collect(p, sh, ws, t / p.n_tiles, tl.row0, tl.rows, shares);
                 __threadfence();
                 TRACE(3, it, 2);
                 TRACE_ADD(3, it, 3, sh->n_work[ws]);
@@ -1365,9 +1504,11 @@ cudaError_t launch_variant(const Plan &plan, const KParams &kp, cudaStream_t str
     attr[0].val.clusterDim.x = CTAS;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    XMaps maps_x;
+    for (int i = 0; i < X_MAPS; ++i) maps_x.box[i] = plan.map_x[i];
     cfg.attrs = attr;
     cfg.numAttrs = CTAS == 2 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, plan.map_x, plan.map_w, kp);
+    return cudaLaunchKernelEx(&cfg, kern, maps_x, plan.map_w, kp);
 }
 
 template <int MODE, int BL, int EPI>
@@ -1416,55 +1557,58 @@ cudaError_t sm100_encode_maps(const Problem &p, Plan &plan)
 {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
-    {
+    // x: boxes of 32, 64 and 128 rows, of which the producer takes the one that covers a tile's share
+    for (int i = 0; i < X_MAPS; ++i) {
         cuuint64_t dims[2] = {(cuuint64_t)p.K, (cuuint64_t)p.M};
         cuuint64_t strides[1] = {(cuuint64_t)p.K};
-        cuuint32_t box[2] = {BK, BM};
+        cuuint32_t box[2] = {BK, 32u << i};
         cuuint32_t estr[2] = {1, 1};
-        CUresult r = enc(&plan.map_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t *>(p.x), dims, strides, box, estr,
+        CUresult r = enc(&plan.map_x[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t *>(p.x), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     }
+    // weights: a box is 128 channels x 128 K; with swiglu_quant 64 (pair) or 128 channels of either half of the
+    // columns, the halves being a dimension of their own
+    const cuuint32_t halves = p.mode == kModeSwigluQuant ? 2 : 1, box_ch = halves == 2 && plan.ctas == 2 ? BC / 2 : BC;
+    const cuuint64_t K = (cuuint64_t)p.K, N = (cuuint64_t)p.N, cols = N / halves, E = (cuuint64_t)p.E;
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUresult r;
     if (p.w_layout == kBFractalNz) {
-        // FRACTAL_NZ [E, N/32, K/16, 16, 32]: element (k, n) at ((n/32 * K/16 + k/16) * 16 + k%16) * 32 + n%32
-        cuuint64_t dims[5] = {32, 16, (cuuint64_t)(p.K / 16), (cuuint64_t)(p.N / 32), (cuuint64_t)p.E};
-        cuuint64_t strides[4] = {32, 512, (cuuint64_t)p.K * 32, (cuuint64_t)p.K * (cuuint64_t)p.N};
-        cuuint32_t box[5] = {32, 16, BK / 16, 4, 1};
-        cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-        CUresult r = enc(&plan.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<int8_t *>(p.w), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    } else {
-        const bool tr = p.w_layout == kBTransposed;
-        const cuuint64_t inner = tr ? p.K : p.N, mid = tr ? p.N : p.K;
-        cuuint64_t dims[3] = {inner, mid, (cuuint64_t)p.E};
-        cuuint64_t strides[2] = {inner, inner * mid};
-        cuuint32_t box[3] = {128, 128, 1};
-        cuuint32_t estr[3] = {1, 1, 1};
-        CUresult r = enc(&plan.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t *>(p.w), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+        // FRACTAL_NZ [E, N/32, K/16, 16, 32]: element (k, n) at (n/32 * K + k) * 32 + n%32
+        cuuint64_t dims[5] = {32, K, cols / 32, halves, E};
+        cuuint64_t strides[4] = {32, K * 32, K * cols, K * N};
+        cuuint32_t box[5] = {32, BK, box_ch / 32, halves, 1};
+        r = enc(&plan.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<int8_t *>(p.w), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    } else if (p.w_layout == kBTransposed) {  // [E, N, K]
+        cuuint64_t dims[4] = {K, cols, halves, E};
+        cuuint64_t strides[3] = {K, K * cols, K * N};
+        cuuint32_t box[4] = {BK, box_ch, halves, 1};
+        r = enc(&plan.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<int8_t *>(p.w), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    } else {  // [E, K, N]
+        cuuint64_t dims[4] = {cols, K, halves, E};
+        cuuint64_t strides[3] = {N, cols, K * N};
+        cuuint32_t box[4] = {box_ch, BK, halves, 1};
+        r = enc(&plan.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<int8_t *>(p.w), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, box_ch == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
-    plan.maps_ready = true;
+    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     return cudaSuccess;
 }
 
 cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStream_t stream)
 {
-    if (!plan.maps_ready) {
-        cudaError_t e = sm100_encode_maps(p, plan);
-        if (e != cudaSuccess) return e;
-    }
     plan.num_sms = device_sm_count();
     if (plan.num_sms <= 0) return cudaErrorNoDevice;
     if (p.opt.max_ctas > 0 && p.opt.max_ctas < plan.num_sms) plan.num_sms = p.opt.max_ctas;
-    if (plan.num_sms < 2) {  // a CTA pair needs two CTAs
-        plan.ctas = 1;
-        plan.hybrid = false;
-    }
+    if (plan.ctas != 2 || plan.num_sms < 2) plan.ctas = 1;  // a CTA pair needs two CTAs
+    cudaError_t e = sm100_encode_maps(p, plan);
+    if (e != cudaSuccess) return e;
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     KParams kp;
     kp.group_list = p.group_list;
@@ -1474,8 +1618,8 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     kp.K = (int)p.K;
     kp.N = (int)p.N;
     kp.half_n = (int)(p.N / 2);
-    if (plan.ctas != 2) plan.ctas = 1;
-    kp.n_tiles = p.mode == kModeSwigluQuant ? (int)((p.N / 2 + BN / 2 - 1) / (BN / 2)) : (int)((p.N + BN - 1) / BN);
+    const int64_t tile_cols = p.mode == kModeSwigluQuant ? BC : BC * plan.ctas, cols = p.mode == kModeSwigluQuant ? p.N / 2 : p.N;
+    kp.n_tiles = (int)((cols + tile_cols - 1) / tile_cols);
     kp.num_k_blocks = (int)((p.K + BK - 1) / BK);
     kp.w_scale = p.w_scale;
     kp.w_scale_dtype = p.w_scale_dtype;
@@ -1492,7 +1636,6 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     kp.q_scale_out = reinterpret_cast<float *>(p.out1);
     kp.out = p.mode == kModeSwigluQuant ? static_cast<void *>(ws + plan.off_stage) : p.out0;
 
-    cudaError_t e;
     const bool lean = !p.bias && p.act_type == 0 && !p.out_f16 && (p.mode != kModeDequantBf16 || p.x_scale);
     const int epi = p.combine ? kEpiCombine : !lean ? kEpiGeneric : (p.out_row_index ? kEpiScatter : kEpiPlain);
     kp.logit = p.logit;
@@ -1505,7 +1648,8 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     for (int i = 0; i < 8; ++i) kp.out_peers[i] = i < kp.num_peers ? p.out_peers[i] : nullptr;
     if (kp.num_peers > 0 && epi != kEpiScatter) return cudaErrorInvalidValue;
     // Pacing (see the producer): needs one zeroed word per wave; the plan reserves them only where it pays.
-    kp.wave_cnt = plan.off_wave ? reinterpret_cast<int *>(ws + plan.off_wave) : nullptr;
+    // One counter per wave is reserved for pairs; a single one-CTA unit has more waves and nobody to keep pace with.
+    kp.wave_cnt = plan.off_wave && plan.num_sms >= 2 ? reinterpret_cast<int *>(ws + plan.off_wave) : nullptr;
     kp.pace_cycles = kp.num_k_blocks * 1200 + 20000;   // about one tile's duration
 #ifdef GMM_TRACE
     kp.trace = getenv("GMM_TRACE_PTR") ? reinterpret_cast<long long *>(strtoull(getenv("GMM_TRACE_PTR"), nullptr, 0)) : nullptr;
@@ -1517,22 +1661,9 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     kp.wait_limit = p.opt.wait_limit_cycles > 0 ? p.opt.wait_limit_cycles : WAIT_LIMIT_CYCLES;
     kp.skip_k_blocks = p.opt.test_skip_k_blocks > 0 ? (p.opt.test_skip_k_blocks < kp.num_k_blocks ? p.opt.test_skip_k_blocks : kp.num_k_blocks) : 0;
     if (p.opt.ev_start) cudaEventRecord(p.opt.ev_start, stream);
-    // Pair tiles for the bulk of every group, then (plan.hybrid) 128-row tiles for the trailing blocks a pair would half waste.
-    const int launches = plan.ctas == 2 && plan.hybrid ? 2 : 1;
-    Plan one = plan;
-    for (int i = 0; i < launches; ++i) {
-        kp.part = launches == 2 ? i + 1 : 0;
-        kp.rb_base = i == 0 ? 0 : (int)((p.M + 2 * BM - 1) / (2 * BM)) + p.gl_len + 1;
-        const Plan &pl = i == 0 ? plan : one;
-        if (i == 1) {
-            one.ctas = 1;
-            kp.wave_cnt = nullptr;  // the pacing counters belong to the first launch
-        }
-        if (p.mode == kModeSwigluQuant) e = launch_layout<kModeSwigluQuant>(p.w_layout, epi, pl, kp, stream);
-        else if (p.mode == kModeInt32) e = launch_layout<kModeInt32>(p.w_layout, epi, pl, kp, stream);
-        else e = launch_layout<kModeDequantBf16>(p.w_layout, epi, pl, kp, stream);
-        if (e != cudaSuccess) break;
-    }
+    if (p.mode == kModeSwigluQuant) e = launch_layout<kModeSwigluQuant>(p.w_layout, epi, plan, kp, stream);
+    else if (p.mode == kModeInt32) e = launch_layout<kModeInt32>(p.w_layout, epi, plan, kp, stream);
+    else e = launch_layout<kModeDequantBf16>(p.w_layout, epi, plan, kp, stream);
     if (p.opt.ev_stop) cudaEventRecord(p.opt.ev_stop, stream);
     return e;
 }

@@ -423,6 +423,61 @@ def test_swiglu_fractal_nz_n_multiple_of_32_only(oracle):
 
 
 # ----------------------------------------------------------------------------------------------------------
+# edges of the token tiles: the MMA's N side takes any multiple of 32 tokens up to 256 (128 where one CTA keeps both halves
+# of swiglu), longer groups are cut into tiles of nearly equal size
+# ----------------------------------------------------------------------------------------------------------
+
+TILE_EDGE_COUNTS = [1, 31, 32, 33, 0, 63, 65, 96, 127, 128, 129, 160, 255, 256, 257, 385, 513]
+
+
+@pytest.mark.parametrize("ctas", ["1", "2"])
+@pytest.mark.parametrize("kind", ["bf16", "bf16_scatter", "f16_bias_act", "int32", "swiglu", "swiglu_nz", "combine"])
+def test_token_tile_edges(oracle, monkeypatch, ctas, kind):
+    """Every result row on either side of a tile edge, columns that end inside a channel tile, K that ends inside a K block."""
+    monkeypatch.setenv("GMM_B200_CTAS", ctas)
+    counts = np.array(TILE_EDGE_COUNTS, np.int64)
+    E, M, K = len(counts), int(counts.sum()) + 5, 272
+    gl = np.cumsum(counts)
+    if kind.startswith("swiglu"):
+        N = 448     # 224 outputs per row
+        x, w, ws, xs = make_inputs(M, K, N, E, seed=61)
+        check_swiglu(oracle, x, w, ws, xs, gl, w_nz=kind == "swiglu_nz")
+        return
+    N = 288
+    if kind == "combine":
+        check_finalize(oracle, M - 5, K, N, E, counts, 1, 62, shared_rows=M - 5, use_bias=True)
+        return
+    x, w, ws, xs = make_inputs(M, K, N, E, seed=63)
+    if kind == "bf16":
+        check_gmm(oracle, x, w, ws, xs, gl)
+    elif kind == "int32":
+        check_gmm(oracle, x, w, ws, xs, gl, out_dtype="int32")
+    elif kind == "f16_bias_act":
+        bias = np.random.default_rng(5).integers(-3000, 3000, size=(E, N)).astype(np.int32)
+        check_gmm(oracle, x, w, np.ascontiguousarray(ws * 1e-2), xs, gl, bias=bias, act_type=1, out_dtype="f16")
+    else:
+        import ops_transformer_b200 as ops
+        dev = _dev()
+        perm = np.random.default_rng(6).permutation(M).astype(np.int64)
+        t = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
+        out = torch.full((M, N), 0x7fc1, dtype=torch.int16, device=dev).view(torch.bfloat16)
+        _, wsb = ops.grouped_matmul_v4(t(x), t(w), t(ws), t(xs), t(gl), out=out, out_row_index=t(perm), return_workspace=True)
+        ops.check_status(wsb)
+        ref = oracle.gmm_w8a8(x, w, ws, xs, gl, 0)["y"]
+        got, rows = _bf16_bits(out), int(gl[-1])
+        assert np.array_equal(got[perm[:rows]], ref[:rows]) and (got[perm[rows:]] == 0x7fc1).all()
+
+
+def test_swiglu_activations_beyond_the_range_of_exp(oracle):
+    """Activations from -1e4 to 1e4: exp overflows on one side and vanishes on the other; the product stays finite."""
+    counts = np.array([70, 200], np.int64)
+    M, K, N, E = int(counts.sum()), 256, 256, 2
+    x, w, ws, xs = make_inputs(M, K, N, E, seed=64)
+    xs = np.ascontiguousarray(xs * np.logspace(-3, 1, M, dtype=np.float32))
+    check_swiglu(oracle, x, w, ws, xs, np.cumsum(counts))
+
+
+# ----------------------------------------------------------------------------------------------------------
 # grouped_matmul_finalize_routing (down GEMM + weighted combine)
 # ----------------------------------------------------------------------------------------------------------
 
