@@ -50,6 +50,42 @@ typedef struct gmmB200LaunchOptions {
 } gmmB200LaunchOptions;
 ACL_FUNC_VISIBILITY aclnnStatus gmmB200SetExecutorOptions(aclOpExecutor *executor, const gmmB200LaunchOptions *options);
 
+/* Both phases of one operator in one call, from a packed description, for bindings in which every C call and every handle
+ * costs more than the work behind it (a Python call through separate handles spends 45 us, most of it in some twenty ctypes
+ * calls).  Validation, status codes and messages are those of the operator's own GetWorkspaceSize and second-phase calls,
+ * which this one makes.
+ *
+ * words[0 .. count): the operator's tensors in the order listed below, then its attributes.
+ *   tensor     rank (-1: absent), device address, aclDataType, aclFormat, dims[rank], strides[rank] in elements,
+ *              storage rank, storage dims
+ *   int array  length (-1: absent), values;   float   its bits
+ * Operators:
+ *   GMM_V4 / V5 / WEIGHT_NZ: x, weight, bias, scale, perTokenScale, groupList, y; splitItem, groupType, groupListType, actType,
+ *              quantGroupSize, tuningConfig array
+ *   SWIGLU_QUANT / _WEIGHT_NZ: x, weight, bias, offset, weightScale, xScale, groupList, output, outputScale
+ *   FINALIZE_ROUTING / _V2: x1, x2, scale, bias, pertokenScale, groupList, sharedInput, logit, rowIndex, out;
+ *              sharedInputWeight, sharedInputOffset, groupListType, tuningConfig array
+ *   MOE_INIT_ROUTING_V3: x, expertIdx, scale, offset, expandedX, expandedRowIdx, expertTokensCountOrCumsum, expandedScale;
+ *              activeNum, expertCapacity, expertNum, dropPadMode, expertTokensNumType, expertTokensNumFlag, quantMode,
+ *              rowIdxType, activeExpertRange array
+ * If the workspace is too small the first phase's executor comes back (stage PLANNED): the caller allocates
+ * result->workspaceSize bytes and makes the operator's second-phase call, or destroys the executor.  Otherwise stage says
+ * how far the call came when its status is not ACLNN_SUCCESS. */
+enum {
+    GMM_B200_OP_GMM_V4 = 0, GMM_B200_OP_GMM_V5 = 1, GMM_B200_OP_GMM_WEIGHT_NZ = 2, GMM_B200_OP_SWIGLU_QUANT = 3,
+    GMM_B200_OP_SWIGLU_QUANT_WEIGHT_NZ = 4, GMM_B200_OP_FINALIZE_ROUTING = 5, GMM_B200_OP_FINALIZE_ROUTING_V2 = 6,
+    GMM_B200_OP_MOE_INIT_ROUTING_V3 = 7
+};
+enum { GMM_B200_STAGE_PLAN = 0, GMM_B200_STAGE_OPTIONS = 1, GMM_B200_STAGE_PLANNED = 2, GMM_B200_STAGE_RUN = 3 };
+typedef struct gmmB200CallResult {
+    uint64_t workspaceSize;
+    aclOpExecutor *executor;
+    int32_t stage;
+    int32_t reserved;
+} gmmB200CallResult;
+ACL_FUNC_VISIBILITY aclnnStatus gmmB200Call(int32_t op, const int64_t *words, uint64_t count, void *workspace, uint64_t workspaceBytes,
+                                            const gmmB200LaunchOptions *options, aclrtStream stream, gmmB200CallResult *result);
+
 /* Flat form of aclnnGroupedMatmulV4 for the W8A8 path (same arithmetic, same validation of sizes).
  * scaleDtype / biasDtype / yDtype use aclDataType codes; bias may be null (biasDtype ignored);
  * weightTransposed is the weight's layout: 0 = [E, K, N], 1 = [E, N, K], 2 = FRACTAL_NZ [E, N/32, K/16, 16, 32]

@@ -33,7 +33,7 @@ EXPORTED_SYMBOLS = [
     "aclnnMoeInitRoutingV3GetWorkspaceSize", "aclnnMoeInitRoutingV3",
     "aclnnGroupedMatmulSwigluQuantGetWorkspaceSize", "aclnnGroupedMatmulSwigluQuant",
     "aclnnGroupedMatmulSwigluQuantWeightNZGetWorkspaceSize", "aclnnGroupedMatmulSwigluQuantWeightNZ",
-    "gmmB200Version", "gmmB200CheckStatus", "gmmB200SetExecutorOptions", "gmmB200GroupedMatmulW8A8WorkspaceSize", "gmmB200GroupedMatmulW8A8",
+    "gmmB200Version", "gmmB200CheckStatus", "gmmB200SetExecutorOptions", "gmmB200Call", "gmmB200GroupedMatmulW8A8WorkspaceSize", "gmmB200GroupedMatmulW8A8",
     "gmmB200GroupedMatmulSwigluQuantWorkspaceSize", "gmmB200GroupedMatmulSwigluQuant",
     "gmmB200NoAllocScratchBytes", "gmmB200GroupedMatmulSwigluQuantNoAlloc", "gmmB200NoAllocCheckStatus",
     "gmmB200PeerAlloc", "gmmB200PeerFree", "gmmB200PeerExport", "gmmB200PeerImport", "gmmB200PeerRelease", "gmmB200EpDispatch", "gmmB200EpCount", "gmmB200EpRoute", "gmmB200EpInverseMap", "gmmB200EpCombine",
@@ -47,6 +47,15 @@ class LaunchOptions(C.Structure):
 
     def __init__(self, max_ctas: int = 0, start_event=None, stop_event=None, wait_limit_cycles: int = 0, test_skip_k_blocks: int = 0):
         super().__init__(C.sizeof(LaunchOptions), max_ctas, start_event, stop_event, wait_limit_cycles, test_skip_k_blocks, 0)
+
+
+class CallResult(C.Structure):
+    """gmmB200CallResult (include/gmm_b200.h)."""
+    _fields_ = [("workspaceSize", C.c_uint64), ("executor", C.c_void_p), ("stage", C.c_int32), ("reserved", C.c_int32)]
+
+
+OP_GMM, OP_SWIGLU_QUANT, OP_FINALIZE_ROUTING, OP_MOE_INIT_ROUTING = {"V4": 0, "V5": 1, "WeightNz": 2}, {"": 3, "WeightNZ": 4}, {"": 5, "V2": 6}, 7
+STAGE_PLAN, STAGE_OPTIONS, STAGE_PLANNED, STAGE_RUN = range(4)
 
 
 class LibraryMissing(RuntimeError):
@@ -93,6 +102,7 @@ def _load():
     L.aclnnGroupedMatmulSwigluQuant.argtypes = [p, u64, p, p]
     L.gmmB200CheckStatus.argtypes = [p, u64, p, C.POINTER(i32)]
     L.gmmB200SetExecutorOptions.argtypes = [p, po]
+    L.gmmB200Call.argtypes = [i32, p, u64, p, u64, po, p, C.POINTER(CallResult)]
     L.gmmB200GroupedMatmulW8A8WorkspaceSize.argtypes = [i64, i64, i64, i64, i32, C.POINTER(u64)]
     L.gmmB200GroupedMatmulW8A8.argtypes = [p, p, p, i32, p, p, i32, p, i64, i32, i64, i64, i64, i64, i32, i32, p, p, i32, i64, p, i32, p, u64, p, po]
     L.gmmB200GroupedMatmulSwigluQuantWorkspaceSize.argtypes = [i64, i64, i64, i64, C.POINTER(u64)]

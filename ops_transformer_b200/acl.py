@@ -8,7 +8,9 @@ codes raised as ``AclnnError``.  torch is used for device memory and streams onl
 """
 from __future__ import annotations
 
+import array
 import ctypes as C
+import struct
 from typing import Optional, Sequence
 
 import torch
@@ -94,6 +96,11 @@ class _Workspace:
         return b
 
 
+    def peek(self, device: torch.device) -> Optional[torch.Tensor]:
+        """The buffer as it is, whatever its size; None before the first use."""
+        return self._buf.get((device.type, device.index))
+
+
 _WS = _Workspace()
 
 
@@ -115,14 +122,62 @@ def check_status(workspace: Optional[torch.Tensor], stream=None) -> None:
         raise err
 
 
-def _apply_options(executor, options: Optional[LaunchOptions], where: str) -> None:
-    """Attach per-call options to a live executor (between the two phases)."""
-    if options is None:
+def _put(words: list, t: Optional[torch.Tensor], fmt: int = ACL_FORMAT_ND, view_dims: Optional[Sequence[int]] = None) -> None:
+    """Append one tensor to a packed description (gmmB200Call, include/gmm_b200.h); the same view as ``create_tensor``."""
+    if t is None:
+        words.append(-1)
         return
-    rc = _lib.lib().gmmB200SetExecutorOptions(executor, C.byref(options))
+    shape = t.shape
+    rank = len(shape)
+    if rank > 8:
+        raise MemoryError("a tensor of more than 8 dimensions cannot be described")
+    if view_dims is None:
+        words += (rank, t.data_ptr(), _DTYPES[t.dtype], fmt)
+        words += shape
+        words += t.stride()
+    else:
+        strides = [1] * len(view_dims)
+        for i in range(len(view_dims) - 2, -1, -1):
+            strides[i] = strides[i + 1] * view_dims[i + 1]
+        words += (len(view_dims), t.data_ptr(), _DTYPES[t.dtype], fmt)
+        words += view_dims
+        words += strides
+    words.append(rank)
+    words += shape
+
+
+def _put_ints(words: list, values: Optional[Sequence[int]]) -> None:
+    if values is None:
+        words.append(-1)
+    else:
+        words.append(len(values))
+        words += values
+
+
+def _call(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream,
+          options: Optional[LaunchOptions]) -> Optional[torch.Tensor]:
+    """Both phases of operator ``name`` on the packed description; returns the workspace that was used (None if none)."""
+    L = _lib.lib()
+    packed = array.array("q", words)
+    res = _lib.CallResult()
+    # validation needs no device: tensors that are not on one are planned only, so that what is wrong with them is reported first
+    on_gpu = device.type == "cuda"
+    buf = None if not on_gpu else workspace if workspace is not None else _WS.peek(device)
+    handle = _stream_handle(stream) if on_gpu else 0
+    rc = L.gmmB200Call(op, packed.buffer_info()[0], len(packed), buf.data_ptr() if buf is not None else None,
+                       buf.numel() if buf is not None else 0, C.byref(options) if options is not None else None, handle, C.byref(res))
+    if rc == ACLNN_SUCCESS and res.stage == _lib.STAGE_PLANNED:
+        ex = C.c_void_p(res.executor)
+        if workspace is not None and workspace.numel() < res.workspaceSize:
+            L.aclDestroyAclOpExecutor(ex)
+            raise ValueError(f"workspace of {workspace.numel()} bytes is smaller than the {res.workspaceSize} required")
+        buf = workspace if workspace is not None else _WS.get(device, res.workspaceSize)
+        rc = getattr(L, name)(buf.data_ptr(), res.workspaceSize, ex, _stream_handle(stream))
+        res.stage = _lib.STAGE_RUN
     if rc != ACLNN_SUCCESS:
-        _lib.lib().aclDestroyAclOpExecutor(executor)
-        raise AclnnError(rc, where + ": gmmB200SetExecutorOptions")
+        raise AclnnError(rc, name + ("GetWorkspaceSize" if res.stage == _lib.STAGE_PLAN else
+                                     ": gmmB200SetExecutorOptions" if res.stage == _lib.STAGE_OPTIONS else ""))
+    return workspace if workspace is not None else buf if res.workspaceSize else None
 
 
 def grouped_matmul_v4(x: torch.Tensor, weight: torch.Tensor, scale: Optional[torch.Tensor],
@@ -142,7 +197,6 @@ def grouped_matmul_v4(x: torch.Tensor, weight: torch.Tensor, scale: Optional[tor
     reference.  ``out_row_index`` (int64 [M], an extension of this library) scatters result row r to row
     out_row_index[r]; it goes through the flat entry point gmmB200GroupedMatmulW8A8.  ``options``: per-call
     ``LaunchOptions`` (CTA cap, timing events)."""
-    L = _lib.lib()
     nz = weight_format == ACL_FORMAT_FRACTAL_NZ or api == "WeightNz"
     if out is None and not out_peers:
         n_out = weight.shape[1] * 32 if (nz and weight.dim() == 5) else weight.shape[2]
@@ -150,56 +204,16 @@ def grouped_matmul_v4(x: torch.Tensor, weight: torch.Tensor, scale: Optional[tor
     if out_row_index is not None:
         return _grouped_matmul_flat(x, weight, scale, per_token_scale, group_list, bias, group_list_type, act_type, out,
                                     out_row_index, stream, workspace, return_workspace, out_peers, nz, options, out_rows)
-    lists = []
-    tuning = None
-    try:
-        hx = create_tensor_list([x]); lists.append(hx)
-        hw = create_tensor_list([weight], ACL_FORMAT_FRACTAL_NZ if nz else ACL_FORMAT_ND); lists.append(hw)
-        hb = None
-        if bias is not None:
-            hb = create_tensor_list([bias]); lists.append(hb)
-        hs = None
-        if scale is not None:
-            hs = create_tensor_list([scale]); lists.append(hs)
-        hp = None
-        if per_token_scale is not None:
-            hp = create_tensor_list([per_token_scale]); lists.append(hp)
-        hy = create_tensor_list([out]); lists.append(hy)
-        hg = create_tensor(group_list)
-        try:
-            ws_size = C.c_uint64(0)
-            ex = C.c_void_p(0)
-            if tuning_config is not None:
-                tuning = L.aclCreateIntArray(_i64(list(tuning_config)), len(tuning_config))
-            head = (hx, hw, hb, hs, None, None, None, hp, hg, None, None, None, split_item, group_type, group_list_type, act_type)
-            tail = (hy, None, None, C.byref(ws_size), C.byref(ex))
-            if api == "V4":
-                rc = L.aclnnGroupedMatmulV4GetWorkspaceSize(*head, *tail)
-            elif api == "V5":
-                rc = L.aclnnGroupedMatmulV5GetWorkspaceSize(*head, tuning, *tail)
-            elif api == "WeightNz":
-                rc = L.aclnnGroupedMatmulWeightNzGetWorkspaceSize(*head, tuning, quant_group_size, *tail)
-            else:
-                raise ValueError(f"unknown api {api!r}")
-            if rc != ACLNN_SUCCESS:
-                raise AclnnError(rc, f"aclnnGroupedMatmul{api}GetWorkspaceSize")
-            if workspace is None:
-                workspace = _WS.get(x.device, ws_size.value)
-            elif workspace.numel() < ws_size.value:
-                L.aclDestroyAclOpExecutor(ex)
-                raise ValueError(f"workspace of {workspace.numel()} bytes is smaller than the {ws_size.value} required")
-            wptr = C.c_void_p(workspace.data_ptr()) if workspace is not None else None
-            _apply_options(ex, options, "aclnnGroupedMatmul" + api)
-            rc = getattr(L, "aclnnGroupedMatmul" + api)(wptr, ws_size.value, ex, C.c_void_p(_stream_handle(stream)))
-            if rc != ACLNN_SUCCESS:
-                raise AclnnError(rc, "aclnnGroupedMatmul" + api)
-        finally:
-            L.aclDestroyTensor(hg)
-            if tuning:
-                L.aclDestroyIntArray(tuning)
-    finally:
-        for h in lists:
-            L.aclDestroyTensorList(h)
+    if api not in _lib.OP_GMM:
+        raise ValueError(f"unknown api {api!r}")
+    words = []
+    _put(words, x)
+    _put(words, weight, ACL_FORMAT_FRACTAL_NZ if nz else ACL_FORMAT_ND)
+    for t in (bias, scale, per_token_scale, group_list, out):
+        _put(words, t)
+    words += (split_item, group_type, group_list_type, act_type, quant_group_size)
+    _put_ints(words, tuning_config)
+    workspace = _call(_lib.OP_GMM[api], "aclnnGroupedMatmul" + api, words, x.device, workspace, stream, options)
     return (out, workspace) if return_workspace else out
 
 
@@ -252,44 +266,18 @@ def grouped_matmul_swiglu_quant(x: torch.Tensor, weight: torch.Tensor, weight_sc
     ``weight_format`` ACL_FORMAT_FRACTAL_NZ: ``weight`` is the 5-D storage of ``format_cast_nz``; ``api`` "WeightNZ"
     calls aclnnGroupedMatmulSwigluQuantWeightNZ (aclnn_grouped_matmul_swiglu_quant_weight_nz.h:37-54 of the reference),
     which takes the storage as FRACTAL_NZ whatever the format says."""
-    L = _lib.lib()
     M = x.shape[0]
     N = weight_scale.shape[1] if weight_scale.dim() == 2 else 0
     if output is None:
         output = torch.empty((M, N // 2), dtype=torch.int8, device=x.device)
     if output_scale is None:
         output_scale = torch.empty((M,), dtype=torch.float32, device=x.device)
-    handles = []
-    try:
-        def mk(t):
-            if t is None:
-                return None
-            h = create_tensor(t)
-            handles.append(h)
-            return h
-        hx, hb, ho = mk(x), mk(bias), mk(offset)
-        hw = create_tensor(weight, weight_format)
-        handles.append(hw)
-        hws, hxs, hg, hq, hqs = mk(weight_scale), mk(x_scale), mk(group_list), mk(output), mk(output_scale)
-        ws_size = C.c_uint64(0)
-        ex = C.c_void_p(0)
-        name = "aclnnGroupedMatmulSwigluQuant" + api
-        rc = getattr(L, name + "GetWorkspaceSize")(hx, hw, hb, ho, hws, hxs, hg, hq, hqs, None, C.byref(ws_size), C.byref(ex))
-        if rc != ACLNN_SUCCESS:
-            raise AclnnError(rc, name + "GetWorkspaceSize")
-        if workspace is None:
-            workspace = _WS.get(x.device, ws_size.value)
-        elif workspace.numel() < ws_size.value:
-            L.aclDestroyAclOpExecutor(ex)
-            raise ValueError(f"workspace of {workspace.numel()} bytes is smaller than the {ws_size.value} required")
-        wptr = C.c_void_p(workspace.data_ptr()) if workspace is not None else None
-        _apply_options(ex, options, name)
-        rc = getattr(L, name)(wptr, ws_size.value, ex, C.c_void_p(_stream_handle(stream)))
-        if rc != ACLNN_SUCCESS:
-            raise AclnnError(rc, name)
-    finally:
-        for h in handles:
-            L.aclDestroyTensor(h)
+    words = []
+    _put(words, x)
+    _put(words, weight, weight_format)
+    for t in (bias, offset, weight_scale, x_scale, group_list, output, output_scale):
+        _put(words, t)
+    workspace = _call(_lib.OP_SWIGLU_QUANT[api], "aclnnGroupedMatmulSwigluQuant" + api, words, x.device, workspace, stream, options)
     return (output, output_scale, workspace) if return_workspace else (output, output_scale)
 
 
@@ -306,54 +294,19 @@ def grouped_matmul_finalize_routing(x: torch.Tensor, weight_nz: torch.Tensor, sc
     ``shared_input`` rows (gmm/grouped_matmul_finalize_routing/op_host/op_api/aclnn_grouped_matmul_finalize_routing_weight_nz.h:48-64
     of the reference).  ``weight_nz`` is the FRACTAL_NZ storage [E, N/32, K/16, 16, 32] (``format_cast_nz``); with
     ``view_3d`` it is described to the operator as the reference's callers do, a view [E, K, N] over that storage."""
-    L = _lib.lib()
     E, n1, k1 = weight_nz.shape[0], weight_nz.shape[1], weight_nz.shape[2]
     N, K = n1 * 32, k1 * 16
     if out is None:
         out = torch.empty((batch, N), dtype=torch.float32, device=x.device)
-    handles = []
-    tuning = None
-    try:
-        def mk(t, **kw):
-            if t is None:
-                return None
-            h = create_tensor(t, **kw)
-            handles.append(h)
-            return h
-        hx = mk(x)
-        hw = mk(weight_nz, fmt=ACL_FORMAT_FRACTAL_NZ, view_dims=[E, K, N] if view_3d else None)
-        hs, hb, hp, hg = mk(scale), mk(bias), mk(pertoken_scale), mk(group_list)
-        hsh, hl, hr, hy = mk(shared_input), mk(logit), mk(row_index), mk(out)
-        ws_size = C.c_uint64(0)
-        ex = C.c_void_p(0)
-        name = "aclnnGroupedMatmulFinalizeRoutingWeightNz" + api
-        if api == "V2":
-            if tuning_config is not None:
-                tuning = L.aclCreateIntArray(_i64(list(tuning_config)), len(tuning_config))
-            rc = L.aclnnGroupedMatmulFinalizeRoutingWeightNzV2GetWorkspaceSize(
-                hx, hw, hs, hb, None, None, None, hp, hg, hsh, hl, hr, 0, shared_input_weight, shared_input_offset, False, False,
-                group_list_type, tuning, hy, C.byref(ws_size), C.byref(ex))
-        else:
-            rc = L.aclnnGroupedMatmulFinalizeRoutingWeightNzGetWorkspaceSize(
-                hx, hw, hs, hb, hp, hg, hsh, hl, hr, 0, shared_input_weight, shared_input_offset, False, False, group_list_type,
-                hy, C.byref(ws_size), C.byref(ex))
-        if rc != ACLNN_SUCCESS:
-            raise AclnnError(rc, name + "GetWorkspaceSize")
-        if workspace is None:
-            workspace = _WS.get(x.device, ws_size.value)
-        elif workspace.numel() < ws_size.value:
-            L.aclDestroyAclOpExecutor(ex)
-            raise ValueError(f"workspace of {workspace.numel()} bytes is smaller than the {ws_size.value} required")
-        wptr = C.c_void_p(workspace.data_ptr()) if workspace is not None else None
-        _apply_options(ex, options, name)
-        rc = getattr(L, name)(wptr, ws_size.value, ex, C.c_void_p(_stream_handle(stream)))
-        if rc != ACLNN_SUCCESS:
-            raise AclnnError(rc, name)
-    finally:
-        for h in handles:
-            L.aclDestroyTensor(h)
-        if tuning:
-            L.aclDestroyIntArray(tuning)
+    words = []
+    _put(words, x)
+    _put(words, weight_nz, ACL_FORMAT_FRACTAL_NZ, [E, K, N] if view_3d else None)
+    for t in (scale, bias, pertoken_scale, group_list, shared_input, logit, row_index, out):
+        _put(words, t)
+    words += (struct.unpack("<I", bytes(C.c_float(shared_input_weight)))[0], shared_input_offset, group_list_type)
+    _put_ints(words, tuning_config)
+    workspace = _call(_lib.OP_FINALIZE_ROUTING[api], "aclnnGroupedMatmulFinalizeRoutingWeightNz" + api, words, x.device, workspace, stream,
+                      options)
     return (out, workspace) if return_workspace else out
 
 
@@ -390,7 +343,6 @@ def moe_init_routing_v3(x: torch.Tensor, expert_idx: torch.Tensor, *, expert_num
     """aclnnMoeInitRoutingV3 (moe/moe_init_routing_v3/op_host/op_api/aclnn_moe_init_routing_v3.h:24-47 of the reference):
     returns (expandedX, expandedRowIdx, expertTokensCountOrCumsum, expandedScale).  With ``quant_mode`` 1 expandedX is int8
     and expandedScale the per-row scale, i.e. the x / per-token scale of the grouped GEMM operators."""
-    L = _lib.lib()
     n, h = x.shape
     k = expert_idx.shape[1]
     start, end = active_expert_range
@@ -401,31 +353,11 @@ def moe_init_routing_v3(x: torch.Tensor, expert_idx: torch.Tensor, *, expert_num
         es = torch.empty((n * k,), dtype=torch.float32, device=x.device)
     else:
         ex, ri, cnt, es = outputs
-    handles = []
-    rng = L.aclCreateIntArray(_i64(list(active_expert_range)), len(active_expert_range))
-    try:
-        def mk(t):
-            if t is None:
-                return None
-            hh = create_tensor(t)
-            handles.append(hh)
-            return hh
-        hx, hi, hs, ho, hex_, hri, hc, hes = (mk(t) for t in (x, expert_idx, scale, offset, ex, ri, cnt, es))
-        ws_size = C.c_uint64(0)
-        exr = C.c_void_p(0)
-        rc = L.aclnnMoeInitRoutingV3GetWorkspaceSize(hx, hi, hs, ho, n * k if active_num is None else active_num, expert_capacity,
-                                                     expert_num, drop_pad_mode, expert_tokens_num_type, expert_tokens_num_flag,
-                                                     quant_mode, rng, row_idx_type, hex_, hri, hc, hes, C.byref(ws_size), C.byref(exr))
-        if rc != ACLNN_SUCCESS:
-            raise AclnnError(rc, "aclnnMoeInitRoutingV3GetWorkspaceSize")
-        if workspace is None:
-            workspace = _WS.get(x.device, ws_size.value)
-        wptr = C.c_void_p(workspace.data_ptr()) if workspace is not None else None
-        rc = L.aclnnMoeInitRoutingV3(wptr, ws_size.value, exr, C.c_void_p(_stream_handle(stream)))
-        if rc != ACLNN_SUCCESS:
-            raise AclnnError(rc, "aclnnMoeInitRoutingV3")
-    finally:
-        for hh in handles:
-            L.aclDestroyTensor(hh)
-        L.aclDestroyIntArray(rng)
+    words = []
+    for t in (x, expert_idx, scale, offset, ex, ri, cnt, es):
+        _put(words, t)
+    words += (n * k if active_num is None else active_num, expert_capacity, expert_num, drop_pad_mode, expert_tokens_num_type,
+              1 if expert_tokens_num_flag else 0, quant_mode, row_idx_type)
+    _put_ints(words, active_expert_range)
+    _call(_lib.OP_MOE_INIT_ROUTING, "aclnnMoeInitRoutingV3", words, x.device, workspace, stream, None)
     return ex, ri, cnt, es

@@ -1093,4 +1093,197 @@ aclnnStatus gmmB200GroupedMatmulFinalizeRouting(const void *x, const void *weigh
     return ACLNN_SUCCESS;
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// Both phases of one operator from a packed description (include/gmm_b200.h)
+// ---------------------------------------------------------------------------------------------------------
+
+namespace {
+
+struct WordReader {
+    const int64_t *p, *end;
+    bool ok = true;
+    int64_t next()
+    {
+        if (p == end) { ok = false; return 0; }
+        return *p++;
+    }
+};
+
+// One tensor: rank (-1: absent), data, dtype, format, dims, strides, storage rank, storage dims.
+struct PackedTensor {
+    aclTensor t;
+    bool present = false;
+    const aclTensor *get() const { return present ? &t : nullptr; }
+    aclTensor *out() { return present ? &t : nullptr; }
+    void read(WordReader &r)
+    {
+        const int64_t rank = r.next();
+        if (rank < 0) return;
+        if (rank > 8) { r.ok = false; return; }
+        present = true;
+        t.data = reinterpret_cast<void *>((uintptr_t)r.next());
+        t.dtype = (aclDataType)r.next();
+        t.format = (aclFormat)r.next();
+        t.view_dims.resize((size_t)rank);
+        t.strides.resize((size_t)rank);
+        for (int64_t &d : t.view_dims) d = r.next();
+        for (int64_t &d : t.strides) d = r.next();
+        const int64_t storage = r.next();
+        if (storage < 0 || storage > 8) { r.ok = false; return; }
+        t.storage_dims.resize((size_t)storage);
+        for (int64_t &d : t.storage_dims) d = r.next();
+    }
+};
+
+struct PackedList {
+    aclTensorList list;
+    PackedTensor tensor;
+    void read(WordReader &r)
+    {
+        tensor.read(r);
+        if (tensor.present) list.items.assign(1, &tensor.t);
+    }
+    const aclTensorList *get() const { return tensor.present ? &list : nullptr; }
+};
+
+struct PackedInts {
+    aclIntArray a;
+    bool present = false;
+    void read(WordReader &r)
+    {
+        const int64_t n = r.next();
+        if (n < 0) return;
+        if (n > r.end - r.p) { r.ok = false; return; }
+        present = true;
+        a.values.assign(r.p, r.p + n);
+        r.p += n;
+    }
+    aclIntArray *get() { return present ? &a : nullptr; }
+};
+
+float float_of_bits(int64_t v)
+{
+    const uint32_t b = (uint32_t)v;
+    float f;
+    std::memcpy(&f, &b, sizeof(f));
+    return f;
+}
+
+typedef aclnnStatus (*RunFn)(void *, uint64_t, aclOpExecutor *, aclrtStream);
+
+aclnnStatus plan_packed(int32_t op, WordReader &r, uint64_t *size, aclOpExecutor **ex, RunFn *run)
+{
+    const auto malformed = [] { return fail(ACLNN_ERR_PARAM_INVALID, "gmmB200Call: malformed description."); };
+    switch (op) {
+        case GMM_B200_OP_GMM_V4: case GMM_B200_OP_GMM_V5: case GMM_B200_OP_GMM_WEIGHT_NZ: {
+            PackedList x, w, bias, scale, pts, y;
+            PackedTensor gl;
+            PackedInts tuning;
+            x.read(r); w.read(r); bias.read(r); scale.read(r); pts.read(r); gl.read(r); y.read(r);
+            const int64_t split = r.next(), group_type = r.next(), gl_type = r.next(), act = r.next(), qgroup = r.next();
+            tuning.read(r);
+            if (!r.ok) return malformed();
+            aclTensorList *py = y.tensor.present ? &y.list : nullptr;
+            if (op == GMM_B200_OP_GMM_V4) {
+                *run = aclnnGroupedMatmulV4;
+                return aclnnGroupedMatmulV4GetWorkspaceSize(x.get(), w.get(), bias.get(), scale.get(), nullptr, nullptr, nullptr, pts.get(),
+                                                            gl.get(), nullptr, nullptr, nullptr, split, group_type, gl_type, act, py, nullptr,
+                                                            nullptr, size, ex);
+            }
+            if (op == GMM_B200_OP_GMM_V5) {
+                *run = aclnnGroupedMatmulV5;
+                return aclnnGroupedMatmulV5GetWorkspaceSize(x.get(), w.get(), bias.get(), scale.get(), nullptr, nullptr, nullptr, pts.get(),
+                                                            gl.get(), nullptr, nullptr, nullptr, split, group_type, gl_type, act,
+                                                            tuning.get(), py, nullptr, nullptr, size, ex);
+            }
+            *run = aclnnGroupedMatmulWeightNz;
+            return aclnnGroupedMatmulWeightNzGetWorkspaceSize(x.get(), w.get(), bias.get(), scale.get(), nullptr, nullptr, nullptr, pts.get(),
+                                                              gl.get(), nullptr, nullptr, nullptr, split, group_type, gl_type, act,
+                                                              tuning.get(), qgroup, py, nullptr, nullptr, size, ex);
+        }
+        case GMM_B200_OP_SWIGLU_QUANT: case GMM_B200_OP_SWIGLU_QUANT_WEIGHT_NZ: {
+            PackedTensor x, w, bias, offset, ws, xs, gl, q, qs;
+            for (PackedTensor *t : {&x, &w, &bias, &offset, &ws, &xs, &gl, &q, &qs}) t->read(r);
+            if (!r.ok) return malformed();
+            if (op == GMM_B200_OP_SWIGLU_QUANT) {
+                *run = aclnnGroupedMatmulSwigluQuant;
+                return aclnnGroupedMatmulSwigluQuantGetWorkspaceSize(x.get(), w.get(), bias.get(), offset.get(), ws.get(), xs.get(), gl.get(),
+                                                                     q.out(), qs.out(), nullptr, size, ex);
+            }
+            *run = aclnnGroupedMatmulSwigluQuantWeightNZ;
+            return aclnnGroupedMatmulSwigluQuantWeightNZGetWorkspaceSize(x.get(), w.get(), bias.get(), offset.get(), ws.get(), xs.get(),
+                                                                         gl.get(), q.out(), qs.out(), nullptr, size, ex);
+        }
+        case GMM_B200_OP_FINALIZE_ROUTING: case GMM_B200_OP_FINALIZE_ROUTING_V2: {
+            PackedTensor x, w, scale, bias, pts, gl, shared, logit, row, y;
+            for (PackedTensor *t : {&x, &w, &scale, &bias, &pts, &gl, &shared, &logit, &row, &y}) t->read(r);
+            const float weight = float_of_bits(r.next());
+            const int64_t offset = r.next(), gl_type = r.next();
+            PackedInts tuning;
+            tuning.read(r);
+            if (!r.ok) return malformed();
+            if (op == GMM_B200_OP_FINALIZE_ROUTING) {
+                *run = aclnnGroupedMatmulFinalizeRoutingWeightNz;
+                return aclnnGroupedMatmulFinalizeRoutingWeightNzGetWorkspaceSize(x.get(), w.get(), scale.get(), bias.get(), pts.get(), gl.get(),
+                                                                                 shared.get(), logit.get(), row.get(), 0, weight, offset,
+                                                                                 false, false, gl_type, y.out(), size, ex);
+            }
+            *run = aclnnGroupedMatmulFinalizeRoutingWeightNzV2;
+            return aclnnGroupedMatmulFinalizeRoutingWeightNzV2GetWorkspaceSize(x.get(), w.out(), scale.get(), bias.get(), nullptr, nullptr,
+                                                                               nullptr, pts.get(), gl.get(), shared.get(), logit.get(),
+                                                                               row.get(), 0, weight, offset, false, false, gl_type,
+                                                                               tuning.get(), y.out(), size, ex);
+        }
+        case GMM_B200_OP_MOE_INIT_ROUTING_V3: {
+            PackedTensor x, idx, scale, offset, ex_out, row_idx, counts, ex_scale;
+            for (PackedTensor *t : {&x, &idx, &scale, &offset, &ex_out, &row_idx, &counts, &ex_scale}) t->read(r);
+            const int64_t active = r.next(), capacity = r.next(), experts = r.next(), drop_pad = r.next(), num_type = r.next();
+            const bool num_flag = r.next() != 0;
+            const int64_t quant = r.next(), row_type = r.next();
+            PackedInts range;
+            range.read(r);
+            if (!r.ok) return malformed();
+            *run = aclnnMoeInitRoutingV3;
+            return aclnnMoeInitRoutingV3GetWorkspaceSize(x.get(), idx.get(), scale.get(), offset.get(), active, capacity, experts, drop_pad,
+                                                         num_type, num_flag, quant, range.get(), row_type, ex_out.get(), row_idx.get(),
+                                                         counts.get(), ex_scale.get(), size, ex);
+        }
+        default: return fail(ACLNN_ERR_PARAM_INVALID, "gmmB200Call: unknown operator %d.", op);
+    }
+}
+
+}  // namespace
+
+aclnnStatus gmmB200Call(int32_t op, const int64_t *words, uint64_t count, void *workspace, uint64_t workspaceBytes,
+                        const gmmB200LaunchOptions *options, aclrtStream stream, gmmB200CallResult *result)
+{
+    clear_error();
+    GMM_REQUIRE(result != nullptr && (words != nullptr || count == 0), ACLNN_ERR_PARAM_NULLPTR, "words and result must not be nullptr.");
+    result->workspaceSize = 0;
+    result->executor = nullptr;
+    result->stage = GMM_B200_STAGE_PLAN;
+    WordReader r{words, words + count};
+    uint64_t need = 0;
+    aclOpExecutor *ex = nullptr;
+    RunFn run = nullptr;
+    aclnnStatus rc = plan_packed(op, r, &need, &ex, &run);
+    if (rc != ACLNN_SUCCESS) return rc;
+    result->workspaceSize = need;
+    if (options) {
+        result->stage = GMM_B200_STAGE_OPTIONS;
+        rc = gmmB200SetExecutorOptions(ex, options);
+        if (rc != ACLNN_SUCCESS) {
+            if (claim_executor(ex)) delete ex;
+            return rc;
+        }
+    }
+    if (need > workspaceBytes) {  // the caller finds more and runs the second phase itself
+        result->stage = GMM_B200_STAGE_PLANNED;
+        result->executor = ex;
+        return ACLNN_SUCCESS;
+    }
+    result->stage = GMM_B200_STAGE_RUN;
+    return run(need ? workspace : nullptr, need, ex, stream);
+}
+
 }  // extern "C"

@@ -513,3 +513,53 @@ def test_flat_entry_points_validate_on_the_host():
     assert L.gmmB200GroupedMatmulW8A8(one, one, one, 0, one, None, 0, one, 2, 0, 1, 16, 16, 1, 0, 0, None, None, 0, 0, one, 27, one, 256, None, None) == INVALID
     assert L.gmmB200GroupedMatmulSwigluQuant(one, one, one, 0, one, one, 1, 4, 16, 32, 1, 0, one, one, one, 16, None, None) == INVALID  # workspace too small
     assert "workspaceSize" in _lib.last_error()
+
+
+# ----------------------------------------------------------------------------------------------------------
+# gmmB200Call: both phases from a packed description
+# ----------------------------------------------------------------------------------------------------------
+
+def _packed_call(L, op, words, workspace=None, nbytes=0):
+    import array
+    packed = array.array("q", words)
+    res = _lib.CallResult()
+    rc = L.gmmB200Call(op, packed.buffer_info()[0], len(packed), workspace, nbytes, None, None, C.byref(res))
+    return rc, res
+
+
+def test_packed_call_plans_like_the_separate_handles(gmm_lib):
+    torch = pytest.importorskip("torch")
+    from ops_transformer_b200 import acl
+    L = gmm_lib
+    M, K, N, E = 96, 64, 128, 3
+    x, w = torch.zeros(M, K, dtype=torch.int8), torch.zeros(E, N, K, dtype=torch.int8).transpose(1, 2)   # a strided view
+    ws, xs, gl = torch.ones(E, N), torch.ones(M), torch.full((E,), 32, dtype=torch.int64)
+    q, qs = torch.zeros(M, N // 2, dtype=torch.int8), torch.zeros(M)
+    words = []
+    for t in (x, w, None, None, ws, xs, gl, q, qs):
+        acl._put(words, t)
+    hs = [acl.create_tensor(t) for t in (x, w, ws, xs, gl, q, qs)]
+    size, ex = C.c_uint64(0), C.c_void_p(0)
+    want = L.aclnnGroupedMatmulSwigluQuantGetWorkspaceSize(hs[0], hs[1], None, None, *hs[2:], None, C.byref(size), C.byref(ex))
+    rc, res = _packed_call(L, _lib.OP_SWIGLU_QUANT[""], words)
+    assert (rc, res.workspaceSize) == (want, size.value)
+    if rc == 0:   # no workspace given: planned, not run; the executor is live and can be destroyed once
+        assert res.stage == _lib.STAGE_PLANNED
+        assert L.aclDestroyAclOpExecutor(C.c_void_p(res.executor)) == 0
+        assert L.aclDestroyAclOpExecutor(C.c_void_p(res.executor)) != 0
+        L.aclDestroyAclOpExecutor(ex)
+    for h in hs:
+        L.aclDestroyTensor(h)
+    # an invalid call reports what the operator's first phase reports
+    bad = []
+    for t in (x, w, None, None, ws, xs, gl.to(torch.int32), q, qs):
+        acl._put(bad, t)
+    rc, res = _packed_call(L, _lib.OP_SWIGLU_QUANT[""], bad)
+    assert rc == _lib.ACLNN_ERR_PARAM_INVALID and res.stage == _lib.STAGE_PLAN and not res.executor
+
+
+@pytest.mark.parametrize("words", [[], [2, 0, 2, 2, 4], [9], [1, 0, 2, 2, 4, 1, 12]])
+@pytest.mark.parametrize("op", [0, 3, 5, 7, 99])
+def test_packed_call_refuses_a_malformed_description(gmm_lib, op, words):
+    rc, res = _packed_call(gmm_lib, op, words)
+    assert rc == _lib.ACLNN_ERR_PARAM_INVALID and not res.executor
