@@ -468,6 +468,16 @@ def test_token_tile_edges(oracle, monkeypatch, ctas, kind):
         assert np.array_equal(got[perm[:rows]], ref[:rows]) and (got[perm[rows:]] == 0x7fc1).all()
 
 
+@pytest.mark.parametrize("act_type", [1, 2, 4, 5])
+def test_gmm_activations_beyond_the_range_of_exp(oracle, act_type):
+    """Arguments of the sigmoid from -1e4 to 1e4 (cubed, for GELU): both ends of exp, bf16 results within one rounding step."""
+    counts = np.array([70, 200], np.int64)
+    M, K, N, E = int(counts.sum()), 256, 256, 2
+    x, w, ws, xs = make_inputs(M, K, N, E, seed=65)
+    xs = np.ascontiguousarray(xs * np.logspace(-3, 1, M, dtype=np.float32))
+    check_gmm(oracle, x, w, ws, xs, np.cumsum(counts), act_type=act_type, expect_exact=False)
+
+
 def test_swiglu_activations_beyond_the_range_of_exp(oracle):
     """Activations from -1e4 to 1e4: exp overflows on one side and vanishes on the other; the product stays finite."""
     counts = np.array([70, 200], np.int64)
