@@ -23,7 +23,7 @@
 // CTA pairs (cluster of 2, tcgen05 cta_group::2) compute 256 channels; each CTA stages its own 128 channels and half of the
 // tile's token rows.  A launch confined to one CTA runs the one-CTA instances.  Weight layouts: [E,K,N] (MN-major operand,
 // 128-byte swizzle; 64-byte for swiglu's 64-channel boxes), the transposed view [E,N,K] (K-major) and FRACTAL_NZ
-// [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, 5-D tensor map).
+// [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, fetched by two loader warps instead of TMA).
 // Epilogue: a lane holds one channel (its weight scale stays in a register), the tokens' scales come from shared memory.
 // bf16 / fp16 results are read as 16x256b fragments, packed by token pairs and transposed by stmatrix, so that the four
 // warps of a column half together hold 256 contiguous bytes of every result row; 32-bit results (SwiGLU values, the
@@ -84,9 +84,21 @@ constexpr int EPI_WARPS = 8;                 // two warps per TMEM lane quarter,
 // claims) beside the epilogue, so that none of its round trips to L2 delays the next tile.  It hands the epilogue warps
 // lists of row ranges to requantise through a small ring.
 constexpr int WK_DEPTH = 4;                  // work lists the publishing lane may be ahead of the epilogue warps
-constexpr int RQ_WARPS = 5;                  // swiglu_quant: warps that requantise finished row blocks beside the epilogue
+// Weight loader warps (FRACTAL_NZ only).  A 32-byte row of that storage is a row of its own to TMA, 512 per 16 KB, and the
+// copy engine takes about 1.75 cycles for each: 900 cycles per K block where the MMAs need 512 and HBM 740.  In memory 128
+// K-rows of a 32-column slab are 4 KB in one piece, so two warps fetch them with 16-byte cp.async, 512 contiguous bytes per
+// instruction, and put the halves of every row where the 32-byte swizzle wants them.  Tensor copies / loader warps, us:
+// K=2048 N=7168 with 128 tokens x 8 over 256 experts 532 / 418 (6.6 TB/s), swiglu K=7168 N=4096 with 4096 tokens x 8 over 32
+// experts 955 / 844, gmm K=2048 N=7168 with 32 x 400 rows 204 / 184.
+constexpr int LD_WARPS = 2;
+__host__ __device__ constexpr int ld_warps(int bl) { return bl == 2 /* kBFractalNz */ ? LD_WARPS : 0; }
+// swiglu_quant: warps that requantise finished row blocks beside the epilogue; with 16 warps in all a thread has 128 registers
+__host__ __device__ constexpr int rq_warps(int bl) { return 5 - ld_warps(bl); }
 constexpr int BASE_THREADS = 64 + 32 * EPI_WARPS;
-__host__ __device__ constexpr int num_threads(int mode) { return BASE_THREADS + (mode == kModeSwigluQuant ? 32 + 32 * RQ_WARPS : 0); }
+__host__ __device__ constexpr int num_threads(int mode, int bl)
+{
+    return BASE_THREADS + 32 * ld_warps(bl) + (mode == kModeSwigluQuant ? 32 + 32 * rq_warps(bl) : 0);
+}
 constexpr int TMEM_COLS = 512;
 constexpr long long WAIT_LIMIT_CYCLES = 1ll << 31;   // about a second
 constexpr long long DRAIN_LIMIT_CYCLES = 1ll << 24;  // a few milliseconds
@@ -174,6 +186,7 @@ struct KParams {
     int half_n;        // N/2 (swiglu)
     int n_tiles;       // channel tiles per row block
     int num_k_blocks;  // ceil(K / BK)
+    const void *w_nz;     // FRACTAL_NZ weights, read by the loader warps
     const void *w_scale;
     int w_scale_dtype;
     const float *x_scale;
@@ -222,29 +235,43 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+// CLUSTER: acquires what the other CTA of the pair released (values stored into this CTA's shared memory).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(WAIT_SUSPEND_NS)
-        : "memory");
+    if (CLUSTER)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"(WAIT_SUSPEND_NS)
+            : "memory");
+    else
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"(WAIT_SUSPEND_NS)
+            : "memory");
     return ok != 0;
 }
 
 // Bounded wait.  Returns false when the limit ran out or another role already gave up.
+template <bool CLUSTER>
 __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, Shared *sh, int *status, int who,
                                             long long limit)
 {
     const long long t0 = clock64();
     uint32_t spins = 0;
     while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         if ((++spins & 31u) == 0u) {
             if (*(volatile int *)&sh->abort_flag) return false;
             if (clock64() - t0 > limit) {
@@ -259,11 +286,12 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, Share
         }
     }
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, Shared *sh, int *status, int who)
 {
     const uint32_t a = smem_u32(bar);
-    if (mbar_try_wait(a, parity)) return true;
-    return mbar_wait_slow(a, parity, sh, status, who, sh->wait_limit);
+    if (mbar_try_wait<CLUSTER>(a, parity)) return true;
+    return mbar_wait_slow<CLUSTER>(a, parity, sh, status, who, sh->wait_limit);
 }
 
 // Tiled TMA loads into this CTA's shared memory.  CTAS == 2 is the pair form: the byte count is credited to the mbarrier at
@@ -288,16 +316,19 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
         asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
                      ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
-template <int CTAS>
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4, uint32_t bar)
+// 16 bytes from global to shared memory, past L1; `bytes` 0 writes zeros without reading.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes)
 {
-    if (CTAS == 1)
-        asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar) : "memory");
-    else
-        asm volatile("cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                     ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar) : "memory");
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+// One arrival at `bar` (counted in its initial count) when this thread's copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// What was written to shared memory by ordinary accesses and cp.async is visible to the tensor core's reads.
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // L2 eviction policies for the fp32 SwiGLU staging rows: they are read back exactly once, about one tile after they were
 // written, while the operands of 74 other tiles stream through L2 in between.  Stored with evict_last and read back with
 // evict_first, more of them are still in L2 when they are needed (less DRAM traffic; the time gained is within 1 %).
@@ -670,12 +701,13 @@ __device__ __forceinline__ uint32_t quant4(float4 v, float rcp)
 // pieces (a load instruction covers 512 contiguous bytes, a store 128): the tensor cores read their operands through the
 // same shared-memory / L1 data path, so every extra line these accesses touch is taken from the MMAs.  Sixteen loads
 // per lane are in flight at a time, because they wait for L2 under the full load of the GEMM.
+template <int RQ>
 __device__ void requant_rows(const KParams &p, int r_begin, int r_end, int warp_r, int lane)
 {
     const int H = p.half_n;
     const int nf = H >> 2;  // 16-byte pieces per row
     const float *stage = reinterpret_cast<const float *>(p.out);
-    for (int grow = r_begin + warp_r; grow < r_end; grow += RQ_WARPS) {
+    for (int grow = r_begin + warp_r; grow < r_end; grow += RQ) {
         const float amax = __uint_as_float(__ldcg(p.amax_bits + grow));
         const float4 *src = reinterpret_cast<const float4 *>(stage + (size_t)grow * H);
         uint32_t *dst = reinterpret_cast<uint32_t *>(p.q_out + (size_t)grow * H);
@@ -807,14 +839,15 @@ __device__ void release_pending(const KParams &p, Shared *sh, int ws, int shares
 }
 
 // Requantising warp: the row ranges of the next work list.  Every warp consumes every list, in order, and takes the rows
-// warp, warp + RQ_WARPS, ... of each range.  Returns false when the (bounded) wait for the list gave up.
+// warp, warp + RQ, ... of each range.  Returns false when the (bounded) wait for the list gave up.
+template <int RQ>
 __device__ __forceinline__ bool consume_work(const KParams &p, Shared *sh, int list, int warp_r, int lane)
 {
     const int ws = list % WK_DEPTH;
     const bool ok = mbar_wait(&sh->wk_full[ws], ((uint32_t)(list / WK_DEPTH)) & 1u, sh, p.status, 650 + ws);
     if (!__all_sync(0xffffffffu, ok)) return false;
     const int n = sh->n_work[ws];
-    for (int k = 0; k < n; ++k) requant_rows(p, sh->work_begin[ws][k], sh->work_end[ws][k], warp_r, lane);
+    for (int k = 0; k < n; ++k) requant_rows<RQ>(p, sh->work_begin[ws][k], sh->work_end[ws][k], warp_r, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh->wk_empty[ws]);
     return true;
@@ -900,7 +933,7 @@ struct XMaps {
 // result rows scattered through out_row_index, optionally into other GPUs' memory; kEpiGeneric = every option
 // tested at run time.  CTAS: 1 = one CTA per tile (128 channels), 2 = a cluster of two CTAs (256 channels).
 template <int MODE, int BL, int EPI, int CTAS>
-__global__ void __launch_bounds__(num_threads(MODE), 1)
+__global__ void __launch_bounds__(num_threads(MODE, BL), 1)
 gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constant__ CUtensorMap map_w, const KParams p)
 {
     constexpr bool PLAIN = EPI != kEpiGeneric;   // lean arithmetic
@@ -909,6 +942,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
     constexpr bool SWIGLU = MODE == kModeSwigluQuant;
     constexpr bool OUT16 = MODE == kModeDequantBf16 && !COMBINE;
     using S = Shape<MODE, CTAS>;
+    constexpr bool NZ = BL == kBFractalNz;       // weights come through the loader warps
+    constexpr int RQ = rq_warps(BL), LD0 = num_threads(MODE, BL) / 32 - ld_warps(BL);   // first loader warp
     constexpr bool DUAL = S::kDual;
     constexpr int CH_CTA = S::kCols, MAX_TOK = S::kMaxTok, W_BYTES = S::kWStage;
     extern __shared__ uint8_t smem_raw[];
@@ -923,7 +958,9 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) {
-            mbar_init(&sh->full[s], 1);   // pair: only rank 0's is used; its producer arrives, both CTAs' copies credit it
+            // The producer arrives once and the copies credit their bytes (pair: at rank 0's barrier, for both CTAs); loader
+            // threads arrive each at their own CTA's barrier.
+            mbar_init(&sh->full[s], !NZ ? 1 : rank == 0 ? 1 + 32 * LD_WARPS : 32 * LD_WARPS);
             mbar_init(&sh->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -934,7 +971,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         for (int b = 0; b < 4; ++b) mbar_init(&sh->grp_sync[b], SWIGLU ? 2 : 4);
         for (int b = 0; b < WK_DEPTH; ++b) {
             mbar_init(&sh->wk_full[b], 1);
-            mbar_init(&sh->wk_empty[b], RQ_WARPS);
+            mbar_init(&sh->wk_empty[b], RQ);
         }
         sh->stored_count = 0;
         sh->abort_flag = 0;
@@ -961,7 +998,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
 
     if (warp == 0) {
         // ------------------------------ TMA producer (whole warp, one elected lane issues) ------------------------------
-        {
+        if (!(NZ && rank == 1)) {
             const bool leader = elect_one();
             int stage = 0;
             uint32_t phase = 0;
@@ -999,7 +1036,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                 const int my_row0 = tl.row0 + (int)rank * my_tok;
                 const int x_rows = x_box_rows<CTAS>(my_tok);
                 const CUtensorMap *map_x = &maps_x.box[x_rows >= 128 ? 2 : x_rows >= 64 ? 1 : 0];
-                const uint32_t tx_bytes = (uint32_t)CTAS * (uint32_t)(W_BYTES + x_rows * BK);
+                const uint32_t tx_bytes = (uint32_t)CTAS * (uint32_t)((NZ ? 0 : W_BYTES) + x_rows * BK);
                 const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA;   // first weight column of this CTA
                 // test hook: leaving K blocks out of the last tile makes the MMA issuer's wait run out (nothing else is touched)
                 const int kb_end = p.num_k_blocks - (t + n_units >= total_tiles ? p.skip_k_blocks : 0);
@@ -1015,9 +1052,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                         uint8_t *wdst = smem + stage * stage_bytes;
                         const uint32_t bar = CTAS == 2 ? full_rank0 + (uint32_t)stage * 8u : smem_u32(&sh->full[stage]);
                         if (rank == 0) mbar_arrive_expect_tx(&sh->full[stage], tx_bytes);
-                        if (BL == kBFractalNz) tma_load_5d<CTAS>(wdst, &map_w, 0, kb * BK, c0 >> 5, 0, tl.g, bar);
-                        else if (BL == kBTransposed) tma_load_4d<CTAS>(wdst, &map_w, kb * BK, c0, 0, tl.g, bar);
-                        else tma_load_4d<CTAS>(wdst, &map_w, c0, kb * BK, 0, tl.g, bar);
+                        if (BL == kBTransposed) tma_load_4d<CTAS>(wdst, &map_w, kb * BK, c0, 0, tl.g, bar);
+                        else if (!NZ) tma_load_4d<CTAS>(wdst, &map_w, c0, kb * BK, 0, tl.g, bar);
                         tma_load_2d<CTAS>(wdst + W_BYTES, map_x, kb * BK, my_row0, bar);
                         if (CTAS == 1 && x_rows > 128) tma_load_2d<CTAS>(wdst + W_BYTES + 128 * BK, map_x, kb * BK, my_row0 + 128, bar);
                     }
@@ -1073,13 +1109,14 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
 #ifdef GMM_TRACE
                     const long long tw0 = clock64();
 #endif
-                    if (!__all_sync(0xffffffffu, mbar_wait(&sh->full[stage], phase, sh, p.status, 300 + stage))) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait<NZ && CTAS == 2>(&sh->full[stage], phase, sh, p.status, 300 + stage))) { ok = false; break; }
 #ifdef GMM_TRACE
                     if (lane == 0) {
                         TRACE_ADD(1, ti, 3, clock64() - tw0);
                         TRACE_ADD(1, ti, 4, kb == 0 ? clock64() - tw0 : 0);
                     }
 #endif
+                    if (NZ) fence_async_proxy();
                     tc_fence_after();
                     if (leader) {
                         const uint64_t w_desc = w_desc0 + (uint64_t)(stage * (stage_bytes >> 4));
@@ -1116,6 +1153,76 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                 if (buf == 0) acc_phase ^= 1u;
             }
         }
+        else if (NZ) {
+            // ------------------------------ rank 1, loader warps: token rows, once the stage's weights are there ------------------------------
+            // The loaders' weights are complete at this CTA's barrier; rank 0 has to learn of it.  The copy of this CTA's token
+            // rows says so: it is issued after the weights have been seen complete (and fenced for the tensor core's reads) and
+            // credits rank 0's barrier.  An arrival of a thread would do too, but a cluster-wide release costs it 1450 cycles.
+            const bool leader = elect_one();
+            const uint32_t full_rank0 = map_to_cta(&sh->full[0], 0);
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            int g_prev = 0;
+            for (int t = unit; t < total_tiles && ok; t += n_units) {
+                const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                g_prev = tl.g;
+                const int my_tok = (tl.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP / CTAS;
+                const int x_rows = x_box_rows<CTAS>(my_tok);
+                const CUtensorMap *map_x = &maps_x.box[x_rows >= 128 ? 2 : x_rows >= 64 ? 1 : 0];
+                const int kb_end = p.num_k_blocks - (t + n_units >= total_tiles ? p.skip_k_blocks : 0);
+                for (int kb = 0; kb < kb_end; ++kb) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&sh->full[stage], phase, sh, p.status, 330 + stage))) { ok = false; break; }
+                    fence_async_proxy();
+                    if (leader)
+                        tma_load_2d<CTAS>(smem + stage * stage_bytes + W_BYTES, map_x, kb * BK, tl.row0 + my_tok, full_rank0 + (uint32_t)stage * 8u);
+                    __syncwarp();
+                    if (++stage == stages) { stage = 0; phase ^= 1u; }
+                }
+            }
+        }
+    } else if (NZ && warp >= LD0) {
+        // ------------------------------ weight loaders (FRACTAL_NZ) ------------------------------
+        // Storage [E, N/32, K/16, 16, 32]: element (k, n) at (n/32 * K + k) * 32 + n%32.  A stage is 4 (two accumulators: 8) slabs
+        // of 128 K-rows x 32 bytes; thread l takes 16-byte pieces l, l + 64, ... of each.  In shared memory a slab keeps that
+        // order, except that the 16-byte halves of rows 4..7 of every 8 change places (32-byte swizzle).
+        const int l = (int)threadIdx.x - LD0 * 32;
+        const uint32_t dst0 = smem_u32(smem) + (uint32_t)((l * 16) ^ ((l * 2) & 16));
+        constexpr int SLABS = W_BYTES / 4096;
+        const size_t slab_bytes = (size_t)p.K * 32;
+        const int8_t *w = static_cast<const int8_t *>(p.w_nz);
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        int g_prev = 0;
+        for (int t = unit; t < total_tiles && ok; t += n_units) {
+            const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+            g_prev = tl.g;
+            const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA, cols = SWIGLU ? p.half_n : p.N;
+            const int8_t *src = w + (size_t)tl.g * p.K * p.N + (size_t)(c0 >> 5) * slab_bytes + l * 16;
+            const size_t half_off = SWIGLU ? (size_t)(p.half_n >> 5) * slab_bytes : 0;   // from the activated to the linear half
+            for (int kb = 0; kb < p.num_k_blocks; ++kb) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&sh->empty[stage], phase ^ 1u, sh, p.status, 140 + stage))) { ok = false; break; }
+                const uint32_t dst = dst0 + (uint32_t)(stage * stage_bytes);
+                const int k_left = p.K - kb * BK - (l >> 1);   // > 0: this thread's K-row of the first piece exists
+#pragma unroll
+                for (int sl = 0; sl < SLABS; ++sl) {
+                    constexpr int PER_HALF = SWIGLU ? SLABS / 2 : SLABS;
+                    const int in_half = sl % PER_HALF;
+                    const bool in_n = c0 + in_half * 32 < cols;
+                    const int8_t *sp = src + (sl >= PER_HALF ? half_off : 0) + (size_t)in_half * slab_bytes;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool in = in_n && k_left > i * 32;
+                        cp_async16(dst + (uint32_t)(sl * 4096 + i * 1024), in ? sp + i * 1024 : w, in ? 16u : 0u);
+                    }
+                }
+                cp_async_arrive(&sh->full[stage]);
+                src += BK * 32;
+                if (++stage == stages) { stage = 0; phase ^= 1u; }
+            }
+        }
+        cp_async_wait_all();
     } else if (warp < 2 + EPI_WARPS) {
         // ------------------------------ epilogue: warp -> (TMEM lane quarter, every second chunk of 32 tokens) ------------------------------
         const int quarter = warp & 3;
@@ -1426,7 +1533,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         int lists = 1;
         for (int t = unit; t < total_tiles; t += n_units) ++lists;
         for (int i = 0; i < lists; ++i)
-            if (!consume_work(p, sh, i, warp - 3 - EPI_WARPS, lane)) break;
+            if (!consume_work<RQ>(p, sh, i, warp - 3 - EPI_WARPS, lane)) break;
     }
 
     else if (SWIGLU) {
@@ -1529,7 +1636,7 @@ cudaError_t launch_variant(const Plan &plan, const KParams &kp, cudaStream_t str
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CTAS == 2 ? (plan.num_sms & ~1) : plan.num_sms), 1, 1);
-    cfg.blockDim = dim3(num_threads(MODE), 1, 1);
+    cfg.blockDim = dim3(num_threads(MODE, BL), 1, 1);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1608,14 +1715,10 @@ cudaError_t sm100_encode_maps(const Problem &p, Plan &plan)
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     CUresult r;
     if (p.w_layout == kBFractalNz) {
-        // FRACTAL_NZ [E, N/32, K/16, 16, 32]: element (k, n) at (n/32 * K + k) * 32 + n%32
-        cuuint64_t dims[5] = {32, K, cols / 32, halves, E};
-        cuuint64_t strides[4] = {32, K * 32, K * cols, K * N};
-        cuuint32_t box[5] = {32, BK, box_ch / 32, halves, 1};
-        r = enc(&plan.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<int8_t *>(p.w), dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else if (p.w_layout == kBTransposed) {  // [E, N, K]
+        plan.map_w = plan.map_x[0];  // the loader warps read it; the kernel's map parameter is not used
+        return cudaSuccess;
+    }
+    if (p.w_layout == kBTransposed) {  // [E, N, K]
         cuuint64_t dims[4] = {K, cols, halves, E};
         cuuint64_t strides[3] = {K, K * cols, K * N};
         cuuint32_t box[4] = {BK, box_ch, halves, 1};
@@ -1654,6 +1757,7 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     const int64_t tile_cols = p.mode == kModeSwigluQuant ? BC : BC * plan.ctas, cols = p.mode == kModeSwigluQuant ? p.N / 2 : p.N;
     kp.n_tiles = (int)((cols + tile_cols - 1) / tile_cols);
     kp.num_k_blocks = (int)((p.K + BK - 1) / BK);
+    kp.w_nz = p.w;
     kp.w_scale = p.w_scale;
     kp.w_scale_dtype = p.w_scale_dtype;
     kp.x_scale = p.x_scale;
