@@ -36,9 +36,11 @@
 // idle; the SM clock falls to 1.5-1.6 GHz, at which the tensor pipe alone draws the board's 1 kW); groups of up to 128 rows
 // HBM; short K the epilogue.  Measured before (tokens on the M side, operations issued by one thread of a diverged warp,
 // every epilogue thread fencing for itself, requantisation inside the epilogue warps) and now, us:
-//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 881 (power), 1000 tokens x 8: layer 597 / 514,
-//     128 tokens x 8 over 256 experts 884 / 850 (HBM); K=2048 N=1536, 64 groups of 64 rows 66 / 54, of 400 rows 190 / 121
-//   gmm K=2048 N=7168: 4096 tokens x 8 449 / 430; 32 groups of 192 rows 120 / 105; K=768 N=2048, 64 x 400 rows 76 / 62
+//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 881 (power), 128 tokens x 8 over 256 experts 884 / 850 (HBM);
+//     K=2048 N=1536, 64 groups of 64 rows 66 / 54, of 400 rows 190 / 118
+//   gmm K=2048 N=7168: 4096 tokens x 8 over 32 experts 403 / 366; 32 groups of 160 rows 131 / 102; K=768 N=2048, 64 x 400 rows
+//     76 / 70 (of which 10 % came from moving the second CTA's accumulator release out of its epilogue warps: 374 / 334 for
+//     32 groups of 1000 rows)
 // The producers pace themselves wave by wave so that the units which share x rows and weight boxes through L2 stay
 // together (a bounded hint).
 // Every wait on an mbarrier is bounded; on expiry the CTA records a status word, all roles leave their loops,
@@ -965,7 +967,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sh->acc_full[b], 1);
-            mbar_init(&sh->acc_empty[b], EPI_WARPS * CTAS);  // one arrival per epilogue warp of every CTA of the unit
+            // one arrival per epilogue warp of this CTA; pair: rank 1's, complete, is passed on to rank 0 as one more
+            mbar_init(&sh->acc_empty[b], EPI_WARPS + (CTAS == 2 && rank == 0 ? 1 : 0));
             mbar_init(&sh->tok_ready[b], EPI_THREADS);
         }
         for (int b = 0; b < 4; ++b) mbar_init(&sh->grp_sync[b], SWIGLU ? 2 : 4);
@@ -996,9 +999,24 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
     const uint32_t tmem_base = sh->tmem_base;
     const int L = p.gl_len;
 
-    if (warp == 0) {
+    if (CTAS == 2 && rank == 1 && warp == (NZ ? 0 : 1)) {
+        // ------------------------------ rank 1, a warp without other work: its epilogue's releases to rank 0 ------------------------------
+        // An arrival at the other CTA's barrier with cluster-wide release takes 1450 cycles; here no epilogue warp waits for it.
+        const uint32_t acc_empty_rank0 = map_to_cta(&sh->acc_empty[0], 0);
+        int buf = 0;
+        uint32_t acc_phase = 0;
+        for (int t = unit; t < total_tiles; t += n_units) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[buf], acc_phase, sh, p.status, 210 + buf))) break;
+            tc_fence_after();
+            tc_fence_before();
+            if (lane == 0) mbar_arrive_cluster(acc_empty_rank0 + (uint32_t)buf * 8u);
+            __syncwarp();
+            buf ^= 1;
+            if (buf == 0) acc_phase ^= 1u;
+        }
+    } else if (warp == 0) {
         // ------------------------------ TMA producer (whole warp, one elected lane issues) ------------------------------
-        if (!(NZ && rank == 1)) {
+        {
             const bool leader = elect_one();
             int stage = 0;
             uint32_t phase = 0;
@@ -1240,7 +1258,6 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         int buf = 0, it = 0;
         uint32_t acc_phase = 0;
         const uint64_t pol_last = policy_evict_last();
-        const uint32_t acc_empty_rank0 = CTAS == 2 ? map_to_cta(&sh->acc_empty[0], 0) : 0u;
         bool ok = true;
         int g_prev = 0;
         for (int t = unit; t < total_tiles; t += n_units, ++it) {
@@ -1503,10 +1520,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             if (te == 0) TRACE(2, it, 2);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {  // the accumulator buffer may be overwritten once every epilogue warp of the unit has read it
-                if (CTAS == 1) mbar_arrive(&sh->acc_empty[buf]);
-                else mbar_arrive_cluster(acc_empty_rank0 + (uint32_t)buf * 8u);
-            }
+            if (lane == 0) mbar_arrive(&sh->acc_empty[buf]);  // the buffer may be overwritten once every epilogue warp of the unit has read it
             buf ^= 1;
             if (buf == 0) acc_phase ^= 1u;
 
