@@ -8,7 +8,7 @@
 // RowIdxGather (moe_v3_row_idx_gather.h:141-156), MoeGatherOut (moe_v3_gather_out.h:197-233) and
 // MoeGatherOutDynamicQuant::Compute (moe_v3_gather_dynamic_quant.h:103-143).
 //
-// Four launches, no host read in between:
+// Two to four launches (at most 1024 pairs: scatter and gather only; small tables: no scan), no host read in between:
 //   count   - one histogram of the active experts per block of 1024 pairs
 //   scan    - per expert (one CTA per 32 experts): exclusive prefix over the blocks; the CTA that finishes last then
 //             scans over the experts: start of every expert's rows, the counts output, the number of rows
@@ -49,6 +49,7 @@ struct RoutingParams {
     int *pair_pos;             // [pairs]: output row of every pair, -1 if its expert is not active
     int *total;                // number of output rows
     int nb;
+    int slots;                 // pairs of its token a CTA of the token-major gather stores: k, or 1 with k CTAs per token
 };
 
 // Programmatic dependent launch.  The kernels of one call form a chain (count -> scatter -> gather) in which the next
@@ -182,6 +183,35 @@ __global__ void __launch_bounds__(1024) routing_scan_kernel(const RoutingParams 
     if (threadIdx.x == 0) *p.total = row_carry;
 }
 
+// Scan over the experts (range <= 1024 = blockDim) from their totals in `tot`: first row of every expert into `first` and, if
+// `write_counts`, the counts output in count or key-value form (as the scan kernel writes it) and the number of rows.
+__device__ void expert_scan(const RoutingParams &p, const int *tot, int *first, int *warp_sums, bool write_counts)
+{
+    const int e = threadIdx.x;
+    const int c = e < p.range ? tot[e] : 0;
+    int sum_c, sum_nz;
+    const int inc_c = block_scan_1024(c, warp_sums, &sum_c);
+    const int inc_nz = block_scan_1024(c != 0 ? 1 : 0, warp_sums, &sum_nz);
+    if (e < p.range) first[e] = inc_c - c;
+    if (!write_counts) return;
+    if (e < p.range) {
+        if (p.count_type == 1) {
+            p.counts_out[e] = c;
+        } else if (c != 0) {
+            p.counts_out[2 * (size_t)(inc_nz - 1)] = e + p.e_start;
+            p.counts_out[2 * (size_t)(inc_nz - 1) + 1] = c;
+        }
+    }
+    if (p.count_type == 2) {  // the compact list ends in zero entries (moe_v3_expert_tokens_count.h:126-128, 255-257)
+        const int written_pairs = min(p.range + 1, p.expert_num);
+        for (int i = sum_nz + threadIdx.x; i < written_pairs; i += blockDim.x) {
+            p.counts_out[2 * (size_t)i] = 0;
+            p.counts_out[2 * (size_t)i + 1] = 0;
+        }
+    }
+    if (threadIdx.x == 0) *p.total = sum_c;
+}
+
 constexpr int kWarpTableRange = 256;  // up to this many active experts the scatter keeps one counter per warp and expert
 
 // PER_WARP: shared memory holds [32 warps][range] counters, all warps count at once and a scan over the warps gives every
@@ -190,15 +220,17 @@ constexpr int kWarpTableRange = 256;  // up to this many active experts the scat
 // every block derives what it needs from the block histograms itself - the rows of the earlier blocks and the first row
 // of every expert - while block 0 also writes the counts output.  One launch less per call.
 constexpr int kFoldTable = 8192;
-template <bool PER_WARP, bool FOLD = false>
+// SINGLE (all pairs in one block, at most kWarpTableRange active experts): the count kernel is left out too; the per-warp table
+// holds every expert's total.
+template <bool PER_WARP, bool FOLD = false, bool SINGLE = false>
 __global__ void __launch_bounds__(kPairsPerBlock) routing_scatter_kernel(const RoutingParams p)
 {
     extern __shared__ int running[];
-    __shared__ int s_first[FOLD ? kWarpTableRange : 1], s_off[FOLD ? kWarpTableRange : 1], s_tot[FOLD ? kWarpTableRange : 1];
+    __shared__ int s_first[FOLD || SINGLE ? kWarpTableRange : 1], s_off[FOLD ? kWarpTableRange : 1], s_tot[FOLD || SINGLE ? kWarpTableRange : 1];
     const int slots = PER_WARP ? p.range * (kPairsPerBlock / 32) : p.range;
     pdl_release();
     for (int e = threadIdx.x; e < slots; e += blockDim.x) running[e] = 0;
-    pdl_wait();  // the block histograms (or the scan's tables) are complete
+    if (!SINGLE) pdl_wait();  // the block histograms (or the scan's tables) are complete
     if (FOLD) {
         __shared__ int warp_sums[32];
         for (int e = threadIdx.x; e < p.range; e += blockDim.x) {
@@ -217,33 +249,7 @@ __global__ void __launch_bounds__(kPairsPerBlock) routing_scatter_kernel(const R
             }
         }
         __syncthreads();
-        // scan over the experts (range <= 256 <= blockDim): first row of every expert, and the counts output from block 0
-        {
-            const int e = threadIdx.x;
-            const int c = e < p.range ? s_tot[e] : 0;
-            int sum_c, sum_nz;
-            const int inc_c = block_scan_1024(c, warp_sums, &sum_c);
-            const int inc_nz = block_scan_1024(c != 0 ? 1 : 0, warp_sums, &sum_nz);
-            if (e < p.range) s_first[e] = inc_c - c;
-            if (blockIdx.x == 0) {  // in count or key-value form (as the scan kernel writes it)
-                if (e < p.range) {
-                    if (p.count_type == 1) {
-                        p.counts_out[e] = c;
-                    } else if (c != 0) {
-                        p.counts_out[2 * (size_t)(inc_nz - 1)] = e + p.e_start;
-                        p.counts_out[2 * (size_t)(inc_nz - 1) + 1] = c;
-                    }
-                }
-                if (p.count_type == 2) {  // the compact list ends in zero entries (moe_v3_expert_tokens_count.h:126-128, 255-257)
-                    const int written_pairs = min(p.range + 1, p.expert_num);
-                    for (int i = sum_nz + threadIdx.x; i < written_pairs; i += blockDim.x) {
-                        p.counts_out[2 * (size_t)i] = 0;
-                        p.counts_out[2 * (size_t)i + 1] = 0;
-                    }
-                }
-                if (threadIdx.x == 0) *p.total = sum_c;
-            }
-        }
+        expert_scan(p, s_tot, s_first, warp_sums, blockIdx.x == 0);
     }
     const long long j = (long long)blockIdx.x * kPairsPerBlock + threadIdx.x;
     int e = -1;
@@ -267,8 +273,14 @@ __global__ void __launch_bounds__(kPairsPerBlock) routing_scatter_kernel(const R
                 running[w * p.range + x] = run;
                 run += t;
             }
+            if (SINGLE) s_tot[x] = run;
         }
         __syncthreads();
+        if (SINGLE) {
+            __shared__ int single_sums[32];
+            expert_scan(p, s_tot, s_first, single_sums, true);
+            __syncthreads();
+        }
         if (e >= 0) before = running[warp * p.range + e] + rank;
     } else {
         for (int w = 0; w < kPairsPerBlock / 32; ++w) {
@@ -292,7 +304,8 @@ __global__ void __launch_bounds__(kPairsPerBlock) routing_scatter_kernel(const R
         if (p.row_idx_type == 0) p.expanded_row_idx[j] = -1;
         return;
     }
-    const int pos = FOLD ? s_first[e] + s_off[e] + before
+    const int pos = SINGLE ? s_first[e] + before
+                  : FOLD   ? s_first[e] + s_off[e] + before
                          : p.expert_first[e] + p.block_off[(size_t)blockIdx.x * p.range + e] + before;
     p.sorted_row[pos] = (int)j;
     p.pair_pos[j] = pos;
@@ -452,7 +465,8 @@ __global__ void __launch_bounds__(THREADS, MINB) routing_quant_token_kernel(cons
     constexpr int G = 16 / VEC;  // 16-byte loads that make one 16-byte store of int8: a thread owns G adjacent ones
     static_assert(NCH % G == 0, "whole stores per thread");
     __shared__ float red[THREADS / 32];
-    const int token = blockIdx.x;
+    const int token = p.slots == p.k ? blockIdx.x : blockIdx.x / p.k;
+    const int s0 = p.slots == p.k ? 0 : blockIdx.x - token * p.k;
     const int chunks = p.h / VEC;
     const uint4 *row = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.x) + (size_t)token * p.h);
     float v[NCH][VEC];
@@ -485,7 +499,7 @@ __global__ void __launch_bounds__(THREADS, MINB) routing_quant_token_kernel(cons
                                      quant_fast(v[i][e4 + 2], scale, rcp), quant_fast(v[i][e4 + 3], scale, rcp));
     }
     pdl_wait();  // the row positions are complete
-    for (int s = 0; s < p.k; ++s) {
+    for (int s = s0; s < s0 + p.slots; ++s) {
         const long long j = (long long)token * p.k + s;
         const int pos = p.pair_pos[j];
         if (pos < 0) continue;  // uniform over the CTA
@@ -623,14 +637,20 @@ cudaError_t init_routing_launch(const InitRoutingProblem &r, void *workspace, si
     // GMM_B200_PDL=0 turns the overlap of the chain's kernels off (plain stream order)
     const char *pdl_env = getenv("GMM_B200_PDL");
     const bool overlap = !(pdl_env && pdl_env[0] == '0');
-    routing_count_kernel<<<(unsigned)nb, kPairsPerBlock, smem, stream>>>(p);
-    if (range <= kWarpTableRange && (long long)nb * range <= kFoldTable) {
-        const cudaError_t e = launch_pdl(routing_scatter_kernel<true, true>, (unsigned)nb, kPairsPerBlock, smem * (kPairsPerBlock / 32), stream, overlap, p);
-        if (e != cudaSuccess) return e;
+    p.slots = p.k;
+    const size_t table = smem * (kPairsPerBlock / 32);
+    if (nb == 1 && range <= kWarpTableRange) {
+        routing_scatter_kernel<true, false, true><<<1, kPairsPerBlock, table, stream>>>(p);
     } else {
-        routing_scan_kernel<<<(unsigned)((range + 31) / 32), 1024, 0, stream>>>(p);
-        if (range <= kWarpTableRange) routing_scatter_kernel<true><<<(unsigned)nb, kPairsPerBlock, smem * (kPairsPerBlock / 32), stream>>>(p);
-        else routing_scatter_kernel<false><<<(unsigned)nb, kPairsPerBlock, smem, stream>>>(p);
+        routing_count_kernel<<<(unsigned)nb, kPairsPerBlock, smem, stream>>>(p);
+        if (range <= kWarpTableRange && (long long)nb * range <= kFoldTable) {
+            const cudaError_t e = launch_pdl(routing_scatter_kernel<true, true>, (unsigned)nb, kPairsPerBlock, table, stream, overlap, p);
+            if (e != cudaSuccess) return e;
+        } else {
+            routing_scan_kernel<<<(unsigned)((range + 31) / 32), 1024, 0, stream>>>(p);
+            if (range <= kWarpTableRange) routing_scatter_kernel<true><<<(unsigned)nb, kPairsPerBlock, table, stream>>>(p);
+            else routing_scatter_kernel<false><<<(unsigned)nb, kPairsPerBlock, smem, stream>>>(p);
+        }
     }
     const int eb = r.x_dtype == kF32 ? 4 : (r.x_dtype == kI8 ? 1 : 2);
     const bool aligned = ((reinterpret_cast<uintptr_t>(r.x) | reinterpret_cast<uintptr_t>(r.expanded_x) | reinterpret_cast<uintptr_t>(r.scale)) & 15) == 0;
@@ -638,14 +658,20 @@ cudaError_t init_routing_launch(const InitRoutingProblem &r, void *workspace, si
     if (r.quant) {
         // token-major kernels hold 32 values per thread (256 threads): h <= 8192, and h a multiple of 16 for the 16-byte stores
         const bool fast = aligned && r.h % 16 == 0 && r.h <= 8192 && r.n <= 0x7fffffffll;
+        // Fewer tokens than SMs: one CTA per pair.  A CTA's k pairs are a serial chain, with a smooth scale of two passes over
+        // that expert's scales and a block reduction each; with more tokens than SMs the chains run side by side and the row is
+        // better read once.  128 fp16 tokens, 8 of 256 experts, 64 of them active, h = 7168, smooth scales: 23.2 us a call with
+        // one CTA per token and the count kernel, 19.8 us with one per pair and without it.
+        p.slots = r.n < 148 ? 1 : (int)r.k;
+        const unsigned gather_grid = (unsigned)(p.slots == 1 ? pairs : r.n);
         if (r.x_dtype == kF32) {
-            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<float, 8, 256>, (unsigned)r.n, 256, 0, stream, overlap, p);
+            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<float, 8, 256>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<float><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else if (r.x_dtype == kF16) {
-            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__half, 4, 256, 4>, (unsigned)r.n, 256, 0, stream, overlap, p);
+            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__half, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<__half><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else if (r.x_dtype == kBF16) {
-            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__nv_bfloat16, 4, 256, 4>, (unsigned)r.n, 256, 0, stream, overlap, p);
+            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__nv_bfloat16, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<__nv_bfloat16><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else {
             return cudaErrorInvalidValue;

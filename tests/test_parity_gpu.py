@@ -654,6 +654,19 @@ def test_init_routing_many_blocks_keep_pair_order(oracle):
     check_init_routing(oracle, 9000, 8, 64, 32, (1, 31), 82, count_type=2)     # folded scan over 71 blocks
 
 
+@pytest.mark.parametrize("n,k,E,rng", [
+    (1, 1, 4, (0, 4)), (128, 8, 64, (0, 64)), (128, 8, 256, (64, 128)),    # all pairs in one block (1024): no count kernel
+    (128, 8, 300, (10, 267)),                                              # 257 active experts: too wide for the per-warp table
+    (129, 8, 64, (0, 64)),                                                 # one pair block more
+    (147, 6, 32, (8, 24)), (148, 6, 32, (8, 24)),                          # one CTA per pair / one CTA per token
+])
+@pytest.mark.parametrize("smooth", [False, True])
+def test_init_routing_launch_shape_edges(oracle, n, k, E, rng, smooth):
+    for count_type in (1, 2):
+        check_init_routing(oracle, n, k, 272, E, rng, 70 + n + k, smooth=smooth, x_kind="f16" if smooth else "bf16",
+                           row_idx_type=count_type - 1, count_type=count_type)
+
+
 def test_init_routing_without_quantisation(oracle):
     check_init_routing(oracle, 200, 4, 256, 32, (0, 32), 76, quant=False, per_token_scale=True)
     check_init_routing(oracle, 200, 4, 256, 32, (4, 20), 77, quant=False, x_kind="int8", row_idx_type=0)
