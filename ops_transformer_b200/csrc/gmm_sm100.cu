@@ -321,7 +321,7 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
 // 16 bytes from global to shared memory, past L1; `bytes` 0 writes zeros without reading.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes)
 {
-    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 // One arrival at `bar` (counted in its initial count) when this thread's copies so far have landed.
 __device__ __forceinline__ void cp_async_arrive(uint64_t *bar)
