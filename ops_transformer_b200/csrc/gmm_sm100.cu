@@ -855,16 +855,25 @@ __device__ __forceinline__ bool consume_work(const KParams &p, Shared *sh, int l
     return true;
 }
 
-// v / (1 + exp(-z)), for z < 0 as v e / (1 + e), with e = exp(-|z|) so that nothing overflows:  e = 2^t (1 + d ln 2) with
-// t = fl(-|z| log2 e) and d the remainder of that product (log2 e in two parts), the quotient from an approximate reciprocal
-// r of the denominator in [1, 2] and one correction q + (n - q den) r (Markstein).  As exact as expf and a correctly rounded
-// division (the 2-ulp ex2 is what either form is left with), in half of the instructions and without a branch.  An infinite
-// quotient is kept as it is; NaN stays NaN.
+// v / (1 + exp(-z)), for z < 0 as v e / (1 + e), with e = exp(-|z|) so that nothing overflows.
+//   e = 2^t (1 + d ln 2): t is the rounded product -|z| h of h = fl(log2 e), d = -|z| (h + l) - t what the rounding and the
+//   remainder l of log2 e = h + l left out (an fma each; |d| < 2^-16, so the second-order term is below 2^-33).
+//   The quotient comes from an approximate reciprocal r of the denominator in [1, 2] and one correction q + (n - q den) r
+//   (Markstein, IA-64 and Elementary Functions, 2000).
+// Below z = -64, where 1 + e is 1, e is kept multiplied by 4 until the last step: the flush of ex2 to zero then begins at
+// 2^-128, which is where 1 + expf(-z) of apply_activation overflows and its quotient becomes zero; unscaled it began at 2^-126
+// and took the results for z in [-88.72, -87.34] (about 5e-37) with it.
+// Error: ex2 2 ulp, its correction, n, the denominator, the quotient and its correction a rounding each: below 4 ulp of the
+// exact value down to the point where it vanishes, like expf and a division rounded once (which also sees expf's 2 ulp).  The
+// two differ in the last places, so the SIMT kernels' results (apply_activation) are not bit for bit the same.
+// An infinite quotient is kept as it is; NaN stays NaN.
 __device__ __forceinline__ float times_sigmoid(float v, float z)
 {
+    const bool tail = z < -64.0f;
     const float x = fminf(fabsf(z), 150.0f);
-    const float t = __fmul_rn(x, -1.44269502f);
-    const float d = __fmaf_rn(x, -1.92596303e-8f, __fmaf_rn(x, -1.44269502f, -t));
+    float t = __fmul_rn(x, -1.44269502f);
+    const float d = __fmaf_rn(x, -1.92596299e-8f, __fmaf_rn(x, -1.44269502f, -t));
+    if (tail) t = __fadd_rn(t, 2.0f);   // exact: |t| > 92
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
     e = __fmaf_rn(e, __fmul_rn(d, 0.693147181f), e);
@@ -873,7 +882,8 @@ __device__ __forceinline__ float times_sigmoid(float v, float z)
     const float n = z < 0.0f ? __fmul_rn(v, e) : v;
     const float q = __fmul_rn(n, r);
     const float c = __fmaf_rn(__fmaf_rn(-q, den, n), r, q);
-    return fabsf(q) <= 3.402823466e38f ? c : q;
+    const float res = fabsf(q) <= 3.402823466e38f ? c : q;
+    return tail ? __fmul_rn(res, 0.25f) : res;
 }
 
 // apply_activation (gmm_common.h) over a thread's values, the choice made once: with a switch in every element the unrolled

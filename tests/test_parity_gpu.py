@@ -487,6 +487,70 @@ def test_swiglu_activations_beyond_the_range_of_exp(oracle):
     check_swiglu(oracle, x, w, ws, xs, np.cumsum(counts))
 
 
+def _sigmoid_arguments():
+    """Arguments of the sigmoid: a dense sweep, the strip in which exp(z) leaves the normal range, both far ends, and small."""
+    z = np.concatenate([np.linspace(-100, 100, 40001), np.linspace(-89.5, -86.5, 6001), np.linspace(-66, -62, 2001),
+                        np.linspace(-150, 150, 3001), np.logspace(-6, 3, 4000), -np.logspace(-6, 3, 4000)]).astype(np.float32)
+    return z[z != 0]
+
+
+EXP_END = 88.722839   # expf overflows above: v / (1 + expf(-z)) is zero below -EXP_END (at the limit itself either is right)
+
+
+@pytest.mark.parametrize("K", [16, 17])   # the tensor-core kernel / the SIMT kernel (K that is no multiple of 16)
+def test_sigmoid_of_swiglu_in_fp32(oracle, K):
+    """One product gate * silu(z) per row, read back in fp32 through the row's scale |S| / 127.  Bound: 4 ulp of the sigmoid
+    quotient, one rounding each of the product and of the division by 127."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    z = _sigmoid_arguments()
+    M, N = z.size, 64
+    x, w = np.zeros((M, K), np.int8), np.zeros((1, K, N), np.int8)
+    x[:, 0] = np.sign(z)
+    w[0, 0, 0] = w[0, 0, N // 2] = 1       # S = z * silu(z) in column 0, zero elsewhere
+    t = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
+    _, qs, wsb = ops.grouped_matmul_swiglu_quant(t(x), t(w), torch.ones((1, N), device=dev), t(np.abs(z)),
+                                                 torch.tensor([M], device=dev), return_workspace=True)
+    ops.check_status(wsb)
+    z64 = z.astype(np.float64)
+    want = np.where(z64 > -EXP_END, z64 * z64 / (1 + np.exp(-np.maximum(z64, -100.0))) / 127, 0.0)
+    got = qs.cpu().numpy().astype(np.float64)
+    keep = np.abs(z64 + EXP_END) > 4e-5
+    err = np.abs(got - want) / np.maximum(want, 1e-44)
+    assert err[keep].max() <= 5 * 2.0 ** -23, (z[keep][err[keep].argmax()], err[keep].max())
+
+
+@pytest.mark.parametrize("act_type", [2, 4, 5])
+def test_activations_of_special_values(oracle, act_type):
+    """bf16 results of the tensor-core kernel's activations against 64 bits over the same arguments, and at infinities, NaN
+    and values whose cube overflows against the SIMT kernel (expf and a division)."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    z = _sigmoid_arguments()
+    special = np.array([np.inf, -np.inf, np.nan, 1e13, -1e13, 1e20, -1e20, 3e38, -3e38, 1e-38, -1e-38, 1e-44, -1e-44], np.float32)
+    v = np.concatenate([z, special])
+    M, N = v.size, 32
+    got = {}
+    for K in (16, 17):
+        x, w = np.zeros((M, K), np.int8), np.zeros((1, K, N), np.int8)
+        x[:, 0] = w[0, 0, 0] = 1
+        t = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
+        y, wsb = ops.grouped_matmul_v4(t(x), t(w), torch.ones((1, N), device=dev), t(v), torch.tensor([M], device=dev),
+                                       act_type=act_type, return_workspace=True)
+        ops.check_status(wsb)
+        got[K] = y[:, 0].float().cpu().numpy()
+    n = z.size
+    assert np.array_equal(got[16][n:], got[17][n:], equal_nan=True)
+    a = z.astype(np.float64)
+    arg = {2: 1.59576912 * (a + 0.044715 * a ** 3), 4: 1.702 * a, 5: a}[act_type]
+    want = np.where(arg > -EXP_END, a / (1 + np.exp(-np.maximum(arg, -100.0))), 0.0)
+    keep = np.abs(arg + EXP_END) > 1e-4    # three fp32 roundings of the argument
+    for K in (16, 17):
+        # half a step of bf16 (8 significant bits); the argument's own roundings (2^-22 of at most 89) move exp by 2e-5
+        err = np.abs(got[K][:n] - want) / np.maximum(np.abs(want), 1e-38)
+        assert err[keep].max() <= 2.0 ** -8 + 4e-5, (K, z[keep][err[keep].argmax()], err[keep].max())
+
+
 # ----------------------------------------------------------------------------------------------------------
 # grouped_matmul_finalize_routing (down GEMM + weighted combine)
 # ----------------------------------------------------------------------------------------------------------
