@@ -376,6 +376,13 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr)
 {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
+// The same in two parts: what this thread has done and observed in its CTA's shared memory is released to the cluster by the
+// next arrival, and an arrival that releases nothing by itself.
+__device__ __forceinline__ void fence_release_shared_cluster() { asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar_cluster_addr)
+{
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
 __device__ __forceinline__ uint32_t cluster_cta_rank()
 {
     uint32_t r;
@@ -971,8 +978,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) {
             // The producer arrives once and the copies credit their bytes (pair: at rank 0's barrier, for both CTAs); loader
-            // threads arrive each at their own CTA's barrier.
-            mbar_init(&sh->full[s], !NZ ? 1 : rank == 0 ? 1 + 32 * LD_WARPS : 32 * LD_WARPS);
+            // threads arrive each at their own CTA's barrier, and rank 1's, complete, is passed on to rank 0 as one more.
+            mbar_init(&sh->full[s], !NZ ? 1 : rank == 0 ? 32 * LD_WARPS + CTAS : 32 * LD_WARPS);
             mbar_init(&sh->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -1182,10 +1189,14 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             }
         }
         else if (NZ) {
-            // ------------------------------ rank 1, loader warps: token rows, once the stage's weights are there ------------------------------
-            // The loaders' weights are complete at this CTA's barrier; rank 0 has to learn of it.  The copy of this CTA's token
-            // rows says so: it is issued after the weights have been seen complete (and fenced for the tensor core's reads) and
-            // credits rank 0's barrier.  An arrival of a thread would do too, but a cluster-wide release costs it 1450 cycles.
+            // ------------------------------ rank 1, loader warps: token rows, and word to rank 0 that the stage is there ------------------------------
+            // The loaders' weights are complete at this CTA's barrier; rank 0, which issues the MMA that reads them, has to learn
+            // of it.  The chain, every link a rule of the PTX memory model: the loaders' cp.async are tracked by this CTA's
+            // barrier (cp.async.mbarrier.arrive), whose completed phase this warp acquires; a proxy fence on that path orders
+            // them before reads of the async proxy; a release at cluster scope, cumulative over what this warp has observed, with
+            // the arrival at rank 0's barrier; rank 0's acquire at cluster scope, after which it issues the MMA.  The release
+            // covers shared memory alone (sync_restrict): an arrival with an unrestricted one also waits for global memory, 1450
+            // cycles per K block of 512.  The completion of the token copy would not do: it releases the copy's own bytes only.
             const bool leader = elect_one();
             const uint32_t full_rank0 = map_to_cta(&sh->full[0], 0);
             int stage = 0;
@@ -1202,8 +1213,11 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                 for (int kb = 0; kb < kb_end; ++kb) {
                     if (!__all_sync(0xffffffffu, mbar_wait(&sh->full[stage], phase, sh, p.status, 330 + stage))) { ok = false; break; }
                     fence_async_proxy();
-                    if (leader)
+                    fence_release_shared_cluster();
+                    if (leader) {
                         tma_load_2d<CTAS>(smem + stage * stage_bytes + W_BYTES, map_x, kb * BK, tl.row0 + my_tok, full_rank0 + (uint32_t)stage * 8u);
+                        mbar_arrive_cluster_relaxed(full_rank0 + (uint32_t)stage * 8u);
+                    }
                     __syncwarp();
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }

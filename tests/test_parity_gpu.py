@@ -487,6 +487,38 @@ def test_swiglu_activations_beyond_the_range_of_exp(oracle):
     check_swiglu(oracle, x, w, ws, xs, np.cumsum(counts))
 
 
+@pytest.mark.parametrize("K", [2048, 7168])
+def test_fractal_nz_on_pairs_repeats_bit_for_bit(monkeypatch, K):
+    """The second CTA's weights reach the first one's MMAs through a chain of barriers, 16 or 56 K blocks per tile through a
+    ring of at most 6 stages.  Every repetition equals the row-major layout's exact result (int32 sums, int8 rows of swiglu);
+    full tiles, tiles of one 32-token step and several tiles per group, new weights and a clean ring each time."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    monkeypatch.setenv("GMM_B200_CTAS", "2")
+    E, N = 5, 1536
+    counts = torch.tensor([700, 31, 256, 0, 1040], dtype=torch.int64, device=dev)
+    M = int(counts.sum())
+    gl = counts.cumsum(0)
+    g = torch.Generator(device=dev)
+    g.manual_seed(71)
+    xs, ws = torch.rand(M, device=dev, generator=g) / 32, torch.rand((E, N), device=dev, generator=g) / 1024
+    for _ in range(12):
+        x = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=dev, generator=g)
+        w = torch.randint(-127, 128, (E, K, N), dtype=torch.int8, device=dev, generator=g)
+        nz = ops.format_cast_nz(w)
+        want = ops.grouped_matmul_v4(x, w, None, None, gl, out_dtype=torch.int32)
+        want_q, want_s = ops.grouped_matmul_swiglu_quant(x, w, ws, xs, gl)
+        for _ in range(3):
+            got, wsb = ops.grouped_matmul_v4(x, nz, None, None, gl, out_dtype=torch.int32, weight_format=ops.ACL_FORMAT_FRACTAL_NZ,
+                                             return_workspace=True)
+            ops.check_status(wsb)
+            assert torch.equal(got, want)
+            q, qs, wsb = ops.grouped_matmul_swiglu_quant(x, nz, ws, xs, gl, weight_format=ops.ACL_FORMAT_FRACTAL_NZ,
+                                                         return_workspace=True)
+            ops.check_status(wsb)
+            assert torch.equal(q, want_q) and torch.equal(qs, want_s)
+
+
 def _sigmoid_arguments():
     """Arguments of the sigmoid: a dense sweep, the strip in which exp(z) leaves the normal range, both far ends, and small."""
     z = np.concatenate([np.linspace(-100, 100, 40001), np.linspace(-89.5, -86.5, 6001), np.linspace(-66, -62, 2001),
