@@ -9,8 +9,10 @@ codes raised as ``AclnnError``.  torch is used for device memory and streams onl
 from __future__ import annotations
 
 import array
+import contextlib
 import ctypes as C
 import struct
+import threading
 from typing import Optional, Sequence
 
 import torch
@@ -79,29 +81,93 @@ def create_tensor_list(tensors: Sequence[torch.Tensor], fmt: int = ACL_FORMAT_ND
     return h
 
 
-class _Workspace:
-    """One growing device buffer per device, reused across calls like a framework's workspace pool."""
+class _Slot:
+    """The pooled workspace of one stream.  ``lock`` is held while a call is enqueued with ``buf``: the clear and the kernels of
+    two calls must not interleave on the stream."""
+    __slots__ = ("lock", "buf")
 
     def __init__(self):
-        self._buf = {}
+        self.lock = threading.RLock()
+        self.buf: Optional[torch.Tensor] = None
 
-    def get(self, device: torch.device, nbytes: int) -> Optional[torch.Tensor]:
-        if nbytes == 0:
-            return None
-        key = (device.type, device.index)
-        b = self._buf.get(key)
-        if b is None or b.numel() < nbytes:
+
+class _Workspace:
+    """Growing device buffers for the calls that bring no workspace, one per device and stream: a call uses its buffer until
+    its last kernel is done, so calls that may run at the same time must not share one.  The buffers are allocated on their
+    own stream; one that is outgrown or evicted goes back to the allocator, which reuses it in that stream's order."""
+    MAX_SLOTS = 16   # streams with a buffer; with more of them the oldest slot's goes
+
+    def __init__(self):
+        self._slots = {}
+        self._lock = threading.Lock()
+        self._replayed = {}   # address -> buffer a replay will use (see for_capture)
+
+    def slot(self, device: torch.device, handle: int) -> _Slot:
+        # the per-thread default stream has one handle and is another stream in every thread
+        key = (device.type, device.index, handle, threading.get_ident() if handle == _STREAM_PER_THREAD else 0)
+        s = self._slots.get(key)
+        if s is None:
+            with self._lock:
+                s = self._slots.setdefault(key, _Slot())
+                while len(self._slots) > self.MAX_SLOTS:
+                    del self._slots[next(iter(self._slots))]
+        return s
+
+    @staticmethod
+    def grown(slot: _Slot, device: torch.device, stream, nbytes: int) -> torch.Tensor:
+        """The slot's buffer with room for ``nbytes``."""
+        if slot.buf is None or slot.buf.numel() < nbytes:
+            with _on_stream(stream, device):
+                slot.buf = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        return slot.buf
+
+    def for_capture(self, slot: _Slot, device: torch.device, stream, nbytes: int) -> torch.Tensor:
+        """A workspace for a call that is being captured.  A buffer from the memory pool of a torch graph belongs to that graph
+        as long as it lives, so that its replays share it neither with other graphs nor with calls outside.  A capture that
+        has no such pool gets the stream's buffer, which is kept from then on even if the stream's calls outgrow it."""
+        with _on_stream(stream, device):
             b = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
-            self._buf[key] = b
+        if _in_graph_pool(b):
+            return b
+        b = self.grown(slot, device, stream, nbytes)
+        self._replayed[b.data_ptr()] = b
         return b
 
 
-    def peek(self, device: torch.device) -> Optional[torch.Tensor]:
-        """The buffer as it is, whatever its size; None before the first use."""
-        return self._buf.get((device.type, device.index))
-
-
 _WS = _Workspace()
+_STREAM_PER_THREAD = 2   # cudaStreamPerThread
+
+
+def _on_stream(stream, device: torch.device):
+    """Context in which torch's current stream is ``stream``."""
+    if stream is None or device.type != "cuda":
+        return contextlib.nullcontext()
+    if not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(int(stream.cuda_stream), device=device)
+    return torch.cuda.stream(stream)
+
+
+def _capturing(stream, device: torch.device) -> bool:
+    if device.type != "cuda":
+        return False
+    if stream is None or int(stream.cuda_stream) == int(torch.cuda.current_stream().cuda_stream):
+        return torch.cuda.is_current_stream_capturing()
+    with _on_stream(stream, device):
+        return torch.cuda.is_current_stream_capturing()
+
+
+def _in_graph_pool(t: torch.Tensor) -> bool:
+    p = t.data_ptr()
+    return any(tuple(seg["segment_pool_id"]) != (0, 0) for seg in torch.cuda.memory_snapshot()
+               if seg["address"] <= p < seg["address"] + seg["total_size"])
+
+
+@contextlib.contextmanager
+def _pooled(device: torch.device, stream, nbytes: int):
+    """A workspace of ``nbytes`` for a call on ``stream`` that is enqueued inside the context."""
+    slot = _WS.slot(device, _stream_handle(stream) if device.type == "cuda" else 0)
+    with slot.lock:
+        yield (_WS.for_capture if _capturing(stream, device) else _WS.grown)(slot, device, stream, nbytes)
 
 
 def _stream_handle(stream) -> int:
@@ -157,12 +223,24 @@ def _put_ints(words: list, values: Optional[Sequence[int]]) -> None:
 def _call(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream,
           options: Optional[LaunchOptions]) -> Optional[torch.Tensor]:
     """Both phases of operator ``name`` on the packed description; returns the workspace that was used (None if none)."""
+    if workspace is not None:
+        return _enqueue(op, name, words, device, workspace, stream, options, None)
+    slot = _WS.slot(device, _stream_handle(stream) if device.type == "cuda" else 0)
+    with slot.lock:
+        return _enqueue(op, name, words, device, None, stream, options, slot)
+
+
+def _enqueue(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream,
+             options: Optional[LaunchOptions], slot: Optional[_Slot]) -> Optional[torch.Tensor]:
     L = _lib.lib()
     packed = array.array("q", words)
     res = _lib.CallResult()
     # validation needs no device: tensors that are not on one are planned only, so that what is wrong with them is reported first
     on_gpu = device.type == "cuda"
-    buf = None if not on_gpu else workspace if workspace is not None else _WS.peek(device)
+    capturing = slot is not None and _capturing(stream, device)
+    buf = workspace if workspace is not None else slot.buf
+    if not on_gpu or capturing:
+        buf = None
     handle = _stream_handle(stream) if on_gpu else 0
     rc = L.gmmB200Call(op, packed.buffer_info()[0], len(packed), buf.data_ptr() if buf is not None else None,
                        buf.numel() if buf is not None else 0, C.byref(options) if options is not None else None, handle, C.byref(res))
@@ -171,7 +249,11 @@ def _call(op: int, name: str, words: list, device: torch.device, workspace: Opti
         if workspace is not None and workspace.numel() < res.workspaceSize:
             L.aclDestroyAclOpExecutor(ex)
             raise ValueError(f"workspace of {workspace.numel()} bytes is smaller than the {res.workspaceSize} required")
-        buf = workspace if workspace is not None else _WS.get(device, res.workspaceSize)
+        try:
+            buf = workspace if workspace is not None else (_WS.for_capture if capturing else _WS.grown)(slot, device, stream, res.workspaceSize)
+        except Exception:
+            L.aclDestroyAclOpExecutor(ex)
+            raise
         rc = getattr(L, name)(buf.data_ptr(), res.workspaceSize, ex, _stream_handle(stream))
         res.stage = _lib.STAGE_RUN
     if rc != ACLNN_SUCCESS:
@@ -244,7 +326,9 @@ def _grouped_matmul_flat(x, weight, scale, per_token_scale, group_list, bias, gr
     if rc != ACLNN_SUCCESS:
         raise AclnnError(rc, "gmmB200GroupedMatmulW8A8WorkspaceSize")
     if workspace is None:
-        workspace = _WS.get(x.device, size.value)
+        with _pooled(x.device, stream, size.value) as pooled:
+            return _grouped_matmul_flat(x, weight, scale, per_token_scale, group_list, bias, group_list_type, act_type, out, out_row_index,
+                                        stream, pooled, return_workspace, out_peers, nz, options, out_rows)
     p = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
     rc = L.gmmB200GroupedMatmulW8A8(p(x), p(weight), p(scale), _DTYPES[scale.dtype] if scale is not None else 0, p(per_token_scale),
                                     p(bias), _DTYPES[bias.dtype] if bias is not None else 0, p(group_list), group_list.numel(),
@@ -322,7 +406,11 @@ def grouped_matmul_finalize_routing_flat(x, weight, weight_layout, scale, group_
     else:
         E, _, N = weight.shape
     if workspace is None:
-        workspace = _WS.get(x.device, 256)
+        with _pooled(x.device, stream, 256) as pooled:
+            return grouped_matmul_finalize_routing_flat(
+                x, weight, weight_layout, scale, group_list, row_index, out, bias=bias, pertoken_scale=pertoken_scale,
+                shared_input=shared_input, logit=logit, shared_input_weight=shared_input_weight, shared_input_offset=shared_input_offset,
+                group_list_type=group_list_type, stream=stream, workspace=pooled, options=options)
     p = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
     rc = L.gmmB200GroupedMatmulFinalizeRouting(
         p(x), p(weight), weight_layout, p(scale), _DTYPES[scale.dtype], p(bias), p(pertoken_scale), p(group_list),

@@ -563,3 +563,107 @@ def test_packed_call_plans_like_the_separate_handles(gmm_lib):
 def test_packed_call_refuses_a_malformed_description(gmm_lib, op, words):
     rc, res = _packed_call(gmm_lib, op, words)
     assert rc == _lib.ACLNN_ERR_PARAM_INVALID and not res.executor
+
+
+# ----------------------------------------------------------------------------------------------------------
+# the pooled workspace: which calls may share a buffer
+# ----------------------------------------------------------------------------------------------------------
+
+@pytest.fixture
+def recorded_calls(monkeypatch):
+    """``acl._call`` against a library that records (workspace address, stream, thread) instead of launching; the device is a
+    stand-in and its memory is host memory.  ``need`` is the workspace size that the operator asks for."""
+    torch = pytest.importorskip("torch")
+    import contextlib
+    import threading
+    import types
+    from ops_transformer_b200 import acl
+    rec = types.SimpleNamespace(calls=[], need=1000, inside=0, overlapped=False, capturing=False, alive=[])
+    lock = threading.Lock()
+
+    class Lib:
+        def gmmB200Call(self, op, words, count, ws, nbytes, options, stream, result):
+            import time
+            with lock:
+                rec.inside += 1
+                rec.overlapped |= rec.inside > 1
+            time.sleep(0.002)
+            res = result._obj
+            res.workspaceSize, res.stage = rec.need, _lib.STAGE_RUN if ws and nbytes >= rec.need else _lib.STAGE_PLANNED
+            if res.stage == _lib.STAGE_RUN:
+                rec.calls.append((ws, stream))
+            with lock:
+                rec.inside -= 1
+            return 0
+
+        def anOperator(self, ws, nbytes, executor, stream):
+            rec.calls.append((ws, stream))
+            return 0
+
+    real_empty = torch.empty
+
+    def empty(n, dtype=None, device=None):
+        t = real_empty(n, dtype=dtype)
+        rec.alive.append(t)   # keeps addresses distinct
+        return t
+    fake_torch = types.SimpleNamespace(
+        empty=empty, uint8=torch.uint8, Tensor=torch.Tensor,
+        cuda=types.SimpleNamespace(Stream=types.SimpleNamespace, stream=lambda s: contextlib.nullcontext(),
+                                   current_stream=lambda: types.SimpleNamespace(cuda_stream=7),
+                                   is_current_stream_capturing=lambda: rec.capturing, memory_snapshot=lambda: rec.snapshot()))
+    monkeypatch.setattr(acl, "torch", fake_torch)
+    monkeypatch.setattr(acl._lib, "lib", lambda: Lib())
+    monkeypatch.setattr(acl, "_WS", type(acl._WS)())
+    device = types.SimpleNamespace(type="cuda", index=0)
+    rec.call = lambda handle=None: acl._call(0, "anOperator", [], device, None, None if handle is None else types.SimpleNamespace(cuda_stream=handle), None)
+    rec.acl = acl
+    return rec
+
+
+def test_streams_do_not_share_a_pooled_workspace(recorded_calls):
+    rec = recorded_calls
+    for handle in (11, 12, 11, 12, None):
+        rec.call(handle)
+    ptr = [p for p, _ in rec.calls]
+    assert [s for _, s in rec.calls] == [11, 12, 11, 12, 7]
+    assert ptr[0] == ptr[2] and ptr[1] == ptr[3] and len({ptr[0], ptr[1], ptr[4]}) == 3
+    rec.need = 5000       # grows on one stream only
+    rec.call(11)
+    rec.need = 1000
+    rec.call(11), rec.call(12)
+    assert rec.calls[5][0] == rec.calls[6][0] != ptr[0] and rec.calls[7][0] == ptr[1]
+    for handle in range(100, 200):   # bounded
+        rec.call(handle)
+    assert len(rec.acl._WS._slots) == rec.acl._WS.MAX_SLOTS
+
+
+def test_threads_on_one_stream_enqueue_one_call_at_a_time(recorded_calls):
+    import threading
+    rec = recorded_calls
+    rec.call(11)
+    ts = [threading.Thread(target=lambda: [rec.call(11) for _ in range(5)]) for _ in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not rec.overlapped and len(rec.calls) == 21 and len(set(rec.calls)) == 1
+    per_thread = []
+    ts = [threading.Thread(target=lambda: (rec.call(2), per_thread.append(threading.get_ident()))) for _ in range(2)]   # cudaStreamPerThread
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    if per_thread[0] != per_thread[1]:
+        assert len({p for p, s in rec.calls if s == 2}) == 2
+
+
+def test_captured_calls_keep_their_workspace(recorded_calls):
+    rec = recorded_calls
+    rec.call(11)
+    rec.capturing = True
+    rec.snapshot = lambda: [dict(address=t.data_ptr(), total_size=t.numel(), segment_pool_id=(0, 5)) for t in rec.alive]
+    rec.call(11)   # torch graph: a buffer from the graph's own pool, not the stream's, and not kept by the pool
+    rec.call(11)
+    assert len({p for p, _ in rec.calls}) == 3 and not rec.acl._WS._replayed
+    rec.snapshot = lambda: []
+    rec.call(11)   # a capture without such a pool: the stream's buffer, kept when it is outgrown
+    assert rec.calls[3][0] == rec.calls[0][0]
+    rec.capturing, rec.need = False, 9000
+    rec.call(11)
+    assert rec.calls[4][0] != rec.calls[0][0] and rec.calls[0][0] in rec.acl._WS._replayed

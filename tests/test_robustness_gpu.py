@@ -170,3 +170,95 @@ def test_options_are_per_executor_and_need_a_live_executor(gmm_lib):
     opts = _lib.LaunchOptions(max_ctas=4)
     assert gmm_lib.gmmB200SetExecutorOptions(None, C.byref(opts)) == _lib.ACLNN_ERR_PARAM_NULLPTR
     assert gmm_lib.gmmB200SetExecutorOptions(C.c_void_p(0x1000), C.byref(opts)) == _lib.ACLNN_ERR_PARAM_INVALID
+
+
+def _check_swiglu_bits(oracle, host, gl, q, qs):
+    ref = oracle.swiglu_quant(*host, gl)
+    rel = np.abs(qs.cpu().numpy() - ref["q_scale"]) / np.abs(ref["q_scale"])
+    assert rel.max() <= 1e-6
+    d = np.abs(q.cpu().numpy().astype(np.int32) - ref["q"].astype(np.int32))
+    assert d.max() <= 1 and np.count_nonzero(d) / d.size <= 1e-4
+
+
+@pytest.mark.parametrize("threads", [False, True])
+def test_pooled_workspaces_of_two_streams(oracle, threads):
+    """Calls that bring no workspace, overlapping on two streams, from one thread or from one each."""
+    import threading
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    counts = np.array([700, 300, 0, 1100, 520], np.int64)
+    M, K, N, E = int(counts.sum()), 1024, 2048, 5
+    gl = torch.from_numpy(np.cumsum(counts)).to(dev)
+    sets = [_gmm_inputs(dev, M, K, N, E, 50 + i) for i in range(2)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = [[], []]
+    torch.cuda.synchronize()
+
+    def work(i, reps):
+        with torch.cuda.stream(streams[i]):
+            for _ in range(reps):
+                outs[i].append(ops.grouped_matmul_swiglu_quant(*sets[i][1], gl))
+    if threads:
+        ts = [threading.Thread(target=work, args=(i, 6)) for i in range(2)]
+        [t.start() for t in ts]
+        [t.join() for t in ts]
+    else:
+        for _ in range(6):
+            work(0, 1)
+            work(1, 1)
+    torch.cuda.synchronize()
+    for i in range(2):
+        for q, qs in outs[i]:
+            assert torch.equal(qs, outs[i][0][1]) and torch.equal(q, outs[i][0][0])
+        _check_swiglu_bits(oracle, sets[i][0], np.cumsum(counts), *outs[i][0])
+
+
+def test_threads_share_one_stream(oracle):
+    """The clear and the kernels of a call stay together on the stream, whoever else enqueues on it."""
+    import threading
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    counts = np.array([100, 60], np.int64)
+    M, K, N, E = int(counts.sum()), 256, 512, 2
+    gl = torch.from_numpy(np.cumsum(counts)).to(dev)
+    sets = [_gmm_inputs(dev, M, K, N, E, 60 + i) for i in range(4)]
+    outs = [[] for _ in sets]
+    torch.cuda.synchronize()
+    ts = [threading.Thread(target=lambda i=i: outs[i].extend(ops.grouped_matmul_swiglu_quant(*sets[i][1], gl) for _ in range(50))) for i in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    torch.cuda.synchronize()
+    for (host, _), out in zip(sets, outs):
+        assert all(torch.equal(qs, out[0][1]) and torch.equal(q, out[0][0]) for q, qs in out)
+        _check_swiglu_bits(oracle, host, np.cumsum(counts), *out[0])
+
+
+def test_captured_calls_own_their_workspace(oracle):
+    """Two graphs replayed at the same time on two streams, after calls outside have outgrown the buffers of the capture."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    counts = np.array([700, 300, 0, 1100], np.int64)
+    M, K, N, E = int(counts.sum()), 512, 1024, 4
+    gl = torch.from_numpy(np.cumsum(counts)).to(dev)
+    sets = [_gmm_inputs(dev, M, K, N, E, 70 + i) for i in range(2)]
+    graphs, outs = [], []
+    for _, t in sets:
+        ops.grouped_matmul_swiglu_quant(*t, gl)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(ops.grouped_matmul_swiglu_quant(*t, gl))
+        graphs.append(g)
+    big = torch.zeros((4 * M, K), dtype=torch.int8, device=dev)
+    ops.grouped_matmul_swiglu_quant(big, *sets[0][1][1:3], torch.ones(4 * M, device=dev), gl)
+    junk = [torch.full((1 << 22,), 0x5a, dtype=torch.uint8, device=dev) for _ in range(8)]   # whatever was freed is in use now
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for g, st in zip(graphs, streams):
+            with torch.cuda.stream(st):
+                g.replay()
+        ops.grouped_matmul_swiglu_quant(*sets[0][1], gl)
+    torch.cuda.synchronize()
+    for (host, _), out in zip(sets, outs):
+        _check_swiglu_bits(oracle, host, np.cumsum(counts), *out)
+    assert all(bool((j == 0x5a).all()) for j in junk)
