@@ -17,7 +17,8 @@ ACL_FUNC_VISIBILITY int32_t gmmB200Version(void);
 /* The second-phase calls only enqueue work, so a device-side problem (a bounded wait that ran out) cannot be
  * returned by them.  This call waits for `stream`, copies the 4-word status record that the kernels keep at the
  * start of `workspace` and returns ACLNN_SUCCESS when it is clean, ACLNN_ERR_RUNTIME_ERROR otherwise.
- * record[0] = code (0 clean, 1 wait timed out, 2 bad scatter index), record[1] = CTA, record[2] = waiting role, record[3] = detail.
+ * record[0] = code (0 clean, 1 wait timed out, 2 bad scatter index, 3 a swiglu_quant group list that names the same rows over and
+ * over), record[1] = CTA, record[2] = waiting role, record[3] = detail.
  * `record` may be null.  Plays the role of the reference's aclrtSynchronizeStream + error query after
  * aclnnGroupedMatmulV4 (gmm/grouped_matmul/examples/test_aclnn_grouped_matmul.cpp:180-196). */
 ACL_FUNC_VISIBILITY aclnnStatus gmmB200CheckStatus(const void *workspace, uint64_t workspaceSize, aclrtStream stream,
@@ -205,8 +206,9 @@ ACL_FUNC_VISIBILITY aclnnStatus gmmB200GroupedMatmulSwigluQuant(const void *x, c
  * cudaMalloc / cudaFree imply.  The operator's scratch memory is a fixed array of
  * GMM_B200_NO_ALLOC_SCRATCH_BYTES inside the library image, which every GPU that loads the library keeps until the
  * process ends.  Same arguments and results as gmmB200GroupedMatmulSwigluQuant minus the workspace.
- *   - Limit: the scratch needed is 256 + 4*m + 8*(m/128 + 2*groupListLen + 2) + 4*m*(n/2) bytes, each part rounded up to 256; a larger problem is rejected
- *     with ACLNN_ERR_PARAM_INVALID and a message (e.g. at n = 4096, m = 4096 rows fit and m = 8192 do not).
+ *   - Limit: with b = ceil(m/128) + groupListLen the scratch needed is 256 + 4*m + 8*b + 4*(b*ceil(n/256) + 1) + 4*m*(n/2) bytes,
+ *     each part rounded up to 256 (the term with n/256 only up to b*ceil(n/256) = 262144); a larger problem is rejected with
+ *     ACLNN_ERR_PARAM_INVALID and a message (e.g. at n = 4096, m = 4096 rows fit and m = 8192 do not).
  *   - The first call on each device looks up the array's device address (once, with that device current); make that
  *     first call before any stream capture begins.
  *   - All calls share the one array and it keeps the previous call's contents; the part that must start at zero is

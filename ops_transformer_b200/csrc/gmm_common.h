@@ -24,7 +24,9 @@ enum : int { kPathSm100 = 0, kPathSimt = 1 };
 // Kernel status word (4 x int32 at the start of the workspace).  code 0 = clean.
 // kStatusBadIndex: a scattered result row named a GPU that is no peer or a row outside the result; the row was skipped
 // (record[1] = CTA, record[2] = 800, record[3] = the first such source row).
-enum : int { kStatusOk = 0, kStatusWaitTimeout = 1, kStatusBadIndex = 2 };
+// kStatusBadList: the group list of a swiglu_quant names the same rows so often that its tiles exceed the workspace's counters;
+// the tiles beyond were left out (record[2] = 810, record[3] = length of the list).
+enum : int { kStatusOk = 0, kStatusWaitTimeout = 1, kStatusBadIndex = 2, kStatusBadList = 3 };
 
 // Per-call launch options (the internal form of gmmB200LaunchOptions, include/gmm_b200.h).  They travel with the
 // problem description, so two threads launching on two streams never see each other's settings.
@@ -80,6 +82,7 @@ struct Plan {
     int ctas = 2;                       // 2 = CTA pairs (256 channels per tile), 1 = single CTAs (128 channels)
     size_t ws_bytes = 0;
     size_t off_status = 0, off_amax = 0, off_stage = 0, off_done = 0;
+    int64_t row_blocks = 0;             // row blocks that the counters at off_done cover (swiglu_quant)
     size_t off_wave = 0;                // 0 = no pacing counters in this workspace
     size_t zero_bytes = 0;              // leading bytes of the workspace cleared at launch
     alignas(64) CUtensorMap map_x[3];   // boxes of 32, 64 and 128 rows

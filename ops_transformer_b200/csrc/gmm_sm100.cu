@@ -187,6 +187,7 @@ struct KParams {
     int M, K, N;
     int half_n;        // N/2 (swiglu)
     int n_tiles;       // channel tiles per row block
+    int max_tiles;     // tiles that the workspace's row block counters cover (swiglu)
     int num_k_blocks;  // ceil(K / BK)
     const void *w_nz;     // FRACTAL_NZ weights, read by the loader warps
     const void *w_scale;
@@ -556,7 +557,10 @@ __device__ __forceinline__ int tile_tokens(int rows)
 
 // Row ranges follow GetSplitValueFromGroupList (gmm/grouped_matmul/op_kernel/grouped_matmul_utils.h:243-257):
 // type 0 = running total, type 1 = count, values narrowed to int32; groups with no rows are skipped
-// (grouped_matmul.h:263).  Ranges are clipped to [0, M] so a malformed list cannot address other memory.
+// (grouped_matmul.h:263).  Ranges are clipped to [0, M] so a malformed list cannot address other memory.  Disjoint ranges have
+// at most ceil(M / 128) + L row blocks; a falling running total names rows again and again and can have many times as many.  The
+// swiglu tiles beyond the counters reserved for that many are left out and reported (kStatusBadList): the counters behind them
+// are other data, and a slice claimed from such a word would be an arbitrary range of rows.
 template <int MAX_TOK>
 __device__ void build_schedule(Shared *sh, const KParams &p)
 {
@@ -621,7 +625,12 @@ __device__ void build_schedule(Shared *sh, const KParams &p)
         if (lane == 31) {
             sh->max_tok = max_tok;
             sh->tile_start[L] = incl;
-            sh->total_tiles = incl;
+            sh->total_tiles = min(incl, p.max_tiles);
+            if (incl > p.max_tiles && blockIdx.x == 0 && atomicCAS(p.status, kStatusOk, kStatusBadList) == kStatusOk) {
+                p.status[1] = 0;
+                p.status[2] = 810;
+                p.status[3] = L;
+            }
         }
     }
     __syncthreads();
@@ -1794,6 +1803,7 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     kp.half_n = (int)(p.N / 2);
     const int64_t tile_cols = p.mode == kModeSwigluQuant ? BC : BC * plan.ctas, cols = p.mode == kModeSwigluQuant ? p.N / 2 : p.N;
     kp.n_tiles = (int)((cols + tile_cols - 1) / tile_cols);
+    kp.max_tiles = p.mode == kModeSwigluQuant ? (int)(plan.row_blocks * kp.n_tiles < 0x7fffffffll ? plan.row_blocks * kp.n_tiles : 0x7fffffffll) : 0x7fffffff;
     kp.num_k_blocks = (int)((p.K + BK - 1) / BK);
     kp.w_nz = p.w;
     kp.w_scale = p.w_scale;

@@ -262,3 +262,36 @@ def test_captured_calls_own_their_workspace(oracle):
     for (host, _), out in zip(sets, outs):
         _check_swiglu_bits(oracle, host, np.cumsum(counts), *out)
     assert all(bool((j == 0x5a).all()) for j in junk)
+
+
+@pytest.mark.parametrize("ctas", ["1", "2"])
+def test_overlapping_group_ranges_stay_within_the_counters(oracle, monkeypatch, ctas):
+    """A running total that falls again names the same rows in many groups: 512 times 33 row blocks of 128 rows where the
+    counters are laid out for 33 and one per group.  The tiles beyond them are left out and reported, nothing outside the
+    call's own buffers is written, and the next call on the workspace is right."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    monkeypatch.setenv("GMM_B200_CTAS", ctas)
+    M, K, N, E = 4200, 16, 64, 1024
+    g = torch.Generator(device=dev)
+    g.manual_seed(3)
+    x = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=dev, generator=g)
+    w = torch.randint(-127, 128, (E, K, N), dtype=torch.int8, device=dev, generator=g)
+    ws, xs = torch.rand((E, N), device=dev, generator=g), torch.rand(M, device=dev, generator=g)
+    fence = 1 << 16
+    out = torch.full((2 * fence + M * N // 2,), 77, dtype=torch.int8, device=dev)
+    scale = torch.full((2 * fence + M,), 7.0, device=dev)
+    q, qs = out[fence:fence + M * N // 2].view(M, N // 2), scale[fence:fence + M]
+    falling = torch.tensor([M, 0] * (E // 2), dtype=torch.int64, device=dev)
+    _, _, wsb = ops.grouped_matmul_swiglu_quant(x, w, ws, xs, falling, output=q, output_scale=qs, return_workspace=True)
+    with pytest.raises(ops.AclnnError) as ei:
+        ops.check_status(wsb)
+    assert ei.value.record == (3, 0, 810, E)
+    for t, v in ((out, 77), (scale, 7.0)):
+        assert bool((t[:fence] == v).all()) and bool((t[-fence:] == v).all())
+    # lists at the bound: every group one partial row block
+    rising = torch.arange(1, E + 1, device=dev) * 4
+    rising[-1] = M
+    ops.grouped_matmul_swiglu_quant(x, w, ws, xs, rising, output=q, output_scale=qs, workspace=wsb)
+    ops.check_status(wsb)
+    _check_swiglu_bits(oracle, [t.cpu().numpy() for t in (x, w, ws, xs)], rising.cpu().numpy(), q, qs)
