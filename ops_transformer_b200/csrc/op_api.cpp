@@ -1107,6 +1107,7 @@ struct WordReader {
         if (p == end) { ok = false; return 0; }
         return *p++;
     }
+    bool all_read() const { return ok && p == end; }   // a description with words left over is another operator's
 };
 
 // One tensor: rank (-1: absent), data, dtype, format, dims, strides, storage rank, storage dims.
@@ -1182,7 +1183,7 @@ aclnnStatus plan_packed(int32_t op, WordReader &r, uint64_t *size, aclOpExecutor
             x.read(r); w.read(r); bias.read(r); scale.read(r); pts.read(r); gl.read(r); y.read(r);
             const int64_t split = r.next(), group_type = r.next(), gl_type = r.next(), act = r.next(), qgroup = r.next();
             tuning.read(r);
-            if (!r.ok) return malformed();
+            if (!r.all_read()) return malformed();
             aclTensorList *py = y.tensor.present ? &y.list : nullptr;
             if (op == GMM_B200_OP_GMM_V4) {
                 *run = aclnnGroupedMatmulV4;
@@ -1204,7 +1205,7 @@ aclnnStatus plan_packed(int32_t op, WordReader &r, uint64_t *size, aclOpExecutor
         case GMM_B200_OP_SWIGLU_QUANT: case GMM_B200_OP_SWIGLU_QUANT_WEIGHT_NZ: {
             PackedTensor x, w, bias, offset, ws, xs, gl, q, qs;
             for (PackedTensor *t : {&x, &w, &bias, &offset, &ws, &xs, &gl, &q, &qs}) t->read(r);
-            if (!r.ok) return malformed();
+            if (!r.all_read()) return malformed();
             if (op == GMM_B200_OP_SWIGLU_QUANT) {
                 *run = aclnnGroupedMatmulSwigluQuant;
                 return aclnnGroupedMatmulSwigluQuantGetWorkspaceSize(x.get(), w.get(), bias.get(), offset.get(), ws.get(), xs.get(), gl.get(),
@@ -1221,7 +1222,7 @@ aclnnStatus plan_packed(int32_t op, WordReader &r, uint64_t *size, aclOpExecutor
             const int64_t offset = r.next(), gl_type = r.next();
             PackedInts tuning;
             tuning.read(r);
-            if (!r.ok) return malformed();
+            if (!r.all_read()) return malformed();
             if (op == GMM_B200_OP_FINALIZE_ROUTING) {
                 *run = aclnnGroupedMatmulFinalizeRoutingWeightNz;
                 return aclnnGroupedMatmulFinalizeRoutingWeightNzGetWorkspaceSize(x.get(), w.get(), scale.get(), bias.get(), pts.get(), gl.get(),
@@ -1242,7 +1243,7 @@ aclnnStatus plan_packed(int32_t op, WordReader &r, uint64_t *size, aclOpExecutor
             const int64_t quant = r.next(), row_type = r.next();
             PackedInts range;
             range.read(r);
-            if (!r.ok) return malformed();
+            if (!r.all_read()) return malformed();
             *run = aclnnMoeInitRoutingV3;
             return aclnnMoeInitRoutingV3GetWorkspaceSize(x.get(), idx.get(), scale.get(), offset.get(), active, capacity, experts, drop_pad,
                                                          num_type, num_flag, quant, range.get(), row_type, ex_out.get(), row_idx.get(),

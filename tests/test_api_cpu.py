@@ -527,35 +527,104 @@ def _packed_call(L, op, words, workspace=None, nbytes=0):
     return rc, res
 
 
-def test_packed_call_plans_like_the_separate_handles(gmm_lib):
+def _packed_operators():
+    """Every operator of gmmB200Call: (name, op, words, first phase through separate handles as a function of the two outputs).
+    The weights of the row-major operators are a strided view."""
     torch = pytest.importorskip("torch")
     from ops_transformer_b200 import acl
-    L = gmm_lib
-    M, K, N, E = 96, 64, 128, 3
-    x, w = torch.zeros(M, K, dtype=torch.int8), torch.zeros(E, N, K, dtype=torch.int8).transpose(1, 2)   # a strided view
+    L = _lib.lib()
+    M, K, N, E, T = 96, 64, 128, 3, 24
+    x, w = torch.zeros(M, K, dtype=torch.int8), torch.zeros(E, N, K, dtype=torch.int8).transpose(1, 2)
+    nz = torch.zeros(E, N // 32, K // 16, 16, 32, dtype=torch.int8)
     ws, xs, gl = torch.ones(E, N), torch.ones(M), torch.full((E,), 32, dtype=torch.int64)
-    q, qs = torch.zeros(M, N // 2, dtype=torch.int8), torch.zeros(M)
-    words = []
-    for t in (x, w, None, None, ws, xs, gl, q, qs):
-        acl._put(words, t)
-    hs = [acl.create_tensor(t) for t in (x, w, ws, xs, gl, q, qs)]
-    size, ex = C.c_uint64(0), C.c_void_p(0)
-    want = L.aclnnGroupedMatmulSwigluQuantGetWorkspaceSize(hs[0], hs[1], None, None, *hs[2:], None, C.byref(size), C.byref(ex))
-    rc, res = _packed_call(L, _lib.OP_SWIGLU_QUANT[""], words)
-    assert (rc, res.workspaceSize) == (want, size.value)
-    if rc == 0:   # no workspace given: planned, not run; the executor is live and can be destroyed once
-        assert res.stage == _lib.STAGE_PLANNED
+    q, qs, y = torch.zeros(M, N // 2, dtype=torch.int8), torch.zeros(M), torch.zeros(M, N, dtype=torch.bfloat16)
+    row, logit = torch.arange(M) // 4, torch.ones(M)
+    tokens, idx = torch.zeros(T, K, dtype=torch.bfloat16), torch.zeros(T, 4, dtype=torch.int32)
+    rows, row_idx, counts = torch.zeros(T * 4, K, dtype=torch.int8), torch.zeros(T * 4, dtype=torch.int32), torch.zeros(E, dtype=torch.int64)
+    row_scale = torch.zeros(T * 4)
+    NZ = _lib.ACL_FORMAT_FRACTAL_NZ
+
+    def pack(tensors, nz_at=None, tail=()):
+        words = []
+        for i, t in enumerate(tensors):
+            acl._put(words, t, NZ if i == nz_at else _lib.ACL_FORMAT_ND)
+        return words + list(tail)
+
+    h = lambda t, fmt=_lib.ACL_FORMAT_ND: acl.create_tensor(t, fmt)  # noqa: E731
+    hl = lambda t, fmt=_lib.ACL_FORMAT_ND: acl.create_tensor_list([t], fmt)  # noqa: E731
+    ints = lambda v: L.aclCreateIntArray(acl._i64(v), len(v))  # noqa: E731
+    weight = C.c_float(0.5)
+    bits = int.from_bytes(bytes(weight), "little")
+    for api, op in _lib.OP_GMM.items():
+        weights, at, tuning = (nz, 1, [16]) if api == "WeightNz" else (w, None, None if api == "V4" else [16])
+        words = pack((x, weights, None, ws, xs, gl, y), at, [2, 0, 1, 0, 0] + ([-1] if tuning is None else [1, 16]))
+
+        def gmm(size, ex, api=api, weights=weights, at=at, tuning=tuning):
+            head = (hl(x), hl(weights, NZ if at else _lib.ACL_FORMAT_ND), None, hl(ws), None, None, None, hl(xs), h(gl), None, None, None, 2, 0, 1, 0)
+            mid = {"V4": (), "V5": (ints([16]),), "WeightNz": (ints([16]), 0)}[api]
+            return getattr(L, f"aclnnGroupedMatmul{api}GetWorkspaceSize")(*head, *mid, hl(y), None, None, size, ex)
+        yield "aclnnGroupedMatmul" + api, op, words, gmm
+    for api, op in _lib.OP_SWIGLU_QUANT.items():
+        weights, at = (nz, 1) if api else (w, None)
+
+        def swiglu(size, ex, api=api, weights=weights):
+            return getattr(L, f"aclnnGroupedMatmulSwigluQuant{api}GetWorkspaceSize")(
+                h(x), h(weights, NZ if api else _lib.ACL_FORMAT_ND), None, None, h(ws), h(xs), h(gl), h(q), h(qs), None, size, ex)
+        yield "aclnnGroupedMatmulSwigluQuant" + api, op, pack((x, weights, None, None, ws, xs, gl, q, qs), at), swiglu
+    big = dict(x=x, w=torch.zeros(E, 8, K // 16, 16, 32, dtype=torch.int8), s=torch.ones(E, 256), y=torch.zeros(T, 256),
+               sh=torch.zeros(T, 256, dtype=torch.bfloat16))
+    for api, op in _lib.OP_FINALIZE_ROUTING.items():
+        words = pack((x, big["w"], big["s"], None, xs, gl, big["sh"], logit, row, big["y"]), 1, [bits, 0, 1] + ([1, 16] if api else [-1]))
+
+        def finalize(size, ex, api=api):
+            a = (h(x), h(big["w"], NZ), h(big["s"]), None)
+            b = (h(xs), h(gl), h(big["sh"]), h(logit), h(row), 0, 0.5, 0, False, False, 1)
+            if api:
+                return L.aclnnGroupedMatmulFinalizeRoutingWeightNzV2GetWorkspaceSize(*a, None, None, None, *b, ints([16]), h(big["y"]), size, ex)
+            return L.aclnnGroupedMatmulFinalizeRoutingWeightNzGetWorkspaceSize(*a, *b, h(big["y"]), size, ex)
+        yield "aclnnGroupedMatmulFinalizeRoutingWeightNz" + api, op, words, finalize
+
+    def routing(size, ex):
+        return L.aclnnMoeInitRoutingV3GetWorkspaceSize(h(tokens), h(idx), None, None, T * 4, 0, E, 0, 1, True, 1, ints([0, E]), 1, h(rows),
+                                                       h(row_idx), h(counts), h(row_scale), size, ex)
+    yield ("aclnnMoeInitRoutingV3", _lib.OP_MOE_INIT_ROUTING,
+           pack((tokens, idx, None, None, rows, row_idx, counts, row_scale), None, [T * 4, 0, E, 0, 1, 1, 1, 1, 2, 0, E]), routing)
+
+
+def test_packed_call_plans_like_the_separate_handles(gmm_lib):
+    L = gmm_lib
+    seen = set()
+    for name, op, words, phase1 in _packed_operators():
+        size, ex = C.c_uint64(0), C.c_void_p(0)
+        assert phase1(C.byref(size), C.byref(ex)) == 0, (name, _lib.last_error())
+        rc, res = _packed_call(L, op, words)
+        # no workspace given: planned, not run; the executor is live, is the operator's own and can be destroyed once
+        assert (rc, res.workspaceSize, res.stage) == (0, size.value, _lib.STAGE_PLANNED), (name, _lib.last_error())
+        assert size.value > 0
+        wrong = "aclnnMoeInitRoutingV3" if name != "aclnnMoeInitRoutingV3" else "aclnnGroupedMatmulV4"
+        assert getattr(L, wrong)(None, 0, ex, None) == _lib.ACLNN_ERR_PARAM_INVALID and name in _lib.last_error()
         assert L.aclDestroyAclOpExecutor(C.c_void_p(res.executor)) == 0
         assert L.aclDestroyAclOpExecutor(C.c_void_p(res.executor)) != 0
-        L.aclDestroyAclOpExecutor(ex)
-    for h in hs:
-        L.aclDestroyTensor(h)
-    # an invalid call reports what the operator's first phase reports
-    bad = []
-    for t in (x, w, None, None, ws, xs, gl.to(torch.int32), q, qs):
-        acl._put(bad, t)
-    rc, res = _packed_call(L, _lib.OP_SWIGLU_QUANT[""], bad)
+        # one word more or less is no description of this operator
+        for bad in (words + [0], words[:-1]):
+            rc, res = _packed_call(L, op, bad)
+            assert rc == _lib.ACLNN_ERR_PARAM_INVALID and res.stage == _lib.STAGE_PLAN and not res.executor, name
+            assert "malformed" in _lib.last_error(), name
+        seen.add(op)
+    assert seen == set(range(8))
+
+
+def test_packed_call_reports_what_the_first_phase_reports(gmm_lib):
+    torch = pytest.importorskip("torch")
+    from ops_transformer_b200 import acl
+    M, K, N, E = 96, 64, 128, 3
+    words = []
+    for t in (torch.zeros(M, K, dtype=torch.int8), torch.zeros(E, K, N, dtype=torch.int8), None, None, torch.ones(E, N), torch.ones(M),
+              torch.full((E,), 32, dtype=torch.int32), torch.zeros(M, N // 2, dtype=torch.int8), torch.zeros(M)):
+        acl._put(words, t)
+    rc, res = _packed_call(gmm_lib, _lib.OP_SWIGLU_QUANT[""], words)
     assert rc == _lib.ACLNN_ERR_PARAM_INVALID and res.stage == _lib.STAGE_PLAN and not res.executor
+    assert "malformed" not in _lib.last_error()
 
 
 @pytest.mark.parametrize("words", [[], [2, 0, 2, 2, 4], [9], [1, 0, 2, 2, 4, 1, 12]])
