@@ -16,7 +16,8 @@
 //             (__match_any_sync ranks the lanes of a warp; the warps are ranked through a per-warp counter table, or take
 //             turns when the active range is too wide for one), which keeps the order of equal keys
 //   gather  - one CTA per token: the row is read once into registers, (quantised,) and stored at the output row of each
-//             of its k pairs; shapes that do not fit the register tile take one CTA per output row
+//             of its k pairs; few tokens with smooth scales, and few pairs without, take one CTA per pair; shapes that do not
+//             fit the register tile one CTA per output row
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -658,11 +659,15 @@ cudaError_t init_routing_launch(const InitRoutingProblem &r, void *workspace, si
     if (r.quant) {
         // token-major kernels hold 32 values per thread (256 threads): h <= 8192, and h a multiple of 16 for the 16-byte stores
         const bool fast = aligned && r.h % 16 == 0 && r.h <= 8192 && r.n <= 0x7fffffffll;
-        // Fewer tokens than SMs: one CTA per pair.  A CTA's k pairs are a serial chain, with a smooth scale of two passes over
-        // that expert's scales and a block reduction each; with more tokens than SMs the chains run side by side and the row is
-        // better read once.  128 fp16 tokens, 8 of 256 experts, 64 of them active, h = 7168, smooth scales: 23.2 us a call with
-        // one CTA per token and the count kernel, 19.8 us with one per pair and without it.
-        p.slots = r.n < 148 ? 1 : (int)r.k;
+        // One CTA per token reads the row once and stores it k times; one CTA per pair takes the k stores apart.  With a smooth
+        // scale a CTA's pairs are a serial chain, each two passes over that expert's scales and a block reduction: pairs of
+        // their own until the tokens alone give every SM a chain.  Without one a pair is a 16-byte store per thread, and k CTAs
+        // repeat the row's quantisation for it: only while they find an SM each.  h = 7168, 64 of 256 experts active, us a call
+        // (per token / per pair), bf16, k = 8: with smooth scales 23.1 / 12.2 at 147 tokens; without 4.6 / 4.2 at 16 tokens (128
+        // pairs), 4.8 / 6.4 at 64, 6.5 / 11.1 at 147; k = 2 without 4.2 / 4.2 at 64 tokens, 4.3 / 4.6 at 96.
+        const int sms = device_sm_count();
+        if (sms <= 0) return cudaErrorNoDevice;
+        p.slots = (r.scale ? r.n < sms : pairs <= sms) ? 1 : (int)r.k;
         const unsigned gather_grid = (unsigned)(p.slots == 1 ? pairs : r.n);
         if (r.x_dtype == kF32) {
             if (fast) launch_err = launch_pdl(routing_quant_token_kernel<float, 8, 256>, gather_grid, 256, 0, stream, overlap, p);

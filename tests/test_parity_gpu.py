@@ -754,7 +754,8 @@ def test_init_routing_many_blocks_keep_pair_order(oracle):
     (1, 1, 4, (0, 4)), (128, 8, 64, (0, 64)), (128, 8, 256, (64, 128)),    # all pairs in one block (1024): no count kernel
     (128, 8, 300, (10, 267)),                                              # 257 active experts: too wide for the per-warp table
     (129, 8, 64, (0, 64)),                                                 # one pair block more
-    (147, 6, 32, (8, 24)), (148, 6, 32, (8, 24)),                          # one CTA per pair / one CTA per token
+    (147, 6, 32, (8, 24)), (148, 6, 32, (8, 24)),                          # smooth: one CTA per pair / one CTA per token
+    (37, 4, 32, (8, 24)), (149, 1, 32, (8, 24)), (30, 5, 32, (0, 32)),     # not smooth: the same at 148, 149 and 150 pairs
 ])
 @pytest.mark.parametrize("smooth", [False, True])
 def test_init_routing_launch_shape_edges(oracle, n, k, E, rng, smooth):
