@@ -51,6 +51,10 @@ typedef struct gmmB200LaunchOptions {
 } gmmB200LaunchOptions;
 ACL_FUNC_VISIBILITY aclnnStatus gmmB200SetExecutorOptions(aclOpExecutor *executor, const gmmB200LaunchOptions *options);
 
+/* 1 if `stream` is being captured into a graph (or that cannot be asked), 0 if not: a pool that outlives the call must not lend
+ * its buffers to a capture, whose replays would use them whenever they run. */
+ACL_FUNC_VISIBILITY int32_t gmmB200StreamIsCapturing(aclrtStream stream);
+
 /* Both phases of one operator in one call, from a packed description, for bindings in which every C call and every handle
  * costs more than the work behind it (a Python call through separate handles spends 45 us, most of it in some twenty ctypes
  * calls).  Validation, status codes and messages are those of the operator's own GetWorkspaceSize and second-phase calls,
@@ -69,13 +73,14 @@ ACL_FUNC_VISIBILITY aclnnStatus gmmB200SetExecutorOptions(aclOpExecutor *executo
  *   MOE_INIT_ROUTING_V3: x, expertIdx, scale, offset, expandedX, expandedRowIdx, expertTokensCountOrCumsum, expandedScale;
  *              activeNum, expertCapacity, expertNum, dropPadMode, expertTokensNumType, expertTokensNumFlag, quantMode,
  *              rowIdxType, activeExpertRange array
- * If the workspace is too small the first phase's executor comes back (stage PLANNED): the caller allocates
- * result->workspaceSize bytes and makes the operator's second-phase call, or destroys the executor.  Otherwise stage says
+ * If the workspace is too small, or a pooled one and the stream is being captured, the first phase's executor comes back (stage
+ * PLANNED): the caller allocates result->workspaceSize bytes and makes the operator's second-phase call, or destroys the executor.  Otherwise stage says
  * how far the call came when its status is not ACLNN_SUCCESS. */
 enum {
     GMM_B200_OP_GMM_V4 = 0, GMM_B200_OP_GMM_V5 = 1, GMM_B200_OP_GMM_WEIGHT_NZ = 2, GMM_B200_OP_SWIGLU_QUANT = 3,
     GMM_B200_OP_SWIGLU_QUANT_WEIGHT_NZ = 4, GMM_B200_OP_FINALIZE_ROUTING = 5, GMM_B200_OP_FINALIZE_ROUTING_V2 = 6,
-    GMM_B200_OP_MOE_INIT_ROUTING_V3 = 7
+    GMM_B200_OP_MOE_INIT_ROUTING_V3 = 7,
+    GMM_B200_OP_POOLED = 0x100   /* added to the operator: `workspace` comes from a pool and is not used if `stream` is being captured */
 };
 enum { GMM_B200_STAGE_PLAN = 0, GMM_B200_STAGE_OPTIONS = 1, GMM_B200_STAGE_PLANNED = 2, GMM_B200_STAGE_RUN = 3 };
 typedef struct gmmB200CallResult {

@@ -33,7 +33,7 @@ EXPORTED_SYMBOLS = [
     "aclnnMoeInitRoutingV3GetWorkspaceSize", "aclnnMoeInitRoutingV3",
     "aclnnGroupedMatmulSwigluQuantGetWorkspaceSize", "aclnnGroupedMatmulSwigluQuant",
     "aclnnGroupedMatmulSwigluQuantWeightNZGetWorkspaceSize", "aclnnGroupedMatmulSwigluQuantWeightNZ",
-    "gmmB200Version", "gmmB200CheckStatus", "gmmB200SetExecutorOptions", "gmmB200Call", "gmmB200GroupedMatmulW8A8WorkspaceSize", "gmmB200GroupedMatmulW8A8",
+    "gmmB200Version", "gmmB200CheckStatus", "gmmB200SetExecutorOptions", "gmmB200Call", "gmmB200StreamIsCapturing", "gmmB200GroupedMatmulW8A8WorkspaceSize", "gmmB200GroupedMatmulW8A8",
     "gmmB200GroupedMatmulSwigluQuantWorkspaceSize", "gmmB200GroupedMatmulSwigluQuant",
     "gmmB200NoAllocScratchBytes", "gmmB200GroupedMatmulSwigluQuantNoAlloc", "gmmB200NoAllocCheckStatus",
     "gmmB200PeerAlloc", "gmmB200PeerFree", "gmmB200PeerExport", "gmmB200PeerImport", "gmmB200PeerRelease", "gmmB200EpDispatch", "gmmB200EpCount", "gmmB200EpRoute", "gmmB200EpInverseMap", "gmmB200EpCombine",
@@ -55,6 +55,7 @@ class CallResult(C.Structure):
 
 
 OP_GMM, OP_SWIGLU_QUANT, OP_FINALIZE_ROUTING, OP_MOE_INIT_ROUTING = {"V4": 0, "V5": 1, "WeightNz": 2}, {"": 3, "WeightNZ": 4}, {"": 5, "V2": 6}, 7
+OP_POOLED = 0x100
 STAGE_PLAN, STAGE_OPTIONS, STAGE_PLANNED, STAGE_RUN = range(4)
 
 
@@ -102,6 +103,7 @@ def _load():
     L.aclnnGroupedMatmulSwigluQuant.argtypes = [p, u64, p, p]
     L.gmmB200CheckStatus.argtypes = [p, u64, p, C.POINTER(i32)]
     L.gmmB200SetExecutorOptions.argtypes = [p, po]
+    L.gmmB200StreamIsCapturing.argtypes = [p]
     L.gmmB200Call.argtypes = [i32, p, u64, p, u64, po, p, C.POINTER(CallResult)]
     L.gmmB200GroupedMatmulW8A8WorkspaceSize.argtypes = [i64, i64, i64, i64, i32, C.POINTER(u64)]
     L.gmmB200GroupedMatmulW8A8.argtypes = [p, p, p, i32, p, p, i32, p, i64, i32, i64, i64, i64, i64, i32, i32, p, p, i32, i64, p, i32, p, u64, p, po]

@@ -113,6 +113,10 @@ class _Workspace:
                     del self._slots[next(iter(self._slots))]
         return s
 
+    def lend(self, slot: _Slot, device: torch.device, stream, nbytes: int) -> torch.Tensor:
+        """A workspace of at least ``nbytes`` for the call that is about to be enqueued with the slot's lock held."""
+        return (self.for_capture if device.type == "cuda" and _capturing(stream) else self.grown)(slot, device, stream, nbytes)
+
     @staticmethod
     def grown(slot: _Slot, device: torch.device, stream, nbytes: int) -> torch.Tensor:
         """The slot's buffer with room for ``nbytes``."""
@@ -147,13 +151,10 @@ def _on_stream(stream, device: torch.device):
     return torch.cuda.stream(stream)
 
 
-def _capturing(stream, device: torch.device) -> bool:
-    if device.type != "cuda":
-        return False
-    if stream is None or int(stream.cuda_stream) == int(torch.cuda.current_stream().cuda_stream):
+def _capturing(stream) -> bool:
+    if stream is None:
         return torch.cuda.is_current_stream_capturing()
-    with _on_stream(stream, device):
-        return torch.cuda.is_current_stream_capturing()
+    return _lib.lib().gmmB200StreamIsCapturing(int(stream.cuda_stream)) != 0
 
 
 def _in_graph_pool(t: torch.Tensor) -> bool:
@@ -162,18 +163,24 @@ def _in_graph_pool(t: torch.Tensor) -> bool:
                if seg["address"] <= p < seg["address"] + seg["total_size"])
 
 
-@contextlib.contextmanager
-def _pooled(device: torch.device, stream, nbytes: int):
-    """A workspace of ``nbytes`` for a call on ``stream`` that is enqueued inside the context."""
-    slot = _WS.slot(device, _stream_handle(stream) if device.type == "cuda" else 0)
+def _with_pooled(device: torch.device, stream, handle: int, nbytes: int, call):
+    """``call(workspace)``, which enqueues on ``stream``, with a pooled workspace of ``nbytes``; returns the workspace."""
+    slot = _WS.slot(device, handle)
     with slot.lock:
-        yield (_WS.for_capture if _capturing(stream, device) else _WS.grown)(slot, device, stream, nbytes)
+        workspace = _WS.lend(slot, device, stream, nbytes)
+        call(workspace)
+        return workspace
 
 
 def _stream_handle(stream) -> int:
     if stream is None:
         stream = torch.cuda.current_stream()
     return int(stream.cuda_stream)
+
+
+def _gpu_stream_handle(stream) -> int:
+    """The same where CUDA is known to be up, without the stream object that torch.cuda.current_stream builds."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()) if stream is None else int(stream.cuda_stream)
 
 
 def check_status(workspace: Optional[torch.Tensor], stream=None) -> None:
@@ -223,26 +230,24 @@ def _put_ints(words: list, values: Optional[Sequence[int]]) -> None:
 def _call(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream,
           options: Optional[LaunchOptions]) -> Optional[torch.Tensor]:
     """Both phases of operator ``name`` on the packed description; returns the workspace that was used (None if none)."""
+    on_gpu = device.type == "cuda"
+    handle = _gpu_stream_handle(stream) if on_gpu else 0
     if workspace is not None:
-        return _enqueue(op, name, words, device, workspace, stream, options, None)
-    slot = _WS.slot(device, _stream_handle(stream) if device.type == "cuda" else 0)
+        return _enqueue(op, name, words, device, workspace, stream, handle, options, None)
+    slot = _WS.slot(device, handle)
     with slot.lock:
-        return _enqueue(op, name, words, device, None, stream, options, slot)
+        return _enqueue(op, name, words, device, None, stream, handle, options, slot)
 
 
-def _enqueue(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream,
+def _enqueue(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream, handle: int,
              options: Optional[LaunchOptions], slot: Optional[_Slot]) -> Optional[torch.Tensor]:
     L = _lib.lib()
     packed = array.array("q", words)
     res = _lib.CallResult()
     # validation needs no device: tensors that are not on one are planned only, so that what is wrong with them is reported first
     on_gpu = device.type == "cuda"
-    capturing = slot is not None and _capturing(stream, device)
-    buf = workspace if workspace is not None else slot.buf
-    if not on_gpu or capturing:
-        buf = None
-    handle = _stream_handle(stream) if on_gpu else 0
-    rc = L.gmmB200Call(op, packed.buffer_info()[0], len(packed), buf.data_ptr() if buf is not None else None,
+    buf = None if not on_gpu else workspace if slot is None else slot.buf
+    rc = L.gmmB200Call(op if slot is None else op | _lib.OP_POOLED, packed.buffer_info()[0], len(packed), buf.data_ptr() if buf is not None else None,
                        buf.numel() if buf is not None else 0, C.byref(options) if options is not None else None, handle, C.byref(res))
     if rc == ACLNN_SUCCESS and res.stage == _lib.STAGE_PLANNED:
         ex = C.c_void_p(res.executor)
@@ -250,16 +255,17 @@ def _enqueue(op: int, name: str, words: list, device: torch.device, workspace: O
             L.aclDestroyAclOpExecutor(ex)
             raise ValueError(f"workspace of {workspace.numel()} bytes is smaller than the {res.workspaceSize} required")
         try:
-            buf = workspace if workspace is not None else (_WS.for_capture if capturing else _WS.grown)(slot, device, stream, res.workspaceSize)
+            buf = workspace if slot is None else _WS.lend(slot, device, stream, res.workspaceSize)
+            handle = handle if on_gpu else _stream_handle(stream)
         except Exception:
             L.aclDestroyAclOpExecutor(ex)
             raise
-        rc = getattr(L, name)(buf.data_ptr(), res.workspaceSize, ex, _stream_handle(stream))
+        rc = getattr(L, name)(buf.data_ptr(), res.workspaceSize, ex, handle)
         res.stage = _lib.STAGE_RUN
     if rc != ACLNN_SUCCESS:
         raise AclnnError(rc, name + ("GetWorkspaceSize" if res.stage == _lib.STAGE_PLAN else
                                      ": gmmB200SetExecutorOptions" if res.stage == _lib.STAGE_OPTIONS else ""))
-    return workspace if workspace is not None else buf if res.workspaceSize else None
+    return workspace if slot is None else buf if res.workspaceSize else None
 
 
 def grouped_matmul_v4(x: torch.Tensor, weight: torch.Tensor, scale: Optional[torch.Tensor],
@@ -325,17 +331,21 @@ def _grouped_matmul_flat(x, weight, scale, per_token_scale, group_list, bias, gr
     rc = L.gmmB200GroupedMatmulW8A8WorkspaceSize(M, K, N, E, ydt, C.byref(size))
     if rc != ACLNN_SUCCESS:
         raise AclnnError(rc, "gmmB200GroupedMatmulW8A8WorkspaceSize")
-    if workspace is None:
-        with _pooled(x.device, stream, size.value) as pooled:
-            return _grouped_matmul_flat(x, weight, scale, per_token_scale, group_list, bias, group_list_type, act_type, out, out_row_index,
-                                        stream, pooled, return_workspace, out_peers, nz, options, out_rows)
     p = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
-    rc = L.gmmB200GroupedMatmulW8A8(p(x), p(weight), p(scale), _DTYPES[scale.dtype] if scale is not None else 0, p(per_token_scale),
-                                    p(bias), _DTYPES[bias.dtype] if bias is not None else 0, p(group_list), group_list.numel(),
-                                    group_list_type, M, K, N, E, trans, act_type, p(out_row_index), peers if n_peers else None, n_peers, out_rows, p(out), ydt, p(workspace),
-                                    workspace.numel(), C.c_void_p(_stream_handle(stream)), C.byref(options) if options is not None else None)
-    if rc != ACLNN_SUCCESS:
-        raise AclnnError(rc, "gmmB200GroupedMatmulW8A8")
+    handle = _gpu_stream_handle(stream) if x.device.type == "cuda" else _stream_handle(stream)
+
+    def enqueue(workspace):
+        rc = L.gmmB200GroupedMatmulW8A8(p(x), p(weight), p(scale), _DTYPES[scale.dtype] if scale is not None else 0, p(per_token_scale),
+                                        p(bias), _DTYPES[bias.dtype] if bias is not None else 0, p(group_list), group_list.numel(),
+                                        group_list_type, M, K, N, E, trans, act_type, p(out_row_index), peers if n_peers else None, n_peers, out_rows,
+                                        p(out), ydt, p(workspace), workspace.numel(), handle,
+                                        C.byref(options) if options is not None else None)
+        if rc != ACLNN_SUCCESS:
+            raise AclnnError(rc, "gmmB200GroupedMatmulW8A8")
+    if workspace is None:
+        workspace = _with_pooled(x.device, stream, handle, size.value, enqueue)
+    else:
+        enqueue(workspace)
     return (out, workspace) if return_workspace else out
 
 
@@ -405,21 +415,22 @@ def grouped_matmul_finalize_routing_flat(x, weight, weight_layout, scale, group_
         E, N = weight.shape[0], weight.shape[1] * 32
     else:
         E, _, N = weight.shape
-    if workspace is None:
-        with _pooled(x.device, stream, 256) as pooled:
-            return grouped_matmul_finalize_routing_flat(
-                x, weight, weight_layout, scale, group_list, row_index, out, bias=bias, pertoken_scale=pertoken_scale,
-                shared_input=shared_input, logit=logit, shared_input_weight=shared_input_weight, shared_input_offset=shared_input_offset,
-                group_list_type=group_list_type, stream=stream, workspace=pooled, options=options)
     p = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
-    rc = L.gmmB200GroupedMatmulFinalizeRouting(
-        p(x), p(weight), weight_layout, p(scale), _DTYPES[scale.dtype], p(bias), p(pertoken_scale), p(group_list),
-        group_list.numel(), group_list_type, p(shared_input), 0 if shared_input is None else shared_input.shape[0],
-        shared_input_offset, shared_input_weight, p(logit), p(row_index), _DTYPES[row_index.dtype], M, K, N, E, p(out),
-        out.shape[0], p(workspace), workspace.numel(), C.c_void_p(_stream_handle(stream)),
-        C.byref(options) if options is not None else None)
-    if rc != ACLNN_SUCCESS:
-        raise AclnnError(rc, "gmmB200GroupedMatmulFinalizeRouting")
+    handle = _gpu_stream_handle(stream) if x.device.type == "cuda" else _stream_handle(stream)
+
+    def enqueue(workspace):
+        rc = L.gmmB200GroupedMatmulFinalizeRouting(
+            p(x), p(weight), weight_layout, p(scale), _DTYPES[scale.dtype], p(bias), p(pertoken_scale), p(group_list),
+            group_list.numel(), group_list_type, p(shared_input), 0 if shared_input is None else shared_input.shape[0],
+            shared_input_offset, shared_input_weight, p(logit), p(row_index), _DTYPES[row_index.dtype], M, K, N, E, p(out),
+            out.shape[0], p(workspace), workspace.numel(), handle,
+            C.byref(options) if options is not None else None)
+        if rc != ACLNN_SUCCESS:
+            raise AclnnError(rc, "gmmB200GroupedMatmulFinalizeRouting")
+    if workspace is None:
+        _with_pooled(x.device, stream, handle, 256, enqueue)
+    else:
+        enqueue(workspace)
     return out
 
 

@@ -1093,6 +1093,16 @@ aclnnStatus gmmB200GroupedMatmulFinalizeRouting(const void *x, const void *weigh
     return ACLNN_SUCCESS;
 }
 
+int32_t gmmB200StreamIsCapturing(aclrtStream stream)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &st) != cudaSuccess) {
+        cudaGetLastError();  // the legacy default stream, while another thread captures in global mode
+        return 1;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Both phases of one operator from a packed description (include/gmm_b200.h)
 // ---------------------------------------------------------------------------------------------------------
@@ -1267,7 +1277,7 @@ aclnnStatus gmmB200Call(int32_t op, const int64_t *words, uint64_t count, void *
     uint64_t need = 0;
     aclOpExecutor *ex = nullptr;
     RunFn run = nullptr;
-    aclnnStatus rc = plan_packed(op, r, &need, &ex, &run);
+    aclnnStatus rc = plan_packed(op & ~GMM_B200_OP_POOLED, r, &need, &ex, &run);
     if (rc != ACLNN_SUCCESS) return rc;
     result->workspaceSize = need;
     if (options) {
@@ -1278,7 +1288,7 @@ aclnnStatus gmmB200Call(int32_t op, const int64_t *words, uint64_t count, void *
             return rc;
         }
     }
-    if (need > workspaceBytes) {  // the caller finds more and runs the second phase itself
+    if (need > workspaceBytes || (need && (op & GMM_B200_OP_POOLED) && gmmB200StreamIsCapturing(stream))) {  // the caller finds more and runs the second phase itself
         result->stage = GMM_B200_STAGE_PLANNED;
         result->executor = ex;
         return ACLNN_SUCCESS;

@@ -658,12 +658,16 @@ def recorded_calls(monkeypatch):
                 rec.overlapped |= rec.inside > 1
             time.sleep(0.002)
             res = result._obj
-            res.workspaceSize, res.stage = rec.need, _lib.STAGE_RUN if ws and nbytes >= rec.need else _lib.STAGE_PLANNED
+            held_back = rec.capturing and op & 0x100   # a pooled workspace is not used under capture
+            res.workspaceSize, res.stage = rec.need, _lib.STAGE_RUN if ws and nbytes >= rec.need and not held_back else _lib.STAGE_PLANNED
             if res.stage == _lib.STAGE_RUN:
                 rec.calls.append((ws, stream))
             with lock:
                 rec.inside -= 1
             return 0
+
+        def gmmB200StreamIsCapturing(self, handle):
+            return int(rec.capturing)
 
         def anOperator(self, ws, nbytes, executor, stream):
             rec.calls.append((ws, stream))
@@ -678,9 +682,10 @@ def recorded_calls(monkeypatch):
     fake_torch = types.SimpleNamespace(
         empty=empty, uint8=torch.uint8, Tensor=torch.Tensor,
         cuda=types.SimpleNamespace(Stream=types.SimpleNamespace, stream=lambda s: contextlib.nullcontext(),
-                                   current_stream=lambda: types.SimpleNamespace(cuda_stream=7),
+                                   current_stream=lambda: types.SimpleNamespace(cuda_stream=7),   # if the handle is asked for that way
                                    is_current_stream_capturing=lambda: rec.capturing, memory_snapshot=lambda: rec.snapshot()))
     monkeypatch.setattr(acl, "torch", fake_torch)
+    monkeypatch.setattr(acl, "_gpu_stream_handle", lambda s: 7 if s is None else s.cuda_stream, raising=False)
     monkeypatch.setattr(acl._lib, "lib", lambda: Lib())
     monkeypatch.setattr(acl, "_WS", type(acl._WS)())
     device = types.SimpleNamespace(type="cuda", index=0)
