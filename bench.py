@@ -283,7 +283,7 @@ def cpu_baseline_sample(name="c2", seconds_budget=15.0):
 
 def verify_rows(torch, kind, counts, x, w_nd, ws, xs, out0, out1):
     """Row sample of a finished launch against the CPU oracle: per expert the first and last row, the rows either side of
-    every 128/256-row tile edge and 32 random ones (every row when there are at most 2048)."""
+    every tile edge and 32 random ones (every row when there are at most 2048)."""
     from oracle import oracle as O
     from oracle import sampled_check as SC
     O.build()

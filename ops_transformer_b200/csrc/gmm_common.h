@@ -143,7 +143,8 @@ int device_sm_count();
 //   Gelu(x)       = x / (1 + exp(-1.59576912 * (x + 0.044715 * x^3)))      (tanh form)
 //   FasterGelu(x) = x / (1 + exp(-1.702 * x))
 //   Silu(x)       = x / (1 + exp(-x))
-// evaluated here in fp32 with every operation rounded separately.
+// evaluated here in fp32 with every operation rounded separately, for the SIMT kernels.  The tensor-core epilogue evaluates the
+// same definitions with times_sigmoid (gmm_sm100.cu), which may differ from this in the last places.
 __device__ __forceinline__ float apply_activation(int act_type, float v)
 {
     switch (act_type) {

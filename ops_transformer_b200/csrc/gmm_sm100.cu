@@ -18,8 +18,9 @@
 //                          half): a tile yields 64 outputs per CTA and token; the two halves meet through shared memory.
 //   swiglu_quant, one CTA: both halves of 128 columns in two accumulators of at most 128 tokens; a lane holds both values.
 // K is consumed 128 bytes per pipeline stage (4 MMAs of K=32).
-// Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2-9 = epilogue; swiglu_quant
-// adds warp 10, one lane of which keeps the books of the row blocks in global memory.
+// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2-9 = epilogue (320 threads); swiglu_quant adds
+// warp 10, one lane of which keeps the books of the row blocks in global memory, and requantising warps up to 512 threads;
+// FRACTAL_NZ adds two weight loader warps (384 threads; in swiglu_quant they take the place of two requantising warps).
 // CTA pairs (cluster of 2, tcgen05 cta_group::2) compute 256 channels; each CTA stages its own 128 channels and half of the
 // tile's token rows.  A launch confined to one CTA runs the one-CTA instances.  Weight layouts: [E,K,N] (MN-major operand,
 // 128-byte swizzle; 64-byte for swiglu's 64-channel boxes), the transposed view [E,N,K] (K-major) and FRACTAL_NZ
@@ -83,9 +84,9 @@ struct Shape {
 constexpr int MAX_GROUPS = 1024;
 constexpr int EPI_WARPS = 8;                 // two warps per TMEM lane quarter, each takes every second 32-token chunk
 // swiglu_quant only: one more warp, of which one lane keeps the books of the row blocks in global memory (arrivals, slice
-// claims) beside the epilogue, so that none of its round trips to L2 delays the next tile.  It hands the epilogue warps
-// lists of row ranges to requantise through a small ring.
-constexpr int WK_DEPTH = 4;                  // work lists the publishing lane may be ahead of the epilogue warps
+// claims) beside the epilogue, so that none of its round trips to L2 delays the next tile.  It hands the requantising warps
+// lists of row ranges through a small ring.
+constexpr int WK_DEPTH = 4;                  // work lists the publishing lane may be ahead of the requantising warps
 // Weight loader warps (FRACTAL_NZ only).  A 32-byte row of that storage is a row of its own to TMA, 512 per 16 KB, and the
 // copy engine takes about 1.75 cycles for each: 900 cycles per K block where the MMAs need 512 and HBM 740.  In memory 128
 // K-rows of a 32-column slab are 4 KB in one piece, so two warps fetch them with 16-byte cp.async, 512 contiguous bytes per
@@ -137,7 +138,7 @@ struct Shared {
     long long wait_limit;              // bound of every wait, in cycles
     // swiglu_quant: how many epilogue warps have stored their part of how many tiles; the row blocks this
     // CTA contributed to and has not yet settled (publishing lane only); a ring of work lists: the row ranges to requantise
-    // (written by that lane, read by the epilogue warps after wk_full)
+    // (written by that lane, read by the requantising warps after wk_full)
     unsigned stored_count;
     int pend_n;
     int pend_rb[MAX_PENDING], pend_row0[MAX_PENDING], pend_rows[MAX_PENDING];
@@ -1586,7 +1587,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         // Per tile of this unit, in the epilogue's order: wait until every epilogue thread has stored the tile, arrive at its
         // row block, collect the row slices that fall to this CTA now (publish_and_collect) into the next work list.  After
         // the last tile one more list takes or hands over what is still pending.  Nothing here waits for another CTA; the
-        // only back-pressure is the ring of work lists, which the epilogue warps empty after every tile.
+        // only back-pressure is the ring of work lists, which the requantising warps empty.
         if (lane == 0) {
             const int shares = p.n_tiles * CTAS;
             int it = 0;
@@ -1831,7 +1832,7 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     for (int i = 0; i < 8; ++i) kp.out_peers[i] = i < kp.num_peers ? p.out_peers[i] : nullptr;
     if (kp.num_peers > 0 && epi != kEpiScatter) return cudaErrorInvalidValue;
     // Pacing (see the producer): needs one zeroed word per wave; the plan reserves them only where it pays.
-    // One counter per wave is reserved for pairs; a single one-CTA unit has more waves and nobody to keep pace with.
+    // The plan reserves a counter per tile, so there is one for every wave; a single unit has nobody to keep pace with.
     kp.wave_cnt = plan.off_wave && plan.num_sms >= 2 ? reinterpret_cast<int *>(ws + plan.off_wave) : nullptr;
     kp.pace_cycles = kp.num_k_blocks * 1200 + 20000;   // about one tile's duration
 #ifdef GMM_TRACE

@@ -403,7 +403,7 @@ aclnnStatus aclnnGroupedMatmulV4(void *workspace, uint64_t workspaceSize, aclOpE
 
 // tuningConfigOptional[0] is the number of rows the caller expects per group, a hint for the reference's host tiling
 // (aclnn_grouped_matmul.cpp:1336-1360).  The device scheduler here reads group_list itself; the hint only replaces
-// M / len(group_list) in the choice between 128-row tiles and CTA pairs, which matters when many groups are empty.
+// M / len(group_list) in the choice between single CTAs and CTA pairs (make_plan), which matters when many groups are empty.
 static aclnnStatus check_tuning_config(const aclIntArray *cfg, int64_t *rows_hint)
 {
     *rows_hint = 0;

@@ -20,8 +20,9 @@ Q_LSB_FRACTION = 1e-4
 
 
 def sample_rows(counts, n_random: int = 32, seed: int = 0, edges=(128, 256), max_rows_all: int = 0) -> np.ndarray:
-    """Sorted row numbers to check: per expert its first and last row, the rows either side of every 128- and 256-row
-    tile edge inside it, and ``n_random`` more drawn uniformly.  With at most ``max_rows_all`` rows in total every row."""
+    """Sorted row numbers to check: per expert its first and last row, the rows either side of every tile edge inside it (as
+    few tiles of at most 128 or 256 rows as hold it, of nearly equal size in steps of 32) and of every multiple of 128 and
+    256, and ``n_random`` more drawn uniformly.  With at most ``max_rows_all`` rows in total every row."""
     counts = np.asarray(counts, np.int64)
     starts = np.concatenate([[0], np.cumsum(counts)[:-1]])
     total = int(counts.sum())
@@ -35,9 +36,12 @@ def sample_rows(counts, n_random: int = 32, seed: int = 0, edges=(128, 256), max
             continue
         local = {0, r - 1}
         for e in edges:
-            for m in range(e, r, e):
-                local.add(m - 1)
-                local.add(m)
+            tiles = -(-r // e)
+            tile = -(-(-(-r // tiles)) // 32) * 32
+            for step in (e, tile):
+                for m in range(step, r, step):
+                    local.add(m - 1)
+                    local.add(m)
         if r > len(local):
             local.update(int(v) for v in rng.integers(0, r, size=n_random))
         picks.extend(s + v for v in sorted(local))

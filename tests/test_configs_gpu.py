@@ -3,7 +3,7 @@
 The oracle cannot run 32768 x 7168 x 4096 in seconds, so every full-size launch is compared on a ROW SAMPLE: both
 operators treat each row on its own, hence the oracle applied to the selected rows (same weights, full K and N) must
 reproduce those rows of the large launch.  Per expert the sample holds the first and last row, the rows either side of
-every 128- and 256-row tile edge and 32 random rows; rows beyond group_list[-1] must keep their sentinel values.
+every tile edge and 32 random rows; rows beyond group_list[-1] must keep their sentinel values.
 Bars as everywhere: int32 bit-exact, bf16 within rtol 4e-3 / atol 1e-2 (and expected bit-identical), requant scales 1e-6
 relative, int8 at most 1 LSB apart on at most 0.01 % of elements.
 

@@ -1014,7 +1014,6 @@ def test_random_sweep_of_shapes_and_options(oracle, monkeypatch, seed):
         M = int(counts.sum()) + int(rng.integers(0, 7))
         x, w, ws, xs = make_inputs(M, K, N, E, seed=1000 * seed + it)
         monkeypatch.setenv("GMM_B200_CTAS", str(rng.choice(["1", "2"])))
-        monkeypatch.setenv("GMM_B200_HYBRID", str(rng.choice(["0", "1"])))
         gl_type = int(rng.integers(0, 2))
         gl = counts if gl_type == 1 else np.cumsum(counts)
         nz = bool(rng.random() < 0.4)
