@@ -248,6 +248,8 @@ def test_captured_calls_own_their_workspace(oracle):
         with torch.cuda.graph(g):
             outs.append(ops.grouped_matmul_swiglu_quant(*t, gl))
         graphs.append(g)
+    from ops_transformer_b200 import acl
+    assert not acl._WS._replayed, "a torch graph's calls take their workspace from the graph's pool"
     big = torch.zeros((4 * M, K), dtype=torch.int8, device=dev)
     ops.grouped_matmul_swiglu_quant(big, *sets[0][1][1:3], torch.ones(4 * M, device=dev), gl)
     junk = [torch.full((1 << 22,), 0x5a, dtype=torch.uint8, device=dev) for _ in range(8)]   # whatever was freed is in use now
