@@ -27,8 +27,9 @@
 // [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, fetched by two loader warps instead of TMA).
 // Epilogue: a lane holds one channel (its weight scale stays in a register), the tokens' scales come from shared memory.
 // bf16 / fp16 results are read as 16x256b fragments, packed by token pairs and transposed by stmatrix, so that the four
-// warps of a column half together hold 256 contiguous bytes of every result row; 32-bit results (SwiGLU values, the
-// combine's fp32 rows, int32 accumulators) are transposed 16 tokens at a time, 128 contiguous bytes per row and warp.
+// warps of a column half together hold 256 contiguous bytes of every result row; SwiGLU values and
+// int32 accumulators are stored as they are held, a token's 32 channels (128 bytes) per instruction; the combine's fp32 rows
+// are transposed 16 tokens at a time, so that a lane adds four channels of a row at once.
 // Rows are optionally scattered by a row index, also into other GPUs' buffers; the finalize-routing variant adds weighted
 // fp32 rows into token rows with 16-byte vector reductions; SwiGLU values go to an fp32 staging buffer with a per-row
 // atomic max, and a finished row block is requantised to int8 in row slices that the CTAs which worked on it claim from a
@@ -348,9 +349,9 @@ __device__ __forceinline__ uint64_t policy_evict_last()
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
     return pol;
 }
-__device__ __forceinline__ void st_global_v4_hint(float *a, const float4 v, uint64_t pol)
+__device__ __forceinline__ void st_global_hint(float *a, float v, uint64_t pol)
 {
-    asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(pol) : "memory");
+    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(a), "f"(v), "l"(pol) : "memory");
 }
 __device__ __forceinline__ float4 ld_global_cg_v4_hint(const float4 *a, uint64_t pol)
 {
@@ -1352,25 +1353,24 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * BT;
             const float *tok = sh->tok_scale[buf];
 
-            // 16 tokens of S, one column per lane: fp32 rows to the staging buffer, row maxima
+            // 16 tokens of S, one column per lane: a token's 32 values are one line of the staging buffer, stored straight from
+            // the registers; the row maxima (NaN left out, as fmaxf does) are reduced on their bits.  Through a transpose in shared
+            // memory, whose accesses come out of the MMAs' operand bandwidth (64 of its 128 bytes per cycle are read, 64 written
+            // by the copies), K=1024 N=2048 took 136 us instead of 118 with 64 groups of 400 rows, 20.3 / 18.5 with 4 of 64.
             auto store_s = [&](const uint32_t (&v)[16], int t0) {
-                uint4 o[4];
-                transpose16(my_stage, v, lane, o);
-                const int col = c0 + ch0 + (lane & 7) * 4;
-                float *sout = reinterpret_cast<float *>(p.out);
+                const int col = c0 + ch0 + lane;
+                const bool in = col < p.half_n;
+                float *dst = reinterpret_cast<float *>(p.out) + (size_t)(tl.row0 + t0) * p.half_n + col;
+                uint32_t amax = 0;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int tk = t0 + i * 4 + (lane >> 3);
-                    const float4 val = make_float4(__uint_as_float(o[i].x), __uint_as_float(o[i].y), __uint_as_float(o[i].z), __uint_as_float(o[i].w));
-                    float amax = 0.0f;
-                    if (col < p.half_n) amax = fmaxf(fmaxf(fmaxf(fmaxf(0.0f, fabsf(val.x)), fabsf(val.y)), fabsf(val.z)), fabsf(val.w));
-#pragma unroll
-                    for (int s = 1; s < 8; s <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
-                    if (tk < tl.rows) {
-                        if (col < p.half_n) st_global_v4_hint(sout + (size_t)(tl.row0 + tk) * p.half_n + col, val, pol_last);
-                        if ((lane & 7) == 0) atomicMax(p.amax_bits + tl.row0 + tk, __float_as_uint(amax));
-                    }
+                for (int i = 0; i < 16; ++i) {
+                    const float val = __uint_as_float(v[i]);
+                    if (in && t0 + i < tl.rows) st_global_hint(dst, val, pol_last);
+                    dst += p.half_n;
+                    const uint32_t m = __reduce_max_sync(0xffffffffu, in ? __float_as_uint(fmaxf(fabsf(val), 0.0f)) : 0u);
+                    if (lane == i) amax = m;
                 }
+                if (lane < 16 && t0 + lane < tl.rows) atomicMax(p.amax_bits + tl.row0 + t0 + lane, amax);
             };
             if (DUAL) {
                 for (int tc = chalf * 16; tc < tl.rows; tc += 32) {
@@ -1428,7 +1428,10 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     uint32_t v[32];
                     tmem_ld32(taddr + tc, v);
                     tmem_ld_wait();
-                    const int col = c0 + quarter * 32 + (lane & 7) * 4;
+                    // One channel per lane for int32: a token's 32 values are one line, stored straight from the registers (K=1024
+                    // N=2048, 64 groups of 400 rows: 81 us transposed, 79.5).  Four channels of a token for the combine: L2 does an
+                    // addition of four in the time of one (K=2048 N=7168, 4096 tokens x 8 over 32 experts: 504 us, 580 singly).
+                    const int col = c0 + quarter * 32 + (COMBINE ? (lane & 7) * 4 : lane);
                     uint32_t *const out = reinterpret_cast<uint32_t *>(p.out);   // rows of N 32-bit results
                     unsigned long long row_addr = 0;   // of token tc + lane; 0: not stored
                     if (SCATTER) {
@@ -1452,15 +1455,22 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                                 r[i] = (uint32_t)(!PLAIN ? acc + bias_i[0] : acc);
                             }
                         }
+                        if (!COMBINE) {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                uint32_t *row = SCATTER ? reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, row_addr, h * 16 + i))
+                                                : t0 + i < tl.rows ? out + (size_t)(tl.row0 + t0 + i) * p.N : nullptr;
+                                if (row && col < p.N) row[col] = r[i];
+                            }
+                            continue;
+                        }
                         uint4 o[4];
                         transpose16(my_stage, r, lane, o);
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            const int tk = h * 16 + i * 4 + (lane >> 3);   // of the chunk
-                            uint32_t *row = SCATTER ? reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, row_addr, tk))
-                                            : tc + tk < tl.rows ? out + (size_t)(tl.row0 + tc + tk) * p.N : nullptr;
+                            uint32_t *row = reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, row_addr, h * 16 + i * 4 + (lane >> 3)));
                             if (!row || col >= p.N) continue;
-                            if (COMBINE && p.scatter_add)
+                            if (p.scatter_add)
                                 red_add_v4(reinterpret_cast<float *>(row + col), make_float4(__uint_as_float(o[i].x), __uint_as_float(o[i].y), __uint_as_float(o[i].z), __uint_as_float(o[i].w)));
                             else *reinterpret_cast<uint4 *>(row + col) = o[i];
                         }
