@@ -873,6 +873,35 @@ __device__ __forceinline__ bool consume_work(const KParams &p, Shared *sh, int l
     return true;
 }
 
+// Two fp32 values in one register pair.  The packed operations of sm_100 round each half as the scalar ones do and take one
+// issue slot for both.  (There is no packed addition here: the assembler fused one with the packed product in front of it, so
+// sums that the reference rounds separately stay scalar.)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // v / (1 + exp(-z)), for z < 0 as v e / (1 + e), with e = exp(-|z|) so that nothing overflows.
 //   e = 2^t (1 + d ln 2): t is the rounded product -|z| h of h = fl(log2 e), d = -|z| (h + l) - t what the rounding and the
 //   remainder l of log2 e = h + l left out (an fma each; |d| < 2^-16, so the second-order term is below 2^-33).
@@ -904,6 +933,56 @@ __device__ __forceinline__ float times_sigmoid(float v, float z)
     return tail ? __fmul_rn(res, 0.25f) : res;
 }
 
+// The same for two values with |z| <= kPlainZ: exp(-z) stays between 2^-93 and 2^93, so neither a sign nor the range has to be
+// looked at, and v / (1 + exp(-z)) is formed as it stands: 9 packed instructions and two approximations each instead of twice
+// 20 instructions.  The error is that of times_sigmoid less the rounding of v e.  (K=1024 N=2048, 64 groups of 400 rows: swiglu
+// 118 -> 115 us; K=1424 N=2976, 3055 rows, fp16 with bias and GELU: 41 -> 39.)
+constexpr float kPlainZ = 64.0f;
+__device__ __forceinline__ f32x2 times_sigmoid2(f32x2 v, f32x2 z)
+{
+    const f32x2 log2e = pair2(1.44269502f, 1.44269502f), neg_log2e = pair2(-1.44269502f, -1.44269502f);
+    const f32x2 t = mul2(z, log2e);   // the exponent is -t
+    const f32x2 d = fma2(z, pair2(-1.92596299e-8f, -1.92596299e-8f), fma2(z, neg_log2e, t));
+    const float2 ts = unpair2(t);
+    float e0, e1, r0, r1;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(-ts.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(-ts.y));
+    f32x2 e = pair2(e0, e1);
+    e = fma2(e, mul2(d, pair2(0.693147181f, 0.693147181f)), e);
+    const f32x2 minus1 = pair2(-1.0f, -1.0f);
+    const f32x2 neg_den = fma2(e, minus1, minus1);
+    const float2 nd = unpair2(neg_den);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-nd.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-nd.y));
+    const f32x2 r = pair2(r0, r1), q = mul2(v, r);
+    return fma2(fma2(q, neg_den, v), r, q);
+}
+
+// Over a thread's N values: the short form where z allows it, so that a result does not depend on what is computed beside it,
+// and nothing else where the whole warp's z do, as those of a layer.
+template <int N>
+__device__ __forceinline__ void times_sigmoids(float (&v)[N], const float (&z)[N])
+{
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) m = fmaxf(m, fabsf(z[i]));
+    if (__all_sync(0xffffffffu, m <= kPlainZ)) {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) {
+            const float2 r = unpair2(times_sigmoid2(pair2(v[i], v[i + 1]), pair2(z[i], z[i + 1])));
+            v[i] = r.x;
+            v[i + 1] = r.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) {
+            const float2 r = unpair2(times_sigmoid2(pair2(v[i], v[i + 1]), pair2(z[i], z[i + 1])));
+            v[i] = fabsf(z[i]) <= kPlainZ ? r.x : times_sigmoid(v[i], z[i]);
+            v[i + 1] = fabsf(z[i + 1]) <= kPlainZ ? r.y : times_sigmoid(v[i + 1], z[i + 1]);
+        }
+    }
+}
+
 // apply_activation (gmm_common.h) over a thread's values, the choice made once: with a switch in every element the unrolled
 // epilogue was several thousand instructions long and ran out of the instruction cache (3055 x 2976, K = 1424, fp16: 58 us
 // without an activation and 95 us with GELU, against 30 us for the instance without options).
@@ -914,15 +993,49 @@ __device__ __forceinline__ void activate(int act_type, float (&v)[N])
 #pragma unroll
         for (int i = 0; i < N; ++i) v[i] = v[i] > 0.0f ? v[i] : 0.0f;
     } else if (act_type == 2) {
+        float z[N];
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float v3 = __fmul_rn(__fmul_rn(v[i], v[i]), v[i]);
-            v[i] = times_sigmoid(v[i], __fmul_rn(1.59576912f, __fadd_rn(v[i], __fmul_rn(0.044715f, v3))));
+        for (int i = 0; i < N; i += 2) {
+            const f32x2 x = pair2(v[i], v[i + 1]);
+            const f32x2 x3 = mul2(mul2(x, x), x);
+            const float2 zi = unpair2(mul2(pair2(1.59576912f, 1.59576912f), fma2(pair2(0.044715f, 0.044715f), x3, x)));
+            z[i] = zi.x;
+            z[i + 1] = zi.y;
         }
+        times_sigmoids(v, z);
     } else if (act_type == 4 || act_type == 5) {
         const float f = act_type == 4 ? 1.702f : 1.0f;
+        float z[N];
 #pragma unroll
-        for (int i = 0; i < N; ++i) v[i] = times_sigmoid(v[i], __fmul_rn(f, v[i]));
+        for (int i = 0; i < N; ++i) z[i] = __fmul_rn(f, v[i]);
+        times_sigmoids(v, z);
+    }
+}
+
+// (acc * x_scale) * w_scale of one channel's 16 tokens; `tok` is 16-byte aligned.
+__device__ __forceinline__ void dequant16(const uint32_t (&acc)[16], const float *tok, float w_scale, float (&out)[16])
+{
+    const f32x2 w = pair2(w_scale, w_scale);
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(tok + i);
+        const float2 lo = unpair2(mul2(mul2(pair2(__int2float_rn((int)acc[i]), __int2float_rn((int)acc[i + 1])), pair2(x.x, x.y)), w));
+        const float2 hi = unpair2(mul2(mul2(pair2(__int2float_rn((int)acc[i + 2]), __int2float_rn((int)acc[i + 3])), pair2(x.z, x.w)), w));
+        out[i] = lo.x; out[i + 1] = lo.y; out[i + 2] = hi.x; out[i + 3] = hi.y;
+    }
+}
+// S = gate * (act / (1 + exp(-act))), into act
+__device__ __forceinline__ void swiglu16(float (&act)[16], const float (&gate)[16])
+{
+    float z[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) z[i] = act[i];
+    times_sigmoids(act, z);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        const float2 r = unpair2(mul2(pair2(gate[i], gate[i + 1]), pair2(act[i], act[i + 1])));
+        act[i] = r.x;
+        act[i + 1] = r.y;
     }
 }
 
@@ -1323,7 +1436,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     }
                 }
             }
-            float xs = 1.0f, lg = 1.0f;
+            float xs = te < tl.rows ? 1.0f : 0.0f, lg = 1.0f;   // 0: rows of other groups, never stored, stay small
             if (te < tl.rows) {
                 if (MODE != kModeInt32 && p.x_scale) xs = __ldg(p.x_scale + tl.row0 + te);
                 if (COMBINE && p.logit) lg = __ldg(p.logit + tl.row0 + te);
@@ -1357,14 +1470,14 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             // the registers; the row maxima (NaN left out, as fmaxf does) are reduced on their bits.  Through a transpose in shared
             // memory, whose accesses come out of the MMAs' operand bandwidth (64 of its 128 bytes per cycle are read, 64 written
             // by the copies), K=1024 N=2048 took 136 us instead of 118 with 64 groups of 400 rows, 20.3 / 18.5 with 4 of 64.
-            auto store_s = [&](const uint32_t (&v)[16], int t0) {
+            auto store_s = [&](const float (&v)[16], int t0) {
                 const int col = c0 + ch0 + lane;
                 const bool in = col < p.half_n;
                 float *dst = reinterpret_cast<float *>(p.out) + (size_t)(tl.row0 + t0) * p.half_n + col;
                 uint32_t amax = 0;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float val = __uint_as_float(v[i]);
+                    const float val = v[i];
                     if (in && t0 + i < tl.rows) st_global_hint(dst, val, pol_last);
                     dst += p.half_n;
                     const uint32_t m = __reduce_max_sync(0xffffffffu, in ? __float_as_uint(fmaxf(fabsf(val), 0.0f)) : 0u);
@@ -1378,46 +1491,38 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     tmem_ld16(taddr + tc, va);
                     tmem_ld16(taddr + MAX_TOK + tc, vb);
                     tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        // (acc * x_scale) * w_scale, then S = gate * (act / (1 + exp(-act)))
-                        const float a = __fmul_rn(__fmul_rn(__int2float_rn((int)va[i]), tok[tc + i]), wsc[0]);
-                        const float b = __fmul_rn(__fmul_rn(__int2float_rn((int)vb[i]), tok[tc + i]), wsc_up);
-                        va[i] = __float_as_uint(__fmul_rn(b, times_sigmoid(a, a)));
-                    }
-                    store_s(va, tc);
+                    // (acc * x_scale) * w_scale
+                    float act[16], gate[16];
+                    dequant16(va, tok + tc, wsc[0], act);
+                    dequant16(vb, tok + tc, wsc_up, gate);
+                    swiglu16(act, gate);
+                    store_s(act, tc);
                 }
             }
             for (int tc = chalf * 32; !DUAL && tc < tl.rows && ok; tc += 64) {  // a chunk of 32 tokens
                 if (SWIGLU) {
-                    uint32_t v[32], own[16];
-                    tmem_ld32(taddr + tc, v);
+                    // The gate warp finishes tokens 0..15 of the chunk, the up warp 16..31: each sends the other its values of
+                    // the other's tokens.
+                    const int own0 = tc + (up ? 16 : 0), other0 = tc + (up ? 0 : 16);
+                    uint32_t va[16], vb[16];
+                    tmem_ld16(taddr + other0, vb);
+                    tmem_ld16(taddr + own0, va);
                     tmem_ld_wait();
-                    // (acc * x_scale) * w_scale.  The gate warp finishes tokens 0..15 of the chunk, the up warp 16..31: each
-                    // sends the other its values of the other's tokens.
+                    float mine[16], theirs[16];   // (acc * x_scale) * w_scale
+                    dequant16(vb, tok + other0, wsc[0], theirs);
 #pragma unroll
-                    for (int t4 = 0; t4 < 4; ++t4) {
-                        const float4 s0 = *reinterpret_cast<const float4 *>(tok + tc + t4 * 4);
-                        const float4 s1 = *reinterpret_cast<const float4 *>(tok + tc + 16 + t4 * 4);
-                        const float sl[4] = {s0.x, s0.y, s0.z, s0.w}, sh4[4] = {s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int i = t4 * 4 + k;
-                            const float lo = __fmul_rn(__fmul_rn(__int2float_rn((int)v[i]), sl[k]), wsc[0]);
-                            const float hi = __fmul_rn(__fmul_rn(__int2float_rn((int)v[16 + i]), sh4[k]), wsc[0]);
-                            own[i] = __float_as_uint(up ? hi : lo);
-                            *reinterpret_cast<float *>(partner_stage + i * 128 + lane * 4) = up ? lo : hi;
-                        }
-                    }
+                    for (int i = 0; i < 16; ++i) *reinterpret_cast<float *>(partner_stage + i * 128 + lane * 4) = theirs[i];
+                    dequant16(va, tok + own0, wsc[0], mine);
                     if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 700)) { ok = false; break; }
+                    float act[16], gate[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const float other = *reinterpret_cast<const float *>(my_stage + i * 128 + lane * 4);
-                        const float act = up ? other : __uint_as_float(own[i]);
-                        const float gate = up ? __uint_as_float(own[i]) : other;
-                        own[i] = __float_as_uint(__fmul_rn(gate, times_sigmoid(act, act)));  // S = gate * (act / (1 + exp(-act)))
+                        act[i] = up ? other : mine[i];
+                        gate[i] = up ? mine[i] : other;
                     }
-                    store_s(own, tc + (up ? 16 : 0));
+                    swiglu16(act, gate);
+                    store_s(act, own0);
                     // the partner may write the next chunk's values here
                     if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 710)) { ok = false; break; }
                 } else if (!OUT16) {
@@ -1445,14 +1550,20 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                         if (t0 >= tl.rows) break;
                         uint32_t r[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int acc = (int)v[h * 16 + i];
+                        for (int i = 0; i < 16; i += 2) {
+                            const int a0 = (int)v[h * 16 + i], a1 = (int)v[h * 16 + i + 1];
                             if (COMBINE) {
-                                float tv = __fmul_rn(__fmul_rn(__int2float_rn(acc), wsc[0]), tok[t0 + i]);
-                                if (p.bias_dtype == kBF16) tv = __fadd_rn(tv, __fmul_rn(sh->tok_logit[buf][t0 + i], bias_f[0]));
-                                r[i] = __float_as_uint(tv);
+                                float2 t = unpair2(mul2(mul2(pair2(__int2float_rn(a0), __int2float_rn(a1)), pair2(wsc[0], wsc[0])),
+                                                        *reinterpret_cast<const f32x2 *>(tok + t0 + i)));
+                                if (p.bias_dtype == kBF16) {
+                                    t.x = __fadd_rn(t.x, __fmul_rn(sh->tok_logit[buf][t0 + i], bias_f[0]));
+                                    t.y = __fadd_rn(t.y, __fmul_rn(sh->tok_logit[buf][t0 + i + 1], bias_f[0]));
+                                }
+                                r[i] = __float_as_uint(t.x);
+                                r[i + 1] = __float_as_uint(t.y);
                             } else {
-                                r[i] = (uint32_t)(!PLAIN ? acc + bias_i[0] : acc);
+                                r[i] = (uint32_t)(PLAIN ? a0 : a0 + bias_i[0]);
+                                r[i + 1] = (uint32_t)(PLAIN ? a1 : a1 + bias_i[0]);
                             }
                         }
                         if (!COMBINE) {
@@ -1510,15 +1621,18 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     float o[4][4][2];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float2 ts = *reinterpret_cast<const float2 *>(tok + tc + i * 8 + (lane & 3) * 2);
+                        const f32x2 ts = *reinterpret_cast<const f32x2 *>(tok + tc + i * 8 + (lane & 3) * 2);
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-#pragma unroll
-                            for (int k = 0; k < 2; ++k) {
-                                int acc = (int)(j < 2 ? v0[i * 4 + j * 2 + k] : v1[i * 4 + (j - 2) * 2 + k]);
-                                if (!PLAIN) acc += bias_i[j];
-                                o[i][j][k] = __fmul_rn(__int2float_rn(acc), wsc[j]);
-                                if (PLAIN || p.x_scale) o[i][j][k] = __fmul_rn(o[i][j][k], k ? ts.y : ts.x);
+                            {
+                                int a0 = (int)(j < 2 ? v0[i * 4 + j * 2] : v1[i * 4 + (j - 2) * 2]);
+                                int a1 = (int)(j < 2 ? v0[i * 4 + j * 2 + 1] : v1[i * 4 + (j - 2) * 2 + 1]);
+                                if (!PLAIN) { a0 += bias_i[j]; a1 += bias_i[j]; }
+                                f32x2 t = mul2(pair2(__int2float_rn(a0), __int2float_rn(a1)), pair2(wsc[j], wsc[j]));
+                                if (PLAIN || p.x_scale) t = mul2(t, ts);
+                                const float2 f = unpair2(t);
+                                o[i][j][0] = f.x;
+                                o[i][j][1] = f.y;
                             }
                     }
                     if (!PLAIN) {
