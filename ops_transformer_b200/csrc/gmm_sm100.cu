@@ -132,6 +132,8 @@ struct Shared {
     uint64_t grp_sync[4];              // epilogue warps that exchange values through out_stage (see group_sync)
     uint64_t wk_full[WK_DEPTH];        // a work list is written (swiglu_quant)
     uint64_t wk_empty[WK_DEPTH];       // every requantising warp is done with it
+    int closing_slot;                  // the ring slot of the last list
+    uint64_t wk_closing;               // the last list is written (for the epilogue warps, which help with that one)
     uint32_t tmem_base;
     int abort_flag;
     int total_tiles;
@@ -144,6 +146,7 @@ struct Shared {
     int pend_n;
     int pend_rb[MAX_PENDING], pend_row0[MAX_PENDING], pend_rows[MAX_PENDING];
     int n_work[WK_DEPTH];
+    int work_last[WK_DEPTH];           // no list follows
     int work_begin[WK_DEPTH][MAX_PENDING + 1], work_end[WK_DEPTH][MAX_PENDING + 1];
     int row_start[MAX_GROUPS];
     int rows[MAX_GROUPS];
@@ -701,6 +704,35 @@ __device__ __forceinline__ void red_add_v4(float *p, const float4 v)
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
+// Two fp32 values in one register pair.  The packed operations of sm_100 round each half as the scalar ones do and take one
+// issue slot for both.  (There is no packed addition here: the assembler fused one with the packed product in front of it, so
+// sums that the reference rounds separately stay scalar.)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // q = int8(rint(half(S * (1 / (amax / 127)))))  -- CastFp32ToInt8Template,
 // gmm/grouped_matmul_swiglu_quant/op_kernel/grouped_matmul_swiglu_quant_utils.h:308-316; NaN -> 0, saturating.
 __device__ __forceinline__ uint32_t quant1(float s, float rcp)
@@ -713,6 +745,18 @@ __device__ __forceinline__ uint32_t quant4(float4 v, float rcp)
 {
     return quant1(v.x, rcp) | (quant1(v.y, rcp) << 8) | (quant1(v.z, rcp) << 16) | (quant1(v.w, rcp) << 24);
 }
+// The same for a row whose scale lies in [1e-30, 1e30]: no finite value leaves [-127, 127], so nothing saturates, and adding
+// 1536 to the fp16 value rounds it to the nearest integer (ties to even: the spacing there is 1) and leaves that integer in the
+// low byte.  NaN, which the row maximum left out, becomes 0.
+__device__ __forceinline__ uint32_t quant4_plain(float4 v, f32x2 rcp)
+{
+    const float2 a = unpair2(mul2(pair2(v.x, v.y), rcp)), b = unpair2(mul2(pair2(v.z, v.w), rcp));
+    const __half2 ha = __floats2half2_rn(a.x, a.y), hb = __floats2half2_rn(b.x, b.y);
+    const __half2 magic = __halves2half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600));
+    const __half2 qa = __hadd2(ha, magic), qb = __hadd2(hb, magic);
+    return __byte_perm(*reinterpret_cast<const uint32_t *>(&qa) & __heq2_mask(ha, ha),
+                       *reinterpret_cast<const uint32_t *>(&qb) & __heq2_mask(hb, hb), 0x6420);
+}
 
 // Second half of grouped_matmul_swiglu_quant for rows [r_begin, r_end) of a finished row block (all of its N tiles
 // have stored S and the row maxima): per row  qs = amax / 127, r = 1 / qs, q = int8(half(S * r))
@@ -721,32 +765,36 @@ __device__ __forceinline__ uint32_t quant4(float4 v, float rcp)
 // pieces (a load instruction covers 512 contiguous bytes, a store 128): the tensor cores read their operands through the
 // same shared-memory / L1 data path, so every extra line these accesses touch is taken from the MMAs.  Sixteen loads
 // per lane are in flight at a time, because they wait for L2 under the full load of the GEMM.
-template <int RQ>
-__device__ void requant_rows(const KParams &p, int r_begin, int r_end, int warp_r, int lane)
+// Not inlined: the epilogue warps take part in the last list, and a second copy would only have to be fetched again.  With their
+// help, without empty lists and with fewer instructions per value, the end of a short call got shorter: K=4096 N=4096, 6 groups
+// of about 200 rows 41.6 -> 40.2 us, K=1408 N=1408, 22 groups of 12 rows 22.5 -> 21.9.
+__device__ __noinline__ void requant_rows(const float *stage, const unsigned *amax_bits, int8_t *q_out, float *q_scale_out, int H, int r_begin,
+                                          int r_end, int worker, int workers)
 {
-    const int H = p.half_n;
+    const int lane = threadIdx.x & 31;
     const int nf = H >> 2;  // 16-byte pieces per row
-    const float *stage = reinterpret_cast<const float *>(p.out);
-    for (int grow = r_begin + warp_r; grow < r_end; grow += RQ) {
-        const float amax = __uint_as_float(__ldcg(p.amax_bits + grow));
+    const uint64_t pol_first = policy_evict_first();
+    for (int grow = r_begin + worker; grow < r_end; grow += workers) {
+        const float amax = __uint_as_float(__ldcg(amax_bits + grow));
         const float4 *src = reinterpret_cast<const float4 *>(stage + (size_t)grow * H);
-        uint32_t *dst = reinterpret_cast<uint32_t *>(p.q_out + (size_t)grow * H);
-        float4 v[16];
-        int f = lane;
-        const uint64_t pol_first = policy_evict_first();
-#pragma unroll
-        for (int u = 0; u < 16; ++u) v[u] = f + 32 * u < nf ? ld_global_cg_v4_hint(src + f + 32 * u, pol_first) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float qs = __fdiv_rn(amax, 127.0f);
-        const float rcp = __fdiv_rn(1.0f, qs);
-        if (lane == 0) p.q_scale_out[grow] = qs;
-        while (true) {
-#pragma unroll
-            for (int u = 0; u < 16; ++u)
-                if (f + 32 * u < nf) dst[f + 32 * u] = quant4(v[u], rcp);
-            f += 512;
-            if (f - lane >= nf) break;
+        uint32_t *dst = reinterpret_cast<uint32_t *>(q_out + (size_t)grow * H);
+        for (int f = lane; f - lane < nf; f += 512) {
+            float4 v[16];
 #pragma unroll
             for (int u = 0; u < 16; ++u) v[u] = f + 32 * u < nf ? ld_global_cg_v4_hint(src + f + 32 * u, pol_first) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float qs = __fdiv_rn(amax, 127.0f);
+            const float rcp = __fdiv_rn(1.0f, qs);
+            if (f == 0) q_scale_out[grow] = qs;
+            if (qs >= 1e-30f && qs <= 1e30f) {
+                const f32x2 rcp2 = pair2(rcp, rcp);
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    if (f + 32 * u < nf) dst[f + 32 * u] = quant4_plain(v[u], rcp2);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    if (f + 32 * u < nf) dst[f + 32 * u] = quant4(v[u], rcp);
+            }
         }
     }
 }
@@ -782,7 +830,6 @@ __device__ __forceinline__ int ld_relaxed_gpu(const int *p)
 // `ws`.  The caller fences before (release of the CTA's stores) and after (acquire of the other CTAs' stores).
 __device__ void publish_and_collect(const KParams &p, Shared *sh, int ws, int rb, int row0, int rows, int shares)
 {
-    sh->n_work[ws] = 0;
     int *state = p.rb_counter;
     // the looks at the older blocks and the arrival travel together (one round trip to L2)
     int seen[MAX_PENDING];
@@ -833,7 +880,6 @@ __device__ void publish_and_collect(const KParams &p, Shared *sh, int ws, int rb
 // depends on the other CTAs being resident.
 __device__ void release_pending(const KParams &p, Shared *sh, int ws, int shares, long long patience)
 {
-    sh->n_work[ws] = 0;
     int *state = p.rb_counter;
     const long long t0 = clock64();
     while (sh->pend_n > 0) {
@@ -848,7 +894,7 @@ __device__ void release_pending(const KParams &p, Shared *sh, int ws, int shares
         }
         sh->pend_n = n;
         if (n == 0 || clock64() - t0 > patience) break;
-        __nanosleep(500);
+        __nanosleep(100);
     }
     for (int i = 0; i < sh->pend_n; ++i) {
         const int o = atomicAdd(state + 2 * sh->pend_rb[i], 1 << 16);
@@ -858,48 +904,12 @@ __device__ void release_pending(const KParams &p, Shared *sh, int ws, int shares
     sh->pend_n = 0;
 }
 
-// Requantising warp: the row ranges of the next work list.  Every warp consumes every list, in order, and takes the rows
-// warp, warp + RQ, ... of each range.  Returns false when the (bounded) wait for the list gave up.
-template <int RQ>
-__device__ __forceinline__ bool consume_work(const KParams &p, Shared *sh, int list, int warp_r, int lane)
+// The row ranges of work list `ws`, which the caller has acquired: worker w of n takes rows w, w + n, ... of each.
+__device__ __forceinline__ void work_off(const KParams &p, const Shared *sh, int ws, int worker, int workers)
 {
-    const int ws = list % WK_DEPTH;
-    const bool ok = mbar_wait(&sh->wk_full[ws], ((uint32_t)(list / WK_DEPTH)) & 1u, sh, p.status, 650 + ws);
-    if (!__all_sync(0xffffffffu, ok)) return false;
     const int n = sh->n_work[ws];
-    for (int k = 0; k < n; ++k) requant_rows<RQ>(p, sh->work_begin[ws][k], sh->work_end[ws][k], warp_r, lane);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sh->wk_empty[ws]);
-    return true;
-}
-
-// Two fp32 values in one register pair.  The packed operations of sm_100 round each half as the scalar ones do and take one
-// issue slot for both.  (There is no packed addition here: the assembler fused one with the packed product in front of it, so
-// sums that the reference rounds separately stay scalar.)
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair2(float a, float b)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpair2(f32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
+    for (int k = 0; k < n; ++k)
+        requant_rows(static_cast<const float *>(p.out), p.amax_bits, p.q_out, p.q_scale_out, p.half_n, sh->work_begin[ws][k], sh->work_end[ws][k], worker, workers);
 }
 
 // v / (1 + exp(-z)), for z < 0 as v e / (1 + e), with e = exp(-|z|) so that nothing overflows.
@@ -1117,6 +1127,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             mbar_init(&sh->wk_full[b], 1);
             mbar_init(&sh->wk_empty[b], RQ);
         }
+        mbar_init(&sh->wk_closing, 1);
         sh->stored_count = 0;
         sh->abort_flag = 0;
         sh->total_tiles = 0;
@@ -1692,38 +1703,64 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             }
         }
         if (SCATTER && p.num_peers > 0) __threadfence_system();  // rows stored into other GPUs' memory
+        if (SWIGLU && ok) {  // nothing left to multiply: the last list is worked off by these warps, too
+            const bool got = mbar_wait(&sh->wk_closing, 0u, sh, p.status, 660);
+            if (__all_sync(0xffffffffu, got)) work_off(p, sh, sh->closing_slot, RQ + warp - 2, RQ + EPI_WARPS);
+        }
     }
 
     else if (SWIGLU && warp > 2 + EPI_WARPS) {
         // ------------------------------ requantising warps (swiglu_quant) ------------------------------
-        // One list per tile of this unit plus the closing one.  A list names the row blocks that are complete by then -
-        // normally the block of this unit's previous tile, whose rows are read while they are still in L2.  These warps
-        // spend their time waiting for L2; beside the epilogue that costs nothing, inside it every tile of a C2-sized
-        // launch lost 13 of 36 thousand cycles to it, more than its MMAs take.
-        int lists = 1;
-        for (int t = unit; t < total_tiles; t += n_units) ++lists;
-        for (int i = 0; i < lists; ++i)
-            if (!consume_work<RQ>(p, sh, i, warp - 3 - EPI_WARPS, lane)) break;
+        // A list names the row blocks that are complete by then - normally the block of this unit's previous tile, whose rows
+        // are read while they are still in L2.  These warps spend their time waiting for L2; beside the epilogue that costs
+        // nothing, inside it every tile of a C2-sized launch lost 13 of 36 thousand cycles to it, more than its MMAs take.
+        const int w = warp - 3 - EPI_WARPS;
+        for (int list = 0;; ++list) {
+            const int ws = list % WK_DEPTH;
+            const bool got = mbar_wait(&sh->wk_full[ws], ((uint32_t)(list / WK_DEPTH)) & 1u, sh, p.status, 650 + ws);
+            if (!__all_sync(0xffffffffu, got)) break;
+            const bool last = sh->work_last[ws] != 0;
+            work_off(p, sh, ws, w, last ? RQ + EPI_WARPS : RQ);
+            if (last) break;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->wk_empty[ws]);
+        }
     }
 
     else if (SWIGLU) {
         // ------------------------------ publishing lane (swiglu_quant) ------------------------------
-        // Per tile of this unit, in the epilogue's order: wait until every epilogue thread has stored the tile, arrive at its
-        // row block, collect the row slices that fall to this CTA now (publish_and_collect) into the next work list.  After
-        // the last tile one more list takes or hands over what is still pending.  Nothing here waits for another CTA; the
-        // only back-pressure is the ring of work lists, which the requantising warps empty.
+        // Per tile of this unit, in the epilogue's order: wait until every epilogue warp has stored the tile, arrive at its
+        // row block, collect the row slices that fall to this CTA now (publish_and_collect) into the next work list, and pass
+        // the list on if there is anything in it.  The last list takes or hands over what is still pending as well.  Nothing
+        // here waits for another CTA; the only back-pressure is the ring of work lists, which the requantising warps empty.
         if (lane == 0) {
             const int shares = p.n_tiles * CTAS;
-            int it = 0;
+            int it = 0, list = 0, ws = 0;
             bool ok = true;
             int g_prev = 0;
+            sh->n_work[0] = 0;
+            auto pass_on = [&](bool last) {
+                sh->work_last[ws] = last ? 1 : 0;
+                if (last) sh->closing_slot = ws;
+                __threadfence();
+                mbar_arrive(&sh->wk_full[ws]);
+                if (last) {
+                    mbar_arrive(&sh->wk_closing);
+                    return;
+                }
+                ++list;
+                ws = list % WK_DEPTH;
+                ok = mbar_wait(&sh->wk_empty[ws], (((uint32_t)(list / WK_DEPTH)) & 1u) ^ 1u, sh, p.status, 630 + ws);
+                if (ok) sh->n_work[ws] = 0;
+            };
             for (int t = unit; t < total_tiles && ok; t += n_units, ++it) {
-                const int ws = it % WK_DEPTH;
+                const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                g_prev = tl.g;
                 const unsigned need = (unsigned)(it + 1) * EPI_WARPS;
                 if (*(volatile unsigned *)&sh->stored_count < need) {
                     const long long t0 = clock64();
                     while (*(volatile unsigned *)&sh->stored_count < need) {
-                        __nanosleep(200);
+                        __nanosleep(60);
                         if (*(volatile int *)&sh->abort_flag) { ok = false; break; }
                         if (clock64() - t0 > sh->wait_limit) {
                             *(volatile int *)&sh->abort_flag = 1;
@@ -1739,24 +1776,15 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     if (!ok) break;
                 }
                 TRACE(3, it, 0);
-                if (!mbar_wait(&sh->wk_empty[ws], (((uint32_t)(it / WK_DEPTH)) & 1u) ^ 1u, sh, p.status, 630 + ws)) { ok = false; break; }
-                const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
-                g_prev = tl.g;
-                TRACE(3, it, 1);
                 __threadfence();
                 publish_and_collect(p, sh, ws, t / p.n_tiles, tl.row0, tl.rows, shares);
-                __threadfence();
                 TRACE(3, it, 2);
                 TRACE_ADD(3, it, 3, sh->n_work[ws]);
-                mbar_arrive(&sh->wk_full[ws]);
+                if (sh->n_work[ws] > 0) pass_on(false);
             }
             if (ok && !*(volatile int *)&sh->abort_flag) {
-                const int ws = it % WK_DEPTH;
-                if (mbar_wait(&sh->wk_empty[ws], (((uint32_t)(it / WK_DEPTH)) & 1u) ^ 1u, sh, p.status, 640 + ws)) {
-                    release_pending(p, sh, ws, shares, 2ll * p.pace_cycles);
-                    __threadfence();
-                    mbar_arrive(&sh->wk_full[ws]);
-                }
+                release_pending(p, sh, ws, shares, 2ll * p.pace_cycles);
+                pass_on(true);
             }
         }
     }
