@@ -62,6 +62,7 @@ namespace {
 constexpr int BC = 128;                 // channels (weight columns) per CTA: the MMA's M side, one TMEM lane each
 constexpr int BT = 256;                 // most tokens of a tile: the MMA's N side, one TMEM column each
 constexpr int TOK_STEP = 32;            // the MMA's N is a multiple of this
+constexpr int SPLIT_TOK = 64;           // least tokens of a tile's piece in the last wave, as far as the tile has them
 constexpr int BK = 128;
 constexpr int UMMA_K = 32;
 constexpr int W_STAGE = BC * BK;        // a CTA's channels x 128 bytes of K
@@ -123,6 +124,12 @@ constexpr int ROW16_PITCH = 2 * BC + 16;
 constexpr int OUT_STAGE_BYTES = 2 * 32 * ROW16_PITCH;
 static_assert(OUT_STAGE_BYTES >= EPI_WARPS * WARP_STAGE_BYTES, "one staging area serves both forms");
 
+// A row block some of whose S this CTA has stored (swiglu_quant).
+struct PendingBlock {
+    int rb, row0, rows;
+    int weight, shares;                // the CTA's shares of the block's requantisation, and how many there are
+};
+
 struct Shared {
     uint64_t full[MAX_STAGES];
     uint64_t empty[MAX_STAGES];
@@ -138,13 +145,14 @@ struct Shared {
     int abort_flag;
     int total_tiles;
     int max_tok;                       // tokens of the largest tile
+    int split_from, split;             // tiles from split_from on are cut into `split` pieces of their tokens (see build_schedule)
     long long wait_limit;              // bound of every wait, in cycles
     // swiglu_quant: how many epilogue warps have stored their part of how many tiles; the row blocks this
     // CTA contributed to and has not yet settled (publishing lane only); a ring of work lists: the row ranges to requantise
     // (written by that lane, read by the requantising warps after wk_full)
     unsigned stored_count;
     int pend_n;
-    int pend_rb[MAX_PENDING], pend_row0[MAX_PENDING], pend_rows[MAX_PENDING];
+    PendingBlock pend[MAX_PENDING];
     int n_work[WK_DEPTH];
     int work_last[WK_DEPTH];           // no list follows
     int work_begin[WK_DEPTH][MAX_PENDING + 1], work_end[WK_DEPTH][MAX_PENDING + 1];
@@ -566,8 +574,13 @@ __device__ __forceinline__ int tile_tokens(int rows)
 // at most ceil(M / 128) + L row blocks; a falling running total names rows again and again and can have many times as many.  The
 // swiglu tiles beyond the counters reserved for that many are left out and reported (kStatusBadList): the counters behind them
 // are other data, and a slice claimed from such a word would be an arbitrary range of rows.
+//
+// The last wave: `rem` tiles for n_units units take as long as a full wave.  Where two or more units are there for each of
+// them, they are cut into that many pieces along their tokens, of SPLIT_TOK or more (below, a K block of MMAs does not get
+// shorter any more): the weights come from L2 for all but one of the pieces.  A piece without rows is left out.
+// K=4096 N=4096, 6 groups of about 200 rows, us: grouped_matmul 32.9 -> 31.1, swiglu_quant 40.2 -> 38.5.
 template <int MAX_TOK>
-__device__ void build_schedule(Shared *sh, const KParams &p)
+__device__ void build_schedule(Shared *sh, const KParams &p, int n_units)
 {
     const int tid = threadIdx.x, L = p.gl_len;
     for (int g = tid; g < L; g += (int)blockDim.x) {
@@ -630,7 +643,12 @@ __device__ void build_schedule(Shared *sh, const KParams &p)
         if (lane == 31) {
             sh->max_tok = max_tok;
             sh->tile_start[L] = incl;
-            sh->total_tiles = min(incl, p.max_tiles);
+            const int total = min(incl, p.max_tiles), rem = total % n_units;
+            int split = rem > 0 ? min(n_units / rem, (max_tok + SPLIT_TOK - 1) / SPLIT_TOK) : 1;
+            if (split < 2 || p.n_tiles > 65535 / (2 * split)) split = 1;   // shares of a row block are counted in 16 bits
+            sh->split = split;
+            sh->split_from = split > 1 ? total - rem : total;
+            sh->total_tiles = split > 1 ? total - rem + rem * split : total;
             if (incl > p.max_tiles && blockIdx.x == 0 && atomicCAS(p.status, kStatusOk, kStatusBadList) == kStatusOk) {
                 p.status[1] = 0;
                 p.status[2] = 810;
@@ -649,14 +667,27 @@ __device__ __forceinline__ int x_box_rows(int share)
     return CTAS == 1 && share > 128 ? 256 : share > 64 ? 128 : share > 32 ? 64 : 32;
 }
 
+// Token rows of each piece of a tile of `rows` rows cut into `split` (the last one may have fewer, or none).
+__device__ __forceinline__ int piece_tokens(int rows, int split)
+{
+    return ((rows + split - 1) / split + TOK_STEP - 1) / TOK_STEP * TOK_STEP;
+}
+
 struct Tile {
-    int g, row0, rows, n_idx;
+    int g, row0, rows, n_idx;           // rows <= 0: a piece without rows, always a unit's last one
+    int index, block_row0, block_rows;  // of the whole tile
 };
 
 // `from`: the group of this unit's previous tile (tiles are visited in ascending order); normally the next one is near.
 template <int MAX_TOK>
 __device__ __forceinline__ Tile decode_tile(const Shared *sh, int t, int n_tiles, int L, int from = 0)
 {
+    int piece = -1;
+    if (t >= sh->split_from) {
+        const int v = t - sh->split_from, k = v / sh->split;
+        piece = v - k * sh->split;
+        t = sh->split_from + k;
+    }
     int lo = from, hi = min(from + 4, L);  // largest g in [0, L) with tile_start[g] <= t
     if (sh->tile_start[hi] <= t) { lo = hi; hi = L; }
     while (hi - lo > 1) {
@@ -671,6 +702,14 @@ __device__ __forceinline__ Tile decode_tile(const Shared *sh, int t, int n_tiles
     tl.n_idx = local - mb * n_tiles;
     tl.row0 = sh->row_start[lo] + mb * tt;
     tl.rows = min(tt, sh->rows[lo] - mb * tt);
+    tl.index = t;
+    tl.block_row0 = tl.row0;
+    tl.block_rows = tl.rows;
+    if (piece >= 0) {
+        const int sub = piece_tokens(tl.rows, sh->split);
+        tl.row0 += piece * sub;
+        tl.rows = min(sub, tl.rows - piece * sub);
+    }
     return tl;
 }
 
@@ -812,11 +851,18 @@ __device__ __noinline__ void requant_rows(const float *stage, const unsigned *am
 //     atomic add of 1 << 16.  If that add finds the block already complete it takes its slice itself; otherwise the
 //     completing arrival, which comes later, sees the hand-over in the value its own add returns.
 // Slices are claimed from the claim counter, so every slice is taken exactly once.
-__device__ __forceinline__ void add_work(Shared *sh, int ws, int row0, int rows, int first, int count, int shares)
+__device__ __forceinline__ void add_work(Shared *sh, int ws, const PendingBlock &b, int first, int count)
 {
     const int k = sh->n_work[ws]++;
-    sh->work_begin[ws][k] = row0 + (int)((long long)rows * first / shares);
-    sh->work_end[ws][k] = row0 + (int)((long long)rows * (first + count) / shares);
+    sh->work_begin[ws][k] = b.row0 + (int)((long long)b.rows * first / b.shares);
+    sh->work_end[ws][k] = b.row0 + (int)((long long)b.rows * (first + count) / b.shares);
+}
+
+// This CTA's shares of block `b` go to whoever completes it, or are taken now if that has happened.
+__device__ __forceinline__ void hand_over(const KParams &p, Shared *sh, int ws, const PendingBlock &b)
+{
+    const int o = atomicAdd(p.rb_counter + 2 * b.rb, b.weight << 16);
+    if ((o & 0xffff) == b.shares) add_work(sh, ws, b, atomicAdd(p.rb_counter + 2 * b.rb + 1, b.weight), b.weight);
 }
 
 __device__ __forceinline__ int ld_relaxed_gpu(const int *p)
@@ -826,51 +872,42 @@ __device__ __forceinline__ int ld_relaxed_gpu(const int *p)
     return v;
 }
 
-// Publishing lane, after the whole CTA has stored a tile: arrive at block `rb`, look at the pending blocks, fill work list
+// Publishing lane, after the whole CTA has stored a tile: arrive at its block, look at the pending blocks, fill work list
 // `ws`.  The caller fences before (release of the CTA's stores) and after (acquire of the other CTAs' stores).
-__device__ void publish_and_collect(const KParams &p, Shared *sh, int ws, int rb, int row0, int rows, int shares)
+__device__ void publish_and_collect(const KParams &p, Shared *sh, int ws, const PendingBlock &mine)
 {
     int *state = p.rb_counter;
     // the looks at the older blocks and the arrival travel together (one round trip to L2)
     int seen[MAX_PENDING];
 #pragma unroll
-    for (int i = 0; i < MAX_PENDING; ++i) seen[i] = i < sh->pend_n ? ld_relaxed_gpu(state + 2 * sh->pend_rb[i]) : 0;
-    const int old = atomicAdd(state + 2 * rb, 1);
-    const bool completed = (old & 0xffff) + 1 == shares;
+    for (int i = 0; i < MAX_PENDING; ++i) seen[i] = i < sh->pend_n ? ld_relaxed_gpu(state + 2 * sh->pend[i].rb) : 0;
+    const int old = atomicAdd(state + 2 * mine.rb, mine.weight);
+    const bool completed = (old & 0xffff) + mine.weight == mine.shares;
     // slice claims, again together
     int first[MAX_PENDING];
 #pragma unroll
     for (int i = 0; i < MAX_PENDING; ++i)
-        first[i] = (i < sh->pend_n && (seen[i] & 0xffff) == shares) ? atomicAdd(state + 2 * sh->pend_rb[i] + 1, 1) : -1;
-    const int cnt = 1 + (old >> 16);
-    const int mine = completed ? atomicAdd(state + 2 * rb + 1, cnt) : -1;
+        first[i] = (i < sh->pend_n && (seen[i] & 0xffff) == sh->pend[i].shares) ? atomicAdd(state + 2 * sh->pend[i].rb + 1, sh->pend[i].weight) : -1;
+    const int cnt = mine.weight + (old >> 16);
+    const int my_first = completed ? atomicAdd(state + 2 * mine.rb + 1, cnt) : -1;
     int n = 0;
 #pragma unroll
     for (int i = 0; i < MAX_PENDING; ++i) {
         if (i >= sh->pend_n) break;
-        if (first[i] >= 0) {
-            add_work(sh, ws, sh->pend_row0[i], sh->pend_rows[i], first[i], 1, shares);
-        } else {
-            sh->pend_rb[n] = sh->pend_rb[i]; sh->pend_row0[n] = sh->pend_row0[i]; sh->pend_rows[n] = sh->pend_rows[i];
-            ++n;
-        }
+        if (first[i] >= 0) add_work(sh, ws, sh->pend[i], first[i], sh->pend[i].weight);
+        else sh->pend[n++] = sh->pend[i];
     }
     sh->pend_n = n;
     if (completed) {
-        add_work(sh, ws, row0, rows, mine, cnt, shares);
+        add_work(sh, ws, mine, my_first, cnt);
         return;
     }
     if (sh->pend_n == MAX_PENDING) {  // hand the oldest block's share over (or take it, if the block completed meanwhile)
-        const int o = atomicAdd(state + 2 * sh->pend_rb[0], 1 << 16);
-        if ((o & 0xffff) == shares)
-            add_work(sh, ws, sh->pend_row0[0], sh->pend_rows[0], atomicAdd(state + 2 * sh->pend_rb[0] + 1, 1), 1, shares);
-        for (int i = 1; i < MAX_PENDING; ++i) {
-            sh->pend_rb[i - 1] = sh->pend_rb[i]; sh->pend_row0[i - 1] = sh->pend_row0[i]; sh->pend_rows[i - 1] = sh->pend_rows[i];
-        }
+        hand_over(p, sh, ws, sh->pend[0]);
+        for (int i = 1; i < MAX_PENDING; ++i) sh->pend[i - 1] = sh->pend[i];
         --sh->pend_n;
     }
-    const int k = sh->pend_n++;
-    sh->pend_rb[k] = rb; sh->pend_row0[k] = row0; sh->pend_rows[k] = rows;
+    sh->pend[sh->pend_n++] = mine;
 }
 
 // Publishing lane, after the CTA's last tile: every block still pending is taken once it is complete.  The other units
@@ -878,29 +915,22 @@ __device__ void publish_and_collect(const KParams &p, Shared *sh, int ws, int rb
 // handing the share over at once would leave the last arrival of every block of the final wave with all of its slices,
 // a serial tail of tens of microseconds); what is still incomplete after that is handed over, so the kernel never
 // depends on the other CTAs being resident.
-__device__ void release_pending(const KParams &p, Shared *sh, int ws, int shares, long long patience)
+__device__ void release_pending(const KParams &p, Shared *sh, int ws, long long patience)
 {
     int *state = p.rb_counter;
     const long long t0 = clock64();
     while (sh->pend_n > 0) {
         int n = 0;
         for (int i = 0; i < sh->pend_n; ++i) {
-            if ((ld_relaxed_gpu(state + 2 * sh->pend_rb[i]) & 0xffff) == shares) {
-                add_work(sh, ws, sh->pend_row0[i], sh->pend_rows[i], atomicAdd(state + 2 * sh->pend_rb[i] + 1, 1), 1, shares);
-            } else {
-                sh->pend_rb[n] = sh->pend_rb[i]; sh->pend_row0[n] = sh->pend_row0[i]; sh->pend_rows[n] = sh->pend_rows[i];
-                ++n;
-            }
+            if ((ld_relaxed_gpu(state + 2 * sh->pend[i].rb) & 0xffff) == sh->pend[i].shares)
+                add_work(sh, ws, sh->pend[i], atomicAdd(state + 2 * sh->pend[i].rb + 1, sh->pend[i].weight), sh->pend[i].weight);
+            else sh->pend[n++] = sh->pend[i];
         }
         sh->pend_n = n;
         if (n == 0 || clock64() - t0 > patience) break;
         __nanosleep(100);
     }
-    for (int i = 0; i < sh->pend_n; ++i) {
-        const int o = atomicAdd(state + 2 * sh->pend_rb[i], 1 << 16);
-        if ((o & 0xffff) == shares)
-            add_work(sh, ws, sh->pend_row0[i], sh->pend_rows[i], atomicAdd(state + 2 * sh->pend_rb[i] + 1, 1), 1, shares);
-    }
+    for (int i = 0; i < sh->pend_n; ++i) hand_over(p, sh, ws, sh->pend[i]);
     sh->pend_n = 0;
 }
 
@@ -1141,7 +1171,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         tmem_alloc<CTAS>(&sh->tmem_base, TMEM_COLS);
         tc_fence_before();
     }
-    build_schedule<MAX_TOK>(sh, p);  // ends with __syncthreads()
+    build_schedule<MAX_TOK>(sh, p, n_units);  // ends with __syncthreads()
     if (CTAS == 2) cluster_sync_all();  // the partner's barriers exist before anything is sent to them
     tc_fence_after();
 
@@ -1158,6 +1188,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         int buf = 0;
         uint32_t acc_phase = 0;
         for (int t = unit; t < total_tiles; t += n_units) {
+            if (t >= sh->split_from && decode_tile<MAX_TOK>(sh, t, p.n_tiles, L).rows <= 0) break;
             if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[buf], acc_phase, sh, p.status, 210 + buf))) break;
             tc_fence_after();
             tc_fence_before();
@@ -1187,6 +1218,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             Tile next = unit < total_tiles ? decode_tile<MAX_TOK>(sh, unit, p.n_tiles, L) : Tile{};
             for (int t = unit; t < total_tiles && ok; t += n_units, ++wave) {
                 const Tile tl = next;
+                if (tl.rows <= 0) break;
                 if (pace) {
                     if (lane == 0) {
                         if (wave > 0) {
@@ -1269,6 +1301,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             Tile next = unit < total_tiles ? decode_tile<MAX_TOK>(sh, unit, p.n_tiles, L) : Tile{};
             for (int t = unit; t < total_tiles && ok; t += n_units, ++ti) {
                 const Tile tl = next;
+                if (tl.rows <= 0) break;
                 const uint32_t idesc = idesc0 | (uint32_t)(((tl.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP) >> 3) << 17;
                 if (lane == 0) TRACE(1, ti, 0);
                 if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[buf], acc_phase ^ 1u, sh, p.status, 200 + buf))) { ok = false; break; }
@@ -1340,6 +1373,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             int g_prev = 0;
             for (int t = unit; t < total_tiles && ok; t += n_units) {
                 const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                if (tl.rows <= 0) break;
                 g_prev = tl.g;
                 const int my_tok = (tl.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP / CTAS;
                 const int x_rows = x_box_rows<CTAS>(my_tok);
@@ -1374,6 +1408,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         int g_prev = 0;
         for (int t = unit; t < total_tiles && ok; t += n_units) {
             const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+            if (tl.rows <= 0) break;
             g_prev = tl.g;
             const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA, cols = SWIGLU ? p.half_n : p.N;
             const int8_t *src = w + (size_t)tl.g * p.K * p.N + (size_t)(c0 >> 5) * slab_bytes + l * 16;
@@ -1421,7 +1456,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         int g_prev = 0;
         for (int t = unit; t < total_tiles; t += n_units, ++it) {
             const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
-                g_prev = tl.g;
+            if (tl.rows <= 0) break;
+            g_prev = tl.g;
             const size_t sbase = (size_t)tl.g * p.N;
             const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA;   // first result column of this CTA
 
@@ -1734,7 +1770,6 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         // the list on if there is anything in it.  The last list takes or hands over what is still pending as well.  Nothing
         // here waits for another CTA; the only back-pressure is the ring of work lists, which the requantising warps empty.
         if (lane == 0) {
-            const int shares = p.n_tiles * CTAS;
             int it = 0, list = 0, ws = 0;
             bool ok = true;
             int g_prev = 0;
@@ -1755,7 +1790,21 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             };
             for (int t = unit; t < total_tiles && ok; t += n_units, ++it) {
                 const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                if (tl.rows <= 0) break;
                 g_prev = tl.g;
+                // A block with tiles in the last wave that are cut into pieces counts in pieces: a whole tile has the shares of
+                // its pieces, a piece one.
+                PendingBlock mine;
+                mine.rb = tl.index / p.n_tiles;
+                mine.row0 = tl.block_row0;
+                mine.rows = tl.block_rows;
+                int pieces = 1;
+                if ((long long)(mine.rb + 1) * p.n_tiles > sh->split_from) {
+                    const int sub = piece_tokens(tl.block_rows, sh->split);
+                    pieces = (tl.block_rows + sub - 1) / sub;
+                }
+                mine.weight = tl.index < sh->split_from ? pieces : 1;
+                mine.shares = p.n_tiles * CTAS * pieces;
                 const unsigned need = (unsigned)(it + 1) * EPI_WARPS;
                 if (*(volatile unsigned *)&sh->stored_count < need) {
                     const long long t0 = clock64();
@@ -1777,13 +1826,13 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                 }
                 TRACE(3, it, 0);
                 __threadfence();
-                publish_and_collect(p, sh, ws, t / p.n_tiles, tl.row0, tl.rows, shares);
+                publish_and_collect(p, sh, ws, mine);
                 TRACE(3, it, 2);
                 TRACE_ADD(3, it, 3, sh->n_work[ws]);
                 if (sh->n_work[ws] > 0) pass_on(false);
             }
             if (ok && !*(volatile int *)&sh->abort_flag) {
-                release_pending(p, sh, ws, shares, 2ll * p.pace_cycles);
+                release_pending(p, sh, ws, 2ll * p.pace_cycles);
                 pass_on(true);
             }
         }

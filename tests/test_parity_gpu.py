@@ -468,6 +468,37 @@ def test_token_tile_edges(oracle, monkeypatch, ctas, kind):
         assert np.array_equal(got[perm[:rows]], ref[:rows]) and (got[perm[rows:]] == 0x7fc1).all()
 
 
+@pytest.mark.parametrize("ctas,max_ctas", [("1", 5), ("1", 8), ("1", 11), ("1", 37), ("2", 8), ("2", 14), ("2", 30)])
+@pytest.mark.parametrize("kind", ["bf16", "int32", "nz", "swiglu", "swiglu_nz"])
+def test_last_wave_cut_into_pieces(monkeypatch, ctas, max_ctas, kind):
+    """Tiles of the last wave are cut along their tokens where two or more units are free for each: pieces that end inside a
+    32-token step, empty ones, and row blocks of swiglu_quant with whole tiles beside pieces.  A launch on one unit, whose
+    waves are single tiles, cuts nothing; the results are the same bits."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    monkeypatch.setenv("GMM_B200_CTAS", ctas)
+    nz = kind in ("nz", "swiglu_nz")
+    for tail in ([200], [33], [256, 256], [1, 90], [129, 2, 255]):
+        counts = np.array([300, 1, 129, 0, 64, 513] + tail, np.int64)
+        E, M, K, N = len(counts), int(counts.sum()), 272, 448
+        x, w, ws, xs = make_inputs(M, K, N, E, seed=66)
+        t = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
+        gl, wt = t(np.cumsum(counts)), t(nd_to_nz(w) if nz else w)
+        got = []
+        for cap in (1, max_ctas):
+            kw = dict(weight_format=ops.ACL_FORMAT_FRACTAL_NZ if nz else ops.ACL_FORMAT_ND, return_workspace=True,
+                      options=ops.LaunchOptions(max_ctas=cap))
+            if kind.startswith("swiglu"):
+                *r, wsb = ops.grouped_matmul_swiglu_quant(t(x), wt, t(ws), t(xs), gl, **kw)
+            elif kind == "int32":
+                *r, wsb = ops.grouped_matmul_v4(t(x), wt, None, None, gl, out_dtype=torch.int32, **kw)
+            else:
+                *r, wsb = ops.grouped_matmul_v4(t(x), wt, t(ws), t(xs), gl, **kw)
+            ops.check_status(wsb)
+            got.append(r)
+        assert all(torch.equal(a, b) for a, b in zip(*got)), tail
+
+
 @pytest.mark.parametrize("act_type", [1, 2, 4, 5])
 def test_gmm_activations_beyond_the_range_of_exp(oracle, act_type):
     """Arguments of the sigmoid from -1e4 to 1e4 (cubed, for GELU): both ends of exp, bf16 results within one rounding step."""
