@@ -27,9 +27,9 @@
 // [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, fetched by two loader warps instead of TMA).
 // Epilogue: a lane holds one channel (its weight scale stays in a register), the tokens' scales come from shared memory.
 // bf16 / fp16 results are read as 16x256b fragments, packed by token pairs and transposed by stmatrix, so that the four
-// warps of a column half together hold 256 contiguous bytes of every result row; SwiGLU values and
-// int32 accumulators are stored as they are held, a token's 32 channels (128 bytes) per instruction; the combine's fp32 rows
-// are transposed 16 tokens at a time, so that a lane adds four channels of a row at once.
+// warps of a column half together hold 256 contiguous bytes of every result row; SwiGLU values are
+// stored as they are held, a token's 32 channels (128 bytes) per instruction; the combine's fp32 rows and int32 accumulators
+// are transposed 16 tokens at a time, so that a lane adds or stores four channels of a row at once.
 // Rows are optionally scattered by a row index, also into other GPUs' buffers; the finalize-routing variant adds weighted
 // fp32 rows into token rows with 16-byte vector reductions; SwiGLU values go to an fp32 staging buffer with a per-row
 // atomic max, and a finished row block is requantised to int8 in row slices that the CTAs which worked on it claim from a
@@ -1580,10 +1580,11 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     uint32_t v[32];
                     tmem_ld32(taddr + tc, v);
                     tmem_ld_wait();
-                    // One channel per lane for int32: a token's 32 values are one line, stored straight from the registers (K=1024
-                    // N=2048, 64 groups of 400 rows: 81 us transposed, 79.5).  Four channels of a token for the combine: L2 does an
-                    // addition of four in the time of one (K=2048 N=7168, 4096 tokens x 8 over 32 experts: 504 us, 580 singly).
-                    const int col = c0 + quarter * 32 + (COMBINE ? (lane & 7) * 4 : lane);
+                    // Four channels of a token per lane: L2 does an addition of four in the time of one (combine, K=2048 N=7168, 4096
+                    // tokens x 8 over 32 experts: 504 us, 580 singly), and results that go to HBM are better off with four lines per
+                    // store than with one straight from the registers (int32 of the same size 407 / 415; of K=1024 N=2048, 64 groups
+                    // of 400 rows, 81 / 79.5).
+                    const int col = c0 + quarter * 32 + (lane & 7) * 4;
                     uint32_t *const out = reinterpret_cast<uint32_t *>(p.out);   // rows of N 32-bit results
                     unsigned long long row_addr = 0;   // of token tc + lane; 0: not stored
                     if (SCATTER) {
@@ -1613,22 +1614,15 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                                 r[i + 1] = (uint32_t)(PLAIN ? a1 : a1 + bias_i[0]);
                             }
                         }
-                        if (!COMBINE) {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                uint32_t *row = SCATTER ? reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, row_addr, h * 16 + i))
-                                                : t0 + i < tl.rows ? out + (size_t)(tl.row0 + t0 + i) * p.N : nullptr;
-                                if (row && col < p.N) row[col] = r[i];
-                            }
-                            continue;
-                        }
                         uint4 o[4];
                         transpose16(my_stage, r, lane, o);
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            uint32_t *row = reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, row_addr, h * 16 + i * 4 + (lane >> 3)));
+                            const int tk = h * 16 + i * 4 + (lane >> 3);   // of the chunk
+                            uint32_t *row = SCATTER ? reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, row_addr, tk))
+                                            : tc + tk < tl.rows ? out + (size_t)(tl.row0 + tc + tk) * p.N : nullptr;
                             if (!row || col >= p.N) continue;
-                            if (p.scatter_add)
+                            if (COMBINE && p.scatter_add)
                                 red_add_v4(reinterpret_cast<float *>(row + col), make_float4(__uint_as_float(o[i].x), __uint_as_float(o[i].y), __uint_as_float(o[i].z), __uint_as_float(o[i].w)));
                             else *reinterpret_cast<uint4 *>(row + col) = o[i];
                         }
