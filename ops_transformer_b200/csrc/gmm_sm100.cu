@@ -83,6 +83,11 @@ struct Shape {
     static constexpr int kMaxTok = kDual ? BT / 2 : BT;
     static constexpr int kCols = MODE == kModeSwigluQuant && !kDual ? BC / 2 : BC;   // result columns per CTA and tile
 };
+// Row blocks of a group that are worked on together: all their tiles of a channel tile, then the next channel tile.  A group that
+// begins in one wave and ends in the next has its x rows read twice then, instead of its weights, four times as many.  swiglu
+// K=7168 N=4096, 32 groups of 1024 rows: 758 us with one, 740 with four; grouped_matmul, which does not pace its waves, K=2048
+// N=7168: 339 / 343.
+__host__ __device__ constexpr int block_group(int mode) { return mode == kModeSwigluQuant ? 4 : 1; }
 constexpr int MAX_GROUPS = 1024;
 constexpr int EPI_WARPS = 8;                 // two warps per TMEM lane quarter, each takes every second 32-token chunk
 // swiglu_quant only: one more warp, of which one lane keeps the books of the row blocks in global memory (arrivals, slice
@@ -200,7 +205,8 @@ struct KParams {
     int M, K, N;
     int half_n;        // N/2 (swiglu)
     int n_tiles;       // channel tiles per row block
-    int max_tiles;     // tiles that the workspace's row block counters cover (swiglu)
+    int max_blocks;    // row blocks that the workspace's counters cover (swiglu)
+    int max_tiles;     // their tiles
     int num_k_blocks;  // ceil(K / BK)
     const void *w_nz;     // FRACTAL_NZ weights, read by the loader warps
     const void *w_scale;
@@ -559,13 +565,17 @@ __host__ __device__ constexpr uint32_t make_idesc(bool a_mn_major, int m)
 // Tile schedule, rebuilt by every CTA from group_list (<= 1024 entries)
 // ---------------------------------------------------------------------------------------------------------
 
-// Token rows per tile of a group of `rows` rows: as few tiles as MAX_TOK rows allow, of nearly equal size (a multiple of 32).
-// Equal tiles keep the units of a wave together; their sum costs the same as full tiles and a short one.
+// Row blocks of a group of `rows` rows, as few as MAX_TOK rows a tile allow, and the token rows of each: of nearly equal size
+// (a multiple of 32; no more than MAX_TOK, so the count stays the same).  Equal tiles keep the units of a wave together; their
+// sum costs the same as full tiles and a short one.
+template <int MAX_TOK>
+__device__ __forceinline__ int row_blocks(int rows) { return (rows + MAX_TOK - 1) / MAX_TOK; }
 template <int MAX_TOK>
 __device__ __forceinline__ int tile_tokens(int rows)
 {
-    const int nt = (rows + MAX_TOK - 1) / MAX_TOK;
-    return nt == 0 ? TOK_STEP : ((rows + nt - 1) / nt + TOK_STEP - 1) / TOK_STEP * TOK_STEP;
+    const int nt = row_blocks<MAX_TOK>(rows);
+    const int each = nt <= 1 ? max(rows, 1) : (rows + nt - 1) / nt;   // (no division on the way of a short call)
+    return (each + TOK_STEP - 1) / TOK_STEP * TOK_STEP;
 }
 
 // Row ranges follow GetSplitValueFromGroupList (gmm/grouped_matmul/op_kernel/grouped_matmul_utils.h:243-257):
@@ -623,7 +633,7 @@ __device__ void build_schedule(Shared *sh, const KParams &p, int n_units)
             sh->row_start[g] = (int)start;
             sh->rows[g] = (int)rows;
             const int tt = tile_tokens<MAX_TOK>((int)rows);
-            const int tiles = (int)((rows + tt - 1) / tt) * p.n_tiles;
+            const int tiles = row_blocks<MAX_TOK>((int)rows) * p.n_tiles;
             max_tok = max(max_tok, tt);
             sh->tile_start[g] = tiles;
             tsum += tiles;
@@ -643,8 +653,8 @@ __device__ void build_schedule(Shared *sh, const KParams &p, int n_units)
         if (lane == 31) {
             sh->max_tok = max_tok;
             sh->tile_start[L] = incl;
-            const int total = min(incl, p.max_tiles), rem = total % n_units;
-            int split = rem > 0 ? min(n_units / rem, (max_tok + SPLIT_TOK - 1) / SPLIT_TOK) : 1;
+            const int total = min(incl, p.max_tiles), rem = total < n_units ? total : total % n_units;
+            int split = max_tok > SPLIT_TOK && rem > 0 ? min(n_units / rem, (max_tok + SPLIT_TOK - 1) / SPLIT_TOK) : 1;
             if (split < 2 || p.n_tiles > 65535 / (2 * split)) split = 1;   // shares of a row block are counted in 16 bits
             sh->split = split;
             sh->split_from = split > 1 ? total - rem : total;
@@ -676,10 +686,11 @@ __device__ __forceinline__ int piece_tokens(int rows, int split)
 struct Tile {
     int g, row0, rows, n_idx;           // rows <= 0: a piece without rows, always a unit's last one
     int index, block_row0, block_rows;  // of the whole tile
+    int block, block_last;              // its row block, and the last tile of that
 };
 
 // `from`: the group of this unit's previous tile (tiles are visited in ascending order); normally the next one is near.
-template <int MAX_TOK>
+template <int MAX_TOK, int BLOCK_GROUP>
 __device__ __forceinline__ Tile decode_tile(const Shared *sh, int t, int n_tiles, int L, int from = 0)
 {
     int piece = -1;
@@ -694,14 +705,19 @@ __device__ __forceinline__ Tile decode_tile(const Shared *sh, int t, int n_tiles
         const int mid = (lo + hi) >> 1;
         if (sh->tile_start[mid] <= t) lo = mid; else hi = mid;
     }
-    const int local = t - sh->tile_start[lo];
-    const int mb = local / n_tiles;
-    const int tt = tile_tokens<MAX_TOK>(sh->rows[lo]);
+    // BLOCK_GROUP row blocks of a group at a time; of them all row blocks of a channel tile, then the next channel tile
+    const int rows = sh->rows[lo], local = t - sh->tile_start[lo], per = BLOCK_GROUP * n_tiles;
+    const int sg = local < per ? 0 : local / per, rem = local - sg * per;
+    const int side = min(BLOCK_GROUP, row_blocks<MAX_TOK>(rows) - sg * BLOCK_GROUP);
+    const int tt = tile_tokens<MAX_TOK>(rows);
     Tile tl;
     tl.g = lo;
-    tl.n_idx = local - mb * n_tiles;
+    tl.n_idx = side == 1 ? rem : rem / side;
+    const int in_side = rem - tl.n_idx * side, mb = sg * BLOCK_GROUP + in_side;
     tl.row0 = sh->row_start[lo] + mb * tt;
-    tl.rows = min(tt, sh->rows[lo] - mb * tt);
+    tl.rows = min(tt, rows - mb * tt);
+    tl.block = sh->tile_start[lo] / n_tiles + mb;
+    tl.block_last = sh->tile_start[lo] + sg * per + (n_tiles - 1) * side + in_side;
     tl.index = t;
     tl.block_row0 = tl.row0;
     tl.block_rows = tl.rows;
@@ -1129,6 +1145,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
     constexpr int RQ = rq_warps(BL), LD0 = num_threads(MODE, BL) / 32 - ld_warps(BL);   // first loader warp
     constexpr bool DUAL = S::kDual;
     constexpr int CH_CTA = S::kCols, MAX_TOK = S::kMaxTok, W_BYTES = S::kWStage;
+    constexpr int BLOCK_GROUP = block_group(MODE);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     Shared *sh = reinterpret_cast<Shared *>(smem + PIPE_BYTES);
@@ -1188,7 +1205,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         int buf = 0;
         uint32_t acc_phase = 0;
         for (int t = unit; t < total_tiles; t += n_units) {
-            if (t >= sh->split_from && decode_tile<MAX_TOK>(sh, t, p.n_tiles, L).rows <= 0) break;
+            if (t >= sh->split_from && decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t, p.n_tiles, L).rows <= 0) break;
             if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[buf], acc_phase, sh, p.status, 210 + buf))) break;
             tc_fence_after();
             tc_fence_before();
@@ -1215,7 +1232,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             // never needed for correctness: when the wait runs out (units not resident together) pacing is switched off.
             bool pace = p.wave_cnt != nullptr && rank == 0;
             int wave = 0;
-            Tile next = unit < total_tiles ? decode_tile<MAX_TOK>(sh, unit, p.n_tiles, L) : Tile{};
+            Tile next = unit < total_tiles ? decode_tile<MAX_TOK, BLOCK_GROUP>(sh, unit, p.n_tiles, L) : Tile{};
             for (int t = unit; t < total_tiles && ok; t += n_units, ++wave) {
                 const Tile tl = next;
                 if (tl.rows <= 0) break;
@@ -1261,7 +1278,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     }
                     __syncwarp();
                     // the next tile is looked up while the ring is full, not between two tiles
-                    if (kb == 0 && t + n_units < total_tiles) next = decode_tile<MAX_TOK>(sh, t + n_units, p.n_tiles, L, tl.g);
+                    if (kb == 0 && t + n_units < total_tiles) next = decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t + n_units, p.n_tiles, L, tl.g);
                     ++issued;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
@@ -1298,7 +1315,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             const uint32_t acc_full_peer = CTAS == 2 ? map_to_cta(&sh->acc_full[0], 1) : 0u;
             int ti = 0;
             if (lane == 0) TRACE_GT(0, 0, 0);
-            Tile next = unit < total_tiles ? decode_tile<MAX_TOK>(sh, unit, p.n_tiles, L) : Tile{};
+            Tile next = unit < total_tiles ? decode_tile<MAX_TOK, BLOCK_GROUP>(sh, unit, p.n_tiles, L) : Tile{};
             for (int t = unit; t < total_tiles && ok; t += n_units, ++ti) {
                 const Tile tl = next;
                 if (tl.rows <= 0) break;
@@ -1346,7 +1363,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                         }
                     }
                     __syncwarp();
-                    if (kb == 0 && t + n_units < total_tiles) next = decode_tile<MAX_TOK>(sh, t + n_units, p.n_tiles, L, tl.g);
+                    if (kb == 0 && t + n_units < total_tiles) next = decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t + n_units, p.n_tiles, L, tl.g);
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
@@ -1372,7 +1389,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             bool ok = true;
             int g_prev = 0;
             for (int t = unit; t < total_tiles && ok; t += n_units) {
-                const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                const Tile tl = decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t, p.n_tiles, L, g_prev);
                 if (tl.rows <= 0) break;
                 g_prev = tl.g;
                 const int my_tok = (tl.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP / CTAS;
@@ -1407,7 +1424,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         bool ok = true;
         int g_prev = 0;
         for (int t = unit; t < total_tiles && ok; t += n_units) {
-            const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+            const Tile tl = decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t, p.n_tiles, L, g_prev);
             if (tl.rows <= 0) break;
             g_prev = tl.g;
             const int c0 = (tl.n_idx * CTAS + (int)rank) * CH_CTA, cols = SWIGLU ? p.half_n : p.N;
@@ -1455,7 +1472,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         bool ok = true;
         int g_prev = 0;
         for (int t = unit; t < total_tiles; t += n_units, ++it) {
-            const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+            const Tile tl = decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t, p.n_tiles, L, g_prev);
             if (tl.rows <= 0) break;
             g_prev = tl.g;
             const size_t sbase = (size_t)tl.g * p.N;
@@ -1783,17 +1800,17 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                 if (ok) sh->n_work[ws] = 0;
             };
             for (int t = unit; t < total_tiles && ok; t += n_units, ++it) {
-                const Tile tl = decode_tile<MAX_TOK>(sh, t, p.n_tiles, L, g_prev);
+                const Tile tl = decode_tile<MAX_TOK, BLOCK_GROUP>(sh, t, p.n_tiles, L, g_prev);
                 if (tl.rows <= 0) break;
                 g_prev = tl.g;
                 // A block with tiles in the last wave that are cut into pieces counts in pieces: a whole tile has the shares of
                 // its pieces, a piece one.
                 PendingBlock mine;
-                mine.rb = tl.index / p.n_tiles;
+                mine.rb = tl.block;
                 mine.row0 = tl.block_row0;
                 mine.rows = tl.block_rows;
                 int pieces = 1;
-                if ((long long)(mine.rb + 1) * p.n_tiles > sh->split_from) {
+                if (tl.block_last >= sh->split_from) {
                     const int sub = piece_tokens(tl.block_rows, sh->split);
                     pieces = (tl.block_rows + sub - 1) / sub;
                 }
@@ -1820,7 +1837,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                 }
                 TRACE(3, it, 0);
                 __threadfence();
-                publish_and_collect(p, sh, ws, mine);
+                if (mine.rb < p.max_blocks) publish_and_collect(p, sh, ws, mine);   // beyond: a list that is reported (build_schedule)
                 TRACE(3, it, 2);
                 TRACE_ADD(3, it, 3, sh->n_work[ws]);
                 if (sh->n_work[ws] > 0) pass_on(false);
@@ -1997,6 +2014,7 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     kp.half_n = (int)(p.N / 2);
     const int64_t tile_cols = p.mode == kModeSwigluQuant ? BC : BC * plan.ctas, cols = p.mode == kModeSwigluQuant ? p.N / 2 : p.N;
     kp.n_tiles = (int)((cols + tile_cols - 1) / tile_cols);
+    kp.max_blocks = plan.row_blocks < 0x7fffffffll ? (int)plan.row_blocks : 0x7fffffff;
     kp.max_tiles = p.mode == kModeSwigluQuant ? (int)(plan.row_blocks * kp.n_tiles < 0x7fffffffll ? plan.row_blocks * kp.n_tiles : 0x7fffffffll) : 0x7fffffff;
     kp.num_k_blocks = (int)((p.K + BK - 1) / BK);
     kp.w_nz = p.w;
