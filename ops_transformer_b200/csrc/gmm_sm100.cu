@@ -89,7 +89,14 @@ struct Shape {
 // N=7168: 339 / 343.
 __host__ __device__ constexpr int block_group(int mode) { return mode == kModeSwigluQuant ? 4 : 1; }
 constexpr int MAX_GROUPS = 1024;
-constexpr int EPI_WARPS = 8;                 // two warps per TMEM lane quarter, each takes every second 32-token chunk
+enum : int { kEpiPlain = 0, kEpiScatter = 1, kEpiGeneric = 2, kEpiCombine = 3 };
+// Epilogue warps, and the tokens of the chunks that they take in turns: two warps per TMEM lane quarter and 32 tokens; with
+// options (bias, activation) four and 16.  The options' chains of dependent instructions left the schedulers idle with two warps
+// each (K=1424 N=2976, 3055 rows, fp16, bias, GELU: 38.8 us, now 37.4; K=2048 N=2048, 16 groups of 250 rows, bias, SiLU: 36.7 /
+// 35.2); the plain epilogue, which the MMAs hide, only got in their way (K=2048 N=7168, 32 groups of 1024 rows: 360 / 364).
+__host__ __device__ constexpr bool wide_epilogue(int mode, int epi) { return mode == kModeDequantBf16 && epi == kEpiGeneric; }
+__host__ __device__ constexpr int epi_warps(int mode, int epi) { return wide_epilogue(mode, epi) ? 16 : 8; }
+__host__ __device__ constexpr int chunk_tokens(int mode, int epi) { return wide_epilogue(mode, epi) ? 16 : 32; }
 // swiglu_quant only: one more warp, of which one lane keeps the books of the row blocks in global memory (arrivals, slice
 // claims) beside the epilogue, so that none of its round trips to L2 delays the next tile.  It hands the requantising warps
 // lists of row ranges through a small ring.
@@ -104,10 +111,9 @@ constexpr int LD_WARPS = 2;
 __host__ __device__ constexpr int ld_warps(int bl) { return bl == 2 /* kBFractalNz */ ? LD_WARPS : 0; }
 // swiglu_quant: warps that requantise finished row blocks beside the epilogue; with 16 warps in all a thread has 128 registers
 __host__ __device__ constexpr int rq_warps(int bl) { return 5 - ld_warps(bl); }
-constexpr int BASE_THREADS = 64 + 32 * EPI_WARPS;
-__host__ __device__ constexpr int num_threads(int mode, int bl)
+__host__ __device__ constexpr int num_threads(int mode, int bl, int epi)
 {
-    return BASE_THREADS + 32 * ld_warps(bl) + (mode == kModeSwigluQuant ? 32 + 32 * rq_warps(bl) : 0);
+    return 64 + 32 * epi_warps(mode, epi) + 32 * ld_warps(bl) + (mode == kModeSwigluQuant ? 32 + 32 * rq_warps(bl) : 0);
 }
 constexpr int TMEM_COLS = 512;
 constexpr long long WAIT_LIMIT_CYCLES = 1ll << 31;   // about a second
@@ -117,17 +123,15 @@ constexpr long long DRAIN_LIMIT_CYCLES = 1ll << 24;  // a few milliseconds
 // instead of the default C3 runs 0.399 instead of 0.414 ms, C2 0.80-0.81 instead of 0.82-0.83 ms (same box, alternating).
 constexpr uint32_t WAIT_SUSPEND_NS = 2000;
 
-constexpr int EPI_THREADS = 32 * EPI_WARPS;
-enum : int { kEpiPlain = 0, kEpiScatter = 1, kEpiGeneric = 2, kEpiCombine = 3 };
 // Weight layouts: [E,K,N]; [E,N,K] (the transposed view); FRACTAL_NZ [E, N/32, K/16, 16, 32] (32-byte runs along N).
 enum : int { kBRowMajor = 0, kBTransposed = 1, kBFractalNz = 2 };
 constexpr int MAX_PENDING = 6;         // unsettled row blocks a CTA keeps track of before it hands its share over
-// Epilogue staging: 32-bit results 16 tokens x 128 bytes per warp; 16-bit results 32 tokens per column half (four warps) of
-// 256 bytes each, 16 bytes apart so that the eight 16-byte rows of a stmatrix fall into different banks.
+// Epilogue staging: 32-bit results 16 tokens x 128 bytes per warp; 16-bit results 64 tokens of 256 bytes each (a chunk for
+// every four warps), 16 bytes apart so that the eight 16-byte rows of a stmatrix fall into different banks.
 constexpr int WARP_STAGE_BYTES = 2048;
 constexpr int ROW16_PITCH = 2 * BC + 16;
-constexpr int OUT_STAGE_BYTES = 2 * 32 * ROW16_PITCH;
-static_assert(OUT_STAGE_BYTES >= EPI_WARPS * WARP_STAGE_BYTES, "one staging area serves both forms");
+constexpr int OUT_STAGE_BYTES = 64 * ROW16_PITCH;
+static_assert(OUT_STAGE_BYTES >= 8 * WARP_STAGE_BYTES, "one staging area serves both forms");
 
 // A row block some of whose S this CTA has stored (swiglu_quant).
 struct PendingBlock {
@@ -502,9 +506,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// 16 TMEM lanes x 32 consecutive columns as matrix fragments: of every 8 columns thread t receives row t/4 in v[4i], v[4i+1]
+// 16 TMEM lanes x 16 or 32 consecutive columns as matrix fragments: of every 8 columns thread t receives row t/4 in v[4i], v[4i+1]
 // and row t/4 + 8 in v[4i+2], v[4i+3], columns 8i + 2 (t%4) and the next one.
-__device__ __forceinline__ void tmem_ld16x256b_x4(uint32_t taddr, uint32_t (&v)[16])
+__device__ __forceinline__ void tmem_ld16x256b(uint32_t taddr, uint32_t (&v)[8])   // 16 columns
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16x256b(uint32_t taddr, uint32_t (&v)[16])   // 32 columns
 {
     asm volatile(
         "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
@@ -1132,7 +1144,7 @@ struct XMaps {
 // result rows scattered through out_row_index, optionally into other GPUs' memory; kEpiGeneric = every option
 // tested at run time.  CTAS: 1 = one CTA per tile (128 channels), 2 = a cluster of two CTAs (256 channels).
 template <int MODE, int BL, int EPI, int CTAS>
-__global__ void __launch_bounds__(num_threads(MODE, BL), 1)
+__global__ void __launch_bounds__(num_threads(MODE, BL, EPI), 1)
 gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constant__ CUtensorMap map_w, const KParams p)
 {
     constexpr bool PLAIN = EPI != kEpiGeneric;   // lean arithmetic
@@ -1142,7 +1154,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
     constexpr bool OUT16 = MODE == kModeDequantBf16 && !COMBINE;
     using S = Shape<MODE, CTAS>;
     constexpr bool NZ = BL == kBFractalNz;       // weights come through the loader warps
-    constexpr int RQ = rq_warps(BL), LD0 = num_threads(MODE, BL) / 32 - ld_warps(BL);   // first loader warp
+    constexpr int EPI_WARPS = epi_warps(MODE, EPI), EPI_THREADS = 32 * EPI_WARPS, CHUNK = chunk_tokens(MODE, EPI);
+    constexpr int RQ = rq_warps(BL), LD0 = num_threads(MODE, BL, EPI) / 32 - ld_warps(BL);   // first loader warp
     constexpr bool DUAL = S::kDual;
     constexpr int CH_CTA = S::kCols, MAX_TOK = S::kMaxTok, W_BYTES = S::kWStage;
     constexpr int BLOCK_GROUP = block_group(MODE);
@@ -1456,9 +1469,10 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         // ------------------------------ epilogue: warp -> (TMEM lane quarter, every second chunk of 32 tokens) ------------------------------
         const int quarter = warp & 3;
         const int chalf = (warp - 2) >> 2;
-        const int te = (int)threadIdx.x - 64;  // 0 .. EPI_THREADS-1: the token whose factors this thread fetches
+        const int te = (int)threadIdx.x - 64;  // the token whose factors this thread fetches (below BT)
         uint8_t *my_stage = sh->out_stage + (warp - 2) * WARP_STAGE_BYTES;
-        uint8_t *half_stage = sh->out_stage + chalf * (32 * ROW16_PITCH);
+        uint8_t *half_stage = sh->out_stage + chalf * (CHUNK * ROW16_PITCH);
+        constexpr int CHUNK_STEP = CHUNK * EPI_WARPS / 4;   // tokens from one of a warp's chunks to its next
         // swiglu: the warp of the other half (gate / up) with the same columns and tokens, two lane quarters on; the two share a
         // barrier
         const bool up = !DUAL && quarter >= 2;
@@ -1509,21 +1523,23 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             // all 32), loads its index a chunk ahead - the first one here, while the MMAs run - and settles the address once; the
             // lanes that store a row get it by a shuffle.  With four indices loaded and tested by every lane inside the chunk,
             // scattered rows cost the call a third (K=1024 N=2048, 32 groups of 1000 rows, us: plain 70, scattered 95, now 82).
-            const int my_tk = OUT16 ? quarter * 8 + (lane & 7) : lane;
+            const int my_tk = OUT16 ? quarter * (CHUNK / 4) + (lane & (CHUNK / 4 - 1)) : lane;
             auto load_dest = [&](int tk) -> long long {   // row of the result, -1 for no token
                 if (tk >= tl.rows) return -1;
                 if (COMBINE) return p.row_index_i32 ? (long long)__ldg(reinterpret_cast<const int *>(p.row_index) + tl.row0 + tk)
                                                     : __ldg(reinterpret_cast<const long long *>(p.row_index) + tl.row0 + tk);
                 return p.out_row_index ? __ldg(p.out_row_index + tl.row0 + tk) : (long long)(tl.row0 + tk);
             };
-            long long next_dest = SCATTER ? load_dest(chalf * 32 + my_tk) : 0;
+            long long next_dest = SCATTER ? load_dest(chalf * CHUNK + my_tk) : 0;
             if (te == 0) TRACE(2, it, 0);
             if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[buf], acc_phase, sh, p.status, 400 + buf))) { ok = false; break; }
             if (te == 0) TRACE(2, it, 1);
             tc_fence_after();
             if (MODE != kModeInt32) {
-                sh->tok_scale[buf][te] = COMBINE && p.logit ? (p.x_scale ? __fmul_rn(xs, lg) : lg) : xs;
-                if (COMBINE) sh->tok_logit[buf][te] = lg;
+                if (EPI_THREADS == BT || te < BT) {
+                    sh->tok_scale[buf][te] = COMBINE && p.logit ? (p.x_scale ? __fmul_rn(xs, lg) : lg) : xs;
+                    if (COMBINE) sh->tok_logit[buf][te] = lg;
+                }
                 mbar_arrive(&sh->tok_ready[buf]);
                 if (!__all_sync(0xffffffffu, mbar_wait(&sh->tok_ready[buf], acc_phase, sh, p.status, 500 + buf))) { ok = false; break; }
             }
@@ -1563,7 +1579,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     store_s(act, tc);
                 }
             }
-            for (int tc = chalf * 32; !DUAL && tc < tl.rows && ok; tc += 64) {  // a chunk of 32 tokens
+            for (int tc = chalf * CHUNK; !DUAL && tc < tl.rows && ok; tc += CHUNK_STEP) {
                 if (SWIGLU) {
                     // The gate warp finishes tokens 0..15 of the chunk, the up warp 16..31: each sends the other its values of
                     // the other's tokens.
@@ -1606,7 +1622,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     unsigned long long row_addr = 0;   // of token tc + lane; 0: not stored
                     if (SCATTER) {
                         const long long row = next_dest;
-                        next_dest = load_dest(tc + 64 + lane);
+                        next_dest = load_dest(tc + CHUNK_STEP + lane);
                         if ((unsigned long long)row < p.row_limit) row_addr = reinterpret_cast<unsigned long long>(out + (size_t)row * p.N);
                     }
 #pragma unroll
@@ -1646,16 +1662,17 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     }
                 } else {
                     // 16-bit results.  After the exchange lane l of this warp stores 16 bytes (8 channels) of rows
-                    // quarter * 8 + 2 i + l / 16 of the chunk: a store instruction covers 256 contiguous bytes of two rows.
+                    // 2 i + l / 16 of its quarter of the chunk: a store instruction covers 256 contiguous bytes of two rows.
                     const int pc = lane & 15;
                     const int col = c0 + pc * 8;
-                    uint32_t v0[16], v1[16];
-                    tmem_ld16x256b_x4(taddr + tc, v0);
-                    tmem_ld16x256b_x4(taddr + (16u << 16) + tc, v1);
+                    constexpr int N8 = CHUNK / 8;   // 8-token pieces of the chunk
+                    uint32_t v0[4 * N8], v1[4 * N8];
+                    tmem_ld16x256b(taddr + tc, v0);
+                    tmem_ld16x256b(taddr + (16u << 16) + tc, v1);
                     unsigned long long row_addr = 0;   // of token tc + my_tk; 0: not stored
                     if (SCATTER) {
                         long long row = next_dest, gpu_field = 0;
-                        next_dest = load_dest(tc + 64 + my_tk);
+                        next_dest = load_dest(tc + CHUNK_STEP + my_tk);
                         uint16_t *obase = reinterpret_cast<uint16_t *>(p.out);
                         if (p.num_peers > 0) {  // high bits: which GPU's buffer, low 40 bits: row in it
                             gpu_field = row >> 40;
@@ -1666,7 +1683,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                         if (tc + my_tk < tl.rows) {
                             if ((unsigned long long)row < p.row_limit && (p.num_peers <= 0 || (unsigned long long)gpu_field < (unsigned long long)p.num_peers)) {
                                 row_addr = reinterpret_cast<unsigned long long>(obase + (size_t)row * p.N);
-                            } else if (lane < 8 && atomicCAS(p.status, kStatusOk, kStatusBadIndex) == kStatusOk) {
+                            } else if (lane < CHUNK / 4 && atomicCAS(p.status, kStatusOk, kStatusBadIndex) == kStatusOk) {
                                 p.status[1] = (int)blockIdx.x;
                                 p.status[2] = 800;
                                 p.status[3] = tl.row0 + tc + my_tk;
@@ -1676,38 +1693,37 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     tmem_ld_wait();
                     // Of every 8 tokens this lane holds two (4 i + its column pair) for four channels (lane / 4 + 8 j):
                     // (acc * w_scale) * x_scale, optional bias, optional activation, then one rounding
-                    float o[4][4][2];
+                    float o[N8][4][2];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < N8; ++i) {
                         const f32x2 ts = *reinterpret_cast<const f32x2 *>(tok + tc + i * 8 + (lane & 3) * 2);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            {
-                                int a0 = (int)(j < 2 ? v0[i * 4 + j * 2] : v1[i * 4 + (j - 2) * 2]);
-                                int a1 = (int)(j < 2 ? v0[i * 4 + j * 2 + 1] : v1[i * 4 + (j - 2) * 2 + 1]);
-                                if (!PLAIN) { a0 += bias_i[j]; a1 += bias_i[j]; }
-                                f32x2 t = mul2(pair2(__int2float_rn(a0), __int2float_rn(a1)), pair2(wsc[j], wsc[j]));
-                                if (PLAIN || p.x_scale) t = mul2(t, ts);
-                                const float2 f = unpair2(t);
-                                o[i][j][0] = f.x;
-                                o[i][j][1] = f.y;
-                            }
+                        for (int j = 0; j < 4; ++j) {
+                            int a0 = (int)(j < 2 ? v0[i * 4 + j * 2] : v1[i * 4 + (j - 2) * 2]);
+                            int a1 = (int)(j < 2 ? v0[i * 4 + j * 2 + 1] : v1[i * 4 + (j - 2) * 2 + 1]);
+                            if (!PLAIN) { a0 += bias_i[j]; a1 += bias_i[j]; }
+                            f32x2 t = mul2(pair2(__int2float_rn(a0), __int2float_rn(a1)), pair2(wsc[j], wsc[j]));
+                            if (PLAIN || p.x_scale) t = mul2(t, ts);
+                            const float2 f = unpair2(t);
+                            o[i][j][0] = f.x;
+                            o[i][j][1] = f.y;
+                        }
                     }
                     if (!PLAIN) {
                         if (p.bias_dtype == kBF16) {
 #pragma unroll
-                            for (int i = 0; i < 4; ++i)
+                            for (int i = 0; i < N8; ++i)
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) {
                                     o[i][j][0] = __fadd_rn(o[i][j][0], bias_f[j]);
                                     o[i][j][1] = __fadd_rn(o[i][j][1], bias_f[j]);
                                 }
                         }
-                        activate(p.act_type, reinterpret_cast<float(&)[32]>(o));
+                        activate(p.act_type, reinterpret_cast<float(&)[8 * N8]>(o));
                     }
                     const bool f16 = !PLAIN && p.out_f16;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < N8; ++i) {
                         uint32_t pk[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) pk[j] = f16 ? pack_f16x2(o[i][j][0], o[i][j][1]) : pack_bf16x2(o[i][j][0], o[i][j][1]);
@@ -1716,8 +1732,8 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     }
                     if (!group_sync(grp_bar, grp_phase, sh, p.status, lane, 720)) { ok = false; break; }
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int r = quarter * 8 + i * 2 + (lane >> 4);
+                    for (int i = 0; i < N8; ++i) {
+                        const int r = quarter * (CHUNK / 4) + i * 2 + (lane >> 4);
                         const uint4 val = *reinterpret_cast<const uint4 *>(half_stage + r * ROW16_PITCH + pc * 16);
                         if (SCATTER) {
                             uint16_t *row = reinterpret_cast<uint16_t *>(__shfl_sync(0xffffffffu, row_addr, i * 2 + (lane >> 4)));
@@ -1894,7 +1910,7 @@ cudaError_t launch_variant(const Plan &plan, const KParams &kp, cudaStream_t str
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CTAS == 2 ? (plan.num_sms & ~1) : plan.num_sms), 1, 1);
-    cfg.blockDim = dim3(num_threads(MODE, BL), 1, 1);
+    cfg.blockDim = dim3(num_threads(MODE, BL, EPI), 1, 1);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
