@@ -79,6 +79,7 @@ struct Problem {
 struct Plan {
     int path = kPathSimt;
     int num_sms = 0;
+    bool beside_init = false;           // the combine's kernel follows the one that initialises its result
     int ctas = 2;                       // 2 = CTA pairs (256 channels per tile), 1 = single CTAs (128 channels)
     size_t ws_bytes = 0;
     size_t off_status = 0, off_amax = 0, off_stage = 0, off_done = 0;
@@ -130,8 +131,9 @@ bool sm100_shape_ok(const Problem &p);
 cudaError_t sm100_encode_maps(const Problem &p, Plan &plan);
 cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStream_t stream);
 // gmm_simt.cu
-// Initial contents of the combined result (PreProcess of grouped_matmul_finalize_routing.h:208-258).
-cudaError_t combine_init_launch(const Problem &p, cudaStream_t stream);
+// Initial contents of the combined result (PreProcess of grouped_matmul_finalize_routing.h:208-258) and of the status record (256
+// bytes).
+cudaError_t combine_init_launch(const Problem &p, int *status, cudaStream_t stream);
 cudaError_t simt_launch(const Problem &p, Plan &plan, void *workspace, cudaStream_t stream);
 
 // SMs of the current device (cached per device); 0 on error.
