@@ -13,11 +13,11 @@
 //   scan    - per expert (one CTA per 32 experts): exclusive prefix over the blocks; the CTA that finishes last then
 //             scans over the experts: start of every expert's rows, the counts output, the number of rows
 //   scatter - every pair finds its place: expert start + earlier blocks + earlier pairs of its block
-//             (__match_any_sync ranks the lanes of a warp; the warps are ranked through a per-warp counter table, or take
+//             (ballots rank the lanes of a warp; the warps are ranked through a per-warp counter table, or take
 //             turns when the active range is too wide for one), which keeps the order of equal keys
 //   gather  - one CTA per token: the row is read once into registers, (quantised,) and stored at the output row of each
-//             of its k pairs; few tokens with smooth scales, and few pairs without, take one CTA per pair; shapes that do not
-//             fit the register tile one CTA per output row
+//             of its k pairs; few tokens with smooth scales, and few pairs without, take one CTA per pair; many tokens with few
+//             slots one CTA per SM, rows staged in shared memory; shapes that do not fit the register tile one CTA per output row
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -190,11 +190,11 @@ __device__ void expert_scan(const RoutingParams &p, const int *tot, int *first, 
 {
     const int e = threadIdx.x;
     const int c = e < p.range ? tot[e] : 0;
-    int sum_c, sum_nz;
+    int sum_c, sum_nz = 0, inc_nz = 0;
     const int inc_c = block_scan_1024(c, warp_sums, &sum_c);
-    const int inc_nz = block_scan_1024(c != 0 ? 1 : 0, warp_sums, &sum_nz);
     if (e < p.range) first[e] = inc_c - c;
     if (!write_counts) return;
+    if (p.count_type == 2) inc_nz = block_scan_1024(c != 0 ? 1 : 0, warp_sums, &sum_nz);
     if (e < p.range) {
         if (p.count_type == 1) {
             p.counts_out[e] = c;
@@ -211,6 +211,19 @@ __device__ void expert_scan(const RoutingParams &p, const int *tot, int *first, 
         }
     }
     if (threadIdx.x == 0) *p.total = sum_c;
+}
+
+// The lanes whose expert `e` (below `range`) is this lane's, one ballot per bit of its number; lanes without one (-1) keep to
+// themselves through the sign.  With 32 warps on one SM __match_any_sync takes about 2 us.
+__device__ __forceinline__ unsigned same_expert(int e, int range)
+{
+    unsigned peers = __ballot_sync(0xffffffffu, e >= 0);
+    if (e < 0) peers = ~peers;
+    for (int b = 0; (range - 1) >> b; ++b) {
+        const unsigned ones = __ballot_sync(0xffffffffu, (e >> b) & 1);
+        peers &= (e >> b) & 1 ? ones : ~ones;
+    }
+    return peers;
 }
 
 constexpr int kWarpTableRange = 256;  // up to this many active experts the scatter keeps one counter per warp and expert
@@ -262,7 +275,7 @@ __global__ void __launch_bounds__(kPairsPerBlock) routing_scatter_kernel(const R
     int before = 0;  // pairs of this block with the same expert that come earlier
     __syncthreads();
     if (PER_WARP) {
-        const unsigned peers = __match_any_sync(0xffffffffu, e);
+        const unsigned peers = same_expert(e, p.range);
         const int rank = __popc(peers & ((1u << lane) - 1u));
         if (e >= 0 && rank == 0) running[warp * p.range + e] = __popc(peers);
         __syncthreads();
@@ -549,6 +562,204 @@ __global__ void __launch_bounds__(THREADS, MINB) routing_quant_token_kernel(cons
     }
 }
 
+// Two values of quant_fast where its reciprocal is not 0: |v / scale| rounds to at most 127 then, so nothing is clamped.
+__device__ __forceinline__ unsigned long long pack_f32x2(float a, float b)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ void quant_pair(float v0, float v1, unsigned long long neg_scale, unsigned long long rcp, int &q0, int &q1)
+{
+    const unsigned long long v = pack_f32x2(v0, v1);
+    unsigned long long q = mul_f32x2(v, rcp);
+    q = fma_f32x2(fma_f32x2(q, neg_scale, v), rcp, q);
+    q = fma_f32x2(fma_f32x2(q, neg_scale, v), rcp, q);
+    const uint32_t a = (uint32_t)q & 0xffffe000u, b = (uint32_t)(q >> 32) & 0xffffe000u;
+    q0 = __float2int_rz(__fadd_rn(__uint_as_float(a), __uint_as_float(0x3f000000u | (a & 0x80000000u))));
+    q1 = __float2int_rz(__fadd_rn(__uint_as_float(b), __uint_as_float(0x3f000000u | (b & 0x80000000u))));
+}
+
+// Largest magnitude of 16 bytes of a row and `m`, as bits of T pairs; NaN is passed over, as fmaxf does.
+template <typename T>
+__device__ __forceinline__ uint32_t max_abs16(const uint4 &u, uint32_t m);
+template <>
+__device__ __forceinline__ uint32_t max_abs16<float>(const uint4 &u, uint32_t m)
+{
+    float f = fmaxf(__uint_as_float(m), fabsf(__uint_as_float(u.x)));
+    f = fmaxf(fmaxf(f, fabsf(__uint_as_float(u.y))), fmaxf(fabsf(__uint_as_float(u.z)), fabsf(__uint_as_float(u.w))));
+    return __float_as_uint(f);
+}
+template <>
+__device__ __forceinline__ uint32_t max_abs16<__nv_bfloat16>(const uint4 &u, uint32_t m)
+{
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t a = w[i] & 0x7fff7fffu;
+        const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162 *>(&m), *reinterpret_cast<const __nv_bfloat162 *>(&a));
+        m = *reinterpret_cast<const uint32_t *>(&r);
+    }
+    return m;
+}
+template <>
+__device__ __forceinline__ uint32_t max_abs16<__half>(const uint4 &u, uint32_t m)
+{
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t a = w[i] & 0x7fff7fffu;
+        const __half2 r = __hmax2(*reinterpret_cast<const __half2 *>(&m), *reinterpret_cast<const __half2 *>(&a));
+        m = *reinterpret_cast<const uint32_t *>(&r);
+    }
+    return m;
+}
+template <typename T>
+__device__ __forceinline__ float max_of_bits(uint32_t m);
+template <>
+__device__ __forceinline__ float max_of_bits<float>(uint32_t m) { return __uint_as_float(m); }
+template <>
+__device__ __forceinline__ float max_of_bits<__nv_bfloat16>(uint32_t m) { return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)); }
+template <>
+__device__ __forceinline__ float max_of_bits<__half>(uint32_t m)
+{
+    const float2 t = __half22float2(*reinterpret_cast<const __half2 *>(&m));
+    return fmaxf(t.x, t.y);
+}
+
+// The quantising gather without smooth scales where the rows read are a good part of the traffic (see the rule at its launch):
+// one CTA per SM, two teams of 256 threads.  A team quantises one token after the other into a ring of batches in shared memory
+// (the next row is on its way meanwhile); a batch's rows go out by bulk copies of whole rows, one per (token, slot) pair.  Only
+// the copies need the row positions: the first batches are read and quantised while the kernels that place the pairs still run,
+// for which one CTA per token had room for 592 tokens on the whole chip.
+constexpr int kTeams = 2, kTeam = 256;
+constexpr int kStageBytes = 184 * 1024;         // leaves room for a block of the placing kernels on the same SM
+constexpr int kRing = 6, kFirstSend = 4;        // batches in shared memory; batches that are quantised before the positions are waited for
+constexpr int kMaxBatch = 8;                    // tokens
+template <typename T, int NCH>
+__global__ void __launch_bounds__(kTeams * kTeam, sizeof(T) == 2 ? 2 : 1) routing_quant_stage_kernel(const RoutingParams p, int batch)
+{
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int G = 16 / VEC;  // 16-byte loads that make one 16-byte store of int8: a thread owns G adjacent ones
+    extern __shared__ __align__(16) uint8_t stage[];   // [team][ring][batch][h]
+    __shared__ float red[kTeams][2][kTeam / 32];
+    __shared__ float row_scale[kTeams][kRing][kMaxBatch];
+    const int team = threadIdx.x / kTeam, tid = threadIdx.x % kTeam, lane = threadIdx.x & 31;
+    const int n = (int)(p.pairs / p.k), chunks = p.h / VEC;
+    const int first = blockIdx.x * kTeams + team, step = gridDim.x * kTeams;
+    uint8_t *const rows = stage + (size_t)team * kRing * batch * p.h;
+    auto load = [&](int token, uint4 (&r)[NCH]) {
+        const uint4 *row = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.x) + (size_t)token * p.h);
+#pragma unroll
+        for (int i = 0; i < NCH; ++i) {
+            const int c = (tid + (i / G) * kTeam) * G + (i % G);
+            r[i] = c < chunks ? __ldg(row + c) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(kTeam) : "memory"); };
+    // the copies of batch b's `cnt` tokens, one lane each of the team's first warp, as one bulk group
+    auto send = [&](int b, int cnt) {
+        const int at = b % kRing, token0 = first + b * batch * step;
+        for (int i = lane; i < cnt * p.k; i += 32) {
+            const int slot = i / p.k, token = token0 + slot * step;
+            const int pos = p.pair_pos[(long long)token * p.k + (i - slot * p.k)];
+            if (pos < 0) continue;
+            p.expanded_scale[pos] = row_scale[team][at][slot];
+            const uint32_t src = (uint32_t)__cvta_generic_to_shared(rows + (size_t)(at * batch + slot) * p.h);
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                         ::"l"(reinterpret_cast<int8_t *>(p.expanded_x) + (size_t)pos * p.h), "r"(src), "r"(p.h) : "memory");
+        }
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    };
+    uint4 raw[NCH], next[NCH];
+    if (first < n) load(first, next);
+    int at = 0, slot = 0, b = 0;
+    for (int token = first, i = 0; token < n; token += step, ++i) {
+        // the slots' copies of a ring ago have been read (the issuing lanes wait, the barrier below tells the others)
+        if (slot == 0 && b >= kRing && tid < 32) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kRing - 1) : "memory");
+        uint32_t mbits = 0;
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            raw[c] = next[c];
+            mbits = max_abs16<T>(raw[c], mbits);
+        }
+        if (token + step < n) load(token + step, next);
+        float amax = max_of_bits<T>(mbits);
+        amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));   // never negative, never NaN
+        if (lane == 0) red[team][i & 1][tid >> 5] = amax;
+        team_sync();
+#pragma unroll
+        for (int w = 0; w < kTeam / 32; ++w) amax = fmaxf(amax, red[team][i & 1][w]);
+        const float scale = __fdiv_rn(amax, 127.0f), rcp = exact_div_rcp(scale);
+        if (tid == 0) row_scale[team][at][slot] = scale;
+        uint32_t w[NCH][VEC / 4];
+        if (rcp != 0.0f) {
+            const unsigned long long ns = pack_f32x2(-scale, -scale), r2 = pack_f32x2(rcp, rcp);
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                float v[VEC];
+                unpack16<T>(raw[c], v);
+#pragma unroll
+                for (int e4 = 0; e4 < VEC; e4 += 4) {
+                    int q[4];
+                    quant_pair(v[e4], v[e4 + 1], ns, r2, q[0], q[1]);
+                    quant_pair(v[e4 + 2], v[e4 + 3], ns, r2, q[2], q[3]);
+                    w[c][e4 / 4] = pack4(q[0], q[1], q[2], q[3]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                float v[VEC];
+                unpack16<T>(raw[c], v);
+#pragma unroll
+                for (int e4 = 0; e4 < VEC; e4 += 4)
+                    w[c][e4 / 4] = pack4(quant_fast(v[e4], scale, 0.0f), quant_fast(v[e4 + 1], scale, 0.0f),
+                                         quant_fast(v[e4 + 2], scale, 0.0f), quant_fast(v[e4 + 3], scale, 0.0f));
+            }
+        }
+        uint8_t *const dst = rows + (size_t)(at * batch + slot) * p.h;
+#pragma unroll
+        for (int c = 0; c < NCH; c += G) {
+            const int pc = (tid + (c / G) * kTeam) * G;
+            if (pc < chunks) {
+                uint4 o;
+                if (VEC == 8) o = make_uint4(w[c][0], w[c][VEC / 4 - 1], w[c + G - 1][0], w[c + G - 1][VEC / 4 - 1]);
+                else o = make_uint4(w[c][0], w[c + 1 < NCH ? c + 1 : c][0], w[c + 2 < NCH ? c + 2 : c][0], w[c + G - 1][0]);
+                *reinterpret_cast<uint4 *>(dst + (size_t)pc * VEC) = o;
+            }
+        }
+        const bool last = token + step >= n;
+        if (++slot == batch || last) {  // the batch is complete
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // its rows, before the copies read them
+            team_sync();
+            if (tid < 32 && (b >= kFirstSend - 1 || last)) {
+                if (b < kFirstSend) {
+                    pdl_wait();  // the row positions are complete
+                    for (int e = 0; e < b; ++e) send(e, batch);
+                }
+                send(b, slot);
+            }
+            if (++at == kRing) at = 0;
+            slot = 0;
+            ++b;
+        }
+    }
+    if (tid < 32) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // One CTA per token: the row is read once, 16 bytes per thread and step, and stored at the output row of each pair.
 __global__ void __launch_bounds__(128) routing_copy_token_kernel(const RoutingParams p, int row_bytes)
 {
@@ -595,6 +806,21 @@ __global__ void __launch_bounds__(128) routing_copy_kernel(const RoutingParams p
         for (size_t c = threadIdx.x; c < row_bytes; c += blockDim.x) dst[c] = src[c];
     }
     if (p.scale && p.expanded_scale && threadIdx.x == 0) p.expanded_scale[pos] = __ldg(p.scale + j / p.k);
+}
+
+template <typename T, int NCH>
+cudaError_t launch_staged(const RoutingParams &p, int batch, int sms, cudaStream_t stream, bool overlap)
+{
+    auto kern = routing_quant_stage_kernel<T, NCH>;
+    static unsigned long long done_mask = 0;   // per device; the attribute is idempotent, so a race only repeats the call
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!((done_mask >> (dev & 63)) & 1ull)) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
+        if (e != cudaSuccess) return e;
+        done_mask |= 1ull << (dev & 63);
+    }
+    return launch_pdl(kern, (unsigned)sms, kTeams * kTeam, (size_t)kRing * kTeams * batch * p.h, stream, overlap, p, batch);
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
@@ -668,15 +894,26 @@ cudaError_t init_routing_launch(const InitRoutingProblem &r, void *workspace, si
         const int sms = device_sm_count();
         if (sms <= 0) return cudaErrorNoDevice;
         p.slots = (r.scale ? r.n < sms : pairs <= sms) ? 1 : (int)r.k;
+        // Rows through shared memory where reading is a good part of the traffic, k up to 4 with 16-bit rows and up to 8 with 32-bit
+        // ones: with more slots the pass is nothing but writes, which gain nothing from rows that were read ahead.  Rows below 4 KB
+        // leave threads idle, fewer than four tokens per SM leave teams idle.  us (per token / staged), 4096 tokens, h = 7168: bf16
+        // k=1 33.7 / 30.0, k=4 40.9 / 39.2, k=8 54.7 / 57.6, f32 k=4 51.5 / 42.8, k=8 65.6 / 62.3; h = 2048 bf16 k=2 32.5 / 27.7, k=4
+        // 35.6 / 30.8; h = 1024 f32 k=2 35.0 / 25.3, k=8 45.9 / 32.8, bf16 k=4 34.2 / 42.7; 600 tokens h = 7168 bf16 k=4 12.2 / 11.7,
+        // k=8 14.5 / 16.0, h = 2048 f32 k=8 11.7 / 10.3.
+        const bool staged = fast && !r.scale && r.n >= 4ll * sms && r.h * eb >= 4096 && r.k <= (eb == 4 ? 8 : 4);
+        const int fit = (int)(kStageBytes / (kRing * kTeams * r.h)), batch = staged ? (fit < kMaxBatch ? fit : kMaxBatch) : 0;
         const unsigned gather_grid = (unsigned)(p.slots == 1 ? pairs : r.n);
         if (r.x_dtype == kF32) {
-            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<float, 8, 256>, gather_grid, 256, 0, stream, overlap, p);
+            if (staged) launch_err = launch_staged<float, 8>(p, batch, sms, stream, overlap);
+            else if (fast) launch_err = launch_pdl(routing_quant_token_kernel<float, 8, 256>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<float><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else if (r.x_dtype == kF16) {
-            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__half, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
+            if (staged) launch_err = launch_staged<__half, 4>(p, batch, sms, stream, overlap);
+            else if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__half, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<__half><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else if (r.x_dtype == kBF16) {
-            if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__nv_bfloat16, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
+            if (staged) launch_err = launch_staged<__nv_bfloat16, 4>(p, batch, sms, stream, overlap);
+            else if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__nv_bfloat16, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<__nv_bfloat16><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else {
             return cudaErrorInvalidValue;

@@ -795,6 +795,38 @@ def test_init_routing_launch_shape_edges(oracle, n, k, E, rng, smooth):
                            row_idx_type=count_type - 1, count_type=count_type)
 
 
+@pytest.mark.parametrize("n,k,h,x_kind", [
+    (591, 4, 2048, "bf16"), (592, 4, 2048, "bf16"), (592, 5, 2048, "bf16"), (592, 4, 2032, "bf16"),   # either side of the staging rule
+    (593, 3, 7168, "bf16"), (4500, 1, 7168, "f16"),     # one ring of slots per team, and slots that are used again
+    (2000, 2, 8192, "f32"), (700, 8, 1024, "f32"),      # widest and narrowest rows
+])
+def test_init_routing_staged_rows(oracle, n, k, h, x_kind):
+    check_init_routing(oracle, n, k, h, 64, (8, 56), 90 + k, x_kind=x_kind, row_idx_type=k & 1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_init_routing_staged_special_rows(dtype):
+    """Rows of infinities, NaN, denormals and the type's largest value: the staged kernel gives what the one for few tokens does."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    big, tiny = torch.finfo(dtype).max, torch.finfo(dtype).smallest_normal
+    g = torch.Generator(device=dev)
+    g.manual_seed(3)
+    rows = torch.randn(12, 2048, device=dev, generator=g).to(dtype)
+    rows[0] = 0
+    rows[1, 5], rows[2, 5], rows[3, 7] = float("inf"), float("-inf"), float("nan")
+    rows[4] = float("nan")
+    rows[5, 9], rows[6, 9] = big, -big
+    rows[7] = rows[7] * tiny
+    rows[8] = tiny / 4
+    rows[9, 1], rows[9, 2] = float("inf"), float("nan")
+    idx = torch.zeros(12, 1, dtype=torch.int32, device=dev)
+    q, _, _, s = ops.moe_init_routing_v3(rows, idx, expert_num=2, active_expert_range=(0, 2))
+    q2, _, _, s2 = ops.moe_init_routing_v3(rows.repeat(60, 1), idx.repeat(60, 1), expert_num=2, active_expert_range=(0, 2))
+    torch.cuda.synchronize()
+    assert torch.equal(q2, q.repeat(60, 1)) and torch.equal(s2.view(torch.int32), s.repeat(60).view(torch.int32))
+
+
 def test_init_routing_without_quantisation(oracle):
     check_init_routing(oracle, 200, 4, 256, 32, (0, 32), 76, quant=False, per_token_scale=True)
     check_init_routing(oracle, 200, 4, 256, 32, (4, 20), 77, quant=False, x_kind="int8", row_idx_type=0)
