@@ -1,4 +1,4 @@
-"""Builds libgmm_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libgmm_b200.so (the C-ABI library) in-tree with nvcc for sm_100a, and the extension module that describes tensors to it.
 
 Run as ``python -m ops_transformer_b200._build`` or through ``__graft_entry__.build()``.
 """
@@ -13,6 +13,8 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG_DIR)
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libgmm_b200.so")
+DESCRIBE_PATH = os.path.join(PKG_DIR, "_describe.so")
+DESCRIBE_SOURCE = os.path.join(CSRC, "describe.cpp")
 
 SOURCES = ["gmm_sm100.cu", "gmm_simt.cu", "gmm_noalloc.cu", "ep_peer.cu", "moe_init_routing.cu", "view_copy.cu", "acl_shim.cpp", "op_api.cpp"]
 HEADERS = ["gmm_common.h", "acl_shim.h"]
@@ -44,7 +46,29 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_describe(force: bool = False) -> str:
+    """The extension module that writes a call's tensors into its description; g++ against torch's headers."""
+    import sysconfig
+
+    import torch
+    stale = not os.path.exists(DESCRIBE_PATH) or os.path.getmtime(DESCRIBE_PATH) < os.path.getmtime(DESCRIBE_SOURCE)
+    if not force and not stale:
+        return DESCRIBE_PATH
+    root = os.path.dirname(torch.__file__)
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"),
+           "-o", DESCRIBE_PATH, DESCRIBE_SOURCE, "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed building _describe.so")
+    return DESCRIBE_PATH
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
+    build_describe(force)
     if not force and not needs_build():
         return LIB_PATH
     extra = os.environ.get("GMM_B200_NVCC_EXTRA", "").split()  # e.g. -DGMM_DEBUG_KNOBS for kernel experiments

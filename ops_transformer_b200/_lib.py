@@ -135,5 +135,20 @@ def lib():
     return _LIB
 
 
+_DESCRIBE = None
+
+
+def describe(*items) -> bytes:
+    """The packed description of ``items`` (csrc/describe.cpp): int64 words as gmmB200Call takes them."""
+    global _DESCRIBE
+    if _DESCRIBE is None:
+        try:
+            from . import _describe
+        except ImportError as e:
+            raise LibraryMissing(f"the native description module is missing ({e}): build it with `python -m ops_transformer_b200._build`.") from e
+        _DESCRIBE = _describe.describe
+    return _DESCRIBE(*items)
+
+
 def last_error() -> str:
     return lib().aclGetRecentErrMsg().decode("utf-8", "replace")

@@ -197,39 +197,19 @@ def check_status(workspace: Optional[torch.Tensor], stream=None) -> None:
 
 def _put(words: list, t: Optional[torch.Tensor], fmt: int = ACL_FORMAT_ND, view_dims: Optional[Sequence[int]] = None) -> None:
     """Append one tensor to a packed description (gmmB200Call, include/gmm_b200.h); the same view as ``create_tensor``."""
-    if t is None:
-        words.append(-1)
-        return
-    shape = t.shape
-    rank = len(shape)
-    if rank > 8:
-        raise MemoryError("a tensor of more than 8 dimensions cannot be described")
-    if view_dims is None:
-        words += (rank, t.data_ptr(), _DTYPES[t.dtype], fmt)
-        words += shape
-        words += t.stride()
-    else:
-        strides = [1] * len(view_dims)
-        for i in range(len(view_dims) - 2, -1, -1):
-            strides[i] = strides[i + 1] * view_dims[i + 1]
-        words += (len(view_dims), t.data_ptr(), _DTYPES[t.dtype], fmt)
-        words += view_dims
-        words += strides
-    words.append(rank)
-    words += shape
+    words += array.array("q", _lib.describe((t, fmt, view_dims)))
 
 
-def _put_ints(words: list, values: Optional[Sequence[int]]) -> None:
-    if values is None:
-        words.append(-1)
-    else:
-        words.append(len(values))
-        words += values
+def _ints(values: Optional[Sequence[int]]) -> Optional[list]:
+    return None if values is None else list(values)
 
 
-def _call(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream,
+def _call(op: int, name: str, words, device: torch.device, workspace: Optional[torch.Tensor], stream,
           options: Optional[LaunchOptions]) -> Optional[torch.Tensor]:
-    """Both phases of operator ``name`` on the packed description; returns the workspace that was used (None if none)."""
+    """Both phases of operator ``name`` on the packed description (bytes or a list of its words); returns the workspace that was
+    used (None if none)."""
+    if not isinstance(words, bytes):
+        words = array.array("q", words).tobytes()
     on_gpu = device.type == "cuda"
     handle = _gpu_stream_handle(stream) if on_gpu else 0
     if workspace is not None:
@@ -239,15 +219,14 @@ def _call(op: int, name: str, words: list, device: torch.device, workspace: Opti
         return _enqueue(op, name, words, device, None, stream, handle, options, slot)
 
 
-def _enqueue(op: int, name: str, words: list, device: torch.device, workspace: Optional[torch.Tensor], stream, handle: int,
+def _enqueue(op: int, name: str, words: bytes, device: torch.device, workspace: Optional[torch.Tensor], stream, handle: int,
              options: Optional[LaunchOptions], slot: Optional[_Slot]) -> Optional[torch.Tensor]:
     L = _lib.lib()
-    packed = array.array("q", words)
     res = _lib.CallResult()
     # validation needs no device: tensors that are not on one are planned only, so that what is wrong with them is reported first
     on_gpu = device.type == "cuda"
     buf = None if not on_gpu else workspace if slot is None else slot.buf
-    rc = L.gmmB200Call(op if slot is None else op | _lib.OP_POOLED, packed.buffer_info()[0], len(packed), buf.data_ptr() if buf is not None else None,
+    rc = L.gmmB200Call(op if slot is None else op | _lib.OP_POOLED, words, len(words) // 8, buf.data_ptr() if buf is not None else None,
                        buf.numel() if buf is not None else 0, C.byref(options) if options is not None else None, handle, C.byref(res))
     if rc == ACLNN_SUCCESS and res.stage == _lib.STAGE_PLANNED:
         ex = C.c_void_p(res.executor)
@@ -288,19 +267,14 @@ def grouped_matmul_v4(x: torch.Tensor, weight: torch.Tensor, scale: Optional[tor
     nz = weight_format == ACL_FORMAT_FRACTAL_NZ or api == "WeightNz"
     if out is None and not out_peers:
         n_out = weight.shape[1] * 32 if (nz and weight.dim() == 5) else weight.shape[2]
-        out = torch.empty((x.shape[0], n_out), dtype=out_dtype, device=x.device)
+        out = x.new_empty((x.shape[0], n_out), dtype=out_dtype)
     if out_row_index is not None:
         return _grouped_matmul_flat(x, weight, scale, per_token_scale, group_list, bias, group_list_type, act_type, out,
                                     out_row_index, stream, workspace, return_workspace, out_peers, nz, options, out_rows)
     if api not in _lib.OP_GMM:
         raise ValueError(f"unknown api {api!r}")
-    words = []
-    _put(words, x)
-    _put(words, weight, ACL_FORMAT_FRACTAL_NZ if nz else ACL_FORMAT_ND)
-    for t in (bias, scale, per_token_scale, group_list, out):
-        _put(words, t)
-    words += (split_item, group_type, group_list_type, act_type, quant_group_size)
-    _put_ints(words, tuning_config)
+    words = _lib.describe(x, (weight, ACL_FORMAT_FRACTAL_NZ if nz else ACL_FORMAT_ND, None), bias, scale, per_token_scale, group_list, out,
+                          split_item, group_type, group_list_type, act_type, quant_group_size, _ints(tuning_config))
     workspace = _call(_lib.OP_GMM[api], "aclnnGroupedMatmul" + api, words, x.device, workspace, stream, options)
     return (out, workspace) if return_workspace else out
 
@@ -363,14 +337,10 @@ def grouped_matmul_swiglu_quant(x: torch.Tensor, weight: torch.Tensor, weight_sc
     M = x.shape[0]
     N = weight_scale.shape[1] if weight_scale.dim() == 2 else 0
     if output is None:
-        output = torch.empty((M, N // 2), dtype=torch.int8, device=x.device)
+        output = x.new_empty((M, N // 2), dtype=torch.int8)
     if output_scale is None:
-        output_scale = torch.empty((M,), dtype=torch.float32, device=x.device)
-    words = []
-    _put(words, x)
-    _put(words, weight, weight_format)
-    for t in (bias, offset, weight_scale, x_scale, group_list, output, output_scale):
-        _put(words, t)
+        output_scale = x.new_empty((M,), dtype=torch.float32)
+    words = _lib.describe(x, (weight, weight_format, None), bias, offset, weight_scale, x_scale, group_list, output, output_scale)
     workspace = _call(_lib.OP_SWIGLU_QUANT[api], "aclnnGroupedMatmulSwigluQuant" + api, words, x.device, workspace, stream, options)
     return (output, output_scale, workspace) if return_workspace else (output, output_scale)
 
@@ -391,14 +361,10 @@ def grouped_matmul_finalize_routing(x: torch.Tensor, weight_nz: torch.Tensor, sc
     E, n1, k1 = weight_nz.shape[0], weight_nz.shape[1], weight_nz.shape[2]
     N, K = n1 * 32, k1 * 16
     if out is None:
-        out = torch.empty((batch, N), dtype=torch.float32, device=x.device)
-    words = []
-    _put(words, x)
-    _put(words, weight_nz, ACL_FORMAT_FRACTAL_NZ, [E, K, N] if view_3d else None)
-    for t in (scale, bias, pertoken_scale, group_list, shared_input, logit, row_index, out):
-        _put(words, t)
-    words += (struct.unpack("<I", bytes(C.c_float(shared_input_weight)))[0], shared_input_offset, group_list_type)
-    _put_ints(words, tuning_config)
+        out = x.new_empty((batch, N), dtype=torch.float32)
+    words = _lib.describe(x, (weight_nz, ACL_FORMAT_FRACTAL_NZ, [E, K, N] if view_3d else None), scale, bias, pertoken_scale, group_list,
+                          shared_input, logit, row_index, out, struct.unpack("<I", bytes(C.c_float(shared_input_weight)))[0],
+                          shared_input_offset, group_list_type, _ints(tuning_config))
     workspace = _call(_lib.OP_FINALIZE_ROUTING[api], "aclnnGroupedMatmulFinalizeRoutingWeightNz" + api, words, x.device, workspace, stream,
                       options)
     return (out, workspace) if return_workspace else out
@@ -446,17 +412,14 @@ def moe_init_routing_v3(x: torch.Tensor, expert_idx: torch.Tensor, *, expert_num
     k = expert_idx.shape[1]
     start, end = active_expert_range
     if outputs is None:
-        ex = torch.empty((n * k, h), dtype=torch.int8 if quant_mode == 1 else x.dtype, device=x.device)
-        ri = torch.empty((n * k,), dtype=torch.int32, device=x.device)
-        cnt = torch.empty((end - start,) if expert_tokens_num_type == 1 else (expert_num, 2), dtype=torch.int64, device=x.device)
-        es = torch.empty((n * k,), dtype=torch.float32, device=x.device)
+        ex = x.new_empty((n * k, h), dtype=torch.int8 if quant_mode == 1 else x.dtype)
+        ri = x.new_empty((n * k,), dtype=torch.int32)
+        cnt = x.new_empty((end - start,) if expert_tokens_num_type == 1 else (expert_num, 2), dtype=torch.int64)
+        es = x.new_empty((n * k,), dtype=torch.float32)
     else:
         ex, ri, cnt, es = outputs
-    words = []
-    for t in (x, expert_idx, scale, offset, ex, ri, cnt, es):
-        _put(words, t)
-    words += (n * k if active_num is None else active_num, expert_capacity, expert_num, drop_pad_mode, expert_tokens_num_type,
-              1 if expert_tokens_num_flag else 0, quant_mode, row_idx_type)
-    _put_ints(words, active_expert_range)
+    words = _lib.describe(x, expert_idx, scale, offset, ex, ri, cnt, es, n * k if active_num is None else active_num, expert_capacity,
+                          expert_num, drop_pad_mode, expert_tokens_num_type, 1 if expert_tokens_num_flag else 0, quant_mode,
+                          row_idx_type, _ints(active_expert_range))
     _call(_lib.OP_MOE_INIT_ROUTING, "aclnnMoeInitRoutingV3", words, x.device, workspace, stream, None)
     return ex, ri, cnt, es

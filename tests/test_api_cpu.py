@@ -7,6 +7,7 @@ import ctypes as C
 import os
 import re
 
+import numpy as np
 import pytest
 import torch
 
@@ -632,6 +633,22 @@ def test_packed_call_reports_what_the_first_phase_reports(gmm_lib):
 def test_packed_call_refuses_a_malformed_description(gmm_lib, op, words):
     rc, res = _packed_call(gmm_lib, op, words)
     assert rc == _lib.ACLNN_ERR_PARAM_INVALID and not res.executor
+
+
+def test_native_description_of_arguments():
+    """Every kind of item: tensors as views with their strides, a storage described by other view sizes, integers, lists, None;
+    what is none of these is refused."""
+    t = torch.zeros(4, 6, dtype=torch.int8)[:, 1:4]
+    nz = torch.zeros(2, 2, 3, 16, 32, dtype=torch.int8)
+    got = np.frombuffer(_lib.describe(None, t, (nz, 29, [2, 48, 64]), 5, np.int64(-7), [1, np.int32(2)], torch.zeros((), dtype=torch.int64)),
+                        np.int64).tolist()
+    assert got[:-5] == [-1, 2, t.data_ptr(), _lib.ACL_INT8, _lib.ACL_FORMAT_ND, 4, 3, 6, 1, 2, 4, 3,
+                        3, nz.data_ptr(), _lib.ACL_INT8, 29, 2, 48, 64, 48 * 64, 64, 1, 5, 2, 2, 3, 16, 32, 5, -7, 2, 1, 2]
+    assert got[-5] == 0 and got[-3:] == [_lib.ACL_INT64, _lib.ACL_FORMAT_ND, 0]
+    for bad, error in ((torch.zeros(1, dtype=torch.float64), KeyError), (torch.zeros([1] * 9, dtype=torch.int8), MemoryError),
+                       (1.5, TypeError), ("x", TypeError), ([1.5], TypeError), (2 ** 63, OverflowError)):
+        with pytest.raises(error):
+            _lib.describe(t, bad)
 
 
 # ----------------------------------------------------------------------------------------------------------
