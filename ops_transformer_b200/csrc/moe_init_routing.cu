@@ -16,8 +16,8 @@
 //             (ballots rank the lanes of a warp; the warps are ranked through a per-warp counter table, or take
 //             turns when the active range is too wide for one), which keeps the order of equal keys
 //   gather  - one CTA per token: the row is read once into registers, (quantised,) and stored at the output row of each
-//             of its k pairs; few tokens with smooth scales, and few pairs without, take one CTA per pair; many tokens with few
-//             slots one CTA per SM, rows staged in shared memory; shapes that do not fit the register tile one CTA per output row
+//             of its k pairs; few tokens with smooth scales, and few pairs without, take one CTA per pair; shapes that do not
+//             fit the register tile one CTA per output row
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -465,103 +465,6 @@ __device__ __forceinline__ void unpack16<__half>(const uint4 &u, float *f)
     }
 }
 
-// The fast form of the quantising gather: one CTA per TOKEN.  The row is read once, 16 bytes per thread and step, and
-// stays in registers; without a smooth scale it is quantised once and the int8 row is stored at the output row of each
-// of the token's k pairs; with one, every pair is scaled, reduced and quantised from the registers.  DRAM traffic is the
-// algorithmic minimum: x once, every output row once.  Needs h a multiple of the 16-byte vector, h <= THREADS * NCH * VEC
-// and 16-byte aligned pointers; other shapes take routing_quant_kernel.  MINB CTAs per SM: the 16-bit inputs run with 4
-// (64 registers): 66 instead of 73 us per call on 4096 x 7168 bf16 tokens, because a CTA is a chain of load, block
-// reduction and stores, and only other CTAs fill the gaps.
-template <typename T, int NCH, int THREADS, int MINB = 3>
-__global__ void __launch_bounds__(THREADS, MINB) routing_quant_token_kernel(const RoutingParams p)
-{
-    constexpr int VEC = 16 / (int)sizeof(T);
-    constexpr int G = 16 / VEC;  // 16-byte loads that make one 16-byte store of int8: a thread owns G adjacent ones
-    static_assert(NCH % G == 0, "whole stores per thread");
-    __shared__ float red[THREADS / 32];
-    const int token = p.slots == p.k ? blockIdx.x : blockIdx.x / p.k;
-    const int s0 = p.slots == p.k ? 0 : blockIdx.x - token * p.k;
-    const int chunks = p.h / VEC;
-    const uint4 *row = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.x) + (size_t)token * p.h);
-    float v[NCH][VEC];
-#pragma unroll
-    for (int i = 0; i < NCH; ++i) {
-        const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
-        if (c < chunks) {
-            unpack16<T>(__ldg(row + c), v[i]);
-        } else {
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) v[i][e] = 0.0f;
-        }
-    }
-    const bool smooth = p.scale != nullptr;
-    float scale = 0.0f;
-    uint32_t w[NCH][VEC / 4];  // the quantised row, four int8 per word
-    if (!smooth) {             // one quantisation serves all k pairs of the token
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < NCH; ++i)
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) amax = fmaxf(amax, fabsf(v[i][e]));
-        scale = __fdiv_rn(block_max<THREADS>(amax, red), 127.0f);
-        const float rcp = exact_div_rcp(scale);
-#pragma unroll
-        for (int i = 0; i < NCH; ++i)
-#pragma unroll
-            for (int e4 = 0; e4 < VEC; e4 += 4)
-                w[i][e4 / 4] = pack4(quant_fast(v[i][e4], scale, rcp), quant_fast(v[i][e4 + 1], scale, rcp),
-                                     quant_fast(v[i][e4 + 2], scale, rcp), quant_fast(v[i][e4 + 3], scale, rcp));
-    }
-    pdl_wait();  // the row positions are complete
-    for (int s = s0; s < s0 + p.slots; ++s) {
-        const long long j = (long long)token * p.k + s;
-        const int pos = p.pair_pos[j];
-        if (pos < 0) continue;  // uniform over the CTA
-        if (smooth) {
-            const float *sm = p.scale + (size_t)(__ldg(p.expert_idx + j) - p.e_start) * p.h;
-            float amax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < NCH; ++i) {
-                const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
-                if (c < chunks) {
-#pragma unroll
-                    for (int e4 = 0; e4 < VEC; e4 += 4) {
-                        const float4 m = __ldg(reinterpret_cast<const float4 *>(sm + (size_t)c * VEC + e4));
-                        amax = fmaxf(fmaxf(amax, fabsf(__fmul_rn(v[i][e4], m.x))), fabsf(__fmul_rn(v[i][e4 + 1], m.y)));
-                        amax = fmaxf(fmaxf(amax, fabsf(__fmul_rn(v[i][e4 + 2], m.z))), fabsf(__fmul_rn(v[i][e4 + 3], m.w)));
-                    }
-                }
-            }
-            scale = __fdiv_rn(block_max<THREADS>(amax, red), 127.0f);
-            const float rcp = exact_div_rcp(scale);
-#pragma unroll
-            for (int i = 0; i < NCH; ++i) {  // the products are formed again: keeping them would cost 64 registers
-                const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
-                if (c < chunks) {
-#pragma unroll
-                    for (int e4 = 0; e4 < VEC; e4 += 4) {
-                        const float4 m = __ldg(reinterpret_cast<const float4 *>(sm + (size_t)c * VEC + e4));
-                        w[i][e4 / 4] = pack4(quant_fast(__fmul_rn(v[i][e4], m.x), scale, rcp), quant_fast(__fmul_rn(v[i][e4 + 1], m.y), scale, rcp),
-                                             quant_fast(__fmul_rn(v[i][e4 + 2], m.z), scale, rcp), quant_fast(__fmul_rn(v[i][e4 + 3], m.w), scale, rcp));
-                    }
-                }
-            }
-        }
-        if (threadIdx.x == 0) p.expanded_scale[pos] = scale;
-        int8_t *out = reinterpret_cast<int8_t *>(p.expanded_x) + (size_t)pos * p.h;
-#pragma unroll
-        for (int i = 0; i < NCH; i += G) {
-            const int c = (threadIdx.x + (i / G) * THREADS) * G;
-            if (c < chunks) {
-                uint4 o;
-                if (VEC == 8) o = make_uint4(w[i][0], w[i][VEC / 4 - 1], w[i + G - 1][0], w[i + G - 1][VEC / 4 - 1]);
-                else o = make_uint4(w[i][0], w[i + 1 < NCH ? i + 1 : i][0], w[i + 2 < NCH ? i + 2 : i][0], w[i + G - 1][0]);
-                *reinterpret_cast<uint4 *>(out + (size_t)c * VEC) = o;
-            }
-        }
-    }
-}
-
 // Two values of quant_fast where its reciprocal is not 0: |v / scale| rounds to at most 127 then, so nothing is clamped.
 __device__ __forceinline__ unsigned long long pack_f32x2(float a, float b)
 {
@@ -639,125 +542,134 @@ __device__ __forceinline__ float max_of_bits<__half>(uint32_t m)
     return fmaxf(t.x, t.y);
 }
 
-// The quantising gather without smooth scales where the rows read are a good part of the traffic (see the rule at its launch):
-// one CTA per SM, two teams of 256 threads.  A team quantises one token after the other into a ring of batches in shared memory
-// (the next row is on its way meanwhile); a batch's rows go out by bulk copies of whole rows, one per (token, slot) pair.  Only
-// the copies need the row positions: the first batches are read and quantised while the kernels that place the pairs still run,
-// for which one CTA per token had room for 592 tokens on the whole chip.
-constexpr int kTeams = 2, kTeam = 256;
-constexpr int kStageBytes = 184 * 1024;         // leaves room for a block of the placing kernels on the same SM
-constexpr int kRing = 6, kFirstSend = 4;        // batches in shared memory; batches that are quantised before the positions are waited for
-constexpr int kMaxBatch = 8;                    // tokens
+// A thread's part of a row, quantised with the row's scale: four int8 per word.
 template <typename T, int NCH>
-__global__ void __launch_bounds__(kTeams * kTeam, sizeof(T) == 2 ? 2 : 1) routing_quant_stage_kernel(const RoutingParams p, int batch)
+__device__ __forceinline__ void quant_part(const uint4 (&raw)[NCH], float scale, uint32_t (&w)[NCH][4 / (int)sizeof(T)])
+{
+    constexpr int VEC = 16 / (int)sizeof(T);
+    const float rcp = exact_div_rcp(scale);
+    if (rcp != 0.0f) {
+        const unsigned long long ns = pack_f32x2(-scale, -scale), r2 = pack_f32x2(rcp, rcp);
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            float v[VEC];
+            unpack16<T>(raw[c], v);
+#pragma unroll
+            for (int e4 = 0; e4 < VEC; e4 += 4) {
+                int q[4];
+                quant_pair(v[e4], v[e4 + 1], ns, r2, q[0], q[1]);
+                quant_pair(v[e4 + 2], v[e4 + 3], ns, r2, q[2], q[3]);
+                w[c][e4 / 4] = pack4(q[0], q[1], q[2], q[3]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            float v[VEC];
+            unpack16<T>(raw[c], v);
+#pragma unroll
+            for (int e4 = 0; e4 < VEC; e4 += 4)
+                w[c][e4 / 4] = pack4(quant_fast(v[e4], scale, 0.0f), quant_fast(v[e4 + 1], scale, 0.0f),
+                                     quant_fast(v[e4 + 2], scale, 0.0f), quant_fast(v[e4 + 3], scale, 0.0f));
+        }
+    }
+}
+
+// The fast form of the quantising gather: one CTA per TOKEN.  The row is read once, 16 bytes per thread and step, and
+// stays in registers; without a smooth scale it is quantised once and the int8 row is stored at the output row of each
+// of the token's k pairs; with one, every pair is scaled, reduced and quantised from the registers.  DRAM traffic is the
+// algorithmic minimum: x once, every output row once.  Needs h a multiple of the 16-byte vector, h <= THREADS * NCH * VEC
+// and 16-byte aligned pointers; other shapes take routing_quant_kernel.  MINB CTAs per SM: a CTA is a chain of load, block
+// reduction and stores, and only other CTAs fill the gaps.  Without smooth scales the row stays packed as it was loaded until it
+// is quantised, in pairs, so 16-bit inputs run with 6 CTAs (40 registers); with the row widened first, unpaired and with 4 CTAs the
+// issue slots were the limit.  us per call, before / now: 4096 tokens of h = 7168, bf16, k=8 54.3 / 51.8, k=4 40.9 / 34.0, k=1 33.4 /
+// 24.6, f32 k=4 51.1 / 42.3; h = 2048 bf16 k=2 32.5 / 23.3; 600 x 7168 k=8 14.8 / 13.5.  (8 CTAs: 52.5 for the first.)
+template <typename T, int NCH, int THREADS, bool SMOOTH, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) routing_quant_token_kernel(const RoutingParams p)
 {
     constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int G = 16 / VEC;  // 16-byte loads that make one 16-byte store of int8: a thread owns G adjacent ones
-    extern __shared__ __align__(16) uint8_t stage[];   // [team][ring][batch][h]
-    __shared__ float red[kTeams][2][kTeam / 32];
-    __shared__ float row_scale[kTeams][kRing][kMaxBatch];
-    const int team = threadIdx.x / kTeam, tid = threadIdx.x % kTeam, lane = threadIdx.x & 31;
-    const int n = (int)(p.pairs / p.k), chunks = p.h / VEC;
-    const int first = blockIdx.x * kTeams + team, step = gridDim.x * kTeams;
-    uint8_t *const rows = stage + (size_t)team * kRing * batch * p.h;
-    auto load = [&](int token, uint4 (&r)[NCH]) {
-        const uint4 *row = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.x) + (size_t)token * p.h);
+    static_assert(NCH % G == 0, "whole stores per thread");
+    __shared__ float red[THREADS / 32];
+    const int token = p.slots == p.k ? blockIdx.x : blockIdx.x / p.k;
+    const int s0 = p.slots == p.k ? 0 : blockIdx.x - token * p.k;
+    const int chunks = p.h / VEC;
+    const uint4 *row = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.x) + (size_t)token * p.h);
+    uint4 raw[NCH];
 #pragma unroll
-        for (int i = 0; i < NCH; ++i) {
-            const int c = (tid + (i / G) * kTeam) * G + (i % G);
-            r[i] = c < chunks ? __ldg(row + c) : make_uint4(0, 0, 0, 0);
-        }
-    };
-    auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(kTeam) : "memory"); };
-    // the copies of batch b's `cnt` tokens, one lane each of the team's first warp, as one bulk group
-    auto send = [&](int b, int cnt) {
-        const int at = b % kRing, token0 = first + b * batch * step;
-        for (int i = lane; i < cnt * p.k; i += 32) {
-            const int slot = i / p.k, token = token0 + slot * step;
-            const int pos = p.pair_pos[(long long)token * p.k + (i - slot * p.k)];
-            if (pos < 0) continue;
-            p.expanded_scale[pos] = row_scale[team][at][slot];
-            const uint32_t src = (uint32_t)__cvta_generic_to_shared(rows + (size_t)(at * batch + slot) * p.h);
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                         ::"l"(reinterpret_cast<int8_t *>(p.expanded_x) + (size_t)pos * p.h), "r"(src), "r"(p.h) : "memory");
-        }
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    };
-    uint4 raw[NCH], next[NCH];
-    if (first < n) load(first, next);
-    int at = 0, slot = 0, b = 0;
-    for (int token = first, i = 0; token < n; token += step, ++i) {
-        // the slots' copies of a ring ago have been read (the issuing lanes wait, the barrier below tells the others)
-        if (slot == 0 && b >= kRing && tid < 32) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kRing - 1) : "memory");
+    for (int i = 0; i < NCH; ++i) {
+        const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
+        raw[i] = c < chunks ? __ldg(row + c) : make_uint4(0, 0, 0, 0);
+    }
+    float scale = 0.0f;
+    uint32_t w[NCH][VEC / 4];  // the quantised row, four int8 per word
+    if (!SMOOTH) {             // one quantisation serves all k pairs of the token
         uint32_t mbits = 0;
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-            raw[c] = next[c];
-            mbits = max_abs16<T>(raw[c], mbits);
-        }
-        if (token + step < n) load(token + step, next);
-        float amax = max_of_bits<T>(mbits);
-        amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));   // never negative, never NaN
-        if (lane == 0) red[team][i & 1][tid >> 5] = amax;
-        team_sync();
+        for (int i = 0; i < NCH; ++i) mbits = max_abs16<T>(raw[i], mbits);
+        scale = __fdiv_rn(block_max<THREADS>(max_of_bits<T>(mbits), red), 127.0f);
+        quant_part<T, NCH>(raw, scale, w);
+    }
+    pdl_wait();  // the row positions are complete
+    for (int s = s0; s < s0 + p.slots; ++s) {
+        const long long j = (long long)token * p.k + s;
+        const int pos = p.pair_pos[j];
+        if (pos < 0) continue;  // uniform over the CTA
+        if (SMOOTH) {
+            float v[NCH][VEC];
 #pragma unroll
-        for (int w = 0; w < kTeam / 32; ++w) amax = fmaxf(amax, red[team][i & 1][w]);
-        const float scale = __fdiv_rn(amax, 127.0f), rcp = exact_div_rcp(scale);
-        if (tid == 0) row_scale[team][at][slot] = scale;
-        uint32_t w[NCH][VEC / 4];
-        if (rcp != 0.0f) {
+            for (int i = 0; i < NCH; ++i) unpack16<T>(raw[i], v[i]);
+            const float *sm = p.scale + (size_t)(__ldg(p.expert_idx + j) - p.e_start) * p.h;
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NCH; ++i) {
+                const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
+                if (c < chunks) {
+#pragma unroll
+                    for (int e4 = 0; e4 < VEC; e4 += 4) {
+                        const float4 m = __ldg(reinterpret_cast<const float4 *>(sm + (size_t)c * VEC + e4));
+                        amax = fmaxf(fmaxf(amax, fabsf(__fmul_rn(v[i][e4], m.x))), fabsf(__fmul_rn(v[i][e4 + 1], m.y)));
+                        amax = fmaxf(fmaxf(amax, fabsf(__fmul_rn(v[i][e4 + 2], m.z))), fabsf(__fmul_rn(v[i][e4 + 3], m.w)));
+                    }
+                }
+            }
+            scale = __fdiv_rn(block_max<THREADS>(amax, red), 127.0f);
+            const float rcp = exact_div_rcp(scale);
             const unsigned long long ns = pack_f32x2(-scale, -scale), r2 = pack_f32x2(rcp, rcp);
 #pragma unroll
-            for (int c = 0; c < NCH; ++c) {
-                float v[VEC];
-                unpack16<T>(raw[c], v);
+            for (int i = 0; i < NCH; ++i) {  // the products are formed again: keeping them would cost 64 registers
+                const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
+                if (c < chunks) {
 #pragma unroll
-                for (int e4 = 0; e4 < VEC; e4 += 4) {
-                    int q[4];
-                    quant_pair(v[e4], v[e4 + 1], ns, r2, q[0], q[1]);
-                    quant_pair(v[e4 + 2], v[e4 + 3], ns, r2, q[2], q[3]);
-                    w[c][e4 / 4] = pack4(q[0], q[1], q[2], q[3]);
+                    for (int e4 = 0; e4 < VEC; e4 += 4) {
+                        const float4 m = __ldg(reinterpret_cast<const float4 *>(sm + (size_t)c * VEC + e4));
+                        const float f[4] = {__fmul_rn(v[i][e4], m.x), __fmul_rn(v[i][e4 + 1], m.y), __fmul_rn(v[i][e4 + 2], m.z), __fmul_rn(v[i][e4 + 3], m.w)};
+                        int q[4];
+                        if (rcp != 0.0f) {
+                            quant_pair(f[0], f[1], ns, r2, q[0], q[1]);
+                            quant_pair(f[2], f[3], ns, r2, q[2], q[3]);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) q[e] = quant_fast(f[e], scale, 0.0f);
+                        }
+                        w[i][e4 / 4] = pack4(q[0], q[1], q[2], q[3]);
+                    }
                 }
             }
-        } else {
-#pragma unroll
-            for (int c = 0; c < NCH; ++c) {
-                float v[VEC];
-                unpack16<T>(raw[c], v);
-#pragma unroll
-                for (int e4 = 0; e4 < VEC; e4 += 4)
-                    w[c][e4 / 4] = pack4(quant_fast(v[e4], scale, 0.0f), quant_fast(v[e4 + 1], scale, 0.0f),
-                                         quant_fast(v[e4 + 2], scale, 0.0f), quant_fast(v[e4 + 3], scale, 0.0f));
-            }
         }
-        uint8_t *const dst = rows + (size_t)(at * batch + slot) * p.h;
+        if (threadIdx.x == 0) p.expanded_scale[pos] = scale;
+        int8_t *out = reinterpret_cast<int8_t *>(p.expanded_x) + (size_t)pos * p.h;
 #pragma unroll
-        for (int c = 0; c < NCH; c += G) {
-            const int pc = (tid + (c / G) * kTeam) * G;
-            if (pc < chunks) {
+        for (int i = 0; i < NCH; i += G) {
+            const int c = (threadIdx.x + (i / G) * THREADS) * G;
+            if (c < chunks) {
                 uint4 o;
-                if (VEC == 8) o = make_uint4(w[c][0], w[c][VEC / 4 - 1], w[c + G - 1][0], w[c + G - 1][VEC / 4 - 1]);
-                else o = make_uint4(w[c][0], w[c + 1 < NCH ? c + 1 : c][0], w[c + 2 < NCH ? c + 2 : c][0], w[c + G - 1][0]);
-                *reinterpret_cast<uint4 *>(dst + (size_t)pc * VEC) = o;
+                if (VEC == 8) o = make_uint4(w[i][0], w[i][VEC / 4 - 1], w[i + G - 1][0], w[i + G - 1][VEC / 4 - 1]);
+                else o = make_uint4(w[i][0], w[i + 1 < NCH ? i + 1 : i][0], w[i + 2 < NCH ? i + 2 : i][0], w[i + G - 1][0]);
+                *reinterpret_cast<uint4 *>(out + (size_t)c * VEC) = o;
             }
-        }
-        const bool last = token + step >= n;
-        if (++slot == batch || last) {  // the batch is complete
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // its rows, before the copies read them
-            team_sync();
-            if (tid < 32 && (b >= kFirstSend - 1 || last)) {
-                if (b < kFirstSend) {
-                    pdl_wait();  // the row positions are complete
-                    for (int e = 0; e < b; ++e) send(e, batch);
-                }
-                send(b, slot);
-            }
-            if (++at == kRing) at = 0;
-            slot = 0;
-            ++b;
         }
     }
-    if (tid < 32) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // One CTA per token: the row is read once, 16 bytes per thread and step, and stored at the output row of each pair.
@@ -806,21 +718,6 @@ __global__ void __launch_bounds__(128) routing_copy_kernel(const RoutingParams p
         for (size_t c = threadIdx.x; c < row_bytes; c += blockDim.x) dst[c] = src[c];
     }
     if (p.scale && p.expanded_scale && threadIdx.x == 0) p.expanded_scale[pos] = __ldg(p.scale + j / p.k);
-}
-
-template <typename T, int NCH>
-cudaError_t launch_staged(const RoutingParams &p, int batch, int sms, cudaStream_t stream, bool overlap)
-{
-    auto kern = routing_quant_stage_kernel<T, NCH>;
-    static unsigned long long done_mask = 0;   // per device; the attribute is idempotent, so a race only repeats the call
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!((done_mask >> (dev & 63)) & 1ull)) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
-        if (e != cudaSuccess) return e;
-        done_mask |= 1ull << (dev & 63);
-    }
-    return launch_pdl(kern, (unsigned)sms, kTeams * kTeam, (size_t)kRing * kTeams * batch * p.h, stream, overlap, p, batch);
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
@@ -894,26 +791,15 @@ cudaError_t init_routing_launch(const InitRoutingProblem &r, void *workspace, si
         const int sms = device_sm_count();
         if (sms <= 0) return cudaErrorNoDevice;
         p.slots = (r.scale ? r.n < sms : pairs <= sms) ? 1 : (int)r.k;
-        // Rows through shared memory where reading is a good part of the traffic, k up to 4 with 16-bit rows and up to 8 with 32-bit
-        // ones: with more slots the pass is nothing but writes, which gain nothing from rows that were read ahead.  Rows below 4 KB
-        // leave threads idle, fewer than four tokens per SM leave teams idle.  us (per token / staged), 4096 tokens, h = 7168: bf16
-        // k=1 33.7 / 30.0, k=4 40.9 / 39.2, k=8 54.7 / 57.6, f32 k=4 51.5 / 42.8, k=8 65.6 / 62.3; h = 2048 bf16 k=2 32.5 / 27.7, k=4
-        // 35.6 / 30.8; h = 1024 f32 k=2 35.0 / 25.3, k=8 45.9 / 32.8, bf16 k=4 34.2 / 42.7; 600 tokens h = 7168 bf16 k=4 12.2 / 11.7,
-        // k=8 14.5 / 16.0, h = 2048 f32 k=8 11.7 / 10.3.
-        const bool staged = fast && !r.scale && r.n >= 4ll * sms && r.h * eb >= 4096 && r.k <= (eb == 4 ? 8 : 4);
-        const int fit = (int)(kStageBytes / (kRing * kTeams * r.h)), batch = staged ? (fit < kMaxBatch ? fit : kMaxBatch) : 0;
         const unsigned gather_grid = (unsigned)(p.slots == 1 ? pairs : r.n);
         if (r.x_dtype == kF32) {
-            if (staged) launch_err = launch_staged<float, 8>(p, batch, sms, stream, overlap);
-            else if (fast) launch_err = launch_pdl(routing_quant_token_kernel<float, 8, 256>, gather_grid, 256, 0, stream, overlap, p);
+            if (fast) launch_err = launch_pdl(r.scale ? routing_quant_token_kernel<float, 8, 256, true, 3> : routing_quant_token_kernel<float, 8, 256, false, 4>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<float><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else if (r.x_dtype == kF16) {
-            if (staged) launch_err = launch_staged<__half, 4>(p, batch, sms, stream, overlap);
-            else if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__half, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
+            if (fast) launch_err = launch_pdl(r.scale ? routing_quant_token_kernel<__half, 4, 256, true, 4> : routing_quant_token_kernel<__half, 4, 256, false, 6>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<__half><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else if (r.x_dtype == kBF16) {
-            if (staged) launch_err = launch_staged<__nv_bfloat16, 4>(p, batch, sms, stream, overlap);
-            else if (fast) launch_err = launch_pdl(routing_quant_token_kernel<__nv_bfloat16, 4, 256, 4>, gather_grid, 256, 0, stream, overlap, p);
+            if (fast) launch_err = launch_pdl(r.scale ? routing_quant_token_kernel<__nv_bfloat16, 4, 256, true, 4> : routing_quant_token_kernel<__nv_bfloat16, 4, 256, false, 6>, gather_grid, 256, 0, stream, overlap, p);
             else routing_quant_kernel<__nv_bfloat16><<<(unsigned)pairs, 128, 0, stream>>>(p);
         } else {
             return cudaErrorInvalidValue;

@@ -796,17 +796,18 @@ def test_init_routing_launch_shape_edges(oracle, n, k, E, rng, smooth):
 
 
 @pytest.mark.parametrize("n,k,h,x_kind", [
-    (591, 4, 2048, "bf16"), (592, 4, 2048, "bf16"), (592, 5, 2048, "bf16"), (592, 4, 2032, "bf16"),   # either side of the staging rule
-    (593, 3, 7168, "bf16"), (4500, 1, 7168, "f16"),     # one ring of slots per team, and slots that are used again
-    (2000, 2, 8192, "f32"), (700, 8, 1024, "f32"),      # widest and narrowest rows
+    (149, 1, 16, "bf16"), (300, 2, 4080, "f16"), (593, 3, 7168, "bf16"), (1500, 1, 8192, "f16"),   # widest rows, idle lanes
+    (700, 8, 16, "f32"), (600, 2, 4080, "f32"), (500, 2, 8192, "f32"),
 ])
-def test_init_routing_staged_rows(oracle, n, k, h, x_kind):
+def test_init_routing_rows_kept_packed(oracle, n, k, h, x_kind):
     check_init_routing(oracle, n, k, h, 64, (8, 56), 90 + k, x_kind=x_kind, row_idx_type=k & 1)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-def test_init_routing_staged_special_rows(dtype):
-    """Rows of infinities, NaN, denormals and the type's largest value: the staged kernel gives what the one for few tokens does."""
+@pytest.mark.parametrize("n", [12, 720])
+def test_init_routing_special_rows(dtype, n):
+    """Rows of infinities, NaN, denormals and the type's largest value: without smooth scales (rows kept packed, maxima of pairs)
+    what they give with scales of one (widened values), and each row the same wherever it stands."""
     import ops_transformer_b200 as ops
     dev = _dev()
     big, tiny = torch.finfo(dtype).max, torch.finfo(dtype).smallest_normal
@@ -820,11 +821,13 @@ def test_init_routing_staged_special_rows(dtype):
     rows[7] = rows[7] * tiny
     rows[8] = tiny / 4
     rows[9, 1], rows[9, 2] = float("inf"), float("nan")
-    idx = torch.zeros(12, 1, dtype=torch.int32, device=dev)
-    q, _, _, s = ops.moe_init_routing_v3(rows, idx, expert_num=2, active_expert_range=(0, 2))
-    q2, _, _, s2 = ops.moe_init_routing_v3(rows.repeat(60, 1), idx.repeat(60, 1), expert_num=2, active_expert_range=(0, 2))
+    x, idx = rows.repeat(n // 12, 1), torch.zeros(n, 1, dtype=torch.int32, device=dev)
+    kw = dict(expert_num=2, active_expert_range=(0, 2))
+    q, _, _, s = ops.moe_init_routing_v3(x, idx, **kw)
+    q1, _, _, s1 = ops.moe_init_routing_v3(x, idx, scale=torch.ones(2, 2048, device=dev), **kw)
     torch.cuda.synchronize()
-    assert torch.equal(q2, q.repeat(60, 1)) and torch.equal(s2.view(torch.int32), s.repeat(60).view(torch.int32))
+    assert torch.equal(q, q1) and torch.equal(s.view(torch.int32), s1.view(torch.int32))
+    assert torch.equal(q, q[:12].repeat(n // 12, 1))
 
 
 def test_init_routing_without_quantisation(oracle):
