@@ -18,18 +18,19 @@
 //                          half): a tile yields 64 outputs per CTA and token; the two halves meet through shared memory.
 //   swiglu_quant, one CTA: both halves of 128 columns in two accumulators of at most 128 tokens; a lane holds both values.
 // K is consumed 128 bytes per pipeline stage (4 MMAs of K=32).
-// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2-9 = epilogue (320 threads); swiglu_quant adds
-// warp 10, one lane of which keeps the books of the row blocks in global memory, and requantising warps up to 512 threads;
-// FRACTAL_NZ adds two weight loader warps (384 threads; in swiglu_quant they take the place of two requantising warps).
+// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2-9 = epilogue (320 threads; with bias or
+// activation warps 2-17, 576 threads); swiglu_quant adds warp 10, one lane of which keeps the books of the row blocks in global
+// memory, and requantising warps up to 512 threads; FRACTAL_NZ adds two weight loader warps (in swiglu_quant they take the
+// place of two requantising warps).
 // CTA pairs (cluster of 2, tcgen05 cta_group::2) compute 256 channels; each CTA stages its own 128 channels and half of the
 // tile's token rows.  A launch confined to one CTA runs the one-CTA instances.  Weight layouts: [E,K,N] (MN-major operand,
 // 128-byte swizzle; 64-byte for swiglu's 64-channel boxes), the transposed view [E,N,K] (K-major) and FRACTAL_NZ
 // [E,N/32,K/16,16,32] (MN-major, 32-byte swizzle, fetched by two loader warps instead of TMA).
 // Epilogue: a lane holds one channel (its weight scale stays in a register), the tokens' scales come from shared memory.
 // bf16 / fp16 results are read as 16x256b fragments, packed by token pairs and transposed by stmatrix, so that the four
-// warps of a column half together hold 256 contiguous bytes of every result row; SwiGLU values are
-// stored as they are held, a token's 32 channels (128 bytes) per instruction; the combine's fp32 rows and int32 accumulators
-// are transposed 16 tokens at a time, so that a lane adds or stores four channels of a row at once.
+// warps of a column half together hold 256 contiguous bytes of every result row; SwiGLU values are stored as they are held, a
+// token's 32 channels (128 bytes) per instruction; the combine's fp32 rows and int32 accumulators are transposed 16 tokens at
+// a time, so that a lane adds or stores four channels of a row at once.
 // Rows are optionally scattered by a row index, also into other GPUs' buffers; the finalize-routing variant adds weighted
 // fp32 rows into token rows with 16-byte vector reductions; SwiGLU values go to an fp32 staging buffer with a per-row
 // atomic max, and a finished row block is requantised to int8 in row slices that the CTAs which worked on it claim from a
@@ -38,7 +39,7 @@
 // idle; the SM clock falls to 1.5-1.6 GHz, at which the tensor pipe alone draws the board's 1 kW); groups of up to 128 rows
 // HBM; short K the epilogue.  Measured before (tokens on the M side, operations issued by one thread of a diverged warp,
 // every epilogue thread fencing for itself, requantisation inside the epilogue warps) and now, us:
-//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 881 (power), 128 tokens x 8 over 256 experts 884 / 850 (HBM);
+//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 877 (power), 128 tokens x 8 over 256 experts 884 / 850 (HBM);
 //     K=2048 N=1536, 64 groups of 64 rows 66 / 54, of 400 rows 190 / 118
 //   gmm K=2048 N=7168: 4096 tokens x 8 over 32 experts 403 / 366; 32 groups of 160 rows 131 / 102; K=768 N=2048, 64 x 400 rows
 //     76 / 70 (of which 10 % came from moving the second CTA's accumulator release out of its epilogue warps: 374 / 334 for
@@ -674,7 +675,7 @@ __device__ void build_schedule(Shared *sh, const KParams &p, int n_units)
             sh->tile_start[L] = incl;
             const int total = min(incl, p.max_tiles), rem = total < n_units ? total : total % n_units;
             int split = max_tok > SPLIT_TOK && rem > 0 ? min(n_units / rem, (max_tok + SPLIT_TOK - 1) / SPLIT_TOK) : 1;
-            if (split < 2 || p.n_tiles > 65535 / (2 * split)) split = 1;   // shares of a row block are counted in 16 bits
+            if (split < 2 || p.n_tiles > 32767 / (2 * split)) split = 1;   // shares of a row block are counted in 16 bits
             sh->split = split;
             sh->split_from = split > 1 ? total - rem : total;
             sh->total_tiles = split > 1 ? total - rem + rem * split : total;
