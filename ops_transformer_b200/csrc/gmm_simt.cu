@@ -262,12 +262,13 @@ void make_plan(const Problem &p, Plan *plan)
     plan->path = sm100_shape_ok(p) ? kPathSm100 : kPathSimt;
     // Pairs stage 32 KB per 256 channels x 256 tokens and K block where single CTAs stage 48 KB per 128 x 256, but their CTAs
     // meet at every tile, and a tile of few tokens or few K blocks has nothing to save.  Measured (us, pair / single):
-    //   swiglu K=7168 N=4096, 32 groups: 162 / 157 at 64 rows, 174 / 174 at 128, 195 / 225 at 192, 354 / 401 at 400
-    //   swiglu K=2048 N=1536, 64 groups:  70 /  72 at 160 rows, 118 / 123 at 400, 238 / 237 at 1000
-    //   swiglu K=1024 N=2048, 32 groups:  56 /  55 at 160 rows,  84 /  83 at 400, 148 / 142 at 1000
-    //   gmm    K=2048 N=7168, 32 groups:  86 /  85 at 64 rows,  92 /  91 at 128, 102 / 118 at 160, 334 / 425 at 1000
-    //   gmm    K=1536 N=4096, 32 groups:  48 /  52 at 160 rows,  79 /  91 at 400
-    //   gmm    K=768  N=2048, 64 groups:  40 /  39 at 160 rows,  70 /  70 at 400, 119 / 121 at 1000
+    //   swiglu K=7168 N=4096, 32 groups: 157 / 154 at 64 rows, 170 / 166 at 128, 181 / 206 at 160, 190 / 209 at 192, 338 / 414 at 400
+    //   swiglu K=2048 N=1536, 64 groups:  58 /  52 at 64 rows,  63 /  67 at 160, 112 / 118 at 400, 226 / 224 at 1000
+    //   swiglu K=1024 N=2048, 32 groups:  38 /  39 at 160 rows,  71 /  72 at 400, 133 / 120 at 1000
+    //   gmm    K=2048 N=7168, 32 groups:  84 /  83 at 64 rows,  91 /  90 at 128,  96 / 105 at 160, 329 / 386 at 1000
+    //   gmm    K=1536 N=4096, 32 groups:  48 /  52 at 160 rows,  81 /  90 at 400
+    //   gmm    K=1024 N=2048, 32 groups:  24 /  23 at 160 rows,  39 /  39 at 400,  69 /  71 at 1000
+    //   gmm    K=768  N=2048, 64 groups:  36 /  35 at 160 rows,  62 /  60 at 400, 120 / 122 at 1000
     // GMM_B200_CTAS=1|2 overrides the choice (for measurements and tests).
     const long long avg_rows = p.rows_per_group_hint > 0 ? p.rows_per_group_hint : (p.gl_len > 0 ? p.M / p.gl_len : 0);
     plan->ctas = avg_rows > 128 && p.K >= 1536 ? 2 : 1;

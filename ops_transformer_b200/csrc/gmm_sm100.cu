@@ -40,9 +40,9 @@
 // HBM; short K the epilogue.  Measured before (tokens on the M side, operations issued by one thread of a diverged warp,
 // every epilogue thread fencing for itself, requantisation inside the epilogue warps) and now, us:
 //   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 877 (power), 128 tokens x 8 over 256 experts 884 / 850 (HBM);
-//     K=2048 N=1536, 64 groups of 64 rows 66 / 54, of 400 rows 190 / 118
-//   gmm K=2048 N=7168: 4096 tokens x 8 over 32 experts 403 / 366; 32 groups of 160 rows 131 / 102; K=768 N=2048, 64 x 400 rows
-//     76 / 70 (of which 10 % came from moving the second CTA's accumulator release out of its epilogue warps: 374 / 334 for
+//     K=2048 N=1536, 64 groups of 64 rows 66 / 52, of 400 rows 190 / 112
+//   gmm K=2048 N=7168: 4096 tokens x 8 over 32 experts 403 / 366; 32 groups of 160 rows 131 / 96; K=768 N=2048, 64 x 400 rows
+//     76 / 60 (of which 10 % came from moving the second CTA's accumulator release out of its epilogue warps: 374 / 334 for
 //     32 groups of 1000 rows)
 // The producers pace themselves wave by wave so that the units which share x rows and weight boxes through L2 stay
 // together (a bounded hint).
@@ -85,7 +85,8 @@ struct Shape {
     static constexpr int kCols = MODE == kModeSwigluQuant && !kDual ? BC / 2 : BC;   // result columns per CTA and tile
 };
 // Row blocks of a group that are worked on together: all their tiles of a channel tile, then the next channel tile.  A group that
-// begins in one wave and ends in the next has its x rows read twice then, instead of its weights, four times as many.  swiglu
+// begins in one wave and ends in the next has its x rows read twice then, instead of its weights, four times as many (DRAM reads
+// of 8 groups of 1024 rows, K=7168 N=4096: 403 -> 330 MB).  swiglu
 // K=7168 N=4096, 32 groups of 1024 rows: 758 us with one, 740 with four; grouped_matmul, which does not pace its waves, K=2048
 // N=7168: 339 / 343.
 __host__ __device__ constexpr int block_group(int mode) { return mode == kModeSwigluQuant ? 4 : 1; }
