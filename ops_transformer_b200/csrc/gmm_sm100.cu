@@ -293,7 +293,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 
 // The combine's kernel is launched as a programmatic dependent of the one that initialises its result and the status record, and
 // runs beside it: everything that it reads was complete before that one started.  Nothing is written to global memory before
-// this returns, which is when that kernel has ended and its writes are visible; without such a launch it returns at once.
+// this returns, which is when that kernel has ended and its writes are visible; without such a launch it returns at once.  A warp
+// of every CTA also waits before the CTA leaves, whether it had a tile or not: what the stream runs next is ordered behind this
+// grid alone, so the grid must not end before the initialisation has.
 // (A kernel in the place of every operator's memset would take 2.6 us off a call on the device and cost the host 3.)
 __device__ __forceinline__ void wait_for_init() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -1875,6 +1877,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         }
     }
 
+    if (COMBINE && warp == 0) wait_for_init();
     __syncthreads();
     if (CTAS == 2) cluster_sync_all();  // neither CTA leaves, or frees TMEM, while the other can still reach into it
     if (warp == 1) {

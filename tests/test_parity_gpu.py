@@ -712,6 +712,59 @@ def test_finalize_routing_batch_smaller_than_rows_per_token(oracle):
     check_finalize(oracle, 1024, 128, 256, 2, [500, 524], 16, 66, shared_rows=64, shared_weight=2.0)
 
 
+@pytest.mark.parametrize("ctas", ["1", "2"])
+@pytest.mark.parametrize("captured", [False, True])
+def test_finalize_routing_result_is_whole_for_the_next_kernel(monkeypatch, ctas, captured):
+    """The GEMM starts beside the kernel that initialises the result, so it has to outlast it even without a single row to
+    multiply (a rank that owns none of the chosen experts): a copy enqueued right behind the call sees every shared row and zero,
+    the status record stays clean, and the same holds for a call that is captured and replayed."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    monkeypatch.setenv("GMM_B200_CTAS", ctas)
+    M = batch = 4096
+    K, N, E = 128, 4096, 4                    # 67 MB of result: the initialisation takes longer than an empty GEMM
+    g = torch.Generator(device=dev)
+    g.manual_seed(5)
+    x = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=dev, generator=g)
+    w = torch.randint(-127, 128, (E, N // 32, K // 16, 16, 32), dtype=torch.int8, device=dev, generator=g)
+    ws, xs = torch.rand((E, N), device=dev, generator=g), torch.rand(M, device=dev, generator=g)
+    logit, shared = torch.rand(M, device=dev, generator=g), torch.randn((1000, N), device=dev, generator=g).to(torch.bfloat16)
+    row = torch.randperm(M, device=dev, generator=g)   # one addition per element: the sum has one order
+    counts = torch.zeros(E, dtype=torch.int64, device=dev)
+    y, seen = torch.empty((batch, N), device=dev), torch.empty((batch, N), device=dev)
+    start = torch.zeros((batch, N), device=dev)
+    start[24:1024] = shared.float() * 0.5
+    wsb = torch.empty(4096, dtype=torch.uint8, device=dev)
+
+    def call():
+        ops.grouped_matmul_finalize_routing(x, w, ws, counts, row, batch, pertoken_scale=xs, shared_input=shared, logit=logit,
+                                            shared_input_weight=0.5, shared_input_offset=24, out=y, workspace=wsb)
+        seen.copy_(y)
+
+    graph = None
+    if captured:
+        call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call()
+    for rows in (0, 0, 700, 0):               # the list is read on the device, so a replay sees a new one
+        counts.fill_(rows)
+        y.fill_(7.0)
+        wsb.fill_(0x5a)
+        graph.replay() if graph else call()
+        ops.check_status(wsb)
+        want = start
+        if rows:
+            prod = torch.empty((E * rows, N), device=dev)
+            for e in range(E):
+                part = slice(e * rows, (e + 1) * rows)
+                we = w[e].permute(1, 2, 0, 3).reshape(K, N).double()
+                prod[part] = (x[part].double() @ we).float() * ws[e] * (xs[part] * logit[part])[:, None]
+            want = start.index_add(0, row[:E * rows], prod)
+        assert torch.equal(seen, want), rows
+
+
 # ----------------------------------------------------------------------------------------------------------
 # moe_init_routing_v3 (producer of the path's inputs): every output is integer or exactly rounded, so bit-exact
 # ----------------------------------------------------------------------------------------------------------
