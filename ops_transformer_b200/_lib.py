@@ -138,16 +138,25 @@ def lib():
 _DESCRIBE = None
 
 
-def describe(*items) -> bytes:
-    """The packed description of ``items`` (csrc/describe.cpp): int64 words as gmmB200Call takes them."""
+def _describe_module():
     global _DESCRIBE
     if _DESCRIBE is None:
         try:
             from . import _describe
         except ImportError as e:
             raise LibraryMissing(f"the native description module is missing ({e}): build it with `python -m ops_transformer_b200._build`.") from e
-        _DESCRIBE = _describe.describe
-    return _DESCRIBE(*items)
+        _DESCRIBE = _describe
+    return _DESCRIBE
+
+
+def describe(*items) -> bytes:
+    """The packed description of ``items`` (csrc/describe.cpp): int64 words as gmmB200Call takes them."""
+    return _describe_module().describe(*items)
+
+
+def describe_call(kinds: str, *items) -> bytes:
+    """The same for the arguments of an operator, whose kinds its description fixes (a letter each, csrc/describe.cpp)."""
+    return _describe_module().describe_call(kinds, *items)
 
 
 def last_error() -> str:

@@ -273,8 +273,8 @@ def grouped_matmul_v4(x: torch.Tensor, weight: torch.Tensor, scale: Optional[tor
                                     out_row_index, stream, workspace, return_workspace, out_peers, nz, options, out_rows)
     if api not in _lib.OP_GMM:
         raise ValueError(f"unknown api {api!r}")
-    words = _lib.describe(x, (weight, ACL_FORMAT_FRACTAL_NZ if nz else ACL_FORMAT_ND, None), bias, scale, per_token_scale, group_list, out,
-                          split_item, group_type, group_list_type, act_type, quant_group_size, _ints(tuning_config))
+    words = _lib.describe_call("tftttttiiiiil", x, (weight, ACL_FORMAT_FRACTAL_NZ if nz else ACL_FORMAT_ND, None), bias, scale, per_token_scale,
+                               group_list, out, split_item, group_type, group_list_type, act_type, quant_group_size, _ints(tuning_config))
     workspace = _call(_lib.OP_GMM[api], "aclnnGroupedMatmul" + api, words, x.device, workspace, stream, options)
     return (out, workspace) if return_workspace else out
 
@@ -340,7 +340,7 @@ def grouped_matmul_swiglu_quant(x: torch.Tensor, weight: torch.Tensor, weight_sc
         output = x.new_empty((M, N // 2), dtype=torch.int8)
     if output_scale is None:
         output_scale = x.new_empty((M,), dtype=torch.float32)
-    words = _lib.describe(x, (weight, weight_format, None), bias, offset, weight_scale, x_scale, group_list, output, output_scale)
+    words = _lib.describe_call("tfttttttt", x, (weight, weight_format, None), bias, offset, weight_scale, x_scale, group_list, output, output_scale)
     workspace = _call(_lib.OP_SWIGLU_QUANT[api], "aclnnGroupedMatmulSwigluQuant" + api, words, x.device, workspace, stream, options)
     return (output, output_scale, workspace) if return_workspace else (output, output_scale)
 
@@ -362,9 +362,9 @@ def grouped_matmul_finalize_routing(x: torch.Tensor, weight_nz: torch.Tensor, sc
     N, K = n1 * 32, k1 * 16
     if out is None:
         out = x.new_empty((batch, N), dtype=torch.float32)
-    words = _lib.describe(x, (weight_nz, ACL_FORMAT_FRACTAL_NZ, [E, K, N] if view_3d else None), scale, bias, pertoken_scale, group_list,
-                          shared_input, logit, row_index, out, struct.unpack("<I", bytes(C.c_float(shared_input_weight)))[0],
-                          shared_input_offset, group_list_type, _ints(tuning_config))
+    words = _lib.describe_call("tfttttttttiiil", x, (weight_nz, ACL_FORMAT_FRACTAL_NZ, [E, K, N] if view_3d else None), scale, bias,
+                               pertoken_scale, group_list, shared_input, logit, row_index, out,
+                               struct.unpack("<I", bytes(C.c_float(shared_input_weight)))[0], shared_input_offset, group_list_type, _ints(tuning_config))
     workspace = _call(_lib.OP_FINALIZE_ROUTING[api], "aclnnGroupedMatmulFinalizeRoutingWeightNz" + api, words, x.device, workspace, stream,
                       options)
     return (out, workspace) if return_workspace else out
@@ -418,8 +418,8 @@ def moe_init_routing_v3(x: torch.Tensor, expert_idx: torch.Tensor, *, expert_num
         es = x.new_empty((n * k,), dtype=torch.float32)
     else:
         ex, ri, cnt, es = outputs
-    words = _lib.describe(x, expert_idx, scale, offset, ex, ri, cnt, es, n * k if active_num is None else active_num, expert_capacity,
-                          expert_num, drop_pad_mode, expert_tokens_num_type, 1 if expert_tokens_num_flag else 0, quant_mode,
-                          row_idx_type, _ints(active_expert_range))
+    words = _lib.describe_call("ttttttttiiiiiiiil", x, expert_idx, scale, offset, ex, ri, cnt, es, n * k if active_num is None else active_num,
+                               expert_capacity, expert_num, drop_pad_mode, expert_tokens_num_type, 1 if expert_tokens_num_flag else 0, quant_mode,
+                               row_idx_type, _ints(active_expert_range))
     _call(_lib.OP_MOE_INIT_ROUTING, "aclnnMoeInitRoutingV3", words, x.device, workspace, stream, None)
     return ex, ri, cnt, es

@@ -86,36 +86,63 @@ bool put_tensor(std::vector<int64_t> &w, PyObject *obj, int64_t format, PyObject
     return true;
 }
 
-// describe(item, ...) -> bytes of int64 words.  An item is None or a tensor (row-major format), a tuple (tensor, format,
-// view sizes or None), an integer (one word as it is) or a list of integers (length, then the values).
-PyObject *describe(PyObject *, PyObject *const *args, Py_ssize_t nargs)
+// One argument of a call.  What it has to be follows from its place in the operator's description, not from what is given: an
+// integer may be any object with __index__ (numpy's, a tensor of one element), and only tensors and lists may be None.
+//   't'  a tensor (row-major format) or None          'i'  an integer, one word as it is
+//   'f'  (tensor, format, view sizes or None)         'l'  a list of integers (length, then the values) or None
+bool put_item(std::vector<int64_t> &w, char kind, PyObject *a)
+{
+    if (kind == 't') return put_tensor(w, a, 2, Py_None);
+    if (kind == 'f') {
+        if (!PyTuple_Check(a) || PyTuple_GET_SIZE(a) != 3) {
+            PyErr_SetString(PyExc_TypeError, "(tensor, format, view sizes) is wanted");
+            return false;
+        }
+        const int64_t format = PyLong_AsLongLong(PyTuple_GET_ITEM(a, 1));
+        if (format == -1 && PyErr_Occurred()) return false;
+        return put_tensor(w, PyTuple_GET_ITEM(a, 0), format, PyTuple_GET_ITEM(a, 2));
+    }
+    if (kind == 'i') {
+        PyObject *index = PyNumber_Index(a);
+        const int64_t v = index ? PyLong_AsLongLong(index) : -1;
+        Py_XDECREF(index);
+        if (v == -1 && PyErr_Occurred()) return false;
+        w.push_back(v);
+        return true;
+    }
+    if (kind == 'l') {
+        if (a == Py_None) {
+            w.push_back(-1);
+            return true;
+        }
+        if (!PyList_Check(a)) {
+            PyErr_Format(PyExc_TypeError, "a list of integers or None is wanted, not %s", Py_TYPE(a)->tp_name);
+            return false;
+        }
+        w.push_back((int64_t)PyList_GET_SIZE(a));
+        return read_ints(a, w);
+    }
+    PyErr_SetString(PyExc_ValueError, "unknown kind of argument");
+    return false;
+}
+
+// The kind of an item described by itself: integers are told by their type, tensors stay tensors.
+char kind_of(PyObject *a)
+{
+    if (PyLong_Check(a)) return 'i';
+    if (PyList_Check(a)) return 'l';
+    if (PyTuple_Check(a) && PyTuple_GET_SIZE(a) == 3) return 'f';
+    return a != Py_None && !THPVariable_Check(a) && PyIndex_Check(a) ? 'i' : 't';
+}
+
+template <typename Kind>
+PyObject *packed(PyObject *const *items, Py_ssize_t n, Kind kind)
 {
     try {
         std::vector<int64_t> w;
         w.reserve(192);
-        for (Py_ssize_t i = 0; i < nargs; ++i) {
-            PyObject *a = args[i];
-            if (PyLong_Check(a)) {
-                const int64_t v = PyLong_AsLongLong(a);
-                if (v == -1 && PyErr_Occurred()) return nullptr;
-                w.push_back(v);
-            } else if (PyList_Check(a)) {
-                w.push_back((int64_t)PyList_GET_SIZE(a));
-                if (!read_ints(a, w)) return nullptr;
-            } else if (PyTuple_Check(a) && PyTuple_GET_SIZE(a) == 3) {
-                const int64_t format = PyLong_AsLongLong(PyTuple_GET_ITEM(a, 1));
-                if (format == -1 && PyErr_Occurred()) return nullptr;
-                if (!put_tensor(w, PyTuple_GET_ITEM(a, 0), format, PyTuple_GET_ITEM(a, 2))) return nullptr;
-            } else if (a != Py_None && !THPVariable_Check(a) && PyIndex_Check(a)) {   // an integer of another kind (numpy's)
-                PyObject *index = PyNumber_Index(a);
-                const int64_t v = index ? PyLong_AsLongLong(index) : -1;
-                Py_XDECREF(index);
-                if (v == -1 && PyErr_Occurred()) return nullptr;
-                w.push_back(v);
-            } else if (!put_tensor(w, a, 2, Py_None)) {
-                return nullptr;
-            }
-        }
+        for (Py_ssize_t i = 0; i < n; ++i)
+            if (!put_item(w, kind(i), items[i])) return nullptr;
         return PyBytes_FromStringAndSize(reinterpret_cast<const char *>(w.data()), (Py_ssize_t)(w.size() * sizeof(int64_t)));
     } catch (const std::exception &e) {   // a tensor without storage, for instance
         PyErr_SetString(PyExc_RuntimeError, e.what());
@@ -123,8 +150,28 @@ PyObject *describe(PyObject *, PyObject *const *args, Py_ssize_t nargs)
     }
 }
 
+// describe(item, ...) -> bytes of int64 words
+PyObject *describe(PyObject *, PyObject *const *args, Py_ssize_t nargs)
+{
+    return packed(args, nargs, [&](Py_ssize_t i) { return kind_of(args[i]); });
+}
+
+// describe_call(kinds, item, ...) -> bytes of int64 words: the arguments of one operator, a letter of `kinds` for each
+PyObject *describe_call(PyObject *, PyObject *const *args, Py_ssize_t nargs)
+{
+    Py_ssize_t n = 0;
+    const char *kinds = nargs > 0 ? PyUnicode_AsUTF8AndSize(args[0], &n) : "";
+    if (!kinds) return nullptr;
+    if (nargs < 1 || n != nargs - 1) {
+        PyErr_SetString(PyExc_TypeError, "the kinds of the arguments and as many arguments are wanted");
+        return nullptr;
+    }
+    return packed(args + 1, n, [&](Py_ssize_t i) { return kinds[i]; });
+}
+
 PyMethodDef methods[] = {
-    {"describe", (PyCFunction)(void (*)(void))describe, METH_FASTCALL, "Packed description of a call's arguments."},
+    {"describe", (PyCFunction)(void (*)(void))describe, METH_FASTCALL, "Packed description of items by themselves."},
+    {"describe_call", (PyCFunction)(void (*)(void))describe_call, METH_FASTCALL, "Packed description of an operator's arguments."},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_describe", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

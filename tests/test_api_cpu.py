@@ -651,6 +651,60 @@ def test_native_description_of_arguments():
             _lib.describe(t, bad)
 
 
+def _operator_calls():
+    """Every operator as its Python entry point calls it: (op, tensors, integers, call(tensors, integers)), with the integers at the
+    values of ``_packed_operators``."""
+    import ops_transformer_b200 as ops
+    M, K, N, E, T = 96, 64, 128, 3, 24
+    x, w = torch.zeros(M, K, dtype=torch.int8), torch.zeros(E, N, K, dtype=torch.int8).transpose(1, 2)
+    nz, big = (torch.zeros(E, n // 32, K // 16, 16, 32, dtype=torch.int8) for n in (N, 256))
+    ws, xs, gl = torch.ones(E, N), torch.ones(M), torch.full((E,), 32, dtype=torch.int64)
+    y, q, qs = torch.zeros(M, N, dtype=torch.bfloat16), torch.zeros(M, N // 2, dtype=torch.int8), torch.zeros(M)
+    for api, op in _lib.OP_GMM.items():
+        def gmm(t, i, api=api):
+            return ops.grouped_matmul_v4(*t, out=y, api=api, tuning_config=None if api == "V4" else [16], **i)
+        ints = dict(split_item=2, group_type=0, group_list_type=1, act_type=0, quant_group_size=0)
+        yield op, (x, nz if api == "WeightNz" else w, ws, xs, gl), ints, gmm
+    for api, op in _lib.OP_SWIGLU_QUANT.items():
+        fmt = dict(weight_format=_lib.ACL_FORMAT_FRACTAL_NZ if api else _lib.ACL_FORMAT_ND)
+        yield op, (x, nz if api else w, ws, xs, gl), fmt, lambda t, i, api=api: ops.grouped_matmul_swiglu_quant(*t, api=api, output=q, output_scale=qs, **i)
+    rest = dict(pertoken_scale=xs, shared_input=torch.zeros(T, 256, dtype=torch.bfloat16), logit=torch.ones(M), shared_input_weight=0.5,
+                out=torch.zeros(T, 256), view_3d=False)
+    for api, op in _lib.OP_FINALIZE_ROUTING.items():
+        def finalize(t, i, api=api):
+            return ops.grouped_matmul_finalize_routing(*t, T, api=api, tuning_config=[16] if api else None, **rest, **i)
+        yield op, (x, big, torch.ones(E, 256), gl, torch.arange(M) // 4), dict(shared_input_offset=0, group_list_type=1), finalize
+    outs = (torch.zeros(T * 4, K, dtype=torch.int8), torch.zeros(T * 4, dtype=torch.int32), gl, torch.zeros(T * 4))
+    yield (_lib.OP_MOE_INIT_ROUTING, (torch.zeros(T, K, dtype=torch.bfloat16), torch.zeros(T, 4, dtype=torch.int32)),
+           dict(expert_num=E, drop_pad_mode=0, expert_capacity=0, expert_tokens_num_type=1, quant_mode=1, row_idx_type=1),
+           lambda t, i: ops.moe_init_routing_v3(*t, active_expert_range=(0, E), outputs=outs, **i))
+
+
+def test_operators_describe_their_arguments_by_place(monkeypatch):
+    """Integer arguments may be any object with __index__, 0-dim tensors among them, and nothing else; where a tensor belongs,
+    only a tensor or None goes.  The descriptions are those that the planning tests take, addresses aside."""
+    from ops_transformer_b200 import acl
+    seen = []
+    monkeypatch.setattr(acl, "_call", lambda op, name, words, *rest: seen.append((op, np.frombuffer(words, np.int64).tolist())))
+    host = {op: words for _, op, words, _ in _packed_operators()}
+    for op, tensors, ints, call in _operator_calls():
+        call(tensors, ints)
+        got_op, words = seen.pop()
+        assert got_op == op and len(words) == len(host[op]) and sum(a != b for a, b in zip(words, host[op])) <= 10, op
+        for wrap in (np.int32, torch.tensor, lambda v: torch.tensor([v]), lambda v: torch.tensor(v, dtype=torch.int32)):
+            call(tensors, {k: wrap(v) for k, v in ints.items()})
+            assert seen.pop() == (op, words), op
+        for name, value in ints.items():
+            for bad in (None, 1.0, "1", [value], (value,) * 3, torch.tensor(1.0)):
+                with pytest.raises(TypeError):
+                    call(tensors, {**ints, name: bad})
+        for i in range(len(tensors)):
+            for bad in (5, [1], (tensors[i], 2, None), "x"):
+                with pytest.raises((TypeError, AttributeError)):
+                    call(tensors[:i] + (bad,) + tensors[i + 1:], ints)
+    assert not seen
+
+
 # ----------------------------------------------------------------------------------------------------------
 # the pooled workspace: which calls may share a buffer
 # ----------------------------------------------------------------------------------------------------------
