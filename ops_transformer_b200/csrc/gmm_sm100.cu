@@ -162,6 +162,7 @@ struct Shared {
     // CTA contributed to and has not yet settled (publishing lane only); a ring of work lists: the row ranges to requantise
     // (written by that lane, read by the requantising warps after wk_full)
     unsigned stored_count;
+    unsigned published;                // steps of the publishing lane (see list_wait)
     int pend_n;
     PendingBlock pend[MAX_PENDING];
     int n_work[WK_DEPTH];
@@ -329,6 +330,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, Shared
     const uint32_t a = smem_u32(bar);
     if (mbar_try_wait<CLUSTER>(a, parity)) return true;
     return mbar_wait_slow<CLUSTER>(a, parity, sh, status, who, sh->wait_limit);
+}
+
+// Bounded wait for a work list of swiglu_quant.  Many tiles can lie between two lists - nothing is passed on while none of the
+// CTA's row blocks is complete, four blocks times all their channel tiles at a time with few CTAs - and the last list also waits
+// for other units (`patience`).  The limit is one of a single step, so it starts anew with every step of the publishing lane, which
+// bounds its own waits by it.
+__device__ __noinline__ bool list_wait(uint64_t *bar, uint32_t parity, Shared *sh, int *status, int who, long long patience)
+{
+    const uint32_t a = smem_u32(bar);
+    const long long limit = sh->wait_limit + patience;
+    unsigned seen = *(volatile unsigned *)&sh->published, spins = 0;
+    long long t0 = clock64();
+    while (!mbar_try_wait<false>(a, parity)) {
+        if ((++spins & 31u) != 0u) continue;
+        if (*(volatile int *)&sh->abort_flag) return false;
+        const unsigned now = *(volatile unsigned *)&sh->published;
+        if (now != seen) {
+            seen = now;
+            t0 = clock64();
+        } else if (clock64() - t0 > limit) {
+            *(volatile int *)&sh->abort_flag = 1;
+            if (atomicCAS(status, kStatusOk, kStatusWaitTimeout) == kStatusOk) {
+                status[1] = (int)blockIdx.x;
+                status[2] = who;
+                status[3] = (int)parity;
+            }
+            return false;
+        }
+    }
+    return true;
 }
 
 // Tiled TMA loads into this CTA's shared memory.  CTAS == 2 is the pair form: the byte count is credited to the mbarrier at
@@ -1200,6 +1231,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         }
         mbar_init(&sh->wk_closing, 1);
         sh->stored_count = 0;
+        sh->published = 0;
         sh->abort_flag = 0;
         sh->total_tiles = 0;
         sh->wait_limit = p.wait_limit;
@@ -1779,7 +1811,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         }
         if (SCATTER && p.num_peers > 0) __threadfence_system();  // rows stored into other GPUs' memory
         if (SWIGLU && ok) {  // nothing left to multiply: the last list is worked off by these warps, too
-            const bool got = mbar_wait(&sh->wk_closing, 0u, sh, p.status, 660);
+            const bool got = list_wait(&sh->wk_closing, 0u, sh, p.status, 660, 2ll * p.pace_cycles);
             if (__all_sync(0xffffffffu, got)) work_off(p, sh, sh->closing_slot, RQ + warp - 2, RQ + EPI_WARPS);
         }
     }
@@ -1792,7 +1824,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
         const int w = warp - 3 - EPI_WARPS;
         for (int list = 0;; ++list) {
             const int ws = list % WK_DEPTH;
-            const bool got = mbar_wait(&sh->wk_full[ws], ((uint32_t)(list / WK_DEPTH)) & 1u, sh, p.status, 650 + ws);
+            const bool got = list_wait(&sh->wk_full[ws], ((uint32_t)(list / WK_DEPTH)) & 1u, sh, p.status, 650 + ws, 2ll * p.pace_cycles);
             if (!__all_sync(0xffffffffu, got)) break;
             const bool last = sh->work_last[ws] != 0;
             work_off(p, sh, ws, w, last ? RQ + EPI_WARPS : RQ);
@@ -1813,6 +1845,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             bool ok = true;
             int g_prev = 0;
             sh->n_work[0] = 0;
+            auto step = [&] { *(volatile unsigned *)&sh->published = sh->published + 1; };
             auto pass_on = [&](bool last) {
                 sh->work_last[ws] = last ? 1 : 0;
                 if (last) sh->closing_slot = ws;
@@ -1864,11 +1897,13 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     if (!ok) break;
                 }
                 TRACE(3, it, 0);
+                step();
                 __threadfence();
                 if (mine.rb < p.max_blocks) publish_and_collect(p, sh, ws, mine);   // beyond: a list that is reported (build_schedule)
                 TRACE(3, it, 2);
                 TRACE_ADD(3, it, 3, sh->n_work[ws]);
                 if (sh->n_work[ws] > 0) pass_on(false);
+                step();
             }
             if (ok && !*(volatile int *)&sh->abort_flag) {
                 release_pending(p, sh, ws, 2ll * p.pace_cycles);

@@ -135,6 +135,28 @@ def test_cta_cap_per_call_swiglu_quant(oracle, monkeypatch, max_ctas, ctas):
     assert d.max() <= 1 and np.count_nonzero(d) / d.size <= 1e-4
 
 
+@pytest.mark.parametrize("ctas,rows", [("1", 512), ("2", 1024)])
+def test_wait_limit_is_one_of_a_tile_not_of_the_call(monkeypatch, ctas, rows):
+    """One unit works through four row blocks of 16 channel tiles each, channel tile by channel tile, so that no block is
+    complete before the 61st tile: with 56 K blocks of at least 512 cycles 1.7 million cycles, through which the requantising
+    warps have nothing to do.  A limit of 400,000 cycles, 14 such tiles, does not end the call."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    monkeypatch.setenv("GMM_B200_CTAS", ctas)
+    K, N = 7168, 4096
+    g = torch.Generator(device=dev)
+    g.manual_seed(9)
+    x = torch.randint(-127, 128, (rows, K), dtype=torch.int8, device=dev, generator=g)
+    w = torch.randint(-127, 128, (1, K, N), dtype=torch.int8, device=dev, generator=g)
+    ws, xs = torch.rand((1, N), device=dev, generator=g) * 1e-4, torch.rand(rows, device=dev, generator=g)
+    gl = torch.tensor([rows], dtype=torch.int64, device=dev)
+    q, qs, wsb = ops.grouped_matmul_swiglu_quant(x, w, ws, xs, gl, return_workspace=True,
+                                                 options=ops.LaunchOptions(max_ctas=int(ctas), wait_limit_cycles=400_000))
+    ops.check_status(wsb)
+    want = ops.grouped_matmul_swiglu_quant(x, w, ws, xs, gl)
+    assert torch.equal(q, want[0]) and torch.equal(qs, want[1])
+
+
 def test_two_swiglu_calls_overlapping_on_two_streams(oracle):
     """Two persistent launches that each want every SM: their CTAs are not all resident together.  Nothing in the kernel
     waits for another CTA (the wave pacing is a bounded hint), so both calls finish without a timeout and are correct."""
