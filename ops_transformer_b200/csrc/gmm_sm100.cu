@@ -91,7 +91,7 @@ struct Shape {
 // N=7168: 339 / 343.
 __host__ __device__ constexpr int block_group(int mode) { return mode == kModeSwigluQuant ? 4 : 1; }
 constexpr int MAX_GROUPS = 1024;
-enum : int { kEpiPlain = 0, kEpiScatter = 1, kEpiGeneric = 2, kEpiCombine = 3 };
+enum : int { kEpiPlain = 0, kEpiScatter = 1, kEpiGeneric = 2, kEpiCombine = 3, kEpiHalf = 4, kEpiHalfScatter = 5 };
 // Epilogue warps, and the tokens of the chunks that they take in turns: two warps per TMEM lane quarter and 32 tokens; with
 // options (bias, activation) four and 16.  The options' chains of dependent instructions left the schedulers idle with two warps
 // each (K=1424 N=2976, 3055 rows, fp16, bias, GELU: 38.8 us, now 37.4; K=2048 N=2048, 16 groups of 250 rows, bias, SiLU: 36.7 /
@@ -1181,16 +1181,16 @@ struct XMaps {
     CUtensorMap box[X_MAPS];  // boxes of 32 << i rows
 };
 
-// EPI selects the epilogue variant: kEpiPlain = no bias, no activation, per-token scale present, rows stored in place
-// (the common case, compiled without per-element tests for the options); kEpiScatter = the same arithmetic with the
-// result rows scattered through out_row_index, optionally into other GPUs' memory; kEpiGeneric = every option
-// tested at run time.  CTAS: 1 = one CTA per tile (128 channels), 2 = a cluster of two CTAs (256 channels).
+// EPI selects the epilogue variant: kEpiPlain = no bias, no activation, rows stored in place (the common case, compiled without
+// per-element tests for the options); kEpiScatter = the same arithmetic with the result rows scattered through out_row_index,
+// optionally into other GPUs' memory; kEpiHalf, kEpiHalfScatter = the same two for fp16 results; kEpiCombine = fp32 rows added
+// into row_index; kEpiGeneric = bias or activation, every option tested at run time.  CTAS: 1 = one CTA per tile (128 channels), 2 = a cluster of two CTAs (256 channels).
 template <int MODE, int BL, int EPI, int CTAS>
 __global__ void __launch_bounds__(num_threads(MODE, BL, EPI), 1)
 gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constant__ CUtensorMap map_w, const KParams p)
 {
     constexpr bool PLAIN = EPI != kEpiGeneric;   // lean arithmetic
-    constexpr bool SCATTER = EPI != kEpiPlain;  // rows go where out_row_index says
+    constexpr bool SCATTER = EPI != kEpiPlain && EPI != kEpiHalf;  // rows go where out_row_index says
     constexpr bool COMBINE = EPI == kEpiCombine;  // fp32 rows combined into row_index[r] of a [out_rows, N] result
     constexpr bool SWIGLU = MODE == kModeSwigluQuant;
     constexpr bool OUT16 = MODE == kModeDequantBf16 && !COMBINE;
@@ -1765,7 +1765,7 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                         }
                         activate(p.act_type, reinterpret_cast<float(&)[8 * N8]>(o));
                     }
-                    const bool f16 = !PLAIN && p.out_f16;
+                    const bool f16 = EPI == kEpiHalf || EPI == kEpiHalfScatter || (!PLAIN && p.out_f16);
 #pragma unroll
                     for (int i = 0; i < N8; ++i) {
                         uint32_t pk[4];
@@ -1991,6 +1991,8 @@ cudaError_t launch_epi(int epi, const Plan &plan, const KParams &kp, cudaStream_
 {
     if (MODE == kModeSwigluQuant || epi == kEpiPlain) return launch_ctas<MODE, BL, kEpiPlain>(plan, kp, stream);
     if (epi == kEpiScatter) return launch_ctas<MODE, BL, kEpiScatter>(plan, kp, stream);
+    if (MODE == kModeDequantBf16 && epi == kEpiHalf) return launch_ctas<MODE, BL, MODE == kModeDequantBf16 ? kEpiHalf : kEpiPlain>(plan, kp, stream);
+    if (MODE == kModeDequantBf16 && epi == kEpiHalfScatter) return launch_ctas<MODE, BL, MODE == kModeDequantBf16 ? kEpiHalfScatter : kEpiPlain>(plan, kp, stream);
     if (MODE == kModeDequantBf16 && epi == kEpiCombine) return launch_ctas<MODE, BL, MODE == kModeDequantBf16 ? kEpiCombine : kEpiPlain>(plan, kp, stream);
     return launch_ctas<MODE, BL, kEpiGeneric>(plan, kp, stream);
 }
@@ -2104,8 +2106,12 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     kp.q_scale_out = reinterpret_cast<float *>(p.out1);
     kp.out = p.mode == kModeSwigluQuant ? static_cast<void *>(ws + plan.off_stage) : p.out0;
 
-    const bool lean = !p.bias && p.act_type == 0 && !p.out_f16 && (p.mode != kModeDequantBf16 || p.x_scale);
-    const int epi = p.combine ? kEpiCombine : !lean ? kEpiGeneric : (p.out_row_index ? kEpiScatter : kEpiPlain);
+    // The generic epilogue is for bias and activation alone: its sixteen warps only get in the way of the MMAs where a chunk's
+    // arithmetic is short.  Without the tokens' scales the plain arithmetic multiplies by one; fp16 rows have instances of their own.
+    // K=2048 N=7168, 32 groups of 1024 rows, us with the generic epilogue on eight warps / on sixteen / now: fp16 369 / 379 / 340, scattered
+    // 371 / 381 / 353; bf16 without the tokens' scales 354 / 363 / 326 (bf16 with them 323).
+    const int epi = p.combine ? kEpiCombine : p.bias || p.act_type ? kEpiGeneric
+                  : p.out_f16 ? (p.out_row_index ? kEpiHalfScatter : kEpiHalf) : (p.out_row_index ? kEpiScatter : kEpiPlain);
     kp.logit = p.logit;
     kp.row_index = p.row_index;
     kp.row_index_i32 = p.row_index_i32;
@@ -2114,7 +2120,7 @@ cudaError_t sm100_launch(const Problem &p, Plan &plan, void *workspace, cudaStre
     if (p.combine && (p.mode != kModeDequantBf16 || !p.row_index)) return cudaErrorInvalidValue;
     kp.num_peers = p.mode == kModeDequantBf16 ? p.num_peers : 0;
     for (int i = 0; i < 8; ++i) kp.out_peers[i] = i < kp.num_peers ? p.out_peers[i] : nullptr;
-    if (kp.num_peers > 0 && epi != kEpiScatter) return cudaErrorInvalidValue;
+    if (kp.num_peers > 0 && (epi != kEpiScatter || !p.x_scale)) return cudaErrorInvalidValue;
     // Pacing (see the producer): needs one zeroed word per wave; the plan reserves them only where it pays.
     // The plan reserves a counter per tile, so there is one for every wave; a single unit has nobody to keep pace with.
     kp.wave_cnt = plan.off_wave && plan.num_sms >= 2 ? reinterpret_cast<int *>(ws + plan.off_wave) : nullptr;

@@ -468,6 +468,30 @@ def test_token_tile_edges(oracle, monkeypatch, ctas, kind):
         assert np.array_equal(got[perm[:rows]], ref[:rows]) and (got[perm[rows:]] == 0x7fc1).all()
 
 
+@pytest.mark.parametrize("ctas", ["1", "2"])
+@pytest.mark.parametrize("out_dtype,scales", [("f16", True), ("f16", False), ("bf16", False)])
+def test_token_tile_edges_of_fp16_rows_and_missing_token_scales(oracle, monkeypatch, ctas, out_dtype, scales):
+    """Neither bias nor activation: fp16 rows and rows without the tokens' scales, in place (three weight layouts) and scattered."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    monkeypatch.setenv("GMM_B200_CTAS", ctas)
+    counts = np.array(TILE_EDGE_COUNTS, np.int64)
+    E, M, K, N = len(counts), int(counts.sum()) + 5, 272, 288
+    gl = np.cumsum(counts)
+    x, w, ws, xs = make_inputs(M, K, N, E, seed=64)
+    ws, xs = np.ascontiguousarray(ws * 1e-2), xs if scales else None
+    for layout in ({}, dict(w_trans=True), dict(w_nz=True)):
+        check_gmm(oracle, x, w, ws, xs, gl, out_dtype=out_dtype, **layout)
+    perm = np.random.default_rng(7).permutation(M).astype(np.int64)
+    t = lambda a: None if a is None else torch.from_numpy(a).to(dev)  # noqa: E731
+    out = torch.full((M, N), 0x7fc1, dtype=torch.int16, device=dev).view(torch.float16 if out_dtype == "f16" else torch.bfloat16)
+    _, wsb = ops.grouped_matmul_v4(t(x), t(w), t(ws), t(xs), t(gl), out=out, out_row_index=t(perm), return_workspace=True)
+    ops.check_status(wsb)
+    ref = oracle.gmm_w8a8(x, w, ws, xs, gl, 0, y_dtype=out_dtype)["y"]
+    got, rows = _bf16_bits(out), int(gl[-1])
+    assert np.array_equal(got[perm[:rows]], ref[:rows]) and (got[perm[rows:]] == 0x7fc1).all()
+
+
 @pytest.mark.parametrize("ctas,max_ctas", [("1", 5), ("1", 8), ("1", 11), ("1", 37), ("2", 8), ("2", 14), ("2", 30)])
 @pytest.mark.parametrize("kind", ["bf16", "int32", "nz", "swiglu", "swiglu_nz"])
 def test_last_wave_cut_into_pieces(monkeypatch, ctas, max_ctas, kind):
