@@ -46,24 +46,46 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def build_describe(force: bool = False) -> str:
-    """The extension module that writes a call's tensors into its description; g++ against torch's headers."""
+def described_for() -> str:
+    """What the extension module is bound to beside its source: the C++ interface of this torch and the ABI of this Python.  The
+    module carries it (``built_for``), so that one left over from another installation is told from a fresh one."""
     import sysconfig
 
     import torch
-    stale = not os.path.exists(DESCRIBE_PATH) or os.path.getmtime(DESCRIBE_PATH) < os.path.getmtime(DESCRIBE_SOURCE)
-    if not force and not stale:
+    return f"describe.cpp for torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+
+
+def describe_stale() -> bool:
+    if not os.path.exists(DESCRIBE_PATH) or os.path.getmtime(DESCRIBE_PATH) < os.path.getmtime(DESCRIBE_SOURCE):
+        return True
+    with open(DESCRIBE_PATH, "rb") as f:
+        return described_for().encode() + b"\0" not in f.read()
+
+
+def build_describe(force: bool = False) -> str:
+    """The extension module that writes a call's tensors into its description; g++ against torch's headers.  It is written under
+    another name and moved into place, so that no process loads half of it."""
+    import sysconfig
+
+    import torch
+    if not force and not describe_stale():
         return DESCRIBE_PATH
     root = os.path.dirname(torch.__file__)
+    part = f"{DESCRIBE_PATH}.{os.getpid()}.part"
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DDESCRIBE_BUILT_FOR="{described_for()}"',
            "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
            "-I", sysconfig.get_paths()["include"], "-I", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"),
-           "-o", DESCRIBE_PATH, DESCRIBE_SOURCE, "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        sys.stderr.write(r.stdout + r.stderr)
-        raise RuntimeError("g++ failed building _describe.so")
+           "-o", part, DESCRIBE_SOURCE, "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("g++ failed building _describe.so")
+        os.replace(part, DESCRIBE_PATH)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
     return DESCRIBE_PATH
 
 

@@ -145,6 +145,11 @@ def _describe_module():
             from . import _describe
         except ImportError as e:
             raise LibraryMissing(f"the native description module is missing ({e}): build it with `python -m ops_transformer_b200._build`.") from e
+        from ._build import described_for
+        built_for = getattr(_describe, "built_for", "an earlier source")
+        if built_for != described_for():
+            raise LibraryMissing(f"the native description module was built for another installation ({built_for}; this is "
+                                 f"{described_for()}): build it with `python -m ops_transformer_b200._build`.")
         _DESCRIBE = _describe
     return _DESCRIBE
 

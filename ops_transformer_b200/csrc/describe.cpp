@@ -178,4 +178,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_describe", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__describe(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__describe(void)
+{
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "built_for", DESCRIBE_BUILT_FOR) < 0) Py_CLEAR(m);
+    return m;
+}

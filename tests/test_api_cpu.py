@@ -6,6 +6,7 @@ Phase 1 never dereferences tensor data, so host tensors stand in for device tens
 import ctypes as C
 import os
 import re
+import types
 
 import numpy as np
 import pytest
@@ -703,6 +704,42 @@ def test_operators_describe_their_arguments_by_place(monkeypatch):
                 with pytest.raises((TypeError, AttributeError)):
                     call(tensors[:i] + (bad,) + tensors[i + 1:], ints)
     assert not seen
+
+
+def test_description_module_follows_its_installation(monkeypatch, tmp_path):
+    """A module that was built for another torch or Python is rebuilt, and refused where it is not; the new one takes its place
+    whole, and a build that fails leaves the old one."""
+    from ops_transformer_b200 import _build
+    _lib.describe()
+    here = _build.described_for()
+    assert not _build.describe_stale() and torch.__version__ in here
+    so = tmp_path / "_describe.so"
+    monkeypatch.setattr(_build, "DESCRIBE_PATH", str(so))
+    runs, outcome = [], [0]
+
+    def compile_(cmd, **kw):
+        part = cmd[cmd.index("-o") + 1]
+        runs.append((part, so.exists()))
+        with open(part, "wb") as f:
+            f.write(b"\0" + _build.described_for().encode() + b"\0")
+        return types.SimpleNamespace(returncode=outcome[0], stdout="", stderr="")
+
+    monkeypatch.setattr(_build.subprocess, "run", compile_)
+    for _ in range(2):                                   # built once
+        assert _build.build_describe() == str(so)
+    assert len(runs) == 1 and runs[0][0] != str(so) and not runs[0][1] and [p.name for p in tmp_path.iterdir()] == ["_describe.so"]
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "0")   # one version a prefix of the other
+    assert _build.describe_stale()
+    monkeypatch.setattr(_lib, "_DESCRIBE", None)
+    with pytest.raises(_lib.LibraryMissing, match="another installation"):
+        _lib.describe()
+    old, outcome[0] = so.read_bytes(), 1
+    with pytest.raises(RuntimeError):
+        _build.build_describe()
+    assert so.read_bytes() == old and [p.name for p in tmp_path.iterdir()] == ["_describe.so"]
+    outcome[0] = 0
+    _build.build_describe()
+    assert not _build.describe_stale() and so.read_bytes() != old
 
 
 # ----------------------------------------------------------------------------------------------------------
