@@ -907,6 +907,41 @@ def test_init_routing_special_rows(dtype, n):
     assert torch.equal(q, q[:12].repeat(n // 12, 1))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("smooth", [False, True])
+@pytest.mark.parametrize("n", [40, 1200])
+def test_init_routing_special_rows_as_in_the_general_kernel(dtype, smooth, n):
+    """Infinities, NaN, denormals, the largest values, ties and rows of one sign: the register-tiled kernel gives the bits of the one
+    for any shape and alignment, which divides and converts value by value (an unaligned result selects it)."""
+    import ops_transformer_b200 as ops
+    dev = _dev()
+    h = 2048
+    big, tiny = torch.finfo(dtype).max, torch.finfo(dtype).smallest_normal
+    g = torch.Generator(device=dev)
+    g.manual_seed(4)
+    rows = torch.randn(20, h, device=dev, generator=g).to(dtype)
+    rows[0] = 0
+    rows[1, 5], rows[2, 5], rows[3, 7] = float("inf"), float("-inf"), float("nan")
+    rows[4] = float("nan")
+    rows[5, 9], rows[6, 9] = big, -big
+    rows[7] = rows[7] * tiny
+    rows[8] = tiny / 4
+    rows[9, 1], rows[9, 2] = float("inf"), float("nan")
+    rows[10] = -rows[10].abs()
+    rows[11] = ((torch.arange(h, device=dev) % 509 - 254) / 2).clamp(-127, 127).to(dtype)   # k + 1/2 with a scale of one
+    rows[12] = rows[12] * (1000 if dtype == torch.float16 else big / 8)
+    x = rows.repeat(n // 20, 1)
+    idx = (torch.arange(2 * n, device=dev).view(n, 2) % 3).to(torch.int32)
+    kw = dict(expert_num=3, active_expert_range=(0, 3), scale=torch.rand(3, h, device=dev, generator=g) + 0.5 if smooth else None)
+    q, ri, cnt, s = ops.moe_init_routing_v3(x, idx, **kw)
+    general = [torch.empty(2 * n * h + 1, dtype=torch.int8, device=dev)[1:].view(2 * n, h)] + [torch.empty_like(t) for t in (ri, cnt, s)]
+    ops.moe_init_routing_v3(x, idx, outputs=general, **kw)
+    torch.cuda.synchronize()
+    assert general[0].data_ptr() % 2 == 1
+    for a, b in zip((q, ri, cnt, s.view(torch.int32)), (*general[:3], general[3].view(torch.int32))):
+        assert torch.equal(a, b)
+
+
 def test_init_routing_without_quantisation(oracle):
     check_init_routing(oracle, 200, 4, 256, 32, (0, 32), 76, quant=False, per_token_scale=True)
     check_init_routing(oracle, 200, 4, 256, 32, (4, 20), 77, quant=False, x_kind="int8", row_idx_type=0)
