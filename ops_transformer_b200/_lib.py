@@ -160,8 +160,11 @@ def describe(*items) -> bytes:
 
 
 def describe_call(kinds: str, *items) -> bytes:
-    """The same for the arguments of an operator, whose kinds its description fixes (a letter each, csrc/describe.cpp)."""
-    return _describe_module().describe_call(kinds, *items)
+    """The same for the arguments of an operator, whose kinds its description fixes (a letter each, csrc/describe.cpp).  The first
+    use puts the module's function in this one's place: passing the arguments on costs a fifth of the description."""
+    global describe_call
+    describe_call = _describe_module().describe_call
+    return describe_call(kinds, *items)
 
 
 def last_error() -> str:
