@@ -162,7 +162,7 @@ struct Shared {
     // CTA contributed to and has not yet settled (publishing lane only); a ring of work lists: the row ranges to requantise
     // (written by that lane, read by the requantising warps after wk_full)
     unsigned stored_count;
-    unsigned published;                // steps of the publishing lane (see list_wait)
+    unsigned published;                // tiles that the publishing lane is done with (see list_wait)
     int pend_n;
     PendingBlock pend[MAX_PENDING];
     int n_work[WK_DEPTH];
@@ -300,17 +300,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 // (A kernel in the place of every operator's memset would take 2.6 us off a call on the device and cost the host 3.)
 __device__ __forceinline__ void wait_for_init() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Bounded wait.  Returns false when the limit ran out or another role already gave up.
+// Bounded wait.  Returns false when the limit ran out or another role already gave up.  A change of `*progress` starts the limit
+// anew.
 template <bool CLUSTER>
 __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, Shared *sh, int *status, int who,
-                                            long long limit)
+                                            long long limit, const unsigned *progress = nullptr)
 {
-    const long long t0 = clock64();
-    uint32_t spins = 0;
+    long long t0 = clock64();
+    uint32_t spins = 0, seen = 0;
     while (true) {
         if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         if ((++spins & 31u) == 0u) {
             if (*(volatile int *)&sh->abort_flag) return false;
+            const uint32_t now = progress ? *(const volatile unsigned *)progress : 0u;
+            if (now != seen) {
+                seen = now;
+                t0 = clock64();
+            }
             if (clock64() - t0 > limit) {
                 *(volatile int *)&sh->abort_flag = 1;
                 wait_for_init();
@@ -334,32 +340,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, Shared
 
 // Bounded wait for a work list of swiglu_quant.  Many tiles can lie between two lists - nothing is passed on while none of the
 // CTA's row blocks is complete, four blocks times all their channel tiles at a time with few CTAs - and the last list also waits
-// for other units (`patience`).  The limit is one of a single step, so it starts anew with every step of the publishing lane, which
-// bounds its own waits by it.
-__device__ __noinline__ bool list_wait(uint64_t *bar, uint32_t parity, Shared *sh, int *status, int who, long long patience)
+// for other units (`patience`).  The limit starts anew with every tile that the publishing lane is done with; for each the lane
+// waits twice, and bounds these waits itself.
+__device__ __forceinline__ bool list_wait(uint64_t *bar, uint32_t parity, Shared *sh, int *status, int who, long long patience)
 {
     const uint32_t a = smem_u32(bar);
-    const long long limit = sh->wait_limit + patience;
-    unsigned seen = *(volatile unsigned *)&sh->published, spins = 0;
-    long long t0 = clock64();
-    while (!mbar_try_wait<false>(a, parity)) {
-        if ((++spins & 31u) != 0u) continue;
-        if (*(volatile int *)&sh->abort_flag) return false;
-        const unsigned now = *(volatile unsigned *)&sh->published;
-        if (now != seen) {
-            seen = now;
-            t0 = clock64();
-        } else if (clock64() - t0 > limit) {
-            *(volatile int *)&sh->abort_flag = 1;
-            if (atomicCAS(status, kStatusOk, kStatusWaitTimeout) == kStatusOk) {
-                status[1] = (int)blockIdx.x;
-                status[2] = who;
-                status[3] = (int)parity;
-            }
-            return false;
-        }
-    }
-    return true;
+    if (mbar_try_wait<false>(a, parity)) return true;
+    return mbar_wait_slow<false>(a, parity, sh, status, who, 2 * sh->wait_limit + patience, &sh->published);
 }
 
 // Tiled TMA loads into this CTA's shared memory.  CTAS == 2 is the pair form: the byte count is credited to the mbarrier at
@@ -1845,7 +1832,6 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
             bool ok = true;
             int g_prev = 0;
             sh->n_work[0] = 0;
-            auto step = [&] { *(volatile unsigned *)&sh->published = sh->published + 1; };
             auto pass_on = [&](bool last) {
                 sh->work_last[ws] = last ? 1 : 0;
                 if (last) sh->closing_slot = ws;
@@ -1897,13 +1883,12 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
                     if (!ok) break;
                 }
                 TRACE(3, it, 0);
-                step();
                 __threadfence();
                 if (mine.rb < p.max_blocks) publish_and_collect(p, sh, ws, mine);   // beyond: a list that is reported (build_schedule)
                 TRACE(3, it, 2);
                 TRACE_ADD(3, it, 3, sh->n_work[ws]);
                 if (sh->n_work[ws] > 0) pass_on(false);
-                step();
+                *(volatile unsigned *)&sh->published = (unsigned)it + 1;
             }
             if (ok && !*(volatile int *)&sh->abort_flag) {
                 release_pending(p, sh, ws, 2ll * p.pace_cycles);
