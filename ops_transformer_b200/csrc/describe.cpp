@@ -1,7 +1,7 @@
 // Tensor descriptions for gmmB200Call (include/gmm_b200.h), written from the tensors themselves.
 //
 // In Python the description of a call - address, type, format, sizes, strides and storage sizes of seven to ten tensors - cost
-// 7 us, more than the call's launches; here 0.5.
+// 7 us, more than the call's launches; here 0.6.
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 

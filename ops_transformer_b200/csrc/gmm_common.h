@@ -161,6 +161,35 @@ __device__ __forceinline__ float apply_activation(int act_type, float v)
         default: return v;
     }
 }
+
+// Two fp32 values in one register pair.  The packed operations of sm_100 round each half as the scalar ones do and take one
+// issue slot for both.  (There is no packed addition here: the assembler fused one with the packed product in front of it, so
+// sums that the reference rounds separately stay scalar.)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 #endif
 
 }  // namespace gmm

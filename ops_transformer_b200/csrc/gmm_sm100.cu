@@ -39,7 +39,7 @@
 // idle; the SM clock falls to 1.5-1.6 GHz, at which the tensor pipe alone draws the board's 1 kW); groups of up to 128 rows
 // HBM; short K the epilogue.  Measured before (tokens on the M side, operations issued by one thread of a diverged warp,
 // every epilogue thread fencing for itself, requantisation inside the epilogue warps) and now, us:
-//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 877 (power), 128 tokens x 8 over 256 experts 884 / 850 (HBM);
+//   swiglu K=7168 N=4096: 4096 tokens x 8 over 32 experts 892 / 886 (power), 128 tokens x 8 over 256 experts 884 / 850 (HBM);
 //     K=2048 N=1536, 64 groups of 64 rows 66 / 52, of 400 rows 190 / 112
 //   gmm K=2048 N=7168: 4096 tokens x 8 over 32 experts 403 / 366; 32 groups of 160 rows 131 / 96; K=768 N=2048, 64 x 400 rows
 //     76 / 60 (of which 10 % came from moving the second CTA's accumulator release out of its epilogue warps: 374 / 334 for
@@ -63,7 +63,7 @@ namespace {
 constexpr int BC = 128;                 // channels (weight columns) per CTA: the MMA's M side, one TMEM lane each
 constexpr int BT = 256;                 // most tokens of a tile: the MMA's N side, one TMEM column each
 constexpr int TOK_STEP = 32;            // the MMA's N is a multiple of this
-constexpr int SPLIT_TOK = 64;           // least tokens of a tile's piece in the last wave, as far as the tile has them
+constexpr int SPLIT_TOK = 64;           // the last wave's tiles are cut no further than brings the largest tile to this
 constexpr int BK = 128;
 constexpr int UMMA_K = 32;
 constexpr int W_STAGE = BC * BK;        // a CTA's channels x 128 bytes of K
@@ -86,9 +86,10 @@ struct Shape {
 };
 // Row blocks of a group that are worked on together: all their tiles of a channel tile, then the next channel tile.  A group that
 // begins in one wave and ends in the next has its x rows read twice then, instead of its weights, four times as many (DRAM reads
-// of 8 groups of 1024 rows, K=7168 N=4096: 403 -> 330 MB).  swiglu
-// K=7168 N=4096, 32 groups of 1024 rows: 758 us with one, 740 with four; grouped_matmul, which does not pace its waves, K=2048
-// N=7168: 339 / 343.
+// of 8 groups of 1024 rows, K=7168 N=4096: 403 -> 330 MB).  It is traffic that this saves: the kernel's time stays within the
+// runs' spread, also where four blocks have more tiles than a wave has units (swiglu, us with one / two / four: K=7168 N=4096, 32
+// groups of 1024 rows 664 / 672 / 662; K=4096 N=8192, 16 of 2048 rows 806 / 801 / 796; K=4096 N=10240, 4 of 1024 rows 204 / 191 /
+// 196).  grouped_matmul, which does not pace its waves, K=2048 N=7168: 339 / - / 343.
 __host__ __device__ constexpr int block_group(int mode) { return mode == kModeSwigluQuant ? 4 : 1; }
 constexpr int MAX_GROUPS = 1024;
 enum : int { kEpiPlain = 0, kEpiScatter = 1, kEpiGeneric = 2, kEpiCombine = 3, kEpiHalf = 4, kEpiHalfScatter = 5 };
@@ -627,8 +628,11 @@ __device__ __forceinline__ int tile_tokens(int rows)
 // are other data, and a slice claimed from such a word would be an arbitrary range of rows.
 //
 // The last wave: `rem` tiles for n_units units take as long as a full wave.  Where two or more units are there for each of
-// them, they are cut into that many pieces along their tokens, of SPLIT_TOK or more (below, a K block of MMAs does not get
-// shorter any more): the weights come from L2 for all but one of the pieces.  A piece without rows is left out.
+// them, they are cut into that many pieces along their tokens: the weights come from L2 for all but one of the pieces.  The
+// number of pieces is one for the launch, no more than bring its largest tile down to SPLIT_TOK (below, a K block of MMAs does
+// not get shorter any more); smaller tiles get pieces of a multiple of 32 tokens, and one without rows is left out.  (Pieces of at
+// least SPLIT_TOK whatever the tile take the same time within the runs' spread: K=7168 N=2048, 256 rows and five groups of 100, us
+// as here / so: grouped_matmul 32.0 / 32.8, swiglu_quant 38.5 / 38.5.)
 // K=4096 N=4096, 6 groups of about 200 rows, us: grouped_matmul 32.9 -> 31.1, swiglu_quant 40.2 -> 38.5.
 template <int MAX_TOK>
 __device__ void build_schedule(Shared *sh, const KParams &p, int n_units)
@@ -798,35 +802,6 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi)
 __device__ __forceinline__ void red_add_v4(float *p, const float4 v)
 {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-
-// Two fp32 values in one register pair.  The packed operations of sm_100 round each half as the scalar ones do and take one
-// issue slot for both.  (There is no packed addition here: the assembler fused one with the packed product in front of it, so
-// sums that the reference rounds separately stay scalar.)
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair2(float a, float b)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpair2(f32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
 }
 
 // q = int8(rint(half(S * (1 / (amax / 127)))))  -- CastFp32ToInt8Template,
@@ -1089,7 +1064,7 @@ __device__ __forceinline__ void activate(int act_type, float (&v)[N])
     if (act_type == 1) {
 #pragma unroll
         for (int i = 0; i < N; ++i) v[i] = v[i] > 0.0f ? v[i] : 0.0f;
-    } else if (act_type == 2) {
+    } else if (act_type == 2) {   // z = 1.596 (v + 0.0447 v^3); its sum has one rounding fewer here than in apply_activation
         float z[N];
 #pragma unroll
         for (int i = 0; i < N; i += 2) {
@@ -1805,8 +1780,9 @@ gmm_w8a8_sm100_kernel(const __grid_constant__ XMaps maps_x, const __grid_constan
 
     else if (SWIGLU && warp > 2 + EPI_WARPS) {
         // ------------------------------ requantising warps (swiglu_quant) ------------------------------
-        // A list names the row blocks that are complete by then - normally the block of this unit's previous tile, whose rows
-        // are read while they are still in L2.  These warps spend their time waiting for L2; beside the epilogue that costs
+        // A list names row blocks of which this unit has done tiles and which are complete by then; their rows are read while they
+        // are still in L2.  With block_group row blocks at a time it is normally those of the unit's previous tiles, one after the
+        // other as their last channel tile is done.  These warps spend their time waiting for L2; beside the epilogue that costs
         // nothing, inside it every tile of a C2-sized launch lost 13 of 36 thousand cycles to it, more than its MMAs take.
         const int w = warp - 3 - EPI_WARPS;
         for (int list = 0;; ++list) {

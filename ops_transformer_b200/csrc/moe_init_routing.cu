@@ -466,30 +466,12 @@ __device__ __forceinline__ void unpack16<__half>(const uint4 &u, float *f)
 }
 
 // Two values of quant_fast where its reciprocal is not 0: |v / scale| rounds to at most 127 then, so nothing is clamped.
-__device__ __forceinline__ unsigned long long pack_f32x2(float a, float b)
+__device__ __forceinline__ void quant_pair(float v0, float v1, f32x2 neg_scale, f32x2 rcp, int &q0, int &q1)
 {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c)
-{
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ void quant_pair(float v0, float v1, unsigned long long neg_scale, unsigned long long rcp, int &q0, int &q1)
-{
-    const unsigned long long v = pack_f32x2(v0, v1);
-    unsigned long long q = mul_f32x2(v, rcp);
-    q = fma_f32x2(fma_f32x2(q, neg_scale, v), rcp, q);
-    q = fma_f32x2(fma_f32x2(q, neg_scale, v), rcp, q);
+    const f32x2 v = pair2(v0, v1);
+    f32x2 q = mul2(v, rcp);
+    q = fma2(fma2(q, neg_scale, v), rcp, q);
+    q = fma2(fma2(q, neg_scale, v), rcp, q);
     const uint32_t a = (uint32_t)q & 0xffffe000u, b = (uint32_t)(q >> 32) & 0xffffe000u;
     q0 = __float2int_rz(__fadd_rn(__uint_as_float(a), __uint_as_float(0x3f000000u | (a & 0x80000000u))));
     q1 = __float2int_rz(__fadd_rn(__uint_as_float(b), __uint_as_float(0x3f000000u | (b & 0x80000000u))));
@@ -549,7 +531,7 @@ __device__ __forceinline__ void quant_part(const uint4 (&raw)[NCH], float scale,
     constexpr int VEC = 16 / (int)sizeof(T);
     const float rcp = exact_div_rcp(scale);
     if (rcp != 0.0f) {
-        const unsigned long long ns = pack_f32x2(-scale, -scale), r2 = pack_f32x2(rcp, rcp);
+        const f32x2 ns = pair2(-scale, -scale), r2 = pair2(rcp, rcp);
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
             float v[VEC];
@@ -635,7 +617,7 @@ __global__ void __launch_bounds__(THREADS, MINB) routing_quant_token_kernel(cons
             }
             scale = __fdiv_rn(block_max<THREADS>(amax, red), 127.0f);
             const float rcp = exact_div_rcp(scale);
-            const unsigned long long ns = pack_f32x2(-scale, -scale), r2 = pack_f32x2(rcp, rcp);
+            const f32x2 ns = pair2(-scale, -scale), r2 = pair2(rcp, rcp);
 #pragma unroll
             for (int i = 0; i < NCH; ++i) {  // the products are formed again: keeping them would cost 64 registers
                 const int c = (threadIdx.x + (i / G) * THREADS) * G + (i % G);
