@@ -37,7 +37,8 @@ ACL_FUNC_VISIBILITY aclnnStatus gmmB200CheckStatus(const void *workspace, uint64
  *                    operator.  Null = off.
  *   waitLimitCycles  bound of every device-side wait (SM clock cycles) before a CTA gives up, records a status and returns;
  *                    0 = the default of 2^31 cycles (about a second).  A wait spans at most about a tile of the CTA: where the
- *                    requantising warps of swiglu_quant wait through several tiles, the limit starts anew with each of them.
+ *                    requantising warps of swiglu_quant wait through several tiles, it starts anew with each of them (at twice the
+ *                    limit: the warp that they wait for has two waits of its own per tile).
  *   testSkipKBlocks  test only: the copy-issuing warp leaves this many K blocks out of its last tile, so that the bounded wait
  *                    of the warp that consumes them runs out and the abort path (status record, clean exit) can be exercised
  *                    without touching memory the call does not own.  Results are then undefined.  0 = off. */
